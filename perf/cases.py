@@ -36,6 +36,10 @@ def _tol(case):
 SHAPES = {30: (41, 5, 0.0), 118: (179, 53, 0.10), 300: (411, 69, 0.10), 1354: (1991, 259, 0.10),
           2869: (4582, 509, 0.10), 9241: (16049, 1445, 0.15)}
 
+# outages of the 9241-bus grid after which Newton from the flat start finds no solution or
+# wanders first (of 15,584): their voltages at the iteration limit are not a result
+NO_SOLUTION = {9241: (5938, 7448, 9668, 15311)}
+
 
 def listed():
     return [
@@ -138,6 +142,7 @@ def _outage_cases(branches, nb, n, k, seed, base=False):
     branches); the base case first when asked.  The second outage of a pair is not a
     bridge of what the first one leaves."""
     order = m.select_outages(branches, nb, int((~m.find_bridges(branches, nb)).sum()), seed)
+    order = order[~np.isin(order, NO_SOLUTION.get(nb, ()))]
     cases = [[]] if base else []
     for i in range(n - len(cases)):
         a = int(order[i % len(order)])
