@@ -13,13 +13,14 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmpf.so")
 
 SOURCES = ["engine.cu", "symbolic.cpp", "synth.cpp"]
-HEADERS = ["internal.h", "kernels.cuh"]
+HEADERS = ["internal.h", "kernels.cuh", "kernels_chunk.cuh"]
 
 NVCC_FLAGS = [
     "-O3",
     "-std=c++17",
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo",
+    "--split-compile", "0",
     "-Xcompiler", "-fPIC,-O3",
     "-shared",
 ]

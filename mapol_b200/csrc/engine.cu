@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <memory>
 #include <array>
@@ -27,6 +28,7 @@
 
 #include "internal.h"
 #include "kernels.cuh"
+#include "kernels_chunk.cuh"
 #include "mpf.h"
 
 using namespace mpf;
@@ -87,6 +89,10 @@ enum TaskClass { CLS_S = 0, CLS_M = 1, CLS_L = 2, CLS_M1 = 3, CLS_BIG = 4 };
 // 32-byte chunk would not fit in shared memory (kSmemMax)
 constexpr int kFmaxS = 8, kFmaxM1 = 16, kFmaxM = 24;
 constexpr size_t kSmemMax = 227 * 1024;
+// of it, what the kernels of kernels_chunk.cuh may take dynamically (beside their static
+// reduction buffers)
+constexpr size_t kChunkSmem = kSmemMax - 4096;
+constexpr size_t kChunkScratch = 16 * 1024;  // of it, most for the teams' fronts
 // rounds of PV -> PQ switching per solve (each switches at least one bus of a case)
 constexpr int kMaxQRounds = 20;
 // largest dense front in shared memory: one FP64 lane, f * ((f + 1) | 1) * 8 bytes.
@@ -205,11 +211,22 @@ struct FactorChoice {
   int kind, ge, tt, tpb;
 };
 
+// A block's substitution steps (SweepPlan) on the device
+struct PlanBufs {
+  DevBuf step, step_ptr, idx;
+  size_t scratch = 0, slot = 0;  // as SweepPlan
+  int peak_cb = 0;
+  DevSweep dev() const { return DevSweep{step.as<int4>(), step_ptr.as<int>(), idx.as<int>()}; }
+};
+
 struct LUSystem {
   LUSymbolic sym;
   DevBuf sn_w, sn_f, sn_rptr, sn_rows, child_ptr, child_list, sn_parent, rel_ptr, relmap, ah_ptr, ah_loc;
   DevBuf pan_off, cb_off, cbr_off, lev_sn, child_ref, cb_in;
   DevBuf sn_island;                  // multi-island handles only
+  std::vector<int> h_sn_island;      // the same on the host (empty: one island)
+  // sweep plans by (compact, lanes, value bytes, kilobytes per ring slot)
+  std::map<std::tuple<bool, int, int, int>, std::unique_ptr<PlanBufs>> plans;
   const int* group_island = nullptr; // the handle's current per-group islands (or null)
   std::vector<Launch> factor_sched;  // ascending levels
   std::vector<LaunchDeps> factor_deps;
@@ -279,7 +296,11 @@ struct LUSystem {
           if ((*var_island)[s.sn_rows[q]] != si[k]) throw MpfError{MPF_ERR_INTERNAL, "supernode spans two islands"};
       }
       upload(sn_island, si);
+      h_sn_island = si;
+    } else {
+      h_sn_island.clear();
     }
+    plans.clear();
     upload(sn_w, s.sn_w);
     upload(sn_f, s.sn_f);
     upload(sn_rptr, s.sn_rptr);
@@ -436,6 +457,30 @@ struct LUSystem {
     }
   }
 
+  // The sweep plan for blocks of G lanes of wsize-byte values with ring slots of slot_kb KB,
+  // kept on the device; null when a supernode does not fit
+  const PlanBufs* plan(bool compact, int G, int wsize, int slot_kb) {
+    const auto key = std::make_tuple(compact, G, wsize, slot_kb);
+    auto it = plans.find(key);
+    if (it != plans.end()) return it->second.get();
+    SweepPlan p;
+    const bool ok = slot_kb > 0 && build_sweep_plan(sym, h_sn_island, compact, G, wsize, (size_t)slot_kb * 1024,
+                                                    kChunkScratch, p);
+    auto& slot = plans[key];
+    if (ok) {
+      slot = std::make_unique<PlanBufs>();
+      std::vector<int4> st(p.step.size());
+      for (size_t k = 0; k < st.size(); ++k) st[k] = make_int4(p.step[k].e0, p.step[k].ne, p.step[k].i0, p.step[k].ni);
+      upload(slot->step, st);
+      upload(slot->step_ptr, p.step_ptr);
+      upload(slot->idx, p.idx);
+      slot->scratch = p.scratch;
+      slot->slot = p.slot;
+      slot->peak_cb = p.peak_cb;
+    }
+    return slot.get();
+  }
+
   // A launch's shared memory per team is set by its largest front, while its fronts'
   // sizes spread (a level's supernodes are sorted by front size): a run of fronts
   // 9..16 reserves 16 x 17 entries per lane for fronts averaging 12 x 13.  Shared
@@ -478,7 +523,7 @@ struct LUSystem {
     for (int k = ln.offset; k < ln.offset + ln.count; ++k) {
       const int sn = sym.lev_sn[k];
       const int64_t m = sym.sn_f[sn] - sym.sn_w[sn];
-      e += (ah_host[sn + 1] - ah_host[sn]) + (sym.pan_off[sn + 1] - sym.pan_off[sn]);
+      e += (ah_host[sn + 1] - ah_host[sn]) + (int64_t)sym.sn_w[sn] * (2 * sym.sn_f[sn] - sym.sn_w[sn]);
       if (sym.sn_parent[sn] >= 0) e += m * m;
       for (int c = sym.child_ptr[sn]; c < sym.child_ptr[sn + 1]; ++c) {
         const int64_t mc = sym.sn_f[sym.child_list[c]] - sym.sn_w[sym.child_list[c]];
@@ -575,7 +620,6 @@ void ensure_attrs(int device) {
   CUDA_TRY(cudaFuncSetAttribute(k_mf_bsolve_chunk<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_bsolve_chunk<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_bsolve_chunk<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
-  CUDA_TRY(cudaFuncSetAttribute(k_mf_fsolve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_fsolve_t<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_bsolve_t<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_factor_big<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
@@ -1366,21 +1410,6 @@ void tune_bsolve(LUSystem& sys, int ngroups, const T* pan, T* x, const int* grou
   if (tc.bsolve.emplace(key, best).second) append_tune_file(line + "\n");
 }
 
-template <typename T>
-void launch_fsolve(const LUSystem& sys, int ngroups, const T* pan, T* cbr, T* x, const int* group_active,
-                   cudaStream_t st, int* nlaunch) {
-  for (const Launch& ln : sys.level_sched) {
-    const long long ntasks = (long long)ln.count * ngroups;
-    const int wpb = solve_warps<T>(ln.fcap, 32);
-    long long blocks = std::min<long long>((ntasks + wpb - 1) / wpb, 148LL * 32);
-    const size_t smem = (size_t)wpb * ln.fcap * 32 * sizeof(T);
-    k_mf_fsolve<T><<<(unsigned)blocks, 32 * wpb, smem, st>>>(sys.dev(), sys.lev_sn.as<int>() + ln.offset, ln.count, ngroups,
-                                                        ln.fcap, pan, cbr, x, group_active);
-    CUDA_TRY(cudaGetLastError());
-    ++*nlaunch;
-  }
-}
-
 // ------------------------------------------------------------------ timing
 enum Family { FAM_MIS = 0, FAM_JAC, FAM_FACT, FAM_SOLVE, FAM_UPD, FAM_OTHER, FAM_N };
 
@@ -1510,6 +1539,22 @@ struct mpf_handle {
     }
   } nr_graph[2];
   cudaEvent_t t0 = nullptr, t1 = nullptr;
+
+  // mismatch rows grouped by island
+  DevBuf isl_rows, isl_row_ptr;
+  ChunkRows chunk_rows() {
+    if (!isl_row_ptr.p) {
+      std::vector<int> rows, ptr{0};
+      for (int k = 0; k < std::max(g.n_islands, 1); ++k) {
+        for (int i : g.mis_rows)
+          if (g.n_islands <= 1 || g.bus_island[i] == k) rows.push_back(i);
+        ptr.push_back((int)rows.size());
+      }
+      upload(isl_rows, rows);
+      upload(isl_row_ptr, ptr);
+    }
+    return ChunkRows{isl_rows.as<int>(), isl_row_ptr.as<int>()};
+  }
 
   DevGrid dev() const {
     DevGrid d;
@@ -1945,6 +1990,112 @@ void solve_nr(mpf_handle* h, cudaStream_t st) {
   h->timing.iterations_max = it_total;
 }
 
+// How a chunk kernel runs a set of systems: lanes per block, x and the carried entries in
+// shared memory or not, and the plans
+struct ChunkShape {
+  int G = 0;
+  bool xs = false;
+  int xcap = 0, ccap = 0, scratch = 0, slot = 0;
+  size_t smem = 0;
+  const PlanBufs* plan[2] = {};
+};
+
+// The shape for G lanes: x and the carried entries in shared memory (want_xs) with the rest
+// for the ring, or all of it for the ring; false when a supernode does not fit a slot
+inline bool chunk_shape(const std::vector<LUSystem*>& sys, int G, int wsize, bool want_xs, ChunkShape& out) {
+  out = ChunkShape();
+  out.G = G;
+  size_t held = kChunkScratch;
+  if (want_xs) {
+    for (LUSystem* s : sys) {
+      // any slot size gives the carried entries' slots
+      const PlanBufs* p = s->plan(true, G, wsize, 64);
+      if (!p) return false;
+      out.xcap = std::max(out.xcap, (s->sym.n + 3) / 4 * 4);
+      out.ccap = std::max(out.ccap, (p->peak_cb + 3) / 4 * 4);
+    }
+    held += (size_t)(out.xcap + out.ccap) * G * wsize;
+    out.xs = true;
+  }
+  if (held >= kChunkSmem) return false;
+  const int slot_kb = (int)std::min<size_t>((kChunkSmem - held) / kRingSlots / 1024, 48);
+  size_t scratch = 0, slot = 0;
+  for (size_t k = 0; k < sys.size(); ++k) {
+    out.plan[k] = sys[k]->plan(out.xs, G, wsize, slot_kb);
+    if (!out.plan[k]) return false;
+    scratch = std::max(scratch, out.plan[k]->scratch);
+    slot = std::max(slot, out.plan[k]->slot);
+  }
+  out.scratch = (int)((scratch + 3) / 4 * 4);
+  out.slot = (int)((slot + 15) / 16 * 16);
+  out.smem = (size_t)(out.scratch + out.xcap + out.ccap) * G * wsize + (size_t)kRingSlots * out.slot;
+  return out.smem <= kChunkSmem;
+}
+
+// Widest chunk (at most a 32-byte sector of lanes) that fits and leaves a block for every SM
+inline ChunkShape choose_chunk(const std::vector<LUSystem*>& sys, int widest, int wsize, int ngroups) {
+  ChunkShape sh;
+  if (const char* e = std::getenv("MPF_CHUNK_LANES")) {  // testing
+    const int v = std::atoi(e);
+    for (int xs = std::getenv("MPF_CHUNK_GLOBAL") ? 0 : 1; xs >= 0; --xs)
+      if ((v == 1 || v == 2 || v == 4 || v == 8) && v <= widest && chunk_shape(sys, v, wsize, xs == 1, sh)) return sh;
+  }
+  for (int G = widest; G >= 1; G /= 2) {
+    if (G > 1 && ngroups * (32 / G) < 74) continue;
+    for (int xs = 1; xs >= 0; --xs)
+      if (chunk_shape(sys, G, wsize, xs == 1, sh)) return sh;
+  }
+  throw MpfError{MPF_ERR_INTERNAL, "no chunk plan fits shared memory"};
+}
+
+template <typename T, int G, bool XS>
+void launch_fd_chunk_g(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSystem& Bp, LUSystem& Bpp,
+                       const ChunkShape& sh, cudaStream_t st) {
+  constexpr int P = Prec<T>::idx;
+  static std::mutex mu;
+  static bool done[64] = {};
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (h->device >= 64 || !done[h->device]) {
+      CUDA_TRY(cudaFuncSetAttribute(k_fd_chunk<T, G, XS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmem));
+      if (h->device < 64) done[h->device] = true;
+    }
+  }
+  FdChunk<T> a{};
+  LUSystem* sys[2] = {&Bp, &Bpp};
+  for (int k = 0; k < 2; ++k) {
+    a.sw[k] = sh.plan[k]->dev();
+    a.n[k] = sys[k]->sym.n;
+    a.nnz[k] = sys[k]->sym.nnz;
+    a.sumcbr[k] = sys[k]->sym.cbr_off.back();
+    a.pan[k] = sys[k]->pan[P].as<T>();
+    a.cbr[k] = sys[k]->cbr[P].as<T>();
+    a.x[k] = sys[k]->x[P].as<T>();
+  }
+  a.xcap = sh.xcap;
+  a.ccap = sh.ccap;
+  a.scratch = sh.scratch;
+  a.slot = sh.slot;
+  k_fd_chunk<T, G, XS><<<(unsigned)(h->ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(
+      d, fd, a, h->chunk_rows(), h->opt.max_it_fd, h->opt.tol);
+  CUDA_TRY(cudaGetLastError());
+}
+
+template <typename T>
+void launch_fd_chunk(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSystem& Bp, LUSystem& Bpp, cudaStream_t st) {
+  const ChunkShape sh = choose_chunk({&Bp, &Bpp}, Prec<T>::G, sizeof(T), h->ngroups);
+  auto go = [&](auto g) {
+    constexpr int G = decltype(g)::value;
+    if (sh.xs) launch_fd_chunk_g<T, G, true>(h, d, fd, Bp, Bpp, sh, st);
+    else launch_fd_chunk_g<T, G, false>(h, d, fd, Bp, Bpp, sh, st);
+  };
+  if constexpr (Prec<T>::G >= 8)
+    if (sh.G == 8) return go(std::integral_constant<int, 8>());
+  if (sh.G == 4) go(std::integral_constant<int, 4>());
+  else if (sh.G == 2) go(std::integral_constant<int, 2>());
+  else go(std::integral_constant<int, 1>());
+}
+
 template <typename T>
 void solve_fd(mpf_handle* h, cudaStream_t st, int variant) {
   constexpr int P = Prec<T>::idx;
@@ -2003,53 +2154,15 @@ void solve_fd(mpf_handle* h, cudaStream_t st, int variant) {
                      S.x[P].as<T>(), d.status, d.group_active, 0, st, &nl);
   }
   tm.end(ev);
-  if (h->opt.autotune)
-    for (int k = 0; k < 2; ++k) {
-      LUSystem& S = *systems[k];
-      tune_bsolve<T>(S, h->ngroups, S.pan[P].as<T>(), S.x[P].as<T>(), d.group_active, st);
-    }
-  T* xp = Bp.x[P].as<T>();
-  T* xq = Bpp.x[P].as<T>();
-  const int max_it = h->opt.max_it_fd;
-  auto mismatch = [&]() {
-    int e2 = tm.begin(FAM_MIS);
-    k_mismatch_fd<T><<<rg, 256, 0, st>>>(d, fdd, xp, xq);
-    CUDA_TRY(cudaGetLastError());
-    ++nl;
-    tm.end(e2);
-  };
-  mismatch();
-  ev = tm.begin(FAM_OTHER);
-  check(h, st, 0, max_it, &nl);
+  ev = tm.begin(FAM_SOLVE);
+  launch_fd_chunk<T>(h, d, fdd, Bp, Bpp, st);
+  ++nl;
   tm.end(ev);
-  int i = 0;
-  if (any_active(h, st)) {
-    while (i < max_it) {
-      ++i;
-      for (int half = 0; half < 2; ++half) {
-        LUSystem& S = half == 0 ? Bp : Bpp;
-        ev = tm.begin(FAM_SOLVE);
-        launch_fsolve<T>(S, h->ngroups, S.pan[P].as<T>(), S.cbr[P].as<T>(), S.x[P].as<T>(), d.group_active, st, &nl);
-        launch_bsolve<T>(S, h->ngroups, S.pan[P].as<T>(), S.x[P].as<T>(), d.group_active, st, &nl);
-        tm.end(ev);
-        ev = tm.begin(FAM_UPD);
-        k_update_fd<T><<<rg, 256, 0, st>>>(d, fdd, xp, xq, half);
-        CUDA_TRY(cudaGetLastError());
-        ++nl;
-        tm.end(ev);
-        mismatch();
-        ev = tm.begin(FAM_OTHER);
-        // after the P half only convergence retires a case (fdpf.h:529-540); the
-        // iteration limit is tested after the Q half
-        check(h, st, i, half == 0 ? INT32_MAX : max_it, &nl);
-        tm.end(ev);
-        if (!any_active(h, st)) break;
-      }
-      if (*h->h_any == 0) break;
-    }
-  }
+  // the largest iteration count over the chunks
+  CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaStreamSynchronize(st));
   h->timing.launches = nl;
-  h->timing.iterations_max = i;
+  h->timing.iterations_max = *h->h_any;
 }
 
 }  // namespace

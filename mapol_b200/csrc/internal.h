@@ -61,7 +61,7 @@ struct LUSymbolic {
   int nlevels = 0;
   std::vector<int> lev_ptr, lev_sn;  // supernodes grouped by level, by front size within a level
   std::vector<int> child_ptr, child_list;
-  std::vector<int64_t> pan_off;      // nsn+1, entries
+  std::vector<int64_t> pan_off;      // nsn+1, entries (order_panels); [nsn] = total
   // offsets of each supernode's contribution block ((f-w)^2 entries) and carried
   // right-hand side (f-w); siblings adjacent; [nsn] = the totals
   std::vector<int64_t> cb_off;       // nsn+1
@@ -97,6 +97,11 @@ struct Relax {
 // in the already-permuted variable numbering.
 void lu_symbolic(int n, const std::vector<std::vector<int>>& adj, LUSymbolic& s, const Relax& relax = Relax());
 
+// Panel storage: by island (sn_island, empty: one), level, solo or not, pivots and front size,
+// the order in which a block walks the supernodes (build_sweep_plan), so that a level's panels
+// are adjacent and similar fronts side by side.
+void order_panels(LUSymbolic& s, const std::vector<int>& sn_island);
+
 // Groups matrix entries (rows[e], cols[e]) by the supernode that owns min(row, col)
 // (its arrowhead).  a_index[e] = position of entry e in the grouped ("A-array")
 // order; supernode s owns A-array range [ah_ptr[s], ah_ptr[s+1]); ah_loc[k] is the
@@ -118,6 +123,45 @@ std::vector<int> minimum_degree(int n, const std::vector<std::vector<int>>& adj)
 // of counting fill (which grows with it) passes max_work (0: no limit).
 std::vector<int> minimum_fill(int n, const std::vector<std::vector<int>>& adj, const std::vector<int>* weight,
                               long long max_work = 0);
+
+// Plan of one block's substitutions over the elimination tree (kernels_chunk.cuh): leaves to
+// root, then root to leaves, as one sequence of steps.  A step is a run of supernodes of one
+// level whose panels are adjacent in storage (pan_off is in this order), small enough for a
+// slot of the block's ring buffer.  Supernodes of at most kSoloPivots pivots and kSoloFront
+// rows are solo tasks (1 to 8 threads per lane, no barriers), the others are worked on beside
+// them by nteams teams of `team` threads.
+constexpr int kChunkThreads = 512;
+constexpr int kSoloPivots = 4, kSoloFront = 16;
+constexpr int kRingSlots = 3;
+struct SweepStep {
+  int e0, ne;          // panel entries [e0, e0 + ne)
+  int i0, ni;          // index block: idx[i0 .. i0 + ni), both multiples of 4
+  int up, lsplit;      // 1: leaves to root; log2 of the threads per lane of a solo task
+  int nsolo, nbig;     // tasks of the index block: solo ones first
+  int lteam, nteams;   // log2 of a team's threads
+  int xstride, pad;    // values per lane a team needs for its front
+};
+constexpr int kStepInts = sizeof(SweepStep) / 4;
+inline bool solo_task(int w, int f) { return w <= kSoloPivots && f <= kSoloFront; }
+// Index block of a step: the SweepStep itself, a header of four ints per task, then the
+// tasks' index lists.  Header: panel entry relative to e0; w | f << 12 | layers << 24; start
+// of the task's list in the block; where the rows below the pivots are carried (-1: no
+// parent).  List: the x indices of the pivots [w] (leaves to root) or of the front [f] (root
+// to leaves); leaves to root also `layers` rows of f pairs: the carried entries that front
+// row i adds, two per layer, children in order (-1: none).
+struct SweepPlan {
+  std::vector<SweepStep> step;
+  std::vector<int> step_ptr;   // steps of each island
+  std::vector<int> idx;
+  int peak_cb = 0;             // carried entries alive at once (most over the islands)
+  size_t scratch = 0;          // values per lane of shared memory the teams need
+  size_t slot = 0;             // bytes of the largest step
+};
+// compact_cb: carried entries get slots that are reused once the parent has read them (else
+// their storage in cbr).  G lanes of wsize-byte values; slot: most bytes of a step; scratch:
+// bytes for the teams' fronts.  False when a supernode does not fit.
+bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bool compact_cb, int G, int wsize,
+                      size_t slot, size_t scratch, SweepPlan& out);
 
 // Everything that does not depend on the case batch.
 struct GridSymbolic {

@@ -1,0 +1,536 @@
+// Kernels that keep a chunk of G lanes (cases) on one block for a whole solve (sm_100a).
+//
+// Cases are independent, so a block that owns G lanes of a group can walk every level of
+// the elimination tree by itself: block barriers separate the levels, no block waits for
+// another, and the launch per level (and class of front size) of the level-synchronous
+// kernels, with its latency and its tail, disappears.
+//
+// What bounds such a walk is latency: a level is a handful of tiny fronts, and each would
+// be a chain of round trips to L2 (task, indices, panel).  So x and the carried entries stay
+// in shared memory (where they fit), and everything a level reads that no level writes (its
+// panels and index lists, stored in the order of the walk) streams through a ring buffer in
+// shared memory with cp.async, two steps ahead.  A step then costs a barrier and its
+// arithmetic.  Small supernodes (most of them) take 1 to 8 threads per lane without barriers,
+// and the few larger fronts of a step run beside them on teams of 32 to 1024 threads.
+#pragma once
+
+#include "internal.h"
+#include "kernels.cuh"
+
+namespace mpfk {
+
+using mpf::kChunkThreads;
+using mpf::kRingSlots;
+using mpf::kSoloPivots;
+using mpf::SweepStep;
+
+struct DevSweep {
+  const int4* step;      // per step: e0, ne, i0, ni
+  const int* step_ptr;   // steps of each island
+  const int* idx;
+};
+
+// rows of the mismatch by island
+struct ChunkRows {
+  const int* rows;
+  const int* ptr;  // [islands + 1]
+};
+
+// A team's barrier: a warp, or a named barrier (1 .. 15) of `team` threads; the whole
+// block uses barrier 0
+__device__ __forceinline__ void chunk_sync(int team, int bar) {
+  if (team == 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(team) : "memory");
+}
+
+// x and the carried entries of a chunk: entry i of this thread's lane at x[i * S], c[i * S]
+// (shared memory: S = G; the LU system's arrays: S = 32)
+template <typename T>
+struct ChunkVec {
+  T* x;
+  T* c;
+};
+
+// One substitution step of a supernode.  Leaves to root (UP): L y = b, or with TR U^T z = b,
+// the rows below the pivots carried to the parent; root to leaves: U x = y, or with TR
+// L^T l = z, the ancestors' values known.
+//
+// solo: by `split` threads per lane (thread r of them, G apart in the warp), each with the
+// pivots' values in registers and every split-th of the other rows.  All threads of the warp
+// call it together (on: this one has a task).  pan: the task's panel at this lane, entries G
+// apart.  The loops are kept rolled: a block runs each path once per step, so a kernel larger
+// than the instruction cache is bound by fetching it (334 KB unrolled: 150k cycles per half
+// step of a 300-bus fast-decoupled solve).
+template <typename T, int G, int S, bool UP, bool TR>
+__device__ __forceinline__ void solo_subst(bool on, int4 h, const int* ib, int r, int split, const T* pan,
+                                           const ChunkVec<T>& v) {
+  constexpr int W = kSoloPivots;
+  const int w = on ? h.y & 0xfff : 0, f = on ? (h.y >> 12) & 0xfff : 0;
+  const int* xi = ib + h.z;
+  // entry (a, b) of the pivot block; row / column i beside it: entries sa apart from pivot to
+  // pivot, at side0 + i si
+  const int sa = UP == TR ? f * G : G, si = UP == TR ? G : w * G;
+  const T* side0 = UP == TR ? pan : pan + (w * f - w * w) * G;
+  T y[W];
+  if (UP) {
+    const int2* pr = reinterpret_cast<const int2*>(xi + ((w + 1) & ~1));
+    const int layers = on ? h.y >> 24 : 0;
+    auto carried = [&](int i, T s) {
+#pragma unroll 1
+      for (int k = 0; k < layers; ++k) {
+        const int2 q = pr[k * f + i];
+        if (q.x >= 0) s += v.c[q.x * S];
+        if (q.y >= 0) s += v.c[q.y * S];
+      }
+      return s;
+    };
+#pragma unroll
+    for (int a = 0; a < W; ++a) {
+      y[a] = (T)0;
+      if (a < w) {
+        y[a] = carried(a, v.x[xi[a] * S]);
+#pragma unroll
+        for (int b = 0; b < a; ++b) y[a] -= pan[(TR ? b * f + a : a * f + b) * G] * y[b];
+        if (TR) y[a] = y[a] / pan[(a * f + a) * G];
+      }
+    }
+    if (on && h.w >= 0) {
+#pragma unroll 1
+      for (int i = w + r; i < f; i += split) {
+        T s = carried(i, (T)0);
+        const T* e = side0 + i * si;
+#pragma unroll
+        for (int a = 0; a < W; ++a)
+          if (a < w) s -= e[a * sa] * y[a];
+        v.c[(h.w + i - w) * S] = s;
+      }
+    }
+    __syncwarp();  // the other threads of the task have read x
+  } else {
+    T acc[W];
+#pragma unroll
+    for (int a = 0; a < W; ++a) acc[a] = (T)0;
+#pragma unroll 1
+    for (int i = w + r; i < f; i += split) {
+      const T xv = v.x[xi[i] * S];
+      const T* e = side0 + i * si;
+#pragma unroll
+      for (int a = 0; a < W; ++a)
+        if (a < w) acc[a] += e[a * sa] * xv;
+    }
+#pragma unroll 1
+    for (int o = G; o < split * G; o <<= 1) {
+#pragma unroll
+      for (int a = 0; a < W; ++a) acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], o);
+    }
+#pragma unroll
+    for (int a = W - 1; a >= 0; --a) {
+      y[a] = (T)0;
+      if (a < w) {
+        y[a] = v.x[xi[a] * S] - acc[a];
+#pragma unroll
+        for (int b = a + 1; b < W; ++b)
+          if (b < w) y[a] -= pan[(TR ? b * f + a : a * f + b) * G] * y[b];
+        if (!TR) y[a] = y[a] / pan[(a * f + a) * G];
+      }
+    }
+    __syncwarp();
+  }
+  if (r == 0) {
+#pragma unroll
+    for (int a = 0; a < W; ++a)
+      if (a < w) v.x[xi[a] * S] = y[a];
+  }
+}
+
+// team: slot = thread / G, lane = thread % G; xs: the front's vector, [f][G].  The pivots
+// run one team barrier each; the rows that no later pivot needs take their whole sum
+// without barriers.
+template <typename T, int G, int S, bool UP, bool TR>
+__device__ __forceinline__ void team_subst(int4 h, const int* ib, int team, int tid, int bar, T* xs, const T* us,
+                                           const ChunkVec<T>& v) {
+  const int w = h.y & 0xfff, f = (h.y >> 12) & 0xfff, m = f - w;
+  const int SL = team / G, slot = tid / G;  // shifts: G is a power of two
+  const int* xi = ib + h.z;
+  if (UP) {
+    const int2* pr = reinterpret_cast<const int2*>(xi + ((w + 1) & ~1));
+#pragma unroll 1
+    for (int i = slot; i < f; i += SL) {
+      T b = i < w ? v.x[xi[i] * S] : (T)0;
+#pragma unroll 1
+      for (int k = 0; k < h.y >> 24; ++k) {
+        const int2 q = pr[k * f + i];
+        if (q.x >= 0) b += v.c[q.x * S];
+        if (q.y >= 0) b += v.c[q.y * S];
+      }
+      xs[i * G] = b;
+    }
+  } else {
+#pragma unroll 1
+    for (int q = slot; q < f; q += SL) xs[q * G] = v.x[xi[q] * S];
+  }
+  chunk_sync(team, bar);
+  const T* ul = us + w * f * G;  // L panel below the diagonal block
+  if (UP && !TR) {
+#pragma unroll 1
+    for (int p = 0; p + 1 < w; ++p) {
+      const T yp = xs[p * G];
+#pragma unroll 1
+      for (int i = p + 1 + slot; i < w; i += SL) xs[i * G] -= us[(i * f + p) * G] * yp;
+      chunk_sync(team, bar);
+    }
+#pragma unroll 1
+    for (int i = slot; i < m; i += SL) {
+      T b = xs[(w + i) * G];
+#pragma unroll 2
+      for (int p = 0; p < w; ++p) b -= ul[(i * w + p) * G] * xs[p * G];
+      xs[(w + i) * G] = b;
+    }
+  } else if (UP) {
+#pragma unroll 1
+    for (int p = 0; p < w; ++p) {
+      const T zp = xs[p * G] / us[(p * f + p) * G];
+#pragma unroll 1
+      for (int i = p + 1 + slot; i < w; i += SL) xs[i * G] -= us[(p * f + i) * G] * zp;
+      chunk_sync(team, bar);
+      if (slot == 0) xs[p * G] = zp;
+    }
+    chunk_sync(team, bar);
+#pragma unroll 1
+    for (int i = w + slot; i < f; i += SL) {
+      T b = xs[i * G];
+#pragma unroll 2
+      for (int p = 0; p < w; ++p) b -= us[(p * f + i) * G] * xs[p * G];
+      xs[i * G] = b;
+    }
+  } else if (!TR) {
+#pragma unroll 1
+    for (int r = slot; r < w; r += SL) {
+      T a = xs[r * G], a2 = (T)0;
+      const T* ur = us + r * f * G;
+      int q = w;
+#pragma unroll 1
+      for (; q + 1 < f; q += 2) {
+        a -= ur[q * G] * xs[q * G];
+        a2 -= ur[(q + 1) * G] * xs[(q + 1) * G];
+      }
+      if (q < f) a -= ur[q * G] * xs[q * G];
+      xs[r * G] = a + a2;
+    }
+    chunk_sync(team, bar);
+#pragma unroll 1
+    for (int p = w - 1; p >= 0; --p) {
+      const T xp = xs[p * G] / us[(p * f + p) * G];
+#pragma unroll 1
+      for (int r = slot; r < p; r += SL) xs[r * G] -= us[(r * f + p) * G] * xp;
+      chunk_sync(team, bar);
+      if (slot == 0) xs[p * G] = xp;
+    }
+    chunk_sync(team, bar);
+  } else {
+#pragma unroll 1
+    for (int p = slot; p < w; p += SL) {
+      T a = xs[p * G], a2 = (T)0;
+      int i = 0;
+#pragma unroll 1
+      for (; i + 1 < m; i += 2) {
+        a -= ul[(i * w + p) * G] * xs[(w + i) * G];
+        a2 -= ul[((i + 1) * w + p) * G] * xs[(w + i + 1) * G];
+      }
+      if (i < m) a -= ul[(i * w + p) * G] * xs[(w + i) * G];
+      xs[p * G] = a + a2;
+    }
+    chunk_sync(team, bar);
+#pragma unroll 1
+    for (int p = w - 1; p > 0; --p) {
+      const T xp = xs[p * G];
+#pragma unroll 1
+      for (int r = slot; r < p; r += SL) xs[r * G] -= us[(p * f + r) * G] * xp;
+      chunk_sync(team, bar);
+    }
+  }
+#pragma unroll 1
+  for (int p = slot; p < w; p += SL) v.x[xi[p] * S] = xs[p * G];
+  if (UP && h.w >= 0)
+#pragma unroll 1
+    for (int a = slot; a < m; a += SL) v.c[(h.w + a) * S] = xs[(w + a) * G];
+  chunk_sync(team, bar);
+}
+
+// The block's ring buffer: kRingSlots slots of `slot` bytes
+struct Ring {
+  unsigned char* base;
+  int slot;
+};
+
+// Starts the copies of step rec (e0, ne, i0, ni) into slot k and closes their group
+template <typename T, int G>
+__device__ __forceinline__ void ring_issue(const Ring& R, int k, int4 rec, const int* idx, const T* pan0) {
+  constexpr int V = (int)(16 / sizeof(T)) < G ? (int)(16 / sizeof(T)) : G;
+  constexpr int NV = G / V;
+  unsigned char* at = R.base + (size_t)k * R.slot;
+  const T* src = pan0 + (size_t)rec.x * 32;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < rec.y * NV; i += kChunkThreads)
+    cp_async<T, V>(reinterpret_cast<T*>(at) + (size_t)i * V, src + (size_t)(i / NV) * 32 + (i % NV) * V);
+  int* di = reinterpret_cast<int*>(at + ((size_t)rec.y * G * sizeof(T) + 15) / 16 * 16);
+#pragma unroll 1
+  for (int i = 4 * threadIdx.x; i < rec.w; i += 4 * kChunkThreads) cp_async<int, 4>(di + i, idx + rec.z + i);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// Starts the first two steps of a solve (their data must not change before sweep_run)
+template <typename T, int G>
+__device__ __forceinline__ void sweep_begin(const DevSweep& P, int island, const Ring& R, const T* pan0) {
+  const int s0 = P.step_ptr[island], s1 = P.step_ptr[island + 1];
+#pragma unroll 1
+  for (int k = 0; k < kRingSlots - 1; ++k)
+    ring_issue<T, G>(R, k, s0 + k < s1 ? P.step[s0 + k] : make_int4(0, 0, 0, 0), P.idx, pan0);
+}
+
+// Both substitutions of one island by the block, after sweep_begin (TR: with the transposed
+// factors).  pan0: the panels at the chunk's first lane; v: x and the carried entries at
+// this thread's lane (threadIdx.x % G); xs: the teams' fronts.  Ends with a block barrier;
+// every copy it started has landed.
+template <typename T, int G, int S, bool TR>
+__device__ __forceinline__ void sweep_run(const DevSweep& P, int island, const Ring& R, T* xs, const T* pan0,
+                                          const ChunkVec<T>& v) {
+  constexpr int kLg = G == 8 ? 3 : G == 4 ? 2 : G == 2 ? 1 : 0;
+  const int s0 = P.step_ptr[island], n = P.step_ptr[island + 1] - s0;
+  int slot = 0, free_slot = kRingSlots - 1;
+  int4 next = kRingSlots - 1 < n ? P.step[s0 + kRingSlots - 1] : make_int4(0, 0, 0, 0);
+  static_assert(kRingSlots == 3, "two steps in flight");
+  int ne0 = n > 0 ? P.step[s0].y : 0, ne1 = n > 1 ? P.step[s0 + 1].y : 0;  // their panel entries
+#pragma unroll 1
+  for (int k = 0; k < n; ++k) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kRingSlots - 2) : "memory");
+    __syncthreads();  // step k is in its slot; every thread is done with step k - 1
+    ring_issue<T, G>(R, free_slot, next, P.idx, pan0);
+    const int ne2 = next.y;
+    next = k + kRingSlots < n ? P.step[s0 + k + kRingSlots] : make_int4(0, 0, 0, 0);
+    const unsigned char* at = R.base + (size_t)slot * R.slot;
+    free_slot = slot;
+    slot = slot + 1 == kRingSlots ? 0 : slot + 1;
+    // the step's panels start the slot; its index block follows, the step record first
+    const T* pan = reinterpret_cast<const T*>(at);
+    const int* ib = reinterpret_cast<const int*>(at + ((size_t)ne0 * G * sizeof(T) + 15) / 16 * 16);
+    ne0 = ne1;
+    ne1 = ne2;
+    const int4 q0 = *reinterpret_cast<const int4*>(ib + 4), q1 = *reinterpret_cast<const int4*>(ib + 8);
+    const bool up = q0.x != 0;
+    const int ls = q0.y, nsolo = q0.z, nbig = q0.w, lteam = q1.x, nteams = q1.y, xstride = q1.z;
+    const int4* head = reinterpret_cast<const int4*>(ib + mpf::kStepInts);
+    const int busy = nteams << lteam;  // threads of the teams; the others take the solo tasks
+    if ((int)threadIdx.x < busy) {
+      const int team = 1 << lteam, ti = threadIdx.x >> lteam, tid = threadIdx.x & (team - 1);
+      T* x0 = xs + (size_t)ti * xstride * G + threadIdx.x % G;
+#pragma unroll 1
+      for (int t = ti; t < nbig; t += nteams) {
+        const int4 h = head[nsolo + t];
+        const T* us = pan + h.x * G + threadIdx.x % G;
+        if (up) team_subst<T, G, S, true, TR>(h, ib, team, tid, 1 + ti, x0, us, v);
+        else team_subst<T, G, S, false, TR>(h, ib, team, tid, 1 + ti, x0, us, v);
+      }
+    }
+    // solo tasks: thread -> (task, thread r of the lane, lane); a warp whose first task is past
+    // the last skips them (the trip count is the same for all its threads)
+    const int first = busy < kChunkThreads ? busy : 0;
+    const int lsg = ls + kLg, per = (kChunkThreads - first) >> lsg;
+    int tw = ((int)(threadIdx.x & ~31u) - first) >> lsg;
+    if ((int)threadIdx.x >= first && tw < nsolo) {
+      const int split = 1 << ls, r = (threadIdx.x / G) & (split - 1);
+      int t = ((int)threadIdx.x - first) >> lsg;
+#pragma unroll 1
+      do {
+        const bool on = t < nsolo;
+        const int4 h = head[on ? t : 0];
+        const T* p = pan + h.x * G + threadIdx.x % G;
+        if (up) solo_subst<T, G, S, true, TR>(on, h, ib, r, split, p, v);
+        else solo_subst<T, G, S, false, TR>(on, h, ib, r, split, p, v);
+        t += per;
+        tw += per;
+      } while (tw < nsolo);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+}
+
+// per-lane max over the block's threads (lane = thread % G), left in red[0 .. G)
+template <int G>
+__device__ __forceinline__ void chunk_lane_max(double v, double* red) {
+#pragma unroll
+  for (int o = 16; o >= G; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  const int ln = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (ln < G) red[warp * G + ln] = v;
+  __syncthreads();
+  if (threadIdx.x < G) {
+    double m = red[threadIdx.x];
+    for (int k = 1; k < kChunkThreads / 32; ++k) m = fmax(m, red[k * G + threadIdx.x]);
+    red[threadIdx.x] = m;
+  }
+  __syncthreads();
+}
+
+// Fast-decoupled mismatch of the block's lanes, thread = (row slot, lane):
+// P = Re(mis)/|V| over PV/PQ, Q = Im(mis)/|V| over PQ (fdpf.h:369-414); returns this thread's
+// max over both and writes the side the next half step solves (P, or Q with want_q) to x
+template <typename T, int G>
+__device__ __forceinline__ double chunk_mismatch_fd(const DevGrid& d, const DevFD& fd, const int* rows, int r0, int r1,
+                                                    const LaneOut& o, int g, int lane, T* x, int xs, bool want_q) {
+  double lmax = 0.0;
+#pragma unroll 1
+  for (int r = r0 + threadIdx.x / G; r < r1; r += kChunkThreads / G) {
+    const int i = rows[r];
+    double2 ib = make_double2(0.0, 0.0);
+    const bool touched = row_touched(o, d.y_diag[i]);
+    const double2 vi = d.V[at32(g, d.nb, i, lane)];
+    const int p0 = d.y_rowptr[i], p1 = d.y_rowptr[i + 1];
+    if (touched || d.y_slot) {
+      // the row's entries depend on the case
+#pragma unroll 1
+      for (int p = p0; p < p1; ++p) {
+        const double2 y = yentry(d, o, touched, p, g, lane), u = d.V[at32(g, d.nb, d.y_col[p], lane)];
+        ib.x += y.x * u.x - y.y * u.y;
+        ib.y += y.x * u.y + y.y * u.x;
+      }
+    } else {
+#pragma unroll 1
+      for (int p = p0; p < p1; p += 4) {
+        int jj[4];
+        double2 vv[4], yy[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) jj[u] = p + u < p1 ? d.y_col[p + u] : i;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          vv[u] = jj[u] == i ? vi : d.V[at32(g, d.nb, jj[u], lane)];
+          yy[u] = p + u < p1 ? d.y_val[p + u] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (p + u >= p1) break;
+          ib.x += yy[u].x * vv[u].x - yy[u].y * vv[u].y;
+          ib.y += yy[u].x * vv[u].y + yy[u].y * vv[u].x;
+        }
+      }
+    }
+    const double2 s = d.sbus_case ? d.sbus_case[at32(g, d.nb, i, lane)] : d.sbus0[i];
+    const double av = sqrt(vi.x * vi.x + vi.y * vi.y);
+    const double mr = (vi.x * ib.x + vi.y * ib.y - s.x) / av;
+    const double mi = (vi.y * ib.x - vi.x * ib.y - s.y) / av;
+    const int2 fv = fd.fdvar[i];
+    if (!want_q) x[fv.x * xs] = (T)mr;
+    double m = fabs(mr);
+    if (mr != mr) m = INFINITY;
+    if (fv.y >= 0) {
+      if (want_q) x[fv.y * xs] = (T)mi;
+      m = fmax(m, fabs(mi));
+      if (mi != mi) m = INFINITY;
+    }
+    lmax = fmax(lmax, finite_or_inf(m));
+  }
+  return lmax;
+}
+
+// The whole fast-decoupled iteration (fdpf.h:450-596) of a chunk of G lanes: mismatch,
+// check, then up to max_it iterations of two half steps (forward and backward
+// substitution with the stored factors of B' / B'', update, mismatch, check).  Replaces
+// a launch per level for each of the four substitutions of an iteration and a host read
+// of the "any case running" flag per half step.
+// XS: x and the carried entries of the half step in shared memory (else in the systems' arrays)
+template <typename T>
+struct FdChunk {  // [0]: B' (P half steps), [1]: B'' (Q half steps)
+  DevSweep sw[2];
+  int n[2];
+  long long nnz[2], sumcbr[2];
+  const T* pan[2];
+  T* cbr[2];
+  T* x[2];
+  int xcap, ccap, scratch, slot;  // shared memory: entries per lane of x, of the carried
+                                  // entries and of the teams' fronts; bytes per ring slot
+};
+template <typename T, int G, bool XS>
+__global__ void __launch_bounds__(kChunkThreads, 1) k_fd_chunk(const __grid_constant__ DevGrid d, DevFD fd,
+                                                               const __grid_constant__ FdChunk<T> a, ChunkRows cr,
+                                                               int max_it, double tol) {
+  constexpr int LPG = 32 / G, S = XS ? G : 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[kChunkThreads / 32 * G];
+  __shared__ int st[G];
+  T* const sx = reinterpret_cast<T*>(smem_raw);
+  T* const xs = XS ? sx + (size_t)(a.xcap + a.ccap) * G : sx;  // the teams' fronts
+  const Ring R{reinterpret_cast<unsigned char*>(xs + (size_t)a.scratch * G), a.slot};
+  const int g = blockIdx.x / LPG, lane0 = (blockIdx.x % LPG) * G;
+  const int l = threadIdx.x % G, lane = lane0 + l, c = g * 32 + lane;
+  const int island = d.group_island ? d.group_island[g] : 0;
+  const int r0 = cr.ptr[island], r1 = cr.ptr[island + 1];
+  if (threadIdx.x < G) st[threadIdx.x] = d.status[g * 32 + lane0 + threadIdx.x];
+  __syncthreads();
+  // the mismatch just evaluated decides each running lane (k_check); true while one runs
+  auto check = [&](int it, int limit) {
+    bool active = false;
+    if (threadIdx.x < G && st[threadIdx.x] == ST_RUNNING) {
+      const double m = red[threadIdx.x];
+      d.maxmis[c] = m;
+      d.iters[c] = it;
+      int s = ST_RUNNING;
+      if (!(m <= DBL_MAX)) s = ST_DIVERGED;
+      else if (m < tol) s = ST_CONVERGED;
+      else if (it >= limit) s = ST_MAX_ITER;
+      else active = true;
+      st[threadIdx.x] = s;
+    }
+    return __syncthreads_or(active) != 0;
+  };
+  auto vec = [&](int half) {
+    if (XS) return ChunkVec<T>{sx + l, sx + (size_t)a.xcap * G + l};
+    return ChunkVec<T>{a.x[half] + at32(g, a.n[half], 0, lane), a.cbr[half] + at32(g, a.sumcbr[half], 0, lane)};
+  };
+  // next: the half step that solves for what this mismatch writes
+  auto mismatch = [&](int next) {
+    LaneOut o;
+    load_outages(d, c, o);
+    const ChunkVec<T> v = vec(next);
+    chunk_lane_max<G>(chunk_mismatch_fd<T, G>(d, fd, cr.rows, r0, r1, o, g, lane, v.x, S, next == 1), red);
+  };
+  // a chunk whose lanes were all decided before the solve (padding, cut off) does nothing
+  if (!__syncthreads_or(threadIdx.x < G && st[threadIdx.x] == ST_RUNNING)) return;
+  auto pan0 = [&](int half) { return a.pan[half] + at32(g, a.nnz[half], 0, lane0); };
+  sweep_begin<T, G>(a.sw[0], island, R, pan0(0));
+  int it = 0, half = 0;
+#pragma unroll 1
+  for (;;) {
+    mismatch(half);
+    // after the P half only convergence retires a case (fdpf.h:529-540); the iteration limit
+    // is tested after the Q half (and at the start point)
+    if (!check(it, half == 1 ? INT_MAX : max_it)) break;
+    if (half == 0) ++it;
+    const ChunkVec<T> v = vec(half);
+    sweep_run<T, G, S, false>(a.sw[half], island, R, xs, pan0(half), v);
+    // the next half step's first panels come in while the voltages are updated
+    sweep_begin<T, G>(a.sw[1 - half], island, R, pan0(1 - half));
+    if (st[l] == ST_RUNNING)
+#pragma unroll 1
+      for (int r = r0 + threadIdx.x / G; r < r1; r += kChunkThreads / G) {
+        const int i = cr.rows[r];
+        const int2 fv = fd.fdvar[i];
+        if (half == 1 && fv.y < 0) continue;
+        const size_t k = at32(g, d.nb, i, lane);
+        const double2 u = d.V[k];
+        double mag = sqrt(u.x * u.x + u.y * u.y);
+        double ang = vangle(u, d.angle_mode);
+        if (half == 0) ang -= (double)v.x[fv.x * S];
+        else mag -= (double)v.x[fv.y * S];
+        double sn, cs;
+        sincos(ang, &sn, &cs);
+        d.V[k] = make_double2(mag * cs, mag * sn);
+      }
+    __syncthreads();
+    half = 1 - half;
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");  // the copies of a half step not taken
+  if (threadIdx.x < G) d.status[c] = st[threadIdx.x];
+  if (threadIdx.x == 0) atomicMax(d.it_ptr, it);
+}
+
+}  // namespace mpfk

@@ -11,6 +11,7 @@
 //  * B' and B'' of the fast-decoupled methods (makeB.h:311-501) with their
 //    symbolic LU and base values.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -190,6 +191,24 @@ int64_t LUSymbolic::entry_pos(int row, int col) const {
   return -1;
 }
 
+void order_panels(LUSymbolic& s, const std::vector<int>& sn_island) {
+  std::vector<int> order(s.nsn);
+  for (int q = 0; q < s.nsn; ++q) order[q] = q;
+  auto key = [&](int q) {
+    return std::make_tuple(sn_island.empty() ? 0 : sn_island[q], s.sn_level[q], !solo_task(s.sn_w[q], s.sn_f[q]),
+                           s.sn_w[q], s.sn_f[q]);
+  };
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key(a) < key(b); });
+  s.pan_off.assign(s.nsn + 1, 0);
+  int64_t off = 0;
+  for (int q : order) {
+    const int64_t w = s.sn_w[q], f = s.sn_f[q];
+    s.pan_off[q] = off;
+    off += w * f + (f - w) * w;
+  }
+  s.pan_off[s.nsn] = off;
+}
+
 void lu_symbolic(int n, const std::vector<std::vector<int>>& adj, LUSymbolic& s, const Relax& relax) {
   s = LUSymbolic();
   s.n = n;
@@ -350,13 +369,11 @@ void lu_symbolic(int n, const std::vector<std::vector<int>>& adj, LUSymbolic& s,
                        [&](int a, int b) { return s.sn_f[a] < s.sn_f[b]; });
   }
   // storage offsets, relative maps, flops (of the dense fronts, explicit zeros included)
-  s.pan_off.assign(ns + 1, 0);
   s.cb_off.assign(ns + 1, 0);
   s.cbr_off.assign(ns + 1, 0);
   s.rel_ptr.assign(ns + 1, 0);
   for (int q = 0; q < ns; ++q) {
     const int w = s.sn_w[q], f = s.sn_f[q];
-    s.pan_off[q + 1] = s.pan_off[q] + (int64_t)w * f + (int64_t)(f - w) * w;
     s.cb_off[q + 1] = s.cb_off[q] + (int64_t)(f - w) * (f - w);
     s.cbr_off[q + 1] = s.cbr_off[q] + (f - w);
     s.rel_ptr[q + 1] = s.rel_ptr[q] + (s.sn_parent[q] >= 0 ? f - w : 0);
@@ -386,6 +403,7 @@ void lu_symbolic(int n, const std::vector<std::vector<int>>& adj, LUSymbolic& s,
     s.cb_off[ns] = off;
     s.cbr_off[ns] = roff;
   }
+  order_panels(s, {});
   s.nnz = s.pan_off[ns];
   s.relmap.resize(s.rel_ptr[ns]);
   for (int q = 0; q < ns; ++q) {
@@ -814,7 +832,177 @@ std::string build_symbolic(const mpf_bus* buses, int nb, const mpf_branch* br, i
       build_fd(g, buses, br, false, variant, var_bpp, g.npq, adj_bpp, g.bpp[variant]);
     }
   }
+  if (g.n_islands > 1) {
+    // each island's panels together
+    auto by_island = [&](LUSymbolic& s, const std::vector<int>& var, const std::vector<int>* var2) {
+      std::vector<int> vi(s.n, 0), si(s.nsn);
+      for (int i = 0; i < g.nb; ++i) {
+        if (var[i] >= 0) vi[var[i]] = g.bus_island[i];
+        if (var2 && (*var2)[i] >= 0) vi[(*var2)[i]] = g.bus_island[i];
+      }
+      for (int k = 0; k < s.nsn; ++k) si[k] = vi[s.sn_rows[s.sn_rptr[k]]];
+      order_panels(s, si);
+    };
+    by_island(g.jac, g.var_va, &g.var_vm);
+    for (int v = 0; v < 2; ++v) {
+      by_island(g.bp[v].lu, g.bp[v].var, nullptr);
+      by_island(g.bpp[v].lu, g.bpp[v].var, nullptr);
+    }
+  }
   return std::string();
+}
+
+// ------------------------------------------------------------------ block plans
+bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bool compact_cb, int G, int wsize,
+                      size_t slot, size_t scratch, SweepPlan& out) {
+  out = SweepPlan();
+  if (s.nnz >= INT_MAX) return false;
+  const int nisl = sn_island.empty() ? 1 : 1 + *std::max_element(sn_island.begin(), sn_island.end());
+  std::vector<std::vector<int>> of_island(nisl);
+  for (int n = 0; n < s.nsn; ++n) of_island[sn_island.empty() ? 0 : sn_island[n]].push_back(n);
+  std::vector<int> cb(s.nsn, -1);
+  out.step_ptr.assign(1, 0);
+  auto bytes_of = [&](int64_t ne, size_t ni) { return (size_t)((ne * G * wsize + 15) / 16 * 16) + ni * 4; };
+  for (int isl = 0; isl < nisl; ++isl) {
+    // the island's supernodes by level, in panel order
+    std::vector<int> sn = of_island[isl];
+    std::sort(sn.begin(), sn.end(), [&](int a, int b) {
+      return s.sn_level[a] != s.sn_level[b] ? s.sn_level[a] < s.sn_level[b] : s.pan_off[a] < s.pan_off[b];
+    });
+    std::vector<int> lev{0};
+    for (size_t k = 1; k <= sn.size(); ++k)
+      if (k == sn.size() || s.sn_level[sn[k]] != s.sn_level[sn[k - 1]]) lev.push_back((int)k);
+    if (sn.empty()) lev.assign(1, 0);
+    const int nlev = (int)lev.size() - 1;
+    // carried entries: slots by first fit over the levels at which they are alive
+    std::vector<std::pair<int, int>> free_list{{0, INT_MAX}};  // (offset, length), ascending
+    for (int lv = 0; lv < nlev; ++lv) {
+      for (int k = lev[lv]; k < lev[lv + 1]; ++k) {
+        const int n = sn[k], m = s.sn_f[n] - s.sn_w[n];
+        if (s.sn_parent[n] < 0) continue;
+        if (!compact_cb) {
+          cb[n] = (int)s.cbr_off[n];
+          continue;
+        }
+        for (auto& fr : free_list)
+          if (fr.second >= m) {
+            cb[n] = fr.first;
+            fr.first += m;
+            fr.second -= m;
+            break;
+          }
+        out.peak_cb = std::max(out.peak_cb, cb[n] + m);
+      }
+      if (!compact_cb) continue;
+      for (int k = lev[lv]; k < lev[lv + 1]; ++k)
+        for (int c = s.child_ptr[sn[k]]; c < s.child_ptr[sn[k] + 1]; ++c) {
+          const int ch = s.child_list[c];
+          free_list.push_back({cb[ch], s.sn_f[ch] - s.sn_w[ch]});
+        }
+      std::sort(free_list.begin(), free_list.end());
+      std::vector<std::pair<int, int>> merged;
+      for (auto& fr : free_list) {
+        if (fr.second == 0) continue;
+        if (!merged.empty() && merged.back().first + merged.back().second == fr.first) merged.back().second += fr.second;
+        else merged.push_back(fr);
+      }
+      free_list = merged;
+    }
+    for (int q = 0; q < 2 * nlev; ++q) {
+      const bool up = q < nlev;
+      const int lv = up ? q : 2 * nlev - 1 - q;
+      // index list of a task
+      auto list_of = [&](int n, int* layers) {
+        const int w = s.sn_w[n], f = s.sn_f[n];
+        const int* rows = s.sn_rows.data() + s.sn_rptr[n];
+        std::vector<int> l(rows, rows + (up ? w : f));
+        *layers = 0;
+        if (!up) return l;
+        std::vector<std::vector<int>> src(f);
+        for (int c = s.child_ptr[n]; c < s.child_ptr[n + 1]; ++c) {
+          const int ch = s.child_list[c], m = s.sn_f[ch] - s.sn_w[ch];
+          for (int a = 0; a < m; ++a) src[s.relmap[s.rel_ptr[ch] + a]].push_back(cb[ch] + a);
+        }
+        for (auto& v : src) *layers = std::max(*layers, ((int)v.size() + 1) / 2);
+        l.resize((l.size() + 1) / 2 * 2, 0);  // pairs are read as 8-byte words
+        for (int k = 0; k < *layers; ++k)
+          for (int i = 0; i < f; ++i)
+            for (int e = 2 * k; e < 2 * k + 2; ++e) l.push_back(e < (int)src[i].size() ? src[i][e] : -1);
+        return l;
+      };
+      int k = lev[lv];
+      while (k < lev[lv + 1]) {
+        // as many tasks as the slot holds
+        SweepStep st{};
+        st.up = up;
+        st.e0 = (int)s.pan_off[sn[k]];
+        std::vector<int> head, lists;
+        int k2 = k, fbig = 0, wbig = 0;
+        for (; k2 < lev[lv + 1]; ++k2) {
+          const int n = sn[k2], w = s.sn_w[n], f = s.sn_f[n];
+          int layers = 0;
+          std::vector<int> l = list_of(n, &layers);
+          l.resize((l.size() + 1) / 2 * 2, 0);
+          const int ne = st.ne + w * f + (f - w) * w;
+          const size_t ni = (kStepInts + head.size() + 4 + lists.size() + l.size() + 3) / 4 * 4;
+          if (w > 4095 || f > 4095 || layers > 127) return false;
+          if (s.pan_off[n] != st.e0 + st.ne) return false;
+          if (bytes_of(ne, ni) > slot) break;
+          head.insert(head.end(), {st.ne, w | f << 12 | layers << 24, (int)lists.size(), cb[n]});
+          lists.insert(lists.end(), l.begin(), l.end());
+          st.ne = ne;
+          if (solo_task(w, f)) ++st.nsolo;
+          else {
+            ++st.nbig;
+            fbig = std::max(fbig, f);
+            wbig = std::max(wbig, w);
+          }
+        }
+        if (k2 == k) return false;
+        int team_threads = 32;
+        if (st.nbig > 0) {
+          st.xstride = (fbig + 3) / 4 * 4;
+          const int room = (int)(scratch / ((size_t)st.xstride * G * wsize));
+          // clock cycles: a task's latency, its pivots with a barrier each, its work over
+          // the team's threads
+          double best = -1.0;
+          for (int team : {32, 128, 256, 512, 1024}) {
+            if (team > kChunkThreads) break;
+            const int nt = std::min(std::min(kChunkThreads / team, room), st.nbig);
+            if (nt < 1) break;
+            const double t = (double)((st.nbig + nt - 1) / nt) *
+                             (400.0 + wbig * (team == 32 ? 90.0 : 110.0) + 10.0 * (double)wbig * fbig * G / team);
+            if (best < 0.0 || t < best) {
+              best = t;
+              team_threads = team;
+              st.nteams = nt;
+            }
+          }
+          if (best < 0.0) return false;
+          out.scratch = std::max(out.scratch, (size_t)st.nteams * st.xstride);
+        }
+        // threads per lane of a solo task: as many as the step's tasks leave room for
+        {
+          while (1 << st.lteam < team_threads) ++st.lteam;
+          const int room = kChunkThreads - st.nteams * team_threads;
+          while (st.lsplit < 3 && (2 << st.lsplit) * G <= 32 && st.nsolo * (2 << st.lsplit) * G <= room) ++st.lsplit;
+        }
+        for (size_t t = 0; t < head.size(); t += 4) head[t + 2] += kStepInts + (int)head.size();
+        st.i0 = (int)out.idx.size();
+        st.ni = (int)((kStepInts + head.size() + lists.size() + 3) / 4 * 4);
+        const int* rec = reinterpret_cast<const int*>(&st);
+        out.idx.insert(out.idx.end(), rec, rec + kStepInts);
+        out.idx.insert(out.idx.end(), head.begin(), head.end());
+        out.idx.insert(out.idx.end(), lists.begin(), lists.end());
+        out.idx.resize((size_t)st.i0 + st.ni, 0);
+        out.slot = std::max(out.slot, bytes_of(st.ne, st.ni));
+        out.step.push_back(st);
+        k = k2;
+      }
+    }
+    out.step_ptr.push_back((int)out.step.size());
+  }
+  return out.idx.size() < (size_t)INT_MAX;
 }
 
 }  // namespace mpf

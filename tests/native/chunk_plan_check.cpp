@@ -1,0 +1,222 @@
+// Checks build_sweep_plan on the Newton, B' and B'' systems of synthetic grids (one island
+// and two): a step's panels are adjacent and fit its slot with its index block, its teams fit
+// the block, its warps, its named barriers and the scratch; and both pairs of substitutions
+// walked over the plan, each step reading only its own index block and what earlier steps
+// wrote, equal a plain supernode-by-supernode substitution on random panels.  Prints the number of plans and the
+// largest relative difference.
+#include <cmath>
+#include <cstdio>
+#include <vector>
+
+#include "internal.h"
+
+using namespace mpf;
+
+static long plans = 0;
+static double worst = 0.0;
+
+enum { FWD, BWD, FWD_T, BWD_T };
+
+// plain substitution: supernodes in level order, carried entries in cbr
+static std::vector<double> plain(const LUSymbolic& s, const std::vector<double>& pan, std::vector<double> x, int kind) {
+  const bool up = kind == FWD || kind == FWD_T;
+  std::vector<double> c(s.cbr_off.back() + 1, 0.0);
+  for (int q = 0; q < (int)s.lev_sn.size(); ++q) {
+    const int n = s.lev_sn[up ? q : (int)s.lev_sn.size() - 1 - q];
+    const int w = s.sn_w[n], f = s.sn_f[n];
+    const int* rows = &s.sn_rows[s.sn_rptr[n]];
+    const double* P = &pan[s.pan_off[n]];
+    auto Lv = [&](int i, int p) { return i < w ? P[i * f + p] : P[w * f + (i - w) * w + p]; };
+    std::vector<double> b(f, 0.0);
+    for (int i = 0; i < f; ++i) b[i] = (i < w || !up) ? x[rows[i]] : 0.0;
+    if (up) {
+      for (int e = s.child_ptr[n]; e < s.child_ptr[n + 1]; ++e) {
+        const int ch = s.child_list[e];
+        for (int a = 0; a < s.sn_f[ch] - s.sn_w[ch]; ++a) b[s.relmap[s.rel_ptr[ch] + a]] += c[s.cbr_off[ch] + a];
+      }
+      for (int p = 0; p < w; ++p) {
+        if (kind == FWD_T) b[p] /= P[p * f + p];
+        for (int i = p + 1; i < f; ++i) b[i] -= (kind == FWD ? Lv(i, p) : P[p * f + i]) * b[p];
+      }
+      if (s.sn_parent[n] >= 0)
+        for (int a = 0; a < f - w; ++a) c[s.cbr_off[n] + a] = b[w + a];
+    } else {
+      for (int p = w - 1; p >= 0; --p) {
+        for (int i = p + 1; i < f; ++i) b[p] -= (kind == BWD ? P[p * f + i] : Lv(i, p)) * b[i];
+        if (kind == BWD) b[p] /= P[p * f + p];
+      }
+    }
+    for (int p = 0; p < w; ++p) x[rows[p]] = b[p];
+  }
+  return x;
+}
+
+static bool check(const LUSymbolic& s, const std::vector<int>& isl, bool compact, int G, int wsize, size_t slot, Rng& rng) {
+  const size_t scratch = 16 * 1024;
+  SweepPlan P;
+  if (!build_sweep_plan(s, isl, compact, G, wsize, slot, scratch, P)) {
+    // refused only where one supernode does not fit the slot or the scratch
+    for (int n = 0; n < s.nsn; ++n) {
+      const size_t w = s.sn_w[n], f = s.sn_f[n];
+      if ((w * (2 * f - w)) * G * wsize + 24 * f + 256 > slot || (f + 3) / 4 * 4 * G * wsize > scratch) return true;
+      size_t kids = 0;
+      for (int c = s.child_ptr[n]; c < s.child_ptr[n + 1]; ++c) ++kids;
+      if ((w * (2 * f - w)) * G * wsize + (12 + 4 + w + 2 + (kids + 1) / 2 * 2 * f) * 4 + 96 > slot) return true;
+    }
+    std::printf("refused without a reason\n");
+    return false;
+  }
+  ++plans;
+  std::vector<double> pan(s.nnz), x0(s.n);
+  for (double& v : pan) v = rng.uniform() - 0.5;
+  for (int n = 0; n < s.nsn; ++n)
+    for (int p = 0; p < s.sn_w[n]; ++p) pan[s.pan_off[n] + (size_t)p * s.sn_f[n] + p] = 8.0 + rng.uniform();
+  for (double& v : x0) v = rng.uniform() - 0.5;
+  int nisl = 1;
+  for (int v : isl) nisl = v + 1 > nisl ? v + 1 : nisl;
+  if ((int)P.step_ptr.size() != nisl + 1) return false;
+  size_t most = 0, widest = 0;
+  for (bool tr : {false, true}) {
+    std::vector<double> x = x0;
+    std::vector<int> seen(s.n, 0);
+    for (int k = 0; k < nisl; ++k) {
+      std::vector<double> c(compact ? P.peak_cb + 1 : s.cbr_off.back() + 1, std::nan(""));
+      for (int q = P.step_ptr[k]; q < P.step_ptr[k + 1]; ++q) {
+        // the kernel reads the record's first four ints from the step array, the rest and
+        // everything else from the step's index block
+        const SweepStep& R = P.step[q];
+        if (R.i0 % 4 || R.ni % 4 || R.i0 + R.ni > (int)P.idx.size() || R.e0 + R.ne > s.nnz) return false;
+        const size_t bytes = ((size_t)R.ne * G * wsize + 15) / 16 * 16 + (size_t)R.ni * 4;
+        if (bytes > slot) return false;
+        if (bytes > widest) widest = bytes;
+        const int* ib = &P.idx[R.i0];
+        const bool up = ib[4] != 0;
+        const int split = 1 << ib[5], nsolo = ib[6], nbig = ib[7], team = 1 << ib[8], nteams = ib[9], xstride = ib[10];
+        if (split < 1 || split * G > 32 || (split & (split - 1))) return false;
+        if (nbig > 0) {
+          if (team % 32 || nteams < 1 || team * nteams > kChunkThreads || (team > 32 && nteams > 15)) return false;
+          if ((size_t)nteams * xstride * G * wsize > scratch) return false;
+          if ((size_t)nteams * xstride > most) most = (size_t)nteams * xstride;
+        } else if (nteams != 0) {
+          return false;
+        }
+        const std::vector<double> cr = c, xr = x;  // what earlier steps left
+        std::vector<char> cw(c.size(), 0);
+        for (int t = 0; t < nsolo + nbig; ++t) {
+          const int* h = ib + kStepInts + 4 * t;
+          const int w = h[1] & 0xfff, f = (h[1] >> 12) & 0xfff, layers = h[1] >> 24, cbo = h[3];
+          if ((t < nsolo) != solo_task(w, f) || (t >= nsolo && f > xstride)) return false;
+          if (h[0] + w * (2 * f - w) > R.ne) return false;
+          const int* xi = ib + h[2];
+          const int* pr = xi + ((w + 1) & ~1);
+          if (up && (pr - ib) % 2) return false;
+          if ((up ? pr + 2 * f * layers : xi + f) > ib + R.ni) return false;
+          const double* M = &pan[R.e0 + h[0]];
+          auto Lv = [&](int i, int p) { return i < w ? M[i * f + p] : M[w * f + (i - w) * w + p]; };
+          std::vector<double> b(f, 0.0);
+          for (int i = 0; i < (up ? w : f); ++i) b[i] = xr[xi[i]];
+          if (up) {
+            for (int e = 0; e < layers; ++e)
+              for (int i = 0; i < f; ++i)
+                for (int z = 0; z < 2; ++z)
+                  if (pr[2 * (e * f + i) + z] >= 0) b[i] += cr[pr[2 * (e * f + i) + z]];
+            for (int p = 0; p < w; ++p) {
+              if (tr) b[p] /= M[p * f + p];
+              for (int i = p + 1; i < f; ++i) b[i] -= (tr ? M[p * f + i] : Lv(i, p)) * b[p];
+            }
+            for (int a = 0; a < f - w && cbo >= 0; ++a) {
+              if (cbo + a >= (int)c.size() || cw[cbo + a]) return false;
+              cw[cbo + a] = 1;
+              c[cbo + a] = b[w + a];
+            }
+          } else {
+            for (int p = w - 1; p >= 0; --p) {
+              for (int i = p + 1; i < f; ++i) b[p] -= (tr ? Lv(i, p) : M[p * f + i]) * b[i];
+              if (!tr) b[p] /= M[p * f + p];
+            }
+          }
+          for (int p = 0; p < w; ++p) {
+            x[xi[p]] = b[p];
+            ++seen[xi[p]];
+          }
+        }
+      }
+    }
+    for (int v : seen)
+      if (v != 2) return false;
+    const std::vector<double> ref = plain(s, pan, plain(s, pan, x0, tr ? FWD_T : FWD), tr ? BWD_T : BWD);
+    for (int i = 0; i < s.n; ++i) {
+      const double e = std::fabs(x[i] - ref[i]) / (1.0 + std::fabs(ref[i]));
+      if (!(e < 1e-12)) return false;
+      if (e > worst) worst = e;
+    }
+  }
+  return most == P.scratch && widest == P.slot;
+}
+
+int main() {
+  const int shapes[][4] = {{2, 1, 0, 0}, {30, 41, 5, 0}, {118, 179, 53, 0}, {300, 411, 69, 0},
+                           {1354, 1991, 259, 0}, {1354, 1991, 259, 1}, {2869, 4582, 509, 0}};
+  Rng rng(7);
+  for (auto& sh : shapes) {
+    std::vector<mpf_bus> bus(sh[0]);
+    std::vector<mpf_branch> br(sh[1]);
+    mpf_synth_params p;
+    mpf_synth_default(&p);
+    p.n_bus = sh[0];
+    p.n_branch = sh[1];
+    p.n_pv = sh[2];
+    p.topology = sh[3];
+    p.seed = 3;
+    if (sh[0] == 2) {
+      bus[0] = mpf_bus{MPF_BUS_SLACK, 0, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+      bus[1] = mpf_bus{MPF_BUS_PQ, 0, 1.0, 0.0, -0.1, -0.05, 0.0, 0.0};
+      br[0] = mpf_branch{0, 1, 1, 0, 0.02, 0.1, 0.0, 0.0, 0.0};
+    } else if (mpf_synth_grid(&p, bus.data(), br.data()) != 0) {
+      return 1;
+    }
+    // the grid alone, and twice as two islands of one system
+    for (int copies = 1; copies <= (sh[0] > 2000 ? 1 : 2); ++copies) {
+      std::vector<mpf_bus> b2;
+      std::vector<mpf_branch> r2;
+      for (int k = 0; k < copies; ++k) {
+        b2.insert(b2.end(), bus.begin(), bus.end());
+        for (mpf_branch x : br) {
+          x.from += k * sh[0];
+          x.to += k * sh[0];
+          r2.push_back(x);
+        }
+      }
+      GridSymbolic g;
+      const std::string msg = build_symbolic(b2.data(), (int)b2.size(), r2.data(), (int)r2.size(), g);
+      if (!msg.empty()) {
+        std::printf("%s\n", msg.c_str());
+        return 1;
+      }
+      auto islands = [&](const LUSymbolic& s, const std::vector<int>& var, const std::vector<int>* var2) {
+        std::vector<int> vi(s.n, 0), si;
+        if (g.n_islands <= 1) return si;
+        for (int i = 0; i < g.nb; ++i) {
+          if (var[i] >= 0) vi[var[i]] = g.bus_island[i];
+          if (var2 && (*var2)[i] >= 0) vi[(*var2)[i]] = g.bus_island[i];
+        }
+        for (int k = 0; k < s.nsn; ++k) si.push_back(vi[s.sn_rows[s.sn_rptr[k]]]);
+        return si;
+      };
+      const LUSymbolic* sys[3] = {&g.jac, &g.bp[0].lu, &g.bpp[0].lu};
+      const std::vector<int> isl[3] = {islands(g.jac, g.var_va, &g.var_vm), islands(g.bp[0].lu, g.bp[0].var, nullptr),
+                                       islands(g.bpp[0].lu, g.bpp[0].var, nullptr)};
+      for (int k = 0; k < 3; ++k)
+        for (bool compact : {false, true})
+          for (int G : {8, 1})
+            for (size_t slot : {(size_t)6 * 1024, (size_t)20 * 1024, (size_t)48 * 1024})
+              if (!check(*sys[k], isl[k], compact, G, 4, slot, rng) || !check(*sys[k], isl[k], compact, G / 2 + G % 2, 8, slot, rng)) {
+                std::printf("bad plan: %d buses, copies %d, system %d, compact %d, G %d, slot %zu\n", sh[0], copies, k,
+                            (int)compact, G, slot);
+                return 1;
+              }
+    }
+  }
+  std::printf("plans %ld worst %.2e\n", plans, worst);
+  return 0;
+}

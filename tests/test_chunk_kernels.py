@@ -1,0 +1,52 @@
+"""Kernels that keep a chunk of lanes on one block for a whole solve (kernels_chunk.cuh):
+their plan on the CPU, and on the GPU every lane count against the oracle at the sizes
+where a team, a chunk or a segment ends."""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+import mapol_b200 as m
+from oracle import oracle
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def test_plans_cover_every_supernode_once(built, tmp_path):
+    cxx = shutil.which("g++")
+    if not cxx:
+        pytest.skip("no g++")
+    exe = str(tmp_path / "chunk_plan_check")
+    csrc = os.path.join(ROOT, "mapol_b200", "csrc")
+    subprocess.run([cxx, "-O2", "-std=c++17", "-I" + os.path.join(ROOT, "include"), "-I" + csrc, "-o", exe,
+                    os.path.join(ROOT, "tests", "native", "chunk_plan_check.cpp"), os.path.join(csrc, "symbolic.cpp"),
+                    os.path.join(csrc, "synth.cpp")], check=True)
+    out = subprocess.run([exe], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout
+    assert int(out.stdout.split()[1]) > 400
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("in_shared", [True, False])
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+@pytest.mark.parametrize("prec", [m.FP64, m.MIXED])
+@pytest.mark.parametrize("n_bus,n_cases,topology", [(30, 1, 0), (118, 33, 0), (300, 70, 0), (300, 20, 1)])
+def test_fast_decoupled_chunks_match_oracle(gpu, monkeypatch, in_shared, lanes, prec, n_bus, n_cases, topology):
+    """Tolerance: both sides stop at max |F| < 1e-10; |dV| <= |J^-1| 1e-10 stays below the
+    1e-8 bar of the parity tests."""
+    monkeypatch.setenv("MPF_CHUNK_LANES", str(lanes))
+    if not in_shared:
+        monkeypatch.setenv("MPF_CHUNK_GLOBAL", "1")
+    buses, branches = m.synth_grid(n_bus, int(1.4 * n_bus), max(2, n_bus // 6), 0.1, seed=4, topology=topology)
+    n1 = np.flatnonzero(~m.find_bridges(branches, n_bus))
+    cases = ([[]] + [[int(b)] for b in np.resize(n1, n_cases)])[:n_cases]
+    for alg in (m.FDXB, m.FDBX):
+        ref = oracle.runpf(buses, branches, cases, alg=alg, tol=1e-10)
+        with m.PowerFlow(buses, branches, tol=1e-10) as pf:
+            res = pf.runpf(cases, alg=alg, precision=prec)
+        assert np.array_equal(res.converged, ref["converged"]) and res.converged.all()
+        assert np.abs(res.v - ref["v"]).max() < 1e-8
+        if prec == m.FP64:
+            assert np.array_equal(res.iterations, ref["iterations"])
