@@ -20,7 +20,6 @@ NVCC_FLAGS = [
     "-std=c++17",
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo",
-    "--split-compile", "0",
     "-Xcompiler", "-fPIC,-O3",
     "-shared",
 ]

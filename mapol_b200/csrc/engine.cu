@@ -246,7 +246,7 @@ struct LUSystem {
   std::map<std::pair<int, int>, std::vector<FactorChoice>> tuned;
   // autotuned lane count of every backward-solve level launch (0 = one case per thread)
   std::map<std::pair<int, int>, std::vector<int>> tuned_bs;
-  std::vector<Launch> level_sched;   // one launch per level (fast-decoupled forward and adjoint solves), ascending
+  std::vector<Launch> level_sched;   // one launch per level (adjoint solves of full FP64 batches), ascending
   std::vector<int> ah_host;          // arrowhead ranges (host copy of ah_ptr)
   int nA = 0;
   // values per precision [0] = FP64, [1] = FP32
@@ -345,12 +345,9 @@ struct LUSystem {
     level_sched.clear();
     for (int l = 0; l < s.nlevels; ++l) {
       const int b = s.lev_ptr[l], e = s.lev_ptr[l + 1];
-      int fmax_all = 0, wf = 0;
-      for (int k = b; k < e; ++k) {
-        fmax_all = std::max(fmax_all, s.sn_f[s.lev_sn[k]]);
-        wf = std::max(wf, s.sn_w[s.lev_sn[k]] * s.sn_f[s.lev_sn[k]]);
-      }
-      level_sched.push_back({b, e - b, 0, fmax_all, wf});
+      int fmax_all = 0;
+      for (int k = b; k < e; ++k) fmax_all = std::max(fmax_all, s.sn_f[s.lev_sn[k]]);
+      level_sched.push_back({b, e - b, 0, fmax_all});
       int k = b;
       while (k < e) {
         auto cls_of = [](int f) {
@@ -458,7 +455,7 @@ struct LUSystem {
   }
 
   // The sweep plan for blocks of G lanes of wsize-byte values with ring slots of slot_kb KB,
-  // kept on the device; null when a supernode does not fit
+  // kept on the device; null when a front does not fit the scratch
   const PlanBufs* plan(bool compact, int G, int wsize, int slot_kb) {
     const auto key = std::make_tuple(compact, G, wsize, slot_kb);
     auto it = plans.find(key);
@@ -2001,8 +1998,8 @@ struct ChunkShape {
 };
 
 // The shape for G lanes: x and the carried entries in shared memory (want_xs) with the rest
-// for the ring, or all of it for the ring; false when a supernode does not fit a slot
-inline bool chunk_shape(const std::vector<LUSystem*>& sys, int G, int wsize, bool want_xs, ChunkShape& out) {
+// for the ring, or all of it for the ring; false when that leaves no room
+inline bool chunk_shape(const std::vector<LUSystem*>& sys, int G, int wsize, bool want_xs, size_t budget, ChunkShape& out) {
   out = ChunkShape();
   out.G = G;
   size_t held = kChunkScratch;
@@ -2017,8 +2014,9 @@ inline bool chunk_shape(const std::vector<LUSystem*>& sys, int G, int wsize, boo
     held += (size_t)(out.xcap + out.ccap) * G * wsize;
     out.xs = true;
   }
-  if (held >= kChunkSmem) return false;
-  const int slot_kb = (int)std::min<size_t>((kChunkSmem - held) / kRingSlots / 1024, 48);
+  if (held >= budget) return false;
+  const int slot_kb = (int)std::min<size_t>((budget - held) / kRingSlots / 1024, 48);
+  if (slot_kb < 4) return false;
   size_t scratch = 0, slot = 0;
   for (size_t k = 0; k < sys.size(); ++k) {
     out.plan[k] = sys[k]->plan(out.xs, G, wsize, slot_kb);
@@ -2029,38 +2027,110 @@ inline bool chunk_shape(const std::vector<LUSystem*>& sys, int G, int wsize, boo
   out.scratch = (int)((scratch + 3) / 4 * 4);
   out.slot = (int)((slot + 15) / 16 * 16);
   out.smem = (size_t)(out.scratch + out.xcap + out.ccap) * G * wsize + (size_t)kRingSlots * out.slot;
-  return out.smem <= kChunkSmem;
+  return out.smem <= budget;
 }
 
 // Widest chunk (at most a 32-byte sector of lanes) that fits and leaves a block for every SM
-inline ChunkShape choose_chunk(const std::vector<LUSystem*>& sys, int widest, int wsize, int ngroups) {
+inline ChunkShape choose_chunk(const std::vector<LUSystem*>& sys, int widest, int wsize, int ngroups, int resident) {
   ChunkShape sh;
+  auto budget = [&](int G) { return resident > 1 && ngroups * (32 / G) > 148 ? kChunkSmem / resident : kChunkSmem; };
   if (const char* e = std::getenv("MPF_CHUNK_LANES")) {  // testing
     const int v = std::atoi(e);
     for (int xs = std::getenv("MPF_CHUNK_GLOBAL") ? 0 : 1; xs >= 0; --xs)
-      if ((v == 1 || v == 2 || v == 4 || v == 8) && v <= widest && chunk_shape(sys, v, wsize, xs == 1, sh)) return sh;
+      if ((v == 1 || v == 2 || v == 4 || v == 8) && v <= widest && chunk_shape(sys, v, wsize, xs == 1, budget(v), sh)) return sh;
   }
   for (int G = widest; G >= 1; G /= 2) {
     if (G > 1 && ngroups * (32 / G) < 74) continue;
     for (int xs = 1; xs >= 0; --xs)
-      if (chunk_shape(sys, G, wsize, xs == 1, sh)) return sh;
+      if (chunk_shape(sys, G, wsize, xs == 1, budget(G), sh)) return sh;
   }
   throw MpfError{MPF_ERR_INTERNAL, "no chunk plan fits shared memory"};
+}
+
+// Once per device: a kernel's permission to take the chunk kernels' shared memory
+template <auto Kernel>
+void allow_chunk_smem(int device) {
+  static std::mutex mu;
+  static bool done[64] = {};
+  std::lock_guard<std::mutex> lock(mu);
+  if (device < 64 && done[device]) return;
+  CUDA_TRY(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmem));
+  if (device < 64) done[device] = true;
+}
+
+// f(lanes, x in shared memory) with the shape's as compile-time constants
+template <typename T, class F>
+void with_shape(const ChunkShape& sh, F&& f) {
+  auto lanes = [&](auto g) {
+    if (sh.xs) f(g, std::true_type());
+    else f(g, std::false_type());
+  };
+  if constexpr (Prec<T>::G >= 8)
+    if (sh.G == 8) return lanes(std::integral_constant<int, 8>());
+  if (sh.G == 4) lanes(std::integral_constant<int, 4>());
+  else if (sh.G == 2) lanes(std::integral_constant<int, 2>());
+  else lanes(std::integral_constant<int, 1>());
+}
+
+template <typename T>
+void launch_fsolve_t(const LUSystem& sys, int ngroups, const T* pan, T* cbr, T* x, const int* group_active,
+                     cudaStream_t st) {
+  for (const Launch& ln : sys.level_sched) {
+    const long long ntasks = (long long)ln.count * ngroups;
+    const int wpb = solve_warps<T>(ln.fcap, 32);
+    const long long blocks = std::min<long long>((ntasks + wpb - 1) / wpb, 148LL * 32);
+    const size_t smem = (size_t)wpb * ln.fcap * 32 * sizeof(T);
+    k_mf_fsolve_t<T><<<(unsigned)blocks, 32 * wpb, smem, st>>>(sys.dev(), sys.lev_sn.as<int>() + ln.offset, ln.count,
+                                                          ngroups, ln.fcap, pan, cbr, x, group_active);
+    CUDA_TRY(cudaGetLastError());
+  }
+}
+
+template <typename T>
+void launch_bsolve_t(const LUSystem& sys, int ngroups, const T* pan, T* x, const int* group_active, cudaStream_t st) {
+  for (int k = (int)sys.level_sched.size() - 1; k >= 0; --k) {
+    const Launch& ln = sys.level_sched[k];
+    const long long ntasks = (long long)ln.count * ngroups;
+    const int wpb = solve_warps<T>(ln.fcap, 32);
+    const long long blocks = std::min<long long>((ntasks + wpb - 1) / wpb, 148LL * 32);
+    const size_t smem = (size_t)wpb * ln.fcap * 32 * sizeof(T);
+    k_mf_bsolve_t<T><<<(unsigned)blocks, 32 * wpb, smem, st>>>(sys.dev(), sys.lev_sn.as<int>() + ln.offset, ln.count,
+                                                          ngroups, ln.fcap, pan, x, group_active);
+    CUDA_TRY(cudaGetLastError());
+  }
+}
+
+// x <- (L U)^-T x for every lane: a block per chunk of lanes (k_subst_chunk), or for full
+// batches of plain FP64 whose x does not fit in shared memory a launch per level with a
+// case per thread.  1354 buses, whole adjoint, ms, level launches / chunks: FP64 4096 cases
+// 3.5 / 3.9, FP32 factors 4096 cases 6.2 / 5.2; 300 cases of 2869 buses 9.2 / 4.0, of 9241
+// buses 19.4 / 7.9; 500 of 300 buses 1.47 / 0.52.
+constexpr int kLevelSubstGroups = 64;
+template <typename T>
+void launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, const int* group_active, int device,
+                    cudaStream_t st) {
+  const ChunkShape sh = choose_chunk({&S}, Prec<T>::G, sizeof(T), ngroups, 2);
+  if (sizeof(T) == 8 && !sh.xs && ngroups >= kLevelSubstGroups) {
+    launch_fsolve_t<T>(S, ngroups, pan, cbr, x, group_active, st);
+    launch_bsolve_t<T>(S, ngroups, pan, x, group_active, st);
+    return;
+  }
+  with_shape<T>(sh, [&](auto g, auto xs) {
+    constexpr int G = decltype(g)::value;
+    constexpr bool XS = decltype(xs)::value;
+    allow_chunk_smem<k_subst_chunk<T, G, XS, true>>(device);
+    SubstChunk<T> a{sh.plan[0]->dev(), S.sym.n, S.sym.nnz, S.sym.cbr_off.back(), pan, cbr, x,
+                    sh.xcap, sh.ccap, sh.scratch, sh.slot};
+    k_subst_chunk<T, G, XS, true><<<(unsigned)(ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(a, S.group_island);
+    CUDA_TRY(cudaGetLastError());
+  });
 }
 
 template <typename T, int G, bool XS>
 void launch_fd_chunk_g(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSystem& Bp, LUSystem& Bpp,
                        const ChunkShape& sh, cudaStream_t st) {
   constexpr int P = Prec<T>::idx;
-  static std::mutex mu;
-  static bool done[64] = {};
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (h->device >= 64 || !done[h->device]) {
-      CUDA_TRY(cudaFuncSetAttribute(k_fd_chunk<T, G, XS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmem));
-      if (h->device < 64) done[h->device] = true;
-    }
-  }
+  allow_chunk_smem<k_fd_chunk<T, G, XS>>(h->device);
   FdChunk<T> a{};
   LUSystem* sys[2] = {&Bp, &Bpp};
   for (int k = 0; k < 2; ++k) {
@@ -2083,17 +2153,10 @@ void launch_fd_chunk_g(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSyste
 
 template <typename T>
 void launch_fd_chunk(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSystem& Bp, LUSystem& Bpp, cudaStream_t st) {
-  const ChunkShape sh = choose_chunk({&Bp, &Bpp}, Prec<T>::G, sizeof(T), h->ngroups);
-  auto go = [&](auto g) {
-    constexpr int G = decltype(g)::value;
-    if (sh.xs) launch_fd_chunk_g<T, G, true>(h, d, fd, Bp, Bpp, sh, st);
-    else launch_fd_chunk_g<T, G, false>(h, d, fd, Bp, Bpp, sh, st);
-  };
-  if constexpr (Prec<T>::G >= 8)
-    if (sh.G == 8) return go(std::integral_constant<int, 8>());
-  if (sh.G == 4) go(std::integral_constant<int, 4>());
-  else if (sh.G == 2) go(std::integral_constant<int, 2>());
-  else go(std::integral_constant<int, 1>());
+  const ChunkShape sh = choose_chunk({&Bp, &Bpp}, Prec<T>::G, sizeof(T), h->ngroups, 1);
+  with_shape<T>(sh, [&](auto g, auto xs) {
+    launch_fd_chunk_g<T, decltype(g)::value, decltype(xs)::value>(h, d, fd, Bp, Bpp, sh, st);
+  });
 }
 
 template <typename T>
@@ -2196,34 +2259,6 @@ cudaError_t noalloc_scratch(int device, unsigned long long** out) {
 }  // namespace
 
 // ------------------------------------------------------------------ adjoint
-template <typename T>
-void launch_fsolve_t(const LUSystem& sys, int ngroups, const T* pan, T* cbr, T* x, const int* group_active,
-                     cudaStream_t st) {
-  for (const Launch& ln : sys.level_sched) {
-    const long long ntasks = (long long)ln.count * ngroups;
-    const int wpb = solve_warps<T>(ln.fcap, 32);
-    const long long blocks = std::min<long long>((ntasks + wpb - 1) / wpb, 148LL * 32);
-    const size_t smem = (size_t)wpb * ln.fcap * 32 * sizeof(T);
-    k_mf_fsolve_t<T><<<(unsigned)blocks, 32 * wpb, smem, st>>>(sys.dev(), sys.lev_sn.as<int>() + ln.offset, ln.count,
-                                                          ngroups, ln.fcap, pan, cbr, x, group_active);
-    CUDA_TRY(cudaGetLastError());
-  }
-}
-
-template <typename T>
-void launch_bsolve_t(const LUSystem& sys, int ngroups, const T* pan, T* x, const int* group_active, cudaStream_t st) {
-  for (int k = (int)sys.level_sched.size() - 1; k >= 0; --k) {
-    const Launch& ln = sys.level_sched[k];
-    const long long ntasks = (long long)ln.count * ngroups;
-    const int wpb = solve_warps<T>(ln.fcap, 32);
-    const long long blocks = std::min<long long>((ntasks + wpb - 1) / wpb, 148LL * 32);
-    const size_t smem = (size_t)wpb * ln.fcap * 32 * sizeof(T);
-    k_mf_bsolve_t<T><<<(unsigned)blocks, 32 * wpb, smem, st>>>(sys.dev(), sys.lev_sn.as<int>() + ln.offset, ln.count,
-                                                          ngroups, ln.fcap, pan, x, group_active);
-    CUDA_TRY(cudaGetLastError());
-  }
-}
-
 // Refinement steps of the adjoint solved with FP32 factors (each reduces the error by
 // about the FP32 LU's own accuracy, ~1e-4 relative on the 1354-bus grid).
 constexpr int kAdjRefine = 2;
@@ -2269,8 +2304,7 @@ void adjoint_impl(mpf_handle* h, cudaStream_t st, double* gp, double* gq, double
     CUDA_TRY(cudaMemsetAsync(x, 0, nx * sizeof(T), st));
     k_adj_dldx<T><<<bg, 256, 0, st>>>(d, h->g.nbr, h->rating.as<double>(), x);
     CUDA_TRY(cudaGetLastError());
-    launch_fsolve_t<T>(J, h->ngroups, pan, J.cbr[P].as<T>(), x, d.group_active, st);
-    launch_bsolve_t<T>(J, h->ngroups, pan, x, d.group_active, st);
+    launch_subst_t<T>(J, h->ngroups, pan, J.cbr[P].as<T>(), x, d.group_active, h->device, st);
     gradients(x);
   } else {
     // FP32 factors: solve, then refine with FP64 residuals of the FP64 Jacobian
@@ -2298,8 +2332,7 @@ void adjoint_impl(mpf_handle* h, cudaStream_t st, double* gp, double* gq, double
                                                  h->adj_colent.as<int2>(), A64, lam64, b64, x);
         CUDA_TRY(cudaGetLastError());
       }
-      launch_fsolve_t<T>(J, h->ngroups, pan, J.cbr[P].as<T>(), x, d.group_active, st);
-      launch_bsolve_t<T>(J, h->ngroups, pan, x, d.group_active, st);
+      launch_subst_t<T>(J, h->ngroups, pan, J.cbr[P].as<T>(), x, d.group_active, h->device, st);
       k_adj_accumulate<T><<<eb, 256, 0, st>>>(nx, x, lam64, r > 0);
       CUDA_TRY(cudaGetLastError());
     }

@@ -139,16 +139,18 @@ struct SweepStep {
   int up, lsplit;      // 1: leaves to root; log2 of the threads per lane of a solo task
   int nsolo, nbig;     // tasks of the index block: solo ones first
   int lteam, nteams;   // log2 of a team's threads
-  int xstride, pad;    // values per lane a team needs for its front
+  int xstride;         // values per lane a team needs for its front
+  int direct;          // 1: one team task too large for a slot: its panel and list are read
+                       // where they are (ne = 0; the list follows the block in idx)
 };
 constexpr int kStepInts = sizeof(SweepStep) / 4;
 inline bool solo_task(int w, int f) { return w <= kSoloPivots && f <= kSoloFront; }
 // Index block of a step: the SweepStep itself, a header of four ints per task, then the
-// tasks' index lists.  Header: panel entry relative to e0; w | f << 12 | layers << 24; start
-// of the task's list in the block; where the rows below the pivots are carried (-1: no
-// parent).  List: the x indices of the pivots [w] (leaves to root) or of the front [f] (root
-// to leaves); leaves to root also `layers` rows of f pairs: the carried entries that front
-// row i adds, two per layer, children in order (-1: none).
+// tasks' index lists.  Header: panel entry relative to e0; w | f << 16; start of the task's
+// list in the block; where the rows below the pivots are carried (-1: no parent).  List, root
+// to leaves: the x indices of the front [f].  Leaves to root: the number of layers and a 0,
+// the x indices of the pivots [w] (an even number of ints), and per layer f pairs: the
+// carried entries that front row i adds, two per layer, children in order (-1: none).
 struct SweepPlan {
   std::vector<SweepStep> step;
   std::vector<int> step_ptr;   // steps of each island
@@ -159,7 +161,7 @@ struct SweepPlan {
 };
 // compact_cb: carried entries get slots that are reused once the parent has read them (else
 // their storage in cbr).  G lanes of wsize-byte values; slot: most bytes of a step; scratch:
-// bytes for the teams' fronts.  False when a supernode does not fit.
+// bytes for the teams' fronts.  False when a front does not fit the scratch.
 bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bool compact_cb, int G, int wsize,
                       size_t slot, size_t scratch, SweepPlan& out);
 

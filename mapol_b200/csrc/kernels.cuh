@@ -2010,7 +2010,7 @@ __global__ void k_adj_cast(size_t n_total, const double* __restrict__ b, T* __re
 
 // U^T z = g, supernodes bottom-up (thread per case, warp per (supernode, group)):
 // pivots in order, each pushes U(p, i) z_p into the later rows of its front; the
-// non-pivot rows travel to the parent as a carried vector (as k_mf_fsolve).
+// non-pivot rows travel to the parent as a carried vector.
 template <typename T>
 __global__ void __launch_bounds__(128) k_mf_fsolve_t(DevLU L, const int* __restrict__ task_sn, int nsn_l,
                                                      int ngroups, int fcap, const T* __restrict__ pan,

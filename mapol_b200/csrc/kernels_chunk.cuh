@@ -65,8 +65,8 @@ template <typename T, int G, int S, bool UP, bool TR>
 __device__ __forceinline__ void solo_subst(bool on, int4 h, const int* ib, int r, int split, const T* pan,
                                            const ChunkVec<T>& v) {
   constexpr int W = kSoloPivots;
-  const int w = on ? h.y & 0xfff : 0, f = on ? (h.y >> 12) & 0xfff : 0;
-  const int* xi = ib + h.z;
+  const int w = on ? h.y & 0xffff : 0, f = on ? h.y >> 16 : 0;
+  const int* xi = ib + h.z + (UP ? 2 : 0);
   // entry (a, b) of the pivot block; row / column i beside it: entries sa apart from pivot to
   // pivot, at side0 + i si
   const int sa = UP == TR ? f * G : G, si = UP == TR ? G : w * G;
@@ -74,7 +74,7 @@ __device__ __forceinline__ void solo_subst(bool on, int4 h, const int* ib, int r
   T y[W];
   if (UP) {
     const int2* pr = reinterpret_cast<const int2*>(xi + ((w + 1) & ~1));
-    const int layers = on ? h.y >> 24 : 0;
+    const int layers = on ? xi[-2] : 0;
     auto carried = [&](int i, T s) {
 #pragma unroll 1
       for (int k = 0; k < layers; ++k) {
@@ -143,22 +143,24 @@ __device__ __forceinline__ void solo_subst(bool on, int4 h, const int* ib, int r
   }
 }
 
-// team: slot = thread / G, lane = thread % G; xs: the front's vector, [f][G].  The pivots
+// team: slot = thread / G, lane = thread % G; xs: the front's vector, [f][G]; us: the panel,
+// entries es apart.  The pivots
 // run one team barrier each; the rows that no later pivot needs take their whole sum
 // without barriers.
 template <typename T, int G, int S, bool UP, bool TR>
-__device__ __forceinline__ void team_subst(int4 h, const int* ib, int team, int tid, int bar, T* xs, const T* us,
+__device__ __forceinline__ void team_subst(int4 h, const int* xi, int team, int tid, int bar, T* xs, const T* us, int es,
                                            const ChunkVec<T>& v) {
-  const int w = h.y & 0xfff, f = (h.y >> 12) & 0xfff, m = f - w;
+  const int w = h.y & 0xffff, f = h.y >> 16, m = f - w;
   const int SL = team / G, slot = tid / G;  // shifts: G is a power of two
-  const int* xi = ib + h.z;
+  if (UP) xi += 2;
   if (UP) {
+    const int layers = xi[-2];
     const int2* pr = reinterpret_cast<const int2*>(xi + ((w + 1) & ~1));
 #pragma unroll 1
     for (int i = slot; i < f; i += SL) {
       T b = i < w ? v.x[xi[i] * S] : (T)0;
 #pragma unroll 1
-      for (int k = 0; k < h.y >> 24; ++k) {
+      for (int k = 0; k < layers; ++k) {
         const int2 q = pr[k * f + i];
         if (q.x >= 0) b += v.c[q.x * S];
         if (q.y >= 0) b += v.c[q.y * S];
@@ -170,28 +172,28 @@ __device__ __forceinline__ void team_subst(int4 h, const int* ib, int team, int 
     for (int q = slot; q < f; q += SL) xs[q * G] = v.x[xi[q] * S];
   }
   chunk_sync(team, bar);
-  const T* ul = us + w * f * G;  // L panel below the diagonal block
+  const T* ul = us + w * f * es;  // L panel below the diagonal block
   if (UP && !TR) {
 #pragma unroll 1
     for (int p = 0; p + 1 < w; ++p) {
       const T yp = xs[p * G];
 #pragma unroll 1
-      for (int i = p + 1 + slot; i < w; i += SL) xs[i * G] -= us[(i * f + p) * G] * yp;
+      for (int i = p + 1 + slot; i < w; i += SL) xs[i * G] -= us[(i * f + p) * es] * yp;
       chunk_sync(team, bar);
     }
 #pragma unroll 1
     for (int i = slot; i < m; i += SL) {
       T b = xs[(w + i) * G];
 #pragma unroll 2
-      for (int p = 0; p < w; ++p) b -= ul[(i * w + p) * G] * xs[p * G];
+      for (int p = 0; p < w; ++p) b -= ul[(i * w + p) * es] * xs[p * G];
       xs[(w + i) * G] = b;
     }
   } else if (UP) {
 #pragma unroll 1
     for (int p = 0; p < w; ++p) {
-      const T zp = xs[p * G] / us[(p * f + p) * G];
+      const T zp = xs[p * G] / us[(p * f + p) * es];
 #pragma unroll 1
-      for (int i = p + 1 + slot; i < w; i += SL) xs[i * G] -= us[(p * f + i) * G] * zp;
+      for (int i = p + 1 + slot; i < w; i += SL) xs[i * G] -= us[(p * f + i) * es] * zp;
       chunk_sync(team, bar);
       if (slot == 0) xs[p * G] = zp;
     }
@@ -200,29 +202,29 @@ __device__ __forceinline__ void team_subst(int4 h, const int* ib, int team, int 
     for (int i = w + slot; i < f; i += SL) {
       T b = xs[i * G];
 #pragma unroll 2
-      for (int p = 0; p < w; ++p) b -= us[(p * f + i) * G] * xs[p * G];
+      for (int p = 0; p < w; ++p) b -= us[(p * f + i) * es] * xs[p * G];
       xs[i * G] = b;
     }
   } else if (!TR) {
 #pragma unroll 1
     for (int r = slot; r < w; r += SL) {
       T a = xs[r * G], a2 = (T)0;
-      const T* ur = us + r * f * G;
+      const T* ur = us + r * f * es;
       int q = w;
 #pragma unroll 1
       for (; q + 1 < f; q += 2) {
-        a -= ur[q * G] * xs[q * G];
-        a2 -= ur[(q + 1) * G] * xs[(q + 1) * G];
+        a -= ur[q * es] * xs[q * G];
+        a2 -= ur[(q + 1) * es] * xs[(q + 1) * G];
       }
-      if (q < f) a -= ur[q * G] * xs[q * G];
+      if (q < f) a -= ur[q * es] * xs[q * G];
       xs[r * G] = a + a2;
     }
     chunk_sync(team, bar);
 #pragma unroll 1
     for (int p = w - 1; p >= 0; --p) {
-      const T xp = xs[p * G] / us[(p * f + p) * G];
+      const T xp = xs[p * G] / us[(p * f + p) * es];
 #pragma unroll 1
-      for (int r = slot; r < p; r += SL) xs[r * G] -= us[(r * f + p) * G] * xp;
+      for (int r = slot; r < p; r += SL) xs[r * G] -= us[(r * f + p) * es] * xp;
       chunk_sync(team, bar);
       if (slot == 0) xs[p * G] = xp;
     }
@@ -234,10 +236,10 @@ __device__ __forceinline__ void team_subst(int4 h, const int* ib, int team, int 
       int i = 0;
 #pragma unroll 1
       for (; i + 1 < m; i += 2) {
-        a -= ul[(i * w + p) * G] * xs[(w + i) * G];
-        a2 -= ul[((i + 1) * w + p) * G] * xs[(w + i + 1) * G];
+        a -= ul[(i * w + p) * es] * xs[(w + i) * G];
+        a2 -= ul[((i + 1) * w + p) * es] * xs[(w + i + 1) * G];
       }
-      if (i < m) a -= ul[(i * w + p) * G] * xs[(w + i) * G];
+      if (i < m) a -= ul[(i * w + p) * es] * xs[(w + i) * G];
       xs[p * G] = a + a2;
     }
     chunk_sync(team, bar);
@@ -245,7 +247,7 @@ __device__ __forceinline__ void team_subst(int4 h, const int* ib, int team, int 
     for (int p = w - 1; p > 0; --p) {
       const T xp = xs[p * G];
 #pragma unroll 1
-      for (int r = slot; r < p; r += SL) xs[r * G] -= us[(p * f + r) * G] * xp;
+      for (int r = slot; r < p; r += SL) xs[r * G] -= us[(p * f + r) * es] * xp;
       chunk_sync(team, bar);
     }
   }
@@ -327,9 +329,12 @@ __device__ __forceinline__ void sweep_run(const DevSweep& P, int island, const R
 #pragma unroll 1
       for (int t = ti; t < nbig; t += nteams) {
         const int4 h = head[nsolo + t];
-        const T* us = pan + h.x * G + threadIdx.x % G;
-        if (up) team_subst<T, G, S, true, TR>(h, ib, team, tid, 1 + ti, x0, us, v);
-        else team_subst<T, G, S, false, TR>(h, ib, team, tid, 1 + ti, x0, us, v);
+        // a direct step: ib[0] = e0, ib[2] = i0
+        const T* us = (q1.w ? pan0 + (size_t)ib[0] * 32 : pan + h.x * G) + threadIdx.x % G;
+        const int* xi = q1.w ? P.idx + ib[2] + h.z : ib + h.z;
+        const int es = q1.w ? 32 : G;
+        if (up) team_subst<T, G, S, true, TR>(h, xi, team, tid, 1 + ti, x0, us, es, v);
+        else team_subst<T, G, S, false, TR>(h, xi, team, tid, 1 + ti, x0, us, es, v);
       }
     }
     // solo tasks: thread -> (task, thread r of the lane, lane); a warp whose first task is past
@@ -354,6 +359,40 @@ __device__ __forceinline__ void sweep_run(const DevSweep& P, int island, const R
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
+}
+
+// Both substitutions with the (transposed, TR) factors of one system for a chunk of lanes:
+// x in place.  XS: x and the carried entries in shared memory.
+template <typename T>
+struct SubstChunk {
+  DevSweep sw;
+  int n;
+  long long nnz, sumcbr;
+  const T* pan;
+  T* cbr;
+  T* x;
+  int xcap, ccap, scratch, slot;  // as FdChunk
+};
+template <typename T, int G, bool XS, bool TR>
+__global__ void __launch_bounds__(kChunkThreads, 2) k_subst_chunk(const __grid_constant__ SubstChunk<T> a,
+                                                                  const int* __restrict__ group_island) {
+  constexpr int LPG = 32 / G, S = XS ? G : 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* const sx = reinterpret_cast<T*>(smem_raw);
+  T* const xs = XS ? sx + (size_t)(a.xcap + a.ccap) * G : sx;  // the teams' fronts
+  const Ring R{reinterpret_cast<unsigned char*>(xs + (size_t)a.scratch * G), a.slot};
+  const int g = blockIdx.x / LPG, lane0 = (blockIdx.x % LPG) * G, l = threadIdx.x % G;
+  const int island = group_island ? group_island[g] : 0;
+  const T* pan0 = a.pan + at32(g, a.nnz, 0, lane0);
+  T* const gx = a.x + at32(g, a.n, 0, lane0 + l);
+  sweep_begin<T, G>(a.sw, island, R, pan0);
+  if (XS)
+    for (int i = threadIdx.x / G; i < a.n; i += kChunkThreads / G) sx[i * G + l] = gx[(size_t)i * 32];
+  const ChunkVec<T> v = XS ? ChunkVec<T>{sx + l, sx + (size_t)a.xcap * G + l}
+                           : ChunkVec<T>{gx, a.cbr + at32(g, a.sumcbr, 0, lane0 + l)};
+  sweep_run<T, G, S, TR>(a.sw, island, R, xs, pan0, v);
+  if (XS)
+    for (int i = threadIdx.x / G; i < a.n; i += kChunkThreads / G) gx[(size_t)i * 32] = sx[i * G + l];
 }
 
 // per-lane max over the block's threads (lane = thread % G), left in red[0 .. G)

@@ -912,22 +912,28 @@ bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bo
       const bool up = q < nlev;
       const int lv = up ? q : 2 * nlev - 1 - q;
       // index list of a task
-      auto list_of = [&](int n, int* layers) {
+      auto list_of = [&](int n) {
         const int w = s.sn_w[n], f = s.sn_f[n];
         const int* rows = s.sn_rows.data() + s.sn_rptr[n];
-        std::vector<int> l(rows, rows + (up ? w : f));
-        *layers = 0;
-        if (!up) return l;
-        std::vector<std::vector<int>> src(f);
-        for (int c = s.child_ptr[n]; c < s.child_ptr[n + 1]; ++c) {
-          const int ch = s.child_list[c], m = s.sn_f[ch] - s.sn_w[ch];
-          for (int a = 0; a < m; ++a) src[s.relmap[s.rel_ptr[ch] + a]].push_back(cb[ch] + a);
+        std::vector<int> l;
+        if (up) {
+          std::vector<std::vector<int>> src(f);
+          for (int c = s.child_ptr[n]; c < s.child_ptr[n + 1]; ++c) {
+            const int ch = s.child_list[c], m = s.sn_f[ch] - s.sn_w[ch];
+            for (int a = 0; a < m; ++a) src[s.relmap[s.rel_ptr[ch] + a]].push_back(cb[ch] + a);
+          }
+          int layers = 0;
+          for (auto& v : src) layers = std::max(layers, ((int)v.size() + 1) / 2);
+          l = {layers, 0};
+          l.insert(l.end(), rows, rows + w);
+          l.resize((l.size() + 1) / 2 * 2, 0);  // pairs are read as 8-byte words
+          for (int k = 0; k < layers; ++k)
+            for (int i = 0; i < f; ++i)
+              for (int e = 2 * k; e < 2 * k + 2; ++e) l.push_back(e < (int)src[i].size() ? src[i][e] : -1);
+        } else {
+          l.assign(rows, rows + f);
         }
-        for (auto& v : src) *layers = std::max(*layers, ((int)v.size() + 1) / 2);
-        l.resize((l.size() + 1) / 2 * 2, 0);  // pairs are read as 8-byte words
-        for (int k = 0; k < *layers; ++k)
-          for (int i = 0; i < f; ++i)
-            for (int e = 2 * k; e < 2 * k + 2; ++e) l.push_back(e < (int)src[i].size() ? src[i][e] : -1);
+        l.resize((l.size() + 1) / 2 * 2, 0);
         return l;
       };
       int k = lev[lv];
@@ -936,29 +942,35 @@ bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bo
         SweepStep st{};
         st.up = up;
         st.e0 = (int)s.pan_off[sn[k]];
-        std::vector<int> head, lists;
+        std::vector<int> head, lists, after;
         int k2 = k, fbig = 0, wbig = 0;
         for (; k2 < lev[lv + 1]; ++k2) {
           const int n = sn[k2], w = s.sn_w[n], f = s.sn_f[n];
-          int layers = 0;
-          std::vector<int> l = list_of(n, &layers);
-          l.resize((l.size() + 1) / 2 * 2, 0);
+          if (w > 0x7fff || f > 0x7fff || s.pan_off[n] != st.e0 + st.ne) return false;
+          const std::vector<int> l = list_of(n);
           const int ne = st.ne + w * f + (f - w) * w;
           const size_t ni = (kStepInts + head.size() + 4 + lists.size() + l.size() + 3) / 4 * 4;
-          if (w > 4095 || f > 4095 || layers > 127) return false;
-          if (s.pan_off[n] != st.e0 + st.ne) return false;
-          if (bytes_of(ne, ni) > slot) break;
-          head.insert(head.end(), {st.ne, w | f << 12 | layers << 24, (int)lists.size(), cb[n]});
-          lists.insert(lists.end(), l.begin(), l.end());
-          st.ne = ne;
-          if (solo_task(w, f)) ++st.nsolo;
+          const bool fits = bytes_of(ne, ni) <= slot;
+          if (!fits && k2 > k) break;
+          head.insert(head.end(), {st.ne, w | f << 16, (int)lists.size(), cb[n]});
+          if (fits) {
+            lists.insert(lists.end(), l.begin(), l.end());
+            st.ne = ne;
+          } else {
+            st.direct = 1;
+            after = l;
+          }
+          if (solo_task(w, f) && fits) ++st.nsolo;
           else {
             ++st.nbig;
             fbig = std::max(fbig, f);
             wbig = std::max(wbig, w);
           }
+          if (!fits) {
+            ++k2;
+            break;
+          }
         }
-        if (k2 == k) return false;
         int team_threads = 32;
         if (st.nbig > 0) {
           st.xstride = (fbig + 3) / 4 * 4;
@@ -995,6 +1007,11 @@ bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bo
         out.idx.insert(out.idx.end(), head.begin(), head.end());
         out.idx.insert(out.idx.end(), lists.begin(), lists.end());
         out.idx.resize((size_t)st.i0 + st.ni, 0);
+        if (st.direct) {
+          out.idx[st.i0 + kStepInts + 2] = st.ni;
+          out.idx.insert(out.idx.end(), after.begin(), after.end());
+          out.idx.resize((out.idx.size() + 3) / 4 * 4, 0);
+        }
         out.slot = std::max(out.slot, bytes_of(st.ne, st.ni));
         out.step.push_back(st);
         k = k2;

@@ -55,14 +55,9 @@ static bool check(const LUSymbolic& s, const std::vector<int>& isl, bool compact
   const size_t scratch = 16 * 1024;
   SweepPlan P;
   if (!build_sweep_plan(s, isl, compact, G, wsize, slot, scratch, P)) {
-    // refused only where one supernode does not fit the slot or the scratch
-    for (int n = 0; n < s.nsn; ++n) {
-      const size_t w = s.sn_w[n], f = s.sn_f[n];
-      if ((w * (2 * f - w)) * G * wsize + 24 * f + 256 > slot || (f + 3) / 4 * 4 * G * wsize > scratch) return true;
-      size_t kids = 0;
-      for (int c = s.child_ptr[n]; c < s.child_ptr[n + 1]; ++c) ++kids;
-      if ((w * (2 * f - w)) * G * wsize + (12 + 4 + w + 2 + (kids + 1) / 2 * 2 * f) * 4 + 96 > slot) return true;
-    }
+    // refused only where a front does not fit the scratch
+    for (int n = 0; n < s.nsn; ++n)
+      if ((size_t)(s.sn_f[n] + 3) / 4 * 4 * G * wsize > scratch) return true;
     std::printf("refused without a reason\n");
     return false;
   }
@@ -91,7 +86,8 @@ static bool check(const LUSymbolic& s, const std::vector<int>& isl, bool compact
         if (bytes > widest) widest = bytes;
         const int* ib = &P.idx[R.i0];
         const bool up = ib[4] != 0;
-        const int split = 1 << ib[5], nsolo = ib[6], nbig = ib[7], team = 1 << ib[8], nteams = ib[9], xstride = ib[10];
+        const int split = 1 << ib[5], nsolo = ib[6], nbig = ib[7], team = 1 << ib[8], nteams = ib[9], xstride = ib[10], direct = ib[11];
+        if (direct && (R.ne != 0 || nsolo != 0 || nbig != 1 || ib[0] != R.e0 || ib[2] != R.i0)) return false;
         if (split < 1 || split * G > 32 || (split & (split - 1))) return false;
         if (nbig > 0) {
           if (team % 32 || nteams < 1 || team * nteams > kChunkThreads || (team > 32 && nteams > 15)) return false;
@@ -104,13 +100,14 @@ static bool check(const LUSymbolic& s, const std::vector<int>& isl, bool compact
         std::vector<char> cw(c.size(), 0);
         for (int t = 0; t < nsolo + nbig; ++t) {
           const int* h = ib + kStepInts + 4 * t;
-          const int w = h[1] & 0xfff, f = (h[1] >> 12) & 0xfff, layers = h[1] >> 24, cbo = h[3];
-          if ((t < nsolo) != solo_task(w, f) || (t >= nsolo && f > xstride)) return false;
-          if (h[0] + w * (2 * f - w) > R.ne) return false;
-          const int* xi = ib + h[2];
+          const int w = h[1] & 0xffff, f = h[1] >> 16, cbo = h[3];
+          if ((t < nsolo) != (solo_task(w, f) && !direct) || (t >= nsolo && f > xstride)) return false;
+          if (!direct && h[0] + w * (2 * f - w) > R.ne) return false;
+          const int* xi = ib + h[2] + (up ? 2 : 0);
+          const int layers = up ? xi[-2] : 0;
           const int* pr = xi + ((w + 1) & ~1);
-          if (up && (pr - ib) % 2) return false;
-          if ((up ? pr + 2 * f * layers : xi + f) > ib + R.ni) return false;
+          if (up && (pr - &P.idx[0]) % 2) return false;
+          if ((up ? pr + 2 * f * layers : xi + f) > (direct ? &P.idx[0] + P.idx.size() : ib + R.ni)) return false;
           const double* M = &pan[R.e0 + h[0]];
           auto Lv = [&](int i, int p) { return i < w ? M[i * f + p] : M[w * f + (i - w) * w + p]; };
           std::vector<double> b(f, 0.0);
@@ -156,7 +153,7 @@ static bool check(const LUSymbolic& s, const std::vector<int>& isl, bool compact
 
 int main() {
   const int shapes[][4] = {{2, 1, 0, 0}, {30, 41, 5, 0}, {118, 179, 53, 0}, {300, 411, 69, 0},
-                           {1354, 1991, 259, 0}, {1354, 1991, 259, 1}, {2869, 4582, 509, 0}};
+                           {1354, 1991, 259, 0}, {1354, 1991, 259, 1}, {2869, 4582, 509, 0}, {700, 699, 0, 2}};
   Rng rng(7);
   for (auto& sh : shapes) {
     std::vector<mpf_bus> bus(sh[0]);
@@ -172,6 +169,10 @@ int main() {
       bus[0] = mpf_bus{MPF_BUS_SLACK, 0, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0};
       bus[1] = mpf_bus{MPF_BUS_PQ, 0, 1.0, 0.0, -0.1, -0.05, 0.0, 0.0};
       br[0] = mpf_branch{0, 1, 1, 0, 0.02, 0.1, 0.0, 0.0, 0.0};
+    } else if (sh[3] == 2) {
+      // a hub with hundreds of neighbours: one front row adds hundreds of carried entries
+      for (int i = 0; i < sh[0]; ++i) bus[i] = mpf_bus{i == 1 ? MPF_BUS_SLACK : MPF_BUS_PQ, 0, 1.0, 0.0, -1e-4, 0.0, 0.0, 0.0};
+      for (int i = 1; i < sh[0]; ++i) br[i - 1] = mpf_branch{i < 600 ? 0 : i - 500, i, 1, 0, 0.02, 0.1, 0.0, 0.0, 0.0};
     } else if (mpf_synth_grid(&p, bus.data(), br.data()) != 0) {
       return 1;
     }
