@@ -1477,7 +1477,6 @@ struct mpf_handle {
   // several islands (grids) in one handle: per-bus / per-branch islands, and per
   // batch the island of each group and the case <-> lane maps
   DevBuf bus_island, br_island, group_island, lane_case, case_lane;
-  std::vector<int> h_lane_case;
   // cases whose outages island PV/PQ buses (no path to a slack): per lane, uploaded
   // only when the batch has one; the grid's bridges make the single-outage check O(1)
   DevBuf case_cut;
@@ -1492,11 +1491,11 @@ struct mpf_handle {
   // per-case controls of the current cases (mpf_set_controls)
   struct Controls {
     int nc = 0, navr = 0, noltc = 0, nshc = 0, nslot = 0;
-    DevBuf val, avr, oltc, oltc_par, shc, shc_base, slot_ptr, slot_ent, y_slot, br_ctl, dy, bry, bdy, fdpos[2];
+    DevBuf val, avr, oltc, oltc_par, shc, shc_base, slot_ptr, slot_ent, y_slot, br_ctl, dy, bry, bdy, fdpos[2], vbase, bad;
     void clear() { nc = navr = noltc = nshc = nslot = 0; }
     size_t bytes() const {
       const DevBuf* all[] = {&val, &avr, &oltc, &oltc_par, &shc, &shc_base, &slot_ptr, &slot_ent,
-                             &y_slot, &br_ctl, &dy, &bry, &bdy, &fdpos[0], &fdpos[1]};
+                             &y_slot, &br_ctl, &dy, &bry, &bdy, &fdpos[0], &fdpos[1], &vbase, &bad};
       size_t b = 0;
       for (auto p : all) b += p->bytes;
       return b;
@@ -2289,9 +2288,7 @@ void adjoint_impl(mpf_handle* h, cudaStream_t st, double* gp, double* gq, double
   auto gradients = [&](const auto* lam) {
     using L = std::remove_cv_t<std::remove_pointer_t<decltype(lam)>>;
     if (gp || gq) {
-      const size_t total = (size_t)h->ncases * h->g.nb;
-      k_adj_grad_bus<L><<<(unsigned)std::min<size_t>(148 * 16, total / 256 + 1), 256, 0, st>>>(d, h->ncases, lam, gp,
-                                                                                                 gq);
+      k_adj_grad_bus<L><<<tile_grid(h->g.nb, h->ngroups), dim3(32, kTileRows), 0, st>>>(d, h->ncases, lam, gp, gq);
       CUDA_TRY(cudaGetLastError());
     }
     if (gg || gb) {
@@ -2654,22 +2651,28 @@ int set_cases_impl(mpf_handle* h, int32_t n_cases, const int32_t* island_of_case
           }
       }
     }
-    std::vector<double2> sb;
+    // per-case injections: copied as they are into the Ibus array (scratch between solves)
+    // and checked there, before anything of the current batch changes
+    const size_t per_bus = (size_t)ngroups * g.nb * 32 * sizeof(double2);
     if (sbus) {
-      sb.assign((size_t)ngroups * g.nb * 32, make_double2(0.0, 0.0));
-      for (int c = 0; c < n_cases; ++c)
-        for (int i = 0; i < g.nb; ++i) {
-          const double p = sbus[((size_t)c * g.nb + i) * 2], q = sbus[((size_t)c * g.nb + i) * 2 + 1];
-          if (!std::isfinite(p) || !std::isfinite(q))
-            return fail(h, MPF_ERR_BAD_INPUT, "sbus has a non-finite value");
-          const int ln = case_lane[c];
-          sb[((size_t)(ln >> 5) * g.nb + i) * 32 + (ln & 31)] = make_double2(p, q);
-        }
+      if (h->Ibus.bytes < per_bus) {
+        DevBuf b;
+        b.alloc(per_bus);  // (a failure leaves the current one)
+        std::swap(b.p, h->Ibus.p);
+        std::swap(b.bytes, h->Ibus.bytes);
+      }
+      const size_t n = (size_t)n_cases * g.nb * 2;
+      cudaStream_t st = h->own_stream;
+      CUDA_TRY(cudaMemcpyAsync(h->Ibus.p, sbus, n * sizeof(double), cudaMemcpyHostToDevice, st));
+      CUDA_TRY(cudaMemsetAsync(h->any_active.p, 0, sizeof(int), st));
+      k_any_nonfinite<<<(unsigned)std::min<size_t>(148 * 8, n / 256 + 1), 256, 0, st>>>(n, h->Ibus.as<double>(),
+                                                                                        h->any_active.as<int>());
+      CUDA_TRY(cudaGetLastError());
+      if (any_active(h, st)) return fail(h, MPF_ERR_BAD_INPUT, "sbus has a non-finite value");
     }
     if (ngroups != h->ngroups) {
-      const size_t per_bus = (size_t)ngroups * g.nb * 32 * sizeof(double2);
       h->V.alloc(per_bus);
-      h->Ibus.alloc(per_bus);
+      if (!sbus) h->Ibus.alloc(per_bus);  // (it holds the injections)
       h->status.alloc(lanes * sizeof(int));
       h->iters.alloc(lanes * sizeof(int));
       h->maxmis.alloc(lanes * sizeof(double));
@@ -2686,14 +2689,19 @@ int set_cases_impl(mpf_handle* h, int32_t n_cases, const int32_t* island_of_case
     upload(h->out_br, outs);
     if (any_cut) upload(h->case_cut, cut);
     else h->case_cut.release();
-    if (sbus) upload(h->sbus_case, sb);
-    else h->sbus_case.release();
+    if (sbus && h->sbus_case.bytes < per_bus) h->sbus_case.alloc(per_bus);
+    if (!sbus) h->sbus_case.release();
     if (multi) {
       upload(h->group_island, group_island);
       upload(h->lane_case, lane_case);
       upload(h->case_lane, case_lane);
     }
-    h->h_lane_case = lane_case;
+    if (sbus) {
+      k_scatter_sbus<<<tile_grid(g.nb, ngroups), dim3(32, kTileRows), 0, h->own_stream>>>(
+          g.nb, n_cases, multi ? h->lane_case.as<int>() : nullptr, h->Ibus.as<double2>(), h->sbus_case.as<double2>());
+      CUDA_TRY(cudaGetLastError());
+      CUDA_TRY(cudaStreamSynchronize(h->own_stream));
+    }
     const int* gi = multi ? h->group_island.as<int>() : nullptr;
     h->jac.group_island = gi;
     for (int v = 0; v < 2; ++v) {
@@ -2767,17 +2775,31 @@ int32_t mpf_set_controls(mpf_handle* h, int32_t n_controls, const mpf_control* c
         return fail(h, MPF_ERR_BAD_INPUT, who + ": unknown kind");
       }
     }
-    // values, lane-interleaved; padding lanes hold the base values
-    std::vector<double> val((size_t)h->ngroups * nc * 32);
-    for (int c = 0; c < lanes; ++c)
-      for (int k = 0; k < nc; ++k) {
-        const int uc = h->h_lane_case.empty() ? (c < ncases ? c : -1) : h->h_lane_case[c];
-        const double v = uc >= 0 ? values[(size_t)uc * nc + k] : base[k];
-        if (!std::isfinite(v)) return fail(h, MPF_ERR_BAD_INPUT, "control values must be finite");
-        if (controls[k].kind != MPF_CTRL_SHC && !(v > 0.0))
-          return fail(h, MPF_ERR_BAD_INPUT, "AVR and OLTC values must be > 0");
-        val[((size_t)(c >> 5) * nc + k) * 32 + (c & 31)] = v;
-      }
+    // values, lane-interleaved (padding lanes hold the base values): copied as they are into
+    // the Ibus array (scratch between solves, or a buffer of their own), spread by the device
+    DevBuf raw;
+    cudaStream_t st = h->own_stream;
+    {
+      const size_t vbytes = (size_t)ncases * nc * sizeof(double), obytes = (size_t)lanes * nc * sizeof(double);
+      if (h->Ibus.bytes < vbytes) raw.alloc(vbytes);
+      double* in = raw.p ? raw.as<double>() : h->Ibus.as<double>();
+      std::vector<double2> b2(nc);
+      for (int k = 0; k < nc; ++k) b2[k] = make_double2(base[k], controls[k].kind != MPF_CTRL_SHC ? 1.0 : 0.0);
+      if (!C.vbase.p || C.vbase.bytes < nc * sizeof(double2)) C.vbase.alloc(nc * sizeof(double2));
+      if (!C.bad.p) C.bad.alloc(sizeof(unsigned long long));
+      if (!C.val.p || C.val.bytes < obytes) C.val.alloc(obytes);
+      unsigned long long first = ~0ull;
+      CUDA_TRY(cudaMemcpyAsync(in, values, vbytes, cudaMemcpyHostToDevice, st));
+      CUDA_TRY(cudaMemcpyAsync(C.vbase.p, b2.data(), nc * sizeof(double2), cudaMemcpyHostToDevice, st));
+      CUDA_TRY(cudaMemsetAsync(C.bad.p, 0xff, sizeof first, st));
+      k_scatter_ctl<<<tile_grid(nc, h->ngroups), dim3(32, kTileRows), 0, st>>>(
+          nc, ncases, h->dev().lane_case, in, C.vbase.as<double2>(), C.val.as<double>(), C.bad.as<unsigned long long>());
+      CUDA_TRY(cudaGetLastError());
+      CUDA_TRY(cudaMemcpyAsync(&first, C.bad.p, sizeof first, cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaStreamSynchronize(st));
+      if (first != ~0ull)
+        return fail(h, MPF_ERR_BAD_INPUT, first % 2 ? "AVR and OLTC values must be > 0" : "control values must be finite");
+    }
     // tap parameters: Ys, b/2, cos / sin of the shift, Ys with r = 0 (BX's B'')
     std::vector<double> par(8 * oltc.size(), 0.0);
     std::vector<int> br_ctl(g.nbr, -1);
@@ -2828,7 +2850,6 @@ int32_t mpf_set_controls(mpf_handle* h, int32_t n_controls, const mpf_control* c
     }
     std::vector<double> shc_base(shc.size());
     for (size_t j = 0; j < shc.size(); ++j) shc_base[j] = h->buses[shc[j].x].bsh;
-    upload(C.val, val);
     upload(C.avr, avr);
     upload(C.oltc, oltc);
     upload(C.oltc_par, par);
@@ -2850,7 +2871,6 @@ int32_t mpf_set_controls(mpf_handle* h, int32_t n_controls, const mpf_control* c
     C.noltc = (int)oltc.size();
     C.nshc = (int)shc.size();
     C.nslot = (int)slot_pos.size();
-    cudaStream_t st = h->own_stream;
     const DevCtl t = h->devctl();
     if (C.noltc > 0) {
       const size_t tot = (size_t)h->ngroups * C.noltc * 32;
@@ -3008,9 +3028,8 @@ int32_t mpf_get_results_device(mpf_handle* h, double* v, int32_t* iterations, ui
     CUDA_TRY(cudaSetDevice(h->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : h->own_stream;
     if (v) {
-      const size_t total = (size_t)h->ncases * h->g.nb;
-      k_gather_v<<<(unsigned)std::min<size_t>(148 * 16, total / 256 + 1), 256, 0, st>>>(
-          h->g.nb, h->ncases, h->dev().case_lane, h->V.as<double2>(), reinterpret_cast<double2*>(v));
+      k_gather_v<<<tile_grid(h->g.nb, h->ngroups), dim3(32, kTileRows), 0, st>>>(
+          h->g.nb, h->ncases, h->dev().lane_case, h->V.as<double2>(), reinterpret_cast<double2*>(v));
       CUDA_TRY(cudaGetLastError());
     }
     if (iterations || status || max_mis) {

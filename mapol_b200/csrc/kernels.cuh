@@ -1865,6 +1865,25 @@ __global__ void k_acc_drain(unsigned long long* __restrict__ acc, double* __rest
   acc[c] = 0ull;
 }
 
+// ---------------------------------------------------------------- case-major results
+// [group][entry][32] <-> [case][entry] through a 32 x 32 tile in shared memory, so that both
+// sides move whole 128-byte lines (a thread per entry and case reads 16 of every 512 bytes).
+// Block (32, kTileRows): tile of 32 entries (blockIdx.x) of group blockIdx.y.  Gathering the
+// voltages of 1000 cases of 9241 buses: 69 -> 52 us (296 MB: 5.7 TB/s).
+constexpr int kTileRows = 8;
+inline dim3 tile_grid(int n, int ngroups) { return dim3((unsigned)((n + 31) / 32), (unsigned)ngroups); }
+
+// One block's tile (32 entries of a group from e0 on, [entry][lane]) to out[case][entry]
+template <typename V>
+__device__ __forceinline__ void write_tile(const DevGrid& d, const V (*tile)[33], int g, int e0, int n, int ncases, V* out,
+                                           int warp, int nwarps) {
+  const int lane = threadIdx.x & 31;
+  for (int r = warp; r < 32; r += nwarps) {
+    const int uc = case_of_lane(d, g * 32 + r, ncases);
+    if (uc >= 0 && e0 + lane < n) out[(size_t)uc * n + e0 + lane] = tile[lane][r];
+  }
+}
+
 // ---------------------------------------------------------------- branch flows
 // Per case and branch: Sf = Vf conj(Yff Vf + Yft Vt), St = Vt conj(Ytf Vf + Ytt Vt)
 // (an outaged branch carries nothing).  Per case sums: active loss sum(Re Sf + Re St)
@@ -1881,31 +1900,40 @@ __global__ void __launch_bounds__(256) k_branch_flow(DevGrid d, int nbr, int nca
   LaneOut o;
   load_outages(d, c, o);
   double lsum = 0.0, osum = 0.0;
-  const int k0 = blockIdx.x * 64;
-  const int k1 = min(nbr, k0 + 64);
-  for (int k = k0 + warp; k < k1; k += 8) {
-    double2 sf = make_double2(0.0, 0.0), stt = make_double2(0.0, 0.0);
-    const bool here = branch_here(d, k, g);
-    if (here && !outaged(o, k)) {
-      const int2 ft = d.br_ft[k];
-      double2 y[4];
-      branch_y(d, k, g, lane, y);
-      const double2 vf = d.V[at32(g, d.nb, ft.x, lane)], vt = d.V[at32(g, d.nb, ft.y, lane)];
-      const double2 i_f = make_double2(y[0].x * vf.x - y[0].y * vf.y + y[1].x * vt.x - y[1].y * vt.y,
-                                       y[0].x * vf.y + y[0].y * vf.x + y[1].x * vt.y + y[1].y * vt.x);
-      const double2 i_t = make_double2(y[2].x * vf.x - y[2].y * vf.y + y[3].x * vt.x - y[3].y * vt.y,
-                                       y[2].x * vf.y + y[2].y * vf.x + y[3].x * vt.y + y[3].y * vt.x);
-      sf = make_double2(vf.x * i_f.x + vf.y * i_f.y, vf.y * i_f.x - vf.x * i_f.y);
-      stt = make_double2(vt.x * i_t.x + vt.y * i_t.y, vt.y * i_t.x - vt.x * i_t.y);
+  __shared__ double2 tile[2][32][33];  // Sf and St of 32 branches, written case by case
+  const bool flows = sf_out || st_out;
+  for (int k0 = blockIdx.x * 64; k0 < min(nbr, (int)(blockIdx.x + 1) * 64); k0 += 32) {
+    for (int q = warp; q < 32 && k0 + q < nbr; q += 8) {
+      const int k = k0 + q;
+      double2 sf = make_double2(0.0, 0.0), stt = make_double2(0.0, 0.0);
+      const bool here = branch_here(d, k, g);
+      if (here && !outaged(o, k)) {
+        const int2 ft = d.br_ft[k];
+        double2 y[4];
+        branch_y(d, k, g, lane, y);
+        const double2 vf = d.V[at32(g, d.nb, ft.x, lane)], vt = d.V[at32(g, d.nb, ft.y, lane)];
+        const double2 i_f = make_double2(y[0].x * vf.x - y[0].y * vf.y + y[1].x * vt.x - y[1].y * vt.y,
+                                         y[0].x * vf.y + y[0].y * vf.x + y[1].x * vt.y + y[1].y * vt.x);
+        const double2 i_t = make_double2(y[2].x * vf.x - y[2].y * vf.y + y[3].x * vt.x - y[3].y * vt.y,
+                                         y[2].x * vf.y + y[2].y * vf.x + y[3].x * vt.y + y[3].y * vt.x);
+        sf = make_double2(vf.x * i_f.x + vf.y * i_f.y, vf.y * i_f.x - vf.x * i_f.y);
+        stt = make_double2(vt.x * i_t.x + vt.y * i_t.y, vt.y * i_t.x - vt.x * i_t.y);
+      }
+      lsum += sf.x + stt.x;
+      if (rating && here) {
+        const double ex = sqrt(sf.x * sf.x + sf.y * sf.y) - 0.9 * rating[k];
+        if (ex > 0.0) osum += ex * ex;
+      }
+      if (flows) {
+        tile[0][q][lane] = sf;
+        tile[1][q][lane] = stt;
+      }
     }
-    lsum += sf.x + stt.x;
-    if (rating && here) {
-      const double ex = sqrt(sf.x * sf.x + sf.y * sf.y) - 0.9 * rating[k];
-      if (ex > 0.0) osum += ex * ex;
-    }
-    if (uc >= 0) {
-      if (sf_out) sf_out[(size_t)uc * nbr + k] = sf;
-      if (st_out) st_out[(size_t)uc * nbr + k] = stt;
+    if (flows) {
+      __syncthreads();
+      if (sf_out) write_tile(d, tile[0], g, k0, nbr, ncases, sf_out, warp, 8);
+      if (st_out) write_tile(d, tile[1], g, k0, nbr, ncases, st_out, warp, 8);
+      __syncthreads();
     }
   }
   __shared__ double red[2][8][32];
@@ -2085,17 +2113,21 @@ __global__ void __launch_bounds__(128) k_mf_bsolve_t(DevLU L, const int* __restr
 // dL/dP_i = lambda(P_i row), dL/dQ_i = lambda(Q_i row): F = S(V) - Sbus, so
 // dF/dSbus = -I and dL/dtheta = dL/dtheta|explicit - lambda^T dF/dtheta.
 template <typename T>
-__global__ void k_adj_grad_bus(DevGrid d, int ncases, const T* __restrict__ lam, double* __restrict__ gp,
-                               double* __restrict__ gq) {
-  const size_t total = (size_t)ncases * d.nb;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int uc = (int)(t / d.nb), i = (int)(t % d.nb);
-    const int c = lane_of_case(d, uc);
+__global__ void __launch_bounds__(32 * kTileRows) k_adj_grad_bus(DevGrid d, int ncases, const T* __restrict__ lam,
+                                                               double* __restrict__ gp, double* __restrict__ gq) {
+  __shared__ double tp[32][33], tq[32][33];
+  const int g = blockIdx.y, i0 = blockIdx.x * 32, lane = threadIdx.x;
+  const bool conv = d.status[g * 32 + lane] == ST_CONVERGED;
+  for (int r = threadIdx.y; r < 32 && i0 + r < d.nb; r += kTileRows) {
+    const int i = i0 + r;
     const int2 jv = d.jvar[i];
-    const bool ok = d.status[c] == ST_CONVERGED && row_here(d, i, c >> 5);
-    if (gp) gp[t] = (ok && jv.x >= 0) ? (double)lam[at32(c >> 5, d.n_jac, jv.x, c & 31)] : 0.0;
-    if (gq) gq[t] = (ok && jv.y >= 0 && !still_pv(d, i, c >> 5, c & 31)) ? (double)lam[at32(c >> 5, d.n_jac, jv.y, c & 31)] : 0.0;
+    const bool ok = conv && row_here(d, i, g);
+    tp[r][lane] = (ok && jv.x >= 0) ? (double)lam[at32(g, d.n_jac, jv.x, lane)] : 0.0;
+    tq[r][lane] = (ok && jv.y >= 0 && !still_pv(d, i, g, lane)) ? (double)lam[at32(g, d.n_jac, jv.y, lane)] : 0.0;
   }
+  __syncthreads();
+  if (gp) write_tile(d, tp, g, i0, d.nb, ncases, gp, threadIdx.y, kTileRows);
+  if (gq) write_tile(d, tq, g, i0, d.nb, ncases, gq, threadIdx.y, kTileRows);
 }
 
 // Branch series admittance y = g + jb.  dY/dg for (ff, ft, tf, tt) = a = (1/|t|^2,
@@ -2113,11 +2145,11 @@ __global__ void __launch_bounds__(256) k_adj_grad_branch(DevGrid d, int nbr, int
   const int c = grp * 32 + lane;
   LaneOut o;
   load_outages(d, c, o);
-  const int uc = case_of_lane(d, c, ncases);  // the user's case in this lane, -1 for padding
-  const bool ok = uc >= 0 && d.status[c] == ST_CONVERGED;
-  const int k1 = min(nbr, (int)(blockIdx.x + 1) * 64);
-  for (int k = blockIdx.x * 64 + warp; k < k1; k += 8) {
-    if (uc < 0) continue;
+  const bool ok = case_of_lane(d, c, ncases) >= 0 && d.status[c] == ST_CONVERGED;
+  __shared__ double tg[32][33], tb[32][33];
+  for (int k0 = blockIdx.x * 64; k0 < min(nbr, (int)(blockIdx.x + 1) * 64); k0 += 32) {
+  for (int q = warp; q < 32 && k0 + q < nbr; q += 8) {
+    const int k = k0 + q;
     double rg = 0.0, rb = 0.0;
     if (ok && branch_here(d, k, grp) && !outaged(o, k)) {
       const int2 ft = d.br_ft[k];
@@ -2154,8 +2186,13 @@ __global__ void __launch_bounds__(256) k_adj_grad_branch(DevGrid d, int nbr, int
       rg -= lPf * Df.x + lQf * Df.y + lPt * Dt.x + lQt * Dt.y;
       rb -= lPf * Df.y - lQf * Df.x + lPt * Dt.y - lQt * Dt.x;
     }
-    if (gg) gg[(size_t)uc * nbr + k] = rg;
-    if (gb) gb[(size_t)uc * nbr + k] = rb;
+    tg[q][lane] = rg;
+    tb[q][lane] = rb;
+  }
+  __syncthreads();
+  if (gg) write_tile(d, tg, grp, k0, nbr, ncases, gg, warp, 8);
+  if (gb) write_tile(d, tb, grp, k0, nbr, ncases, gb, warp, 8);
+  __syncthreads();
   }
 }
 
@@ -2375,15 +2412,60 @@ __global__ void k_fill_int(int* p, int n, int v) {
 }
 
 // ---------------------------------------------------------------- results
-// [group][bus][32] -> [case][bus]
-// case_lane (nullable): lane of each case when lanes are grouped by island
-__global__ void k_gather_v(int nb, int ncases, const int* case_lane, const double2* V, double2* out) {
-  const size_t total = (size_t)ncases * nb;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int uc = (int)(t / nb), i = (int)(t % nb);
-    const int c = case_lane ? case_lane[uc] : uc;
-    out[t] = V[at32(c >> 5, nb, i, c & 31)];
+
+// case_lane / lane_case (nullable): lanes grouped by island
+__global__ void __launch_bounds__(32 * kTileRows) k_gather_v(int nb, int ncases, const int* __restrict__ lane_case,
+                                                           const double2* __restrict__ V, double2* __restrict__ out) {
+  __shared__ double2 tile[32][33];
+  const int g = blockIdx.y, i0 = blockIdx.x * 32;
+  for (int r = threadIdx.y; r < 32 && i0 + r < nb; r += kTileRows) tile[r][threadIdx.x] = V[at32(g, nb, i0 + r, threadIdx.x)];
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32; r += kTileRows) {
+    const int c = g * 32 + r, uc = lane_case ? lane_case[c] : (c < ncases ? c : -1);
+    if (uc >= 0 && i0 + (int)threadIdx.x < nb) out[(size_t)uc * nb + i0 + threadIdx.x] = tile[threadIdx.x][r];
   }
+}
+
+// Injections given case by case, [case][bus], into [group][bus][32] (0 in padding lanes)
+__global__ void __launch_bounds__(32 * kTileRows) k_scatter_sbus(int nb, int ncases, const int* __restrict__ lane_case,
+                                                               const double2* __restrict__ in, double2* __restrict__ out) {
+  __shared__ double2 tile[32][33];
+  const int g = blockIdx.y, i0 = blockIdx.x * 32;
+  for (int r = threadIdx.y; r < 32; r += kTileRows) {
+    const int c = g * 32 + r, uc = lane_case ? lane_case[c] : (c < ncases ? c : -1);
+    tile[threadIdx.x][r] = uc >= 0 && i0 + (int)threadIdx.x < nb ? in[(size_t)uc * nb + i0 + threadIdx.x] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32 && i0 + r < nb; r += kTileRows) out[at32(g, nb, i0 + r, threadIdx.x)] = tile[r][threadIdx.x];
+}
+
+// Control values given case by case, [case][control], into [group][control][32] (padding
+// lanes: base); bad gets the smallest 2 (lane nc + control) + (1: not positive, where the
+// kind asks for it; 0: not finite) of the values in error
+__global__ void __launch_bounds__(32 * kTileRows) k_scatter_ctl(int nc, int ncases, const int* __restrict__ lane_case,
+                                                              const double* __restrict__ in, const double2* __restrict__ base,
+                                                              double* __restrict__ out, unsigned long long* __restrict__ bad) {
+  __shared__ double tile[32][33];
+  const int g = blockIdx.y, k0 = blockIdx.x * 32, k = k0 + threadIdx.x;
+  for (int r = threadIdx.y; r < 32 && k < nc; r += kTileRows) {
+    const int c = g * 32 + r, uc = lane_case ? lane_case[c] : (c < ncases ? c : -1);
+    const double2 b = base[k];  // base value; y = 1: must be positive
+    const double v = uc >= 0 ? in[(size_t)uc * nc + k] : b.x;
+    const bool finite = fabs(v) <= DBL_MAX;
+    if (!finite || (b.y != 0.0 && !(v > 0.0)))
+      atomicMin(bad, 2ull * ((unsigned long long)c * nc + k) + (finite ? 1 : 0));
+    tile[threadIdx.x][r] = v;
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32 && k0 + r < nc; r += kTileRows) out[at32(g, nc, k0 + r, threadIdx.x)] = tile[r][threadIdx.x];
+}
+
+// flag |= 1 where a value is infinite or NaN
+__global__ void k_any_nonfinite(size_t n, const double* __restrict__ v, int* __restrict__ flag) {
+  bool bad = false;
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
+    bad |= !(fabs(v[t]) <= DBL_MAX);
+  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flag, 1);
 }
 
 __global__ void k_gather_small(int ncases, const int* case_lane, const int* status, const int* iters,
