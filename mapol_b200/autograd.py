@@ -20,9 +20,9 @@ class PowerFlowLoss(torch.autograd.Function):
         sbus = torch.stack([p.detach(), q.detach()], -1).cpu().numpy()
         pf.set_cases(cases, sbus=sbus)
         pf.solve(T.NR, precision)
-        res = pf.results()
+        status = pf.status()
         over = pf.branch_flows()["overload"]
-        over = np.where(res.status == T.CASE_CONVERGED, over, 0.0)
+        over = np.where(status == T.CASE_CONVERGED, over, 0.0)
         ctx.pf = pf
         ctx.precision = precision
         return torch.as_tensor(over, dtype=torch.float64, device=p.device)

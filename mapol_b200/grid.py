@@ -2,6 +2,7 @@
 load scenarios (all computed by libmpf.so so every machine gets the same inputs).
 """
 import ctypes
+from itertools import chain
 
 import numpy as np
 
@@ -54,11 +55,10 @@ def load_scenarios(buses, n_cases, sigma, seed):
 def cases_to_offsets(cases):
     """List of outage lists -> (offsets[n+1], branches[]) int32 arrays."""
     offs = np.zeros(len(cases) + 1, np.int32)
-    flat = []
-    for i, c in enumerate(cases):
-        offs[i + 1] = offs[i] + len(c)
-        flat.extend(int(b) for b in c)
-    return offs, np.asarray(flat + [0], np.int32)
+    np.cumsum([len(c) for c in cases], out=offs[1:])
+    flat = np.zeros(int(offs[-1]) + 1, np.int32)
+    flat[:-1] = np.fromiter(map(int, chain.from_iterable(cases)), np.int32, int(offs[-1]))
+    return offs, flat
 
 
 def n1_cases(branches, n_bus, n_out, seed, with_base=False):

@@ -144,7 +144,13 @@ class PowerFlow:
         st = np.zeros(self.n_cases, np.uint8)
         mm = np.zeros(self.n_cases)
         self._check(lib().mpf_get_results(self._h, ptr(v), ptr(it), ptr(st), ptr(mm)))
-        return Results(v[..., 0] + 1j * v[..., 1], it, st, mm)
+        return Results(v.view(np.complex128)[..., 0], it, st, mm)
+
+    def status(self):
+        """Per-case status of the last solve alone (no voltages copied)."""
+        st = np.zeros(self.n_cases, np.uint8)
+        self._check(lib().mpf_get_results(self._h, None, None, ptr(st), None))
+        return st
 
     def runpf(self, cases, alg=NR, precision=FP64, sbus=None):
         """End to end from host memory (mpf_runpf_host): cases in, results out."""
@@ -159,7 +165,7 @@ class PowerFlow:
         self._check(lib().mpf_runpf_host(self._h, alg, precision, n, ptr(offs), ptr(flat), ptr(sb),
                                          ptr(v), ptr(it), ptr(st), ptr(mm)))
         self.n_cases = n
-        return Results(v[..., 0] + 1j * v[..., 1], it, st, mm)
+        return Results(v.view(np.complex128)[..., 0], it, st, mm)
 
     def set_ratings(self, rating):
         """Branch ratings (p.u. apparent power, [n_branch]) for the overload loss."""
@@ -207,9 +213,9 @@ class PowerFlow:
     def fitness(self, results=None):
         """The reference's per-case fitness after hybrid_runpf: total active loss when
         the case converged, DBL_MAX otherwise (runpf.h:748-791)."""
-        res = results if results is not None else self.results()
+        status = results.status if results is not None else self.status()
         loss = self.branch_flows()["ploss"]
-        return np.where(res.status == T.CASE_CONVERGED, loss, np.finfo(np.float64).max)
+        return np.where(status == T.CASE_CONVERGED, loss, np.finfo(np.float64).max)
 
     def timing(self):
         t = T.Timing()
