@@ -121,8 +121,9 @@ typedef struct mpf_options {
                           splits the solve by kernel family; 0: direct launches.  All
                           three give the same results bit for bit. */
   int32_t autotune;    /* 1: time the candidate kernels of every factorisation launch on
-                          the first solve of a batch size and keep the fastest (default 1);
-                          0: fixed heuristic */
+                          the first solve of a batch size and keep the fastest, and run
+                          Newton on one block per chunk of cases where that is faster
+                          (default 1); 0: level launches by a fixed heuristic */
   int32_t ordering;    /* fill-reducing bus order of the Newton system, MPF_ORDER_*:
                           0 automatic (default), 1 minimum degree, 2 minimum fill,
                           3 minimum fill weighted by variables per bus */

@@ -211,12 +211,21 @@ struct FactorChoice {
   int kind, ge, tt, tpb;
 };
 
+// A block's factorisation (FactorPlan) on the device
+struct FactorBufs {
+  DevBuf step, idx;
+  int n = 0, peak_cb = 0;
+  size_t most = 0, slot = 0;
+  double cycles = 0.0;
+  DevFactor dev() const { return DevFactor{step.as<int4>(), idx.as<int>(), n}; }
+};
+
 // A block's substitution steps (SweepPlan) on the device
 struct PlanBufs {
-  DevBuf step, step_ptr, idx;
+  DevBuf step, step_ptr, down_ptr, idx;
   size_t scratch = 0, slot = 0;  // as SweepPlan
   int peak_cb = 0;
-  DevSweep dev() const { return DevSweep{step.as<int4>(), step_ptr.as<int>(), idx.as<int>()}; }
+  DevSweep dev() const { return DevSweep{step.as<int4>(), step_ptr.as<int>(), down_ptr.as<int>(), idx.as<int>()}; }
 };
 
 struct LUSystem {
@@ -227,6 +236,8 @@ struct LUSystem {
   std::vector<int> h_sn_island;      // the same on the host (empty: one island)
   // sweep plans by (compact, lanes, value bytes, kilobytes per ring slot)
   std::map<std::tuple<bool, int, int, int>, std::unique_ptr<PlanBufs>> plans;
+  // factorisation plans by (lanes, value bytes, kilobytes of shared memory)
+  std::map<std::tuple<int, int, int>, std::unique_ptr<FactorBufs>> fplans;
   const int* group_island = nullptr; // the handle's current per-group islands (or null)
   std::vector<Launch> factor_sched;  // ascending levels
   std::vector<LaunchDeps> factor_deps;
@@ -247,7 +258,7 @@ struct LUSystem {
   // autotuned lane count of every backward-solve level launch (0 = one case per thread)
   std::map<std::pair<int, int>, std::vector<int>> tuned_bs;
   std::vector<Launch> level_sched;   // one launch per level (adjoint solves of full FP64 batches), ascending
-  std::vector<int> ah_host;          // arrowhead ranges (host copy of ah_ptr)
+  std::vector<int> ah_host, ah_loc_host;  // host copies of ah_ptr and ah_loc
   int nA = 0;
   // values per precision [0] = FP64, [1] = FP32
   DevBuf A[2], pan[2], cb[2], cbr[2], x[2];
@@ -301,6 +312,7 @@ struct LUSystem {
       h_sn_island.clear();
     }
     plans.clear();
+    fplans.clear();
     upload(sn_w, s.sn_w);
     upload(sn_f, s.sn_f);
     upload(sn_rptr, s.sn_rptr);
@@ -313,6 +325,7 @@ struct LUSystem {
     upload(ah_ptr, ahp);
     upload(ah_loc, ahl);
     ah_host = ahp;
+    ah_loc_host = ahl;
     std::vector<long long> po(s.pan_off.begin(), s.pan_off.end()), co(s.cb_off.begin(), s.cb_off.end()),
         ro(s.cbr_off.begin(), s.cbr_off.end());
     upload(pan_off, po);
@@ -470,12 +483,41 @@ struct LUSystem {
       for (size_t k = 0; k < st.size(); ++k) st[k] = make_int4(p.step[k].e0, p.step[k].ne, p.step[k].i0, p.step[k].ni);
       upload(slot->step, st);
       upload(slot->step_ptr, p.step_ptr);
+      upload(slot->down_ptr, p.down_ptr);
       upload(slot->idx, p.idx);
       slot->scratch = p.scratch;
       slot->slot = p.slot;
       slot->peak_cb = p.peak_cb;
     }
     return slot.get();
+  }
+
+  // The factorisation plan for blocks of G lanes of wsize-byte values with kb KB for its ring,
+  // contribution blocks and fronts; null when they do not fit
+  const FactorBufs* fplan(int G, int wsize, int kb) {
+    const auto key = std::make_tuple(G, wsize, kb);
+    auto it = fplans.find(key);
+    if (it != fplans.end()) return it->second.get();
+    FactorPlan p;
+    bool ok = false;
+    // the largest ring slots that leave room for the rest
+    for (size_t slot = 24 * 1024; !ok && slot >= 3 * 1024 && h_sn_island.empty(); slot = slot * 2 / 3 / 16 * 16)
+      ok = (size_t)kb * 1024 > kRingSlots * slot &&
+           build_factor_plan(sym, ah_host, ah_loc_host, G, wsize, slot, (size_t)kb * 1024 - kRingSlots * slot, p);
+    auto& out = fplans[key];
+    if (ok) {
+      out = std::make_unique<FactorBufs>();
+      std::vector<int4> st(p.step.size());
+      for (size_t k = 0; k < st.size(); ++k) st[k] = make_int4(p.step[k].e0, p.step[k].ne, p.step[k].i0, p.step[k].ni);
+      upload(out->step, st);
+      upload(out->idx, p.idx);
+      out->n = (int)st.size();
+      out->peak_cb = p.peak_cb;
+      out->most = p.most;
+      out->slot = p.slot;
+      out->cycles = p.cycles;
+    }
+    return out.get();
   }
 
   // A launch's shared memory per team is set by its largest front, while its fronts'
@@ -1832,160 +1874,6 @@ int enqueue_nr_part(mpf_handle* h, int part, cudaStream_t st, T* A, T* pan, T* c
   return nl;
 }
 
-template <typename T>
-void solve_nr(mpf_handle* h, cudaStream_t st) {
-  constexpr int P = Prec<T>::idx;
-  LUSystem& J = h->jac;
-  J.ensure_values(P, h->ngroups);
-  T* A = J.A[P].as<T>();
-  T* pan = J.pan[P].as<T>();
-  T* cb = J.cb[P].as<T>();
-  T* cbr = J.cbr[P].as<T>();
-  T* x = J.x[P].as<T>();
-  const DevGrid d = h->dev();
-  const dim3 rg = row_grid(h);
-  int nl = 0;
-  EventTimer& tm = h->timer;
-  int ev = tm.begin(FAM_OTHER);
-  k_init<<<std::min(148 * 8, (int)((size_t)h->ngroups * h->g.nb * 32 / 256 + 1)), 256, 0, st>>>(d, h->ncases);
-  CUDA_TRY(cudaGetLastError());
-  ++nl;
-  nl += apply_avr(h, st);
-  if (h->nsw > 0) {
-    const size_t tot = (size_t)h->ngroups * 32 * h->nsw;
-    k_qlim_reset<<<(unsigned)std::min<size_t>(148 * 8, tot / 256 + 1), 256, 0, st>>>(d);
-    CUDA_TRY(cudaGetLastError());
-    ++nl;
-  }
-  tm.end(ev);
-  const int max_it = h->opt.max_it_nr;
-  static const int kFam[4] = {FAM_FACT, FAM_SOLVE, FAM_UPD, FAM_MIS};
-  int it_total = 0;
-  auto& gph = h->nr_graph[P];
-  // one Newton run over the running cases: mismatch at the current voltages, check,
-  // then iterations until no case is running (first: also tune and capture)
-  auto run_newton = [&](bool first) {
-  if (!first) CUDA_TRY(cudaMemsetAsync(h->it_ctr.p, 0, sizeof(int), st));
-  ev = tm.begin(FAM_MIS);
-  launch_mismatch_nr<T>(d, rg, st, x, A, max_it > 0);
-  ++nl;
-  tm.end(ev);
-  ev = tm.begin(FAM_OTHER);
-  check(h, st, 0, max_it, &nl);
-  tm.end(ev);
-  int it = 0;
-  // pick the factorisation kernels of this batch size (first solve only), before
-  // the iteration is captured
-  if (first && h->opt.autotune && max_it > 0 && any_active(h, st)) {
-    tune_factor<T>(J, h->ngroups, A, pan, cb, cbr, x, d.status, d.group_active, st);
-    tune_bsolve<T>(J, h->ngroups, pan, x, d.group_active, st);
-  }
-  const bool dev_loop = h->opt.use_graph == 2;
-  if (h->opt.use_graph) {
-    // the captured kernels hold every device pointer of d by value: capture again
-    // when any of them (or the LU buffers) changed since
-    const void* key[4] = {A, pan, cb, x};
-    if ((gph.exec[0] || gph.loop_exec) &&
-        (gph.ngroups != h->ngroups || std::memcmp(gph.key, key, sizeof(key)) != 0 ||
-         std::memcmp(&gph.dkey, &d, sizeof(d)) != 0))
-      gph.release();
-    if (!gph.captured(dev_loop)) {
-      // capture on a private stream (the caller's may be the legacy one)
-      cudaStream_t cs;
-      CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-      if (!dev_loop) {
-        for (int part = 0; part < 4; ++part) {
-          CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-          gph.launches[part] = enqueue_nr_part<T>(h, part, cs, A, pan, cb, cbr, x);
-          CUDA_TRY(cudaStreamEndCapture(cs, &gph.graph[part]));
-          CUDA_TRY(cudaGraphInstantiate(&gph.exec[part], gph.graph[part], 0));
-        }
-      } else {
-        // head: the condition at entry; then a while node running the four parts and
-        // the condition again.  The update kernel counts iterations on the device, so
-        // the loop ends after at most max_it bodies whatever the cases do.
-        CUDA_TRY(cudaGraphCreate(&gph.loop_graph, 0));
-        cudaGraphConditionalHandle hc;
-        CUDA_TRY(cudaGraphConditionalHandleCreate(&hc, gph.loop_graph, 0, 0));
-        CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, gph.loop_graph, nullptr, nullptr, 0,
-                                               cudaStreamCaptureModeThreadLocal));
-        k_loop_cond<<<1, 1, 0, cs>>>(hc, h->any_active.as<int>(), d.it_ptr, max_it);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaStreamEndCapture(cs, &gph.loop_graph));
-        cudaGraphNode_t head;
-        size_t nn = 1;
-        CUDA_TRY(cudaGraphGetNodes(gph.loop_graph, &head, &nn));
-        if (nn != 1) throw MpfError{MPF_ERR_CUDA, "device loop: the head graph should hold one kernel"};
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = hc;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t loop;
-        CUDA_TRY(cudaGraphAddNode(&loop, gph.loop_graph, &head, 1, &cp));
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        int nlb = 0;
-        for (int part = 0; part < 4; ++part) nlb += enqueue_nr_part<T>(h, part, cs, A, pan, cb, cbr, x);
-        k_loop_cond<<<1, 1, 0, cs>>>(hc, h->any_active.as<int>(), d.it_ptr, max_it);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaStreamEndCapture(cs, &body));
-        CUDA_TRY(cudaGraphInstantiate(&gph.loop_exec, gph.loop_graph, 0));
-        gph.loop_launches = nlb + 1;
-      }
-      CUDA_TRY(cudaStreamDestroy(cs));
-      std::memcpy(gph.key, key, sizeof(key));
-      std::memcpy(&gph.dkey, &d, sizeof(d));
-      gph.ngroups = h->ngroups;
-    }
-  }
-  if (dev_loop) {
-    // one launch for all iterations; their count is read back once
-    const int e = tm.begin(FAM_OTHER);
-    CUDA_TRY(cudaGraphLaunch(gph.loop_exec, st));
-    tm.end(e);
-    CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    it = *h->h_any;
-    nl += 1 + it * gph.loop_launches;
-  }
-  while (!dev_loop && it < max_it && any_active(h, st)) {
-    int e[4];
-    for (int part = 0; part < 4; ++part) {
-      e[part] = tm.begin(kFam[part]);
-      if (h->opt.use_graph) {
-        CUDA_TRY(cudaGraphLaunch(gph.exec[part], st));
-        nl += gph.launches[part];
-      } else {
-        nl += enqueue_nr_part<T>(h, part, st, A, pan, cb, cbr, x);
-      }
-      tm.end(e[part]);
-    }
-    ++it;
-  }
-  it_total += it;
-  };
-  run_newton(true);
-  // reactive limits: switch the violating PV buses of converged cases to PQ and run
-  // those cases again from their voltages, until no case has a new violation
-  if (h->nsw > 0 && max_it > 0) {
-    const size_t tot = (size_t)h->ngroups * h->nsw * 32;
-    const int lanes = h->ngroups * 32;
-    for (int round = 0; round < kMaxQRounds; ++round) {
-      CUDA_TRY(cudaMemsetAsync(h->any_active.p, 0, sizeof(int), st));
-      k_qlim_check<<<(unsigned)std::min<size_t>(148 * 8, tot / 256 + 1), 256, 0, st>>>(
-          d, h->sw_bus.as<int>(), h->q_lim.as<double2>(), h->q_flag.as<int>());
-      k_qlim_restart<<<(lanes + 255) / 256, 256, 0, st>>>(d, h->q_flag.as<int>());
-      CUDA_TRY(cudaGetLastError());
-      nl += 2;
-      if (!any_active(h, st)) break;
-      run_newton(false);
-    }
-  }
-  h->timing.launches = nl;
-  h->timing.iterations_max = it_total;
-}
-
 // How a chunk kernel runs a set of systems: lanes per block, x and the carried entries in
 // shared memory or not, and the plans
 struct ChunkShape {
@@ -2123,6 +2011,277 @@ void launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, const 
     k_subst_chunk<T, G, XS, true><<<(unsigned)(ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(a, S.group_island);
     CUDA_TRY(cudaGetLastError());
   });
+}
+
+// How k_nr_chunk runs the Newton system: lanes per block (0: it does not), shared memory
+struct NrShape {
+  int G = 0, xcap = 0, scratch = 0, slot = 0, fslot = 0, cbs = 0, fronts = 0;
+  size_t smem = 0;
+  const FactorBufs* fac = nullptr;
+  const PlanBufs* sw = nullptr;
+};
+inline bool nr_shape(LUSystem& S, int G, int wsize, NrShape& out) {
+  out = NrShape();
+  out.xcap = (S.sym.n + 3) / 4 * 4;
+  const size_t per = (size_t)G * wsize, held = out.xcap * per;
+  if (held + kChunkScratch + kRingSlots * 4096 > kChunkSmem) return false;
+  out.fac = S.fplan(G, wsize, (int)((kChunkSmem - held) / 1024));
+  if (!out.fac) return false;
+  out.sw = S.plan(false, G, wsize, std::min((int)((kChunkSmem - held - kChunkScratch) / kRingSlots / 1024), 48));
+  if (!out.sw) return false;
+  out.G = G;
+  out.scratch = (int)((out.sw->scratch + 3) / 4 * 4);
+  out.slot = (int)((out.sw->slot + 15) / 16 * 16);
+  out.fslot = (int)((out.fac->slot + 15) / 16 * 16);
+  out.cbs = (int)((kRingSlots * out.fslot + per - 1) / per + 3) / 4 * 4;
+  out.fronts = out.cbs + out.fac->peak_cb;
+  out.smem = held + std::max((out.fronts + out.fac->most) * per, out.scratch * per + (size_t)kRingSlots * out.slot);
+  return out.smem <= kChunkSmem;
+}
+
+// Whether Newton's iteration runs on one block per chunk of lanes, and on how many lanes: by
+// estimated microseconds per iteration, fitted to measurements (30 to 2869 buses, 11 to 4096
+// cases, both precisions).  Chunks: waves of blocks x (20 + 2.2 x the plan's cycles at 1.9
+// GHz + 0.02 n G, 10% more in FP64); level launches: 60 + 6 per launch + the LU entries of
+// the batch.  Measured, ms per solve, level launches / chunks (lanes): 30 buses x 11 cases
+// FP64 0.43 / 0.15 (1); 118 x 167 mixed 0.78 / 0.24 (2); 300 x 257 mixed 1.55 / 0.55 (2), x
+// 1024 1.90 / 0.93 (8), FP64 2.09 / 1.63 (4); 700 x 300 mixed 2.49 / 1.92 (4), x 1000 3.45 /
+// 3.88 (4); 1354 x 200 mixed 3.38 / 2.56 (2), x 1000 4.62 / 10.2 (2).  No grid above
+// kNrChunkEntries LU entries gains (2869 buses x 20 cases 4.0 / 6.0).
+constexpr long long kNrChunkEntries = 50000;
+template <typename T>
+NrShape choose_nr(LUSystem& S, int ngroups) {
+  NrShape sh, best;
+  if (!S.h_sn_island.empty()) return best;
+  for (const char* e : {"MPF_FACTOR_KIND", "MPF_BSOLVE_LANES", "MPF_BSOLVE_TOP"})
+    if (std::getenv(e)) return best;  // testing: a level kernel is forced
+  if (const char* e = std::getenv("MPF_NR_CHUNK")) {  // testing: 0 off, else the lanes per block
+    const int v = std::atoi(e);
+    if (v <= 0 || v > Prec<T>::G || (v & (v - 1)) || !nr_shape(S, v, sizeof(T), sh)) return best;
+    return sh;
+  }
+  if (S.sym.nnz > kNrChunkEntries) return best;
+  const double fp64 = sizeof(T) == 8 ? 1.1 : 1.0;
+  const double lanes = 32.0 * ngroups;
+  double bt = 0.9 * (60.0 + 6.0 * (S.factor_sched.size() + S.bsolve_sched.size()) +
+                     1e-5 * sizeof(T) / 4.0 * (double)S.sym.nnz * lanes);
+  for (int G = Prec<T>::G; G >= 1; G /= 2) {
+    if (!nr_shape(S, G, sizeof(T), sh)) continue;
+    const int waves = (ngroups * (32 / G) + 147) / 148;
+    const double t = fp64 * waves * (20.0 + 2.2 * sh.fac->cycles / 1900.0 + 0.02 * S.sym.n * G);
+    if (t < bt) {
+      bt = t;
+      best = sh;
+    }
+  }
+  return best;
+}
+
+template <typename T>
+void launch_nr_chunk(mpf_handle* h, const NrShape& sh, const DevGrid& d, int what, cudaStream_t st) {
+  constexpr int P = Prec<T>::idx;
+  LUSystem& J = h->jac;
+  const NrChunk<T> a{sh.fac->dev(), sh.sw->dev(),     J.sym.n,  J.nA,    J.sym.nnz, J.A[P].as<T>(), J.pan[P].as<T>(),
+                     J.x[P].as<T>(), sh.xcap, sh.scratch, sh.slot, sh.fslot, sh.cbs,    sh.fronts};
+  ChunkShape cs;
+  cs.G = sh.G;
+  with_shape<T>(cs, [&](auto g, auto) {
+    constexpr int G = decltype(g)::value;
+    auto go = [&](auto ctl, auto ql) {
+      constexpr bool CTL = decltype(ctl)::value, QL = decltype(ql)::value;
+      allow_chunk_smem<k_nr_chunk<T, G, CTL, QL>>(h->device);
+      k_nr_chunk<T, G, CTL, QL><<<(unsigned)(h->ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(
+          d, a, h->chunk_rows(), what, h->opt.max_it_nr, h->opt.tol);
+      CUDA_TRY(cudaGetLastError());
+    };
+    if (d.sw_index) d.y_slot ? go(std::true_type(), std::true_type()) : go(std::false_type(), std::true_type());
+    else d.y_slot ? go(std::true_type(), std::false_type()) : go(std::false_type(), std::false_type());
+  });
+}
+
+template <typename T>
+void solve_nr(mpf_handle* h, cudaStream_t st) {
+  constexpr int P = Prec<T>::idx;
+  LUSystem& J = h->jac;
+  J.ensure_values(P, h->ngroups);
+  T* A = J.A[P].as<T>();
+  T* pan = J.pan[P].as<T>();
+  T* cb = J.cb[P].as<T>();
+  T* cbr = J.cbr[P].as<T>();
+  T* x = J.x[P].as<T>();
+  const DevGrid d = h->dev();
+  const dim3 rg = row_grid(h);
+  int nl = 0;
+  EventTimer& tm = h->timer;
+  int ev = tm.begin(FAM_OTHER);
+  k_init<<<std::min(148 * 8, (int)((size_t)h->ngroups * h->g.nb * 32 / 256 + 1)), 256, 0, st>>>(d, h->ncases);
+  CUDA_TRY(cudaGetLastError());
+  ++nl;
+  nl += apply_avr(h, st);
+  if (h->nsw > 0) {
+    const size_t tot = (size_t)h->ngroups * 32 * h->nsw;
+    k_qlim_reset<<<(unsigned)std::min<size_t>(148 * 8, tot / 256 + 1), 256, 0, st>>>(d);
+    CUDA_TRY(cudaGetLastError());
+    ++nl;
+  }
+  tm.end(ev);
+  const int max_it = h->opt.max_it_nr;
+  static const int kFam[4] = {FAM_FACT, FAM_SOLVE, FAM_UPD, FAM_MIS};
+  int it_total = 0;
+  auto& gph = h->nr_graph[P];
+  // (autotune = 0 keeps the level kernels of the fixed rule)
+  const NrShape chunk = h->opt.autotune ? choose_nr<T>(J, h->ngroups) : NrShape();
+  // one Newton run over the running cases: mismatch at the current voltages, check,
+  // then iterations until no case is running (first: also tune and capture)
+  auto run_newton = [&](bool first) {
+  if (!first) CUDA_TRY(cudaMemsetAsync(h->it_ctr.p, 0, sizeof(int), st));
+  const bool tuned = !first || !h->opt.autotune || (J.tuned.count({P, h->ngroups}) && J.tuned_bs.count({P, h->ngroups}));
+  int it = 0;
+  if (chunk.G == 0 || !tuned) {
+  ev = tm.begin(FAM_MIS);
+  launch_mismatch_nr<T>(d, rg, st, x, A, max_it > 0);
+  ++nl;
+  tm.end(ev);
+  ev = tm.begin(FAM_OTHER);
+  check(h, st, 0, max_it, &nl);
+  tm.end(ev);
+  }
+  // pick the factorisation kernels of this batch size (first solve only), before
+  // the iteration is captured (the chunk kernel needs none, the adjoint does)
+  if (!tuned && max_it > 0 && any_active(h, st)) {
+    tune_factor<T>(J, h->ngroups, A, pan, cb, cbr, x, d.status, d.group_active, st);
+    tune_bsolve<T>(J, h->ngroups, pan, x, d.group_active, st);
+  }
+  if (chunk.G > 0) {
+    auto part = [&](int what, int fam) {
+      const int e = tm.begin(fam);
+      if (what == NR_MISMATCH) CUDA_TRY(cudaMemsetAsync(h->any_active.p, 0, sizeof(int), st));
+      launch_nr_chunk<T>(h, chunk, d, what, st);
+      tm.end(e);
+      ++nl;
+    };
+    if (h->opt.use_graph == 2) {
+      part(NR_ALL, FAM_OTHER);
+      CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaStreamSynchronize(st));
+      it = *h->h_any;
+    } else {  // the same in parts, for the kernel families' times
+      part(NR_MISMATCH, FAM_MIS);
+      while (it < max_it && any_active(h, st)) {
+        part(NR_FACTOR, FAM_FACT);
+        part(NR_SOLVE, FAM_SOLVE);
+        part(NR_UPDATE, FAM_UPD);
+        part(NR_MISMATCH, FAM_MIS);
+        ++it;
+      }
+    }
+    it_total += it;
+    return;
+  }
+  const bool dev_loop = h->opt.use_graph == 2;
+  if (h->opt.use_graph) {
+    // the captured kernels hold every device pointer of d by value: capture again
+    // when any of them (or the LU buffers) changed since
+    const void* key[4] = {A, pan, cb, x};
+    if ((gph.exec[0] || gph.loop_exec) &&
+        (gph.ngroups != h->ngroups || std::memcmp(gph.key, key, sizeof(key)) != 0 ||
+         std::memcmp(&gph.dkey, &d, sizeof(d)) != 0))
+      gph.release();
+    if (!gph.captured(dev_loop)) {
+      // capture on a private stream (the caller's may be the legacy one)
+      cudaStream_t cs;
+      CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+      if (!dev_loop) {
+        for (int part = 0; part < 4; ++part) {
+          CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+          gph.launches[part] = enqueue_nr_part<T>(h, part, cs, A, pan, cb, cbr, x);
+          CUDA_TRY(cudaStreamEndCapture(cs, &gph.graph[part]));
+          CUDA_TRY(cudaGraphInstantiate(&gph.exec[part], gph.graph[part], 0));
+        }
+      } else {
+        // head: the condition at entry; then a while node running the four parts and
+        // the condition again.  The update kernel counts iterations on the device, so
+        // the loop ends after at most max_it bodies whatever the cases do.
+        CUDA_TRY(cudaGraphCreate(&gph.loop_graph, 0));
+        cudaGraphConditionalHandle hc;
+        CUDA_TRY(cudaGraphConditionalHandleCreate(&hc, gph.loop_graph, 0, 0));
+        CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, gph.loop_graph, nullptr, nullptr, 0,
+                                               cudaStreamCaptureModeThreadLocal));
+        k_loop_cond<<<1, 1, 0, cs>>>(hc, h->any_active.as<int>(), d.it_ptr, max_it);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaStreamEndCapture(cs, &gph.loop_graph));
+        cudaGraphNode_t head;
+        size_t nn = 1;
+        CUDA_TRY(cudaGraphGetNodes(gph.loop_graph, &head, &nn));
+        if (nn != 1) throw MpfError{MPF_ERR_CUDA, "device loop: the head graph should hold one kernel"};
+        cudaGraphNodeParams cp = {};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = hc;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        cudaGraphNode_t loop;
+        CUDA_TRY(cudaGraphAddNode(&loop, gph.loop_graph, &head, 1, &cp));
+        cudaGraph_t body = cp.conditional.phGraph_out[0];
+        CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+        int nlb = 0;
+        for (int part = 0; part < 4; ++part) nlb += enqueue_nr_part<T>(h, part, cs, A, pan, cb, cbr, x);
+        k_loop_cond<<<1, 1, 0, cs>>>(hc, h->any_active.as<int>(), d.it_ptr, max_it);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaStreamEndCapture(cs, &body));
+        CUDA_TRY(cudaGraphInstantiate(&gph.loop_exec, gph.loop_graph, 0));
+        gph.loop_launches = nlb + 1;
+      }
+      CUDA_TRY(cudaStreamDestroy(cs));
+      std::memcpy(gph.key, key, sizeof(key));
+      std::memcpy(&gph.dkey, &d, sizeof(d));
+      gph.ngroups = h->ngroups;
+    }
+  }
+  if (dev_loop) {
+    // one launch for all iterations; their count is read back once
+    const int e = tm.begin(FAM_OTHER);
+    CUDA_TRY(cudaGraphLaunch(gph.loop_exec, st));
+    tm.end(e);
+    CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    it = *h->h_any;
+    nl += 1 + it * gph.loop_launches;
+  }
+  while (!dev_loop && it < max_it && any_active(h, st)) {
+    int e[4];
+    for (int part = 0; part < 4; ++part) {
+      e[part] = tm.begin(kFam[part]);
+      if (h->opt.use_graph) {
+        CUDA_TRY(cudaGraphLaunch(gph.exec[part], st));
+        nl += gph.launches[part];
+      } else {
+        nl += enqueue_nr_part<T>(h, part, st, A, pan, cb, cbr, x);
+      }
+      tm.end(e[part]);
+    }
+    ++it;
+  }
+  it_total += it;
+  };
+  run_newton(true);
+  // reactive limits: switch the violating PV buses of converged cases to PQ and run
+  // those cases again from their voltages, until no case has a new violation
+  if (h->nsw > 0 && max_it > 0) {
+    const size_t tot = (size_t)h->ngroups * h->nsw * 32;
+    const int lanes = h->ngroups * 32;
+    for (int round = 0; round < kMaxQRounds; ++round) {
+      CUDA_TRY(cudaMemsetAsync(h->any_active.p, 0, sizeof(int), st));
+      k_qlim_check<<<(unsigned)std::min<size_t>(148 * 8, tot / 256 + 1), 256, 0, st>>>(
+          d, h->sw_bus.as<int>(), h->q_lim.as<double2>(), h->q_flag.as<int>());
+      k_qlim_restart<<<(lanes + 255) / 256, 256, 0, st>>>(d, h->q_flag.as<int>());
+      CUDA_TRY(cudaGetLastError());
+      nl += 2;
+      if (!any_active(h, st)) break;
+      run_newton(false);
+    }
+  }
+  h->timing.launches = nl;
+  h->timing.iterations_max = it_total;
 }
 
 template <typename T, int G, bool XS>

@@ -154,11 +154,46 @@ inline bool solo_task(int w, int f) { return w <= kSoloPivots && f <= kSoloFront
 struct SweepPlan {
   std::vector<SweepStep> step;
   std::vector<int> step_ptr;   // steps of each island
+  std::vector<int> down_ptr;   // of them, the first root-to-leaves step
   std::vector<int> idx;
   int peak_cb = 0;             // carried entries alive at once (most over the islands)
   size_t scratch = 0;          // values per lane of shared memory the teams need
   size_t slot = 0;             // bytes of the largest step
 };
+// Plan of one block's factorisation (one island), streamed like the substitutions: a step is
+// a run of supernodes of one level whose arrowhead values are adjacent.  Its larger fronts go
+// to nteams teams of 1 << lteam threads, the others to the remaining warps, one front per
+// warp; bstride / sstride: shared-memory values per lane of a team's / a warp's front.
+struct FactorStep {
+  int e0, ne;          // arrowhead values [e0, e0 + ne)
+  int i0, ni;          // index block: idx[i0 .. i0 + ni), both multiples of 4
+  int nbig, nsmall;    // tasks of the index block: large fronts first
+  int lteam, nteams;
+  int bstride, sstride;
+  int pad[2];
+};
+static_assert(sizeof(FactorStep) == sizeof(SweepStep), "both records start an index block");
+// Index block: the FactorStep, eight ints per task (first value relative to e0, values; w |
+// f << 16; start of the task's list in the block, where its contribution block goes (-1: no
+// parent), children, panel entry, 0), then the lists: places of the arrowhead values in the
+// front, the pivots' x indices, and per child its contribution block's place, its length m m +
+// m and the place in the front of each of its values: m x m, then the m carried right-hand
+// sides.
+// Row stride of a front in shared memory (front_stride() of the kernels)
+inline int plan_front_stride(int f) { return (f + 1) | 1; }
+struct FactorPlan {
+  std::vector<FactorStep> step;
+  std::vector<int> idx;
+  int peak_cb = 0;             // values per lane of the contribution blocks alive at once
+  size_t most = 0;             // values per lane of the fronts worked on side by side
+  size_t slot = 0;             // bytes of the largest step
+  double cycles = 0.0;         // estimated clock cycles of a factorisation
+};
+// G lanes of wsize-byte values; slot: most bytes of a step; smem: bytes for contribution blocks
+// and fronts.  False when they do not fit.
+bool build_factor_plan(const LUSymbolic& s, const std::vector<int>& ah_ptr, const std::vector<int>& ah_loc, int G,
+                       int wsize, size_t slot, size_t smem, FactorPlan& out);
+
 // compact_cb: carried entries get slots that are reused once the parent has read them (else
 // their storage in cbr).  G lanes of wsize-byte values; slot: most bytes of a step; scratch:
 // bytes for the teams' fronts.  False when a front does not fit the scratch.

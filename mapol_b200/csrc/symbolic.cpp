@@ -337,6 +337,36 @@ void lu_symbolic(int n, const std::vector<std::vector<int>>& adj, LUSymbolic& s,
     s.max_front = std::max(s.max_front, s.sn_f[t]);
     if (parent[last] >= 0) s.sn_parent[t] = s.sn_of[parent[last]];
   }
+  // number the supernodes level by level, solo tasks first, similar ones side by side: the
+  // order in which a block walks them (build_sweep_plan, build_factor_plan), so that a level's
+  // arrowheads and panels are adjacent in storage
+  {
+    std::vector<int> level(ns, 0), order(ns), id(ns);
+    for (int q = 0; q < ns; ++q)  // children come before parents
+      if (s.sn_parent[q] >= 0) level[s.sn_parent[q]] = std::max(level[s.sn_parent[q]], level[q] + 1);
+    for (int q = 0; q < ns; ++q) order[q] = q;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+      return std::make_tuple(level[a], !solo_task(s.sn_w[a], s.sn_f[a]), s.sn_w[a], s.sn_f[a]) <
+             std::make_tuple(level[b], !solo_task(s.sn_w[b], s.sn_f[b]), s.sn_w[b], s.sn_f[b]);
+    });
+    for (int q = 0; q < ns; ++q) id[order[q]] = q;
+    std::vector<int> w(ns), f(ns), par(ns), rptr(ns + 1, 0), rows;
+    rows.reserve(s.sn_rows.size());
+    for (int q = 0; q < ns; ++q) {
+      const int o = order[q];
+      w[q] = s.sn_w[o];
+      f[q] = s.sn_f[o];
+      par[q] = s.sn_parent[o] >= 0 ? id[s.sn_parent[o]] : -1;
+      rows.insert(rows.end(), s.sn_rows.begin() + s.sn_rptr[o], s.sn_rows.begin() + s.sn_rptr[o + 1]);
+      rptr[q + 1] = (int)rows.size();
+    }
+    s.sn_w = w;
+    s.sn_f = f;
+    s.sn_parent = par;
+    s.sn_rptr = rptr;
+    s.sn_rows = rows;
+    for (int& t : s.sn_of) t = id[t];
+  }
   // children lists, levels
   s.child_ptr.assign(ns + 1, 0);
   for (int q = 0; q < ns; ++q)
@@ -910,6 +940,7 @@ bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bo
     }
     for (int q = 0; q < 2 * nlev; ++q) {
       const bool up = q < nlev;
+      if (q == nlev) out.down_ptr.push_back((int)out.step.size());
       const int lv = up ? q : 2 * nlev - 1 - q;
       // index list of a task
       auto list_of = [&](int n) {
@@ -1018,6 +1049,160 @@ bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bo
       }
     }
     out.step_ptr.push_back((int)out.step.size());
+  }
+  return out.idx.size() < (size_t)INT_MAX;
+}
+
+bool build_factor_plan(const LUSymbolic& s, const std::vector<int>& ah_ptr, const std::vector<int>& ah_loc, int G,
+                       int wsize, size_t slot, size_t smem, FactorPlan& out) {
+  out = FactorPlan();
+  if (s.nnz >= INT_MAX) return false;
+  const int nv = std::max(1, G * wsize / 16);  // threads per entry
+  const int warps = kChunkThreads / 32;
+  auto area = [](int f) { return (size_t)(f * ((f + 1) | 1) + 3) / 4 * 4; };  // front_stride()
+  // clock cycles of one front: its barriers and round trips in shared memory, its entries
+  auto cost = [&](int w, int f, int team) {
+    if (team == 32 && f <= (G * wsize <= 16 ? 16 : 8)) return 900.0 + w * (f <= 8 ? 220.0 : 330.0) + 10.0 * nv * 3.0 * f * f / team;
+    return 900.0 + w * (team == 32 ? 600.0 : 500.0) + 10.0 * nv * (0.6 * w * f * f + 3.0 * f * f) / team;
+  };
+  // contribution blocks (and their carried right-hand sides): slots by first fit over the
+  // levels at which they are alive
+  std::vector<int> cb(s.nsn, -1);
+  std::vector<std::pair<int, int>> free_list{{0, INT_MAX}};
+  for (int lv = 0; lv < s.nlevels; ++lv) {
+    for (int k = s.lev_ptr[lv]; k < s.lev_ptr[lv + 1]; ++k) {
+      const int n = s.lev_sn[k], m = s.sn_f[n] - s.sn_w[n];
+      if (s.sn_parent[n] < 0) continue;
+      const int len = (m * m + m + 3) / 4 * 4;
+      for (auto& fr : free_list)
+        if (fr.second >= len) {
+          cb[n] = fr.first;
+          fr.first += len;
+          fr.second -= len;
+          break;
+        }
+      out.peak_cb = std::max(out.peak_cb, cb[n] + len);
+    }
+    for (int k = s.lev_ptr[lv]; k < s.lev_ptr[lv + 1]; ++k)
+      for (int c = s.child_ptr[s.lev_sn[k]]; c < s.child_ptr[s.lev_sn[k] + 1]; ++c) {
+        const int ch = s.child_list[c], m = s.sn_f[ch] - s.sn_w[ch];
+        free_list.push_back({cb[ch], (m * m + m + 3) / 4 * 4});
+      }
+    std::sort(free_list.begin(), free_list.end());
+    std::vector<std::pair<int, int>> merged;
+    for (auto& fr : free_list) {
+      if (fr.second == 0) continue;
+      if (!merged.empty() && merged.back().first + merged.back().second == fr.first) merged.back().second += fr.second;
+      else merged.push_back(fr);
+    }
+    free_list = merged;
+  }
+  if ((size_t)out.peak_cb * G * wsize >= smem) return false;
+  const size_t cap = smem / ((size_t)G * wsize) - out.peak_cb;  // values per lane for the fronts
+  auto bytes_of = [&](int64_t ne, size_t ni) { return (size_t)((ne * G * wsize + 15) / 16 * 16) + ni * 4; };
+  // supernodes are numbered level by level, so a level's arrowheads are adjacent
+  std::vector<int> lev{0};
+  for (int n = 1; n <= s.nsn; ++n)
+    if (n == s.nsn || s.sn_level[n] != s.sn_level[n - 1]) lev.push_back(n);
+  for (int lv = 0; lv + 1 < (int)lev.size(); ++lv) {
+    int k = lev[lv];
+    while (k < lev[lv + 1]) {
+      FactorStep st{};
+      st.e0 = ah_ptr[k];
+      // as many supernodes as the slot holds
+      std::vector<std::vector<int>> lists;
+      size_t ints = kStepInts;
+      int k2 = k;
+      for (; k2 < lev[lv + 1]; ++k2) {
+        const int w = s.sn_w[k2], f = s.sn_f[k2];
+        std::vector<int> l(ah_loc.begin() + ah_ptr[k2], ah_loc.begin() + ah_ptr[k2 + 1]);
+        l.insert(l.end(), s.sn_rows.begin() + s.sn_rptr[k2], s.sn_rows.begin() + s.sn_rptr[k2] + w);
+        for (int c = s.child_ptr[k2]; c < s.child_ptr[k2 + 1]; ++c) {
+          const int ch = s.child_list[c], m = s.sn_f[ch] - s.sn_w[ch];
+          const int* rel = s.relmap.data() + s.rel_ptr[ch];
+          const int rs = plan_front_stride(f);
+          l.push_back(cb[ch]);
+          l.push_back(m * m + m);
+          for (int a = 0; a < m; ++a)
+            for (int b = 0; b < m; ++b) l.push_back(rel[a] * rs + rel[b]);
+          for (int a = 0; a < m; ++a) l.push_back(rel[a] * rs + f);
+        }
+        if (w > 0x7fff || f > 0x7fff) return false;
+        const size_t ni = (ints + 8 + l.size() + 3) / 4 * 4;
+        if (bytes_of(ah_ptr[k2 + 1] - st.e0, ni) > slot) break;
+        ints += 8 + l.size();
+        lists.push_back(l);
+      }
+      if (k2 == k) return false;
+      st.ne = ah_ptr[k2] - st.e0;
+      // large fronts first; the cut and the teams that take the least time
+      std::vector<int> sn;
+      for (int n = k; n < k2; ++n) sn.push_back(n);
+      std::stable_sort(sn.begin(), sn.end(), [&](int a, int b) { return s.sn_f[a] > s.sn_f[b]; });
+      const int n = (int)sn.size();
+      double bt = -1.0;
+      for (int nbig = 0; nbig <= std::min(n, 64); ++nbig) {
+        if (nbig > 0 && nbig < n && s.sn_f[sn[nbig]] == s.sn_f[sn[nbig - 1]]) continue;  // cut between sizes
+        auto worst = [&](int a, int b) {
+          int w = 0, f = 0;
+          for (int q = a; q < b; ++q) {
+            w = std::max(w, s.sn_w[sn[q]]);
+            f = std::max(f, s.sn_f[sn[q]]);
+          }
+          return std::make_pair(w, f);
+        };
+        const auto wb = worst(0, nbig), wsm = worst(nbig, n);
+        const size_t bs = area(wb.second), ss = area(wsm.second);
+        for (int lteam : {5, 7, 8, 9}) {
+          const int team = 1 << lteam;
+          if (team > kChunkThreads || (nbig == 0) != (lteam == 5)) continue;
+          for (int nt = std::min(nbig, kChunkThreads / team); nt >= (nbig > 0 ? 1 : 0); --nt) {
+            const size_t held = (size_t)nt * bs;
+            int free_warps = warps - nt * team / 32;
+            const bool after = nbig < n && free_warps == 0;  // the small fronts follow the large ones
+            if (after) free_warps = warps;
+            const size_t small = nbig < n ? (size_t)free_warps * ss : 0;
+            const size_t need = after ? std::max(held, small) : held + small;
+            if (need > cap) continue;
+            const double tb = nbig > 0 ? (double)((nbig + nt - 1) / nt) * cost(wb.first, wb.second, team) : 0.0;
+            const double ts = nbig < n ? (double)((n - nbig + free_warps - 1) / free_warps) * cost(wsm.first, wsm.second, 32) : 0.0;
+            const double t = after ? tb + ts : std::max(tb, ts);
+            if (bt < 0.0 || t < bt) {
+              bt = t;
+              st.nbig = nbig;
+              st.nsmall = n - nbig;
+              st.lteam = lteam;
+              st.nteams = nt;
+              st.bstride = (int)bs;
+              st.sstride = (int)ss;
+              st.pad[0] = (int)need;
+            }
+            break;  // the most teams that fit
+          }
+        }
+      }
+      if (bt < 0.0) return false;
+      out.cycles += bt;
+      out.most = std::max(out.most, (size_t)st.pad[0]);
+      st.i0 = (int)out.idx.size();
+      std::vector<int> head, body;
+      for (int q : sn) {
+        const std::vector<int>& l = lists[q - k];
+        head.insert(head.end(), {ah_ptr[q] - st.e0, ah_ptr[q + 1] - ah_ptr[q], s.sn_w[q] | s.sn_f[q] << 16,
+                                 (int)(kStepInts + 8 * n + body.size()), cb[q], s.child_ptr[q + 1] - s.child_ptr[q],
+                                 (int)s.pan_off[q], 0});
+        body.insert(body.end(), l.begin(), l.end());
+      }
+      st.ni = (int)((kStepInts + head.size() + body.size() + 3) / 4 * 4);
+      const int* rec = reinterpret_cast<const int*>(&st);
+      out.idx.insert(out.idx.end(), rec, rec + kStepInts);
+      out.idx.insert(out.idx.end(), head.begin(), head.end());
+      out.idx.insert(out.idx.end(), body.begin(), body.end());
+      out.idx.resize((size_t)st.i0 + st.ni, 0);
+      out.slot = std::max(out.slot, bytes_of(st.ne, st.ni));
+      out.step.push_back(st);
+      k = k2;
+    }
   }
   return out.idx.size() < (size_t)INT_MAX;
 }

@@ -69,7 +69,10 @@ static bool check(const LUSymbolic& s, const std::vector<int>& isl, bool compact
   for (double& v : x0) v = rng.uniform() - 0.5;
   int nisl = 1;
   for (int v : isl) nisl = v + 1 > nisl ? v + 1 : nisl;
-  if ((int)P.step_ptr.size() != nisl + 1) return false;
+  if ((int)P.step_ptr.size() != nisl + 1 || (int)P.down_ptr.size() != nisl) return false;
+  for (int k = 0; k < nisl; ++k)  // up to down_ptr leaves to root, then root to leaves
+    for (int q = P.step_ptr[k]; q < P.step_ptr[k + 1]; ++q)
+      if ((P.step[q].up != 0) != (q < P.down_ptr[k])) return false;
   size_t most = 0, widest = 0;
   for (bool tr : {false, true}) {
     std::vector<double> x = x0;
@@ -151,6 +154,119 @@ static bool check(const LUSymbolic& s, const std::vector<int>& isl, bool compact
   return most == P.scratch && widest == P.slot;
 }
 
+// The factorisation's plan: its steps hold every arrowhead value once, in order; a step fits
+// its slot, its teams and warps the block and the shared memory; contribution blocks are
+// written once per slot and step and read only in later steps.  The factorisation walked over
+// the plan equals the dense front-by-front one bit for bit.
+static bool check_factor(const LUSymbolic& s, const std::vector<int>& ah_ptr, const std::vector<int>& ah_loc, int G,
+                         int wsize, size_t slot, size_t smem, Rng& rng) {
+  auto area = [](int f) { return (size_t)f * ((f + 1) | 1); };
+  FactorPlan P;
+  if (!build_factor_plan(s, ah_ptr, ah_loc, G, wsize, slot, smem, P)) return true;
+  ++plans;
+  const int nA = ah_ptr[s.nsn];
+  std::vector<double> A(nA), x0(s.n);
+  for (double& v : A) v = rng.uniform() - 0.5;
+  for (int n = 0; n < s.nsn; ++n)
+    for (int e = ah_ptr[n]; e < ah_ptr[n + 1]; ++e) {
+      const int RS = (s.sn_f[n] + 1) | 1;
+      if (ah_loc[e] / RS == ah_loc[e] % RS) A[e] = 20.0 + rng.uniform();
+    }
+  for (double& v : x0) v = rng.uniform() - 0.5;
+  // a front's partial LU, right-looking (columns f: the right-hand side)
+  auto lu = [](std::vector<double>& F, int f, int w) {
+    const int RS = (f + 1) | 1;
+    for (int p = 0; p < w; ++p) {
+      const double inv = 1.0 / F[p * RS + p];
+      for (int i = p + 1; i < f; ++i) {
+        const double l = F[i * RS + p] * inv;
+        F[i * RS + p] = l;
+        for (int q = p + 1; q <= f; ++q) F[i * RS + q] -= l * F[p * RS + q];
+      }
+    }
+  };
+  std::vector<double> pan(s.nnz, 0.0), ref(s.nnz, 0.0), x = x0, xr = x0;
+  {
+    std::vector<std::vector<double>> cb(s.nsn);
+    for (int q = 0; q < s.nsn; ++q) {
+      const int n = s.lev_sn[q], w = s.sn_w[n], f = s.sn_f[n], m = f - w, RS = (f + 1) | 1;
+      std::vector<double> F((size_t)f * RS, 0.0);
+      for (int e = ah_ptr[n]; e < ah_ptr[n + 1]; ++e) F[ah_loc[e]] = A[e];
+      for (int p = 0; p < w; ++p) F[p * RS + f] = xr[s.sn_rows[s.sn_rptr[n] + p]];
+      for (int c = s.child_ptr[n]; c < s.child_ptr[n + 1]; ++c) {
+        const int ch = s.child_list[c], mc = s.sn_f[ch] - s.sn_w[ch];
+        const int* rel = &s.relmap[s.rel_ptr[ch]];
+        for (int a = 0; a < mc; ++a) {
+          for (int b = 0; b < mc; ++b) F[rel[a] * RS + rel[b]] += cb[ch][a * mc + b];
+          F[rel[a] * RS + f] += cb[ch][mc * mc + a];
+        }
+      }
+      lu(F, f, w);
+      for (int i = 0; i < f; ++i)
+        for (int j = 0; j < (i < w ? f : w); ++j) ref[s.pan_off[n] + (i < w ? i * f + j : w * f + (i - w) * w + j)] = F[i * RS + j];
+      for (int p = 0; p < w; ++p) xr[s.sn_rows[s.sn_rptr[n] + p]] = F[p * RS + f];
+      cb[n].resize(m * m + m);
+      for (int a = 0; a < m; ++a) {
+        for (int b = 0; b < m; ++b) cb[n][a * m + b] = F[(w + a) * RS + w + b];
+        cb[n][m * m + a] = F[(w + a) * RS + f];
+      }
+    }
+  }
+  std::vector<double> cb(P.peak_cb + 1, std::nan(""));
+  int at = 0;
+  size_t most = 0;
+  for (const FactorStep& st : P.step) {
+    if (st.e0 != at || st.i0 % 4 || st.ni % 4 || st.i0 + st.ni > (int)P.idx.size()) return false;
+    at += st.ne;
+    const size_t bytes = ((size_t)st.ne * G * wsize + 15) / 16 * 16 + (size_t)st.ni * 4;
+    if (bytes > slot || bytes > P.slot) return false;
+    const int* ib = &P.idx[st.i0];
+    const int nbig = ib[4], nsmall = ib[5], lteam = ib[6], nteams = ib[7], bstride = ib[8], sstride = ib[9];
+    const int busy = nteams << lteam;
+    if (busy > kChunkThreads || (nbig > 0) != (nteams > 0) || (lteam > 5 && nteams > 15)) return false;
+    if ((size_t)bstride * G * wsize % 16 || (size_t)sstride * G * wsize % 16) return false;
+    const size_t big = (size_t)nteams * bstride;
+    const size_t small = nsmall > 0 ? (kChunkThreads - (busy < kChunkThreads ? busy : 0)) / 32 * (size_t)sstride : 0;
+    const size_t held = busy < kChunkThreads ? big + small : big > small ? big : small;
+    if (held > most) most = held;
+    const std::vector<double> cr = cb, xs = x;
+    std::vector<char> cw(cb.size(), 0);
+    for (int t = 0; t < nbig + nsmall; ++t) {
+      const int* h = ib + kStepInts + 8 * t;
+      const int na = h[1], w = h[2] & 0xffff, f = h[2] >> 16, m = f - w, RS = (f + 1) | 1;
+      if (area(f) > (size_t)(t < nbig ? bstride : sstride) || h[0] < 0 || h[0] + na > st.ne) return false;
+      const int *loc = ib + h[3], *rows = loc + na, *kid = rows + w;
+      std::vector<double> F((size_t)f * RS, 0.0);
+      for (int e = 0; e < na; ++e) F[loc[e]] = A[st.e0 + h[0] + e];
+      for (int p = 0; p < w; ++p) F[p * RS + f] = xs[rows[p]];
+      for (int c = 0; c < h[5]; ++c) {
+        const int ne = kid[1];
+        const int* to = kid + 2;
+        if (to + ne > ib + st.ni) return false;
+        std::vector<char> once(F.size(), 0);
+        for (int e = 0; e < ne; ++e) {
+          if (to[e] < 0 || to[e] >= f * RS || once[to[e]]++) return false;  // distinct within a child
+          F[to[e]] += cr[kid[0] + e];
+        }
+        kid = to + ne;
+      }
+      lu(F, f, w);
+      for (int i = 0; i < f; ++i)
+        for (int j = 0; j < (i < w ? f : w); ++j) pan[h[6] + (i < w ? i * f + j : w * f + (i - w) * w + j)] = F[i * RS + j];
+      for (int p = 0; p < w; ++p) x[rows[p]] = F[p * RS + f];
+      for (int a = 0; a < m && h[4] >= 0; ++a)
+        for (int b = 0; b <= m; ++b) {
+          const int to = h[4] + (b < m ? a * m + b : m * m + a);
+          if (to >= P.peak_cb || cw[to]) return false;
+          cw[to] = 1;
+          cb[to] = F[(w + a) * RS + (b < m ? w + b : f)];
+        }
+    }
+  }
+  if (at != nA || most != P.most || (P.most + P.peak_cb) * G * wsize > smem) return false;
+  return pan == ref && x == xr;
+}
+
 int main() {
   const int shapes[][4] = {{2, 1, 0, 0}, {30, 41, 5, 0}, {118, 179, 53, 0}, {300, 411, 69, 0},
                            {1354, 1991, 259, 0}, {1354, 1991, 259, 1}, {2869, 4582, 509, 0}, {700, 699, 0, 2}};
@@ -207,6 +323,13 @@ int main() {
       const LUSymbolic* sys[3] = {&g.jac, &g.bp[0].lu, &g.bpp[0].lu};
       const std::vector<int> isl[3] = {islands(g.jac, g.var_va, &g.var_vm), islands(g.bp[0].lu, g.bp[0].var, nullptr),
                                        islands(g.bpp[0].lu, g.bpp[0].var, nullptr)};
+      for (int G : {8, 2, 1})
+        for (size_t slot : {(size_t)3 * 1024, (size_t)16 * 1024})
+          for (int ws : {4, 8})
+            if (!check_factor(g.jac, g.ah_ptr, g.ah_loc, G, ws, slot, 170 * 1024, rng)) {
+              std::printf("bad factor plan: %d buses, copies %d, G %d, value %d, slot %zu\n", sh[0], copies, G, ws, slot);
+              return 1;
+            }
       for (int k = 0; k < 3; ++k)
         for (bool compact : {false, true})
           for (int G : {8, 1})

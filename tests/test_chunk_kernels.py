@@ -50,3 +50,28 @@ def test_fast_decoupled_chunks_match_oracle(gpu, monkeypatch, in_shared, lanes, 
         assert np.abs(res.v - ref["v"]).max() < 1e-8
         if prec == m.FP64:
             assert np.array_equal(res.iterations, ref["iterations"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+@pytest.mark.parametrize("prec", [m.FP64, m.MIXED])
+@pytest.mark.parametrize("n_bus,n_cases", [(30, 1), (118, 33), (300, 70), (700, 9)])
+def test_newton_chunks_match_oracle(gpu, monkeypatch, lanes, prec, n_bus, n_cases):
+    """Newton on one block per chunk against the oracle (both to max |F| < 1e-11, so |dV|
+    stays below the parity tests' 1e-8), and in parts (use_graph 1 and 0) bit for bit."""
+    monkeypatch.setenv("MPF_NR_CHUNK", str(lanes))
+    buses, branches = m.synth_grid(n_bus, int(1.5 * n_bus), max(2, n_bus // 6), 0.1, seed=4)
+    n1 = np.flatnonzero(~m.find_bridges(branches, n_bus))
+    cases = ([[]] + [[int(b)] for b in np.resize(n1, n_cases)])[:n_cases]
+    ref = oracle.runpf(buses, branches, cases, alg=m.NR, tol=1e-11)
+    out = []
+    for use_graph in (2, 1, 0):
+        with m.PowerFlow(buses, branches, tol=1e-11, use_graph=use_graph) as pf:
+            out.append(pf.runpf(cases, alg=m.NR, precision=prec))
+    assert out[0].converged.all() and ref["converged"].all()
+    assert np.abs(out[0].v - ref["v"]).max() < 1e-8
+    if prec == m.FP64:
+        assert np.array_equal(out[0].iterations, ref["iterations"])
+    for r in out[1:]:
+        assert np.array_equal(r.v, out[0].v) and np.array_equal(r.iterations, out[0].iterations)
+        assert np.array_equal(r.status, out[0].status) and np.array_equal(r.max_mis, out[0].max_mis)
