@@ -98,7 +98,7 @@ constexpr int kMaxQRounds = 20;
 // largest dense front in shared memory: one FP64 lane, f * ((f + 1) | 1) * 8 bytes.
 // Larger fronts (CLS_BIG, densely meshed grids) keep only their panel, w (2f - w + 1)
 // entries, in shared memory (k_mf_factor_big) and their trailing block in global memory
-constexpr int kFmaxAll = 167;
+constexpr int kFmaxAll = kBigFront;
 inline size_t big_panel(int w, int f) { return (size_t)w * (2 * f - w + 1); }
 // The fronts' limits: every panel of one FP64 lane and one warp's slice of x in the
 // thread-per-case substitutions (f entries of 32 FP64 lanes) fit in shared memory
@@ -140,6 +140,7 @@ struct Launch {
   int wfmax = 0;                 // largest w * f in range (U-panel entries)
   int level = 0;                 // elimination-tree level
   size_t pcap = 0;               // CLS_BIG: largest panel in range, w (2f - w + 1) entries
+  int wcap = 0;                  // CLS_BIG: most pivots in range
   int mcap = 0;                  // CLS_BIG: largest trailing block in range, m = f - w rows
 };
 
@@ -388,6 +389,7 @@ struct LUSystem {
         {
           ln.pcap = std::max(ln.pcap, big_panel(s.sn_w[s.lev_sn[t]], s.sn_f[s.lev_sn[t]]));
           ln.mcap = std::max(ln.mcap, s.sn_f[s.lev_sn[t]] - s.sn_w[s.lev_sn[t]]);
+          ln.wcap = std::max(ln.wcap, (s.sn_w[s.lev_sn[t]] + 3) / 4 * 4);
         }
     for (const Launch& ln : factor_sched) {
       fingerprint = (fingerprint ^ (uint64_t)ln.offset) * 1099511628211ull;
@@ -703,15 +705,16 @@ template <typename T>
 void launch_factor_big(int ge, int S, const LUSystem& sys, const Launch& ln, int ngroups, const T* A, T* pan, T* cb,
                        T* cbr, T* x, int* status, const int* group_active, int with_rhs, cudaStream_t st) {
   const size_t smem = (ln.pcap + (size_t)S * (ln.mcap + 1)) * ge * sizeof(T);
+  const int scap = S * (ln.mcap + 1);
   if (ln.pcap == 0 || S < 1 || smem > kSmemMax) throw MpfError{MPF_ERR_INTERNAL, "big-front panel does not fit"};
   const long long ntasks = (long long)ln.count * ngroups * (32 / ge);
   const unsigned blocks = (unsigned)std::min<long long>(ntasks, 148LL * 32);
   const DevLU dl = sys.dev();
   const int* ts = sys.lev_sn.as<int>() + ln.offset;
   switch (ge) {
-    case 4: k_mf_factor_big<T, 4><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs, (int)ln.pcap, S); break;
-    case 2: k_mf_factor_big<T, 2><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs, (int)ln.pcap, S); break;
-    case 1: k_mf_factor_big<T, 1><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs, (int)ln.pcap, S); break;
+    case 4: k_mf_factor_big<T, 4><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs, (int)ln.pcap, S, scap); break;
+    case 2: k_mf_factor_big<T, 2><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs, (int)ln.pcap, S, scap); break;
+    case 1: k_mf_factor_big<T, 1><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs, (int)ln.pcap, S, scap); break;
     default: throw MpfError{MPF_ERR_INTERNAL, "no big-front kernel for this lane count"};
   }
   CUDA_TRY(cudaGetLastError());
@@ -722,16 +725,16 @@ void launch_factor_big(int ge, int S, const LUSystem& sys, const Launch& ln, int
 template <typename T>
 void launch_factor_big_gt(int ge, const LUSystem& sys, const Launch& ln, int ngroups, const T* A, T* pan, T* cb,
                           T* cbr, T* x, int* status, const int* group_active, int with_rhs, cudaStream_t st) {
-  const size_t smem = ln.pcap * ge * sizeof(T);
+  const size_t smem = (ln.wcap + ln.pcap) * ge * sizeof(T);
   if (ln.pcap == 0 || smem > kSmemMax) throw MpfError{MPF_ERR_INTERNAL, "big-front panel does not fit"};
   const long long ntasks = (long long)ln.count * ngroups * (32 / ge);
   const unsigned blocks = (unsigned)std::min<long long>(ntasks, 148LL * 32);
   const DevLU dl = sys.dev();
   const int* ts = sys.lev_sn.as<int>() + ln.offset;
   switch (ge) {
-    case 4: k_mf_factor_big_gt<T, 4><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs); break;
-    case 2: k_mf_factor_big_gt<T, 2><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs); break;
-    case 1: k_mf_factor_big_gt<T, 1><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs); break;
+    case 4: k_mf_factor_big_gt<T, 4><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs, ln.wcap); break;
+    case 2: k_mf_factor_big_gt<T, 2><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs, ln.wcap); break;
+    case 1: k_mf_factor_big_gt<T, 1><<<blocks, 512, smem, st>>>(dl, ts, ln.count, ngroups, A, pan, cb, cbr, x, status, group_active, with_rhs, ln.wcap); break;
     default: throw MpfError{MPF_ERR_INTERNAL, "no big-front kernel for this lane count"};
   }
   CUDA_TRY(cudaGetLastError());
@@ -874,7 +877,7 @@ std::vector<FactorChoice> factor_candidates(const Launch& ln, int ngroups) {
         if (!dup) c.push_back(x);
       }
       // the trailing block in global memory instead: only the panel in shared memory
-      if (ln.pcap * ge * sizeof(T) <= kSmemMax) c.push_back({7, ge, 0, 1});
+      if ((ln.wcap + ln.pcap) * ge * sizeof(T) <= kSmemMax) c.push_back({7, ge, 0, 1});
     }
     return c;
   }
@@ -1917,7 +1920,8 @@ inline bool chunk_shape(const std::vector<LUSystem*>& sys, int G, int wsize, boo
   return out.smem <= budget;
 }
 
-// Widest chunk (at most a 32-byte sector of lanes) that fits and leaves a block for every SM
+// Widest chunk (at most a 32-byte sector of lanes) that fits and gives at least half of the SMs
+// a block (fewer, wider chunks read the plan less often; below half, a second wave is still free)
 inline ChunkShape choose_chunk(const std::vector<LUSystem*>& sys, int widest, int wsize, int ngroups, int resident) {
   ChunkShape sh;
   auto budget = [&](int G) { return resident > 1 && ngroups * (32 / G) > 148 ? kChunkSmem / resident : kChunkSmem; };

@@ -541,15 +541,20 @@ __device__ __forceinline__ void next_task(int& q, int& r, int sq, int sr, int nc
   }
 }
 
-// First index a < n with rel[a] >= v (rel increasing), or n
-__device__ __forceinline__ int first_at_least(const int* rel, int n, int v) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (rel[mid] < v) lo = mid + 1;
-    else hi = mid;
+// First index a < n with rel[a] >= v (rel increasing), or n, by a whole warp (all 32 threads
+// call it with the same arguments): each round looks at 32 places at once, two dependent loads
+// for up to 1024 entries instead of the ten of a binary search
+__device__ __forceinline__ int warp_first_at_least(const int* rel, int n, int v) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0, len = n;  // the answer lies in [lo, lo + len]
+  while (len > 0) {
+    const int step = (len + 31) >> 5;
+    const int at = lo + (lane + 1) * step - 1;  // the last entry of this thread's share
+    const int below = __popc(__ballot_sync(0xffffffffu, at < lo + len && rel[at] < v));
+    lo += below * step;
+    len = step == 1 ? 0 : min(step, n - lo);
   }
-  return lo;
+  return min(lo, n);
 }
 
 template <int TEAM>
@@ -1133,6 +1138,118 @@ __global__ void __launch_bounds__(TEAM == 32 ? 288 : TEAM, TT > 0 ? 2 : (TEAM > 
   }
 }
 
+// Contribution blocks between two large fronts are stored [lane pair][entry][2] instead of
+// [entry][32]: a large front's task owns 1 to 4 lanes, which are 4 to 16 bytes of every
+// 128-byte row, so its reads and writes of the m x m block moved 32-byte sectors for them, one
+// line per entry (80% of the kernel's time); paired, a warp's accesses are contiguous.  Solve
+// of 250 cases of the uniform 1354-bus grid, mixed: 49.2 -> 34.6 ms, and 30.2 with the blocks
+// asked from DRAM at the task's start.
+// Entry e of lane `lane` of the block at off (len entries): p[e * step].
+constexpr int kBigFront = 167;  // fronts above this many rows are large (kFmaxAll)
+template <typename T>
+struct CbView {
+  T* p;
+  int step;
+};
+template <typename T>
+__device__ __forceinline__ CbView<T> cb_view(T* cb, long long sumcb, int g, long long off, int len, int lane, bool paired) {
+  T* base = cb + at32(g, sumcb, off, 0);
+  if (paired) return CbView<T>{base + (size_t)(lane >> 1) * len * 2 + (lane & 1), 2};
+  return CbView<T>{base + lane, 32};
+}
+
+// Partial LU of a large front's panel in shared memory (entry slots of G lanes; slot, l: this
+// thread's): the w x w pivot block one pivot per barrier, then the other rows' pivot columns
+// (L, a thread per row and lane) and the pivot rows' other columns (U and the right-hand
+// side, a thread per column and lane) side by side, eight entries at a time in registers: one
+// shared-memory read of the pivot block per multiply-add, where the pivot-by-pivot update of
+// the whole panel took three reads, a write and the index arithmetic.  Same operations per
+// entry in the same order.  P: the top part [w][f + 1], then the left part [m][w]; inv: w G
+// values of scratch, or null (the divisions are repeated).  Fronts up to 337 rows, 250 cases,
+// mixed: 2.98 -> 1.52 million cycles of a block per solve.
+template <typename T, int G>
+__device__ __forceinline__ void panel_lu(T* P, T* inv, int f, int w, int ncols, int slot, int l, int slots, int* st_lane) {
+  constexpr int B = 8;
+  const int m = f - w, rs = f + 1;  // row stride of the top part
+  auto D = [&](int i, int j) -> T& { return P[(i * rs + j) * G + l]; };
+  for (int p = 0; p < w; ++p) {
+    T pk = D(p, p);
+    if (bad_pivot(pk)) {
+      if (slot == 0) mark_singular(st_lane);
+      pk = (T)1;
+    }
+    const T iv = (T)1 / pk;
+    if (inv && slot == 0) inv[p * G + l] = iv;
+    const int r = w - 1 - p;
+    if (r > 0) {
+      int i = slot / r, j = slot % r;
+      const int si = slots / r, sj = slots % r;
+      for (; i < r; next_task(i, j, si, sj, r)) {
+        T& b = D(p + 1 + i, p + 1 + j);
+        b = b - (D(p + 1 + i, p) * iv) * D(p, p + 1 + j);
+      }
+    }
+    __syncthreads();
+  }
+  auto inverse = [&](int p) {
+    if (inv) return inv[p * G + l];
+    const T pk = D(p, p);
+    return bad_pivot(pk) ? (T)1 : (T)1 / pk;
+  };
+  // the pivot block's L entries, read unscaled until here
+  for (int e = slot; e < w * w; e += slots) {
+    const int i = e / w, p = e % w;
+    if (p < i) D(i, p) *= inverse(p);
+  }
+  __syncthreads();
+  const int nt = ncols - w;  // columns w .. ncols - 1
+  for (int t = slot; t < m + nt; t += slots) {
+    if (t < m) {
+      T* row = P + ((size_t)w * rs + (size_t)t * w) * G + l;
+      for (int jb = 0; jb < w; jb += B) {
+        T a[B];
+#pragma unroll
+        for (int q = 0; q < B; ++q) a[q] = jb + q < w ? row[(jb + q) * G] : (T)0;
+        for (int p = 0; p < jb; ++p) {
+          const T lp = row[p * G];
+#pragma unroll
+          for (int q = 0; q < B; ++q) a[q] = a[q] - lp * D(p, jb + q);  // (columns past w: not stored)
+        }
+#pragma unroll
+        for (int q = 0; q < B; ++q)
+          if (jb + q < w) {
+            a[q] *= inverse(jb + q);
+#pragma unroll
+            for (int z = q + 1; z < B; ++z) a[z] = a[z] - a[q] * D(jb + q, jb + z);
+            row[(jb + q) * G] = a[q];
+          }
+      }
+    } else {
+      const int j = w + t - m;
+      for (int ib = 0; ib < w; ib += B) {
+        T a[B];
+#pragma unroll
+        for (int q = 0; q < B; ++q) a[q] = ib + q < w ? D(ib + q, j) : (T)0;
+        for (int p = 0; p < ib; ++p) {
+          const T up = D(p, j);
+#pragma unroll
+          for (int q = 0; q < B; ++q)
+            if (ib + q < w) a[q] = a[q] - D(ib + q, p) * up;
+        }
+#pragma unroll
+        for (int q = 0; q < B; ++q)
+          if (ib + q < w) {
+#pragma unroll
+            for (int z = q + 1; z < B; ++z)
+              if (ib + z < w) a[z] = a[z] - D(ib + z, ib + q) * a[q];
+            D(ib + q, j) = a[q];
+          }
+      }
+    }
+  }
+  __syncthreads();
+}
+
 // Fronts too large for a dense front in shared memory (densely meshed grids).  The
 // panel stays in shared memory for the whole task: the w pivot rows with all f columns
 // and the right-hand side (top part, w x (f + 1)) and the pivot columns of the other
@@ -1152,11 +1269,13 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
                                                        T* __restrict__ cbr, T* __restrict__ x,
                                                        int* __restrict__ status,
                                                        const int* __restrict__ group_active, int with_rhs,
-                                                       int pcap, int S) {
+                                                       int pcap, int S, int scap) {
   constexpr int SLOTS = 512 / G, LPG = 32 / G;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* P = reinterpret_cast<T*>(smem_raw);
   const int slot = threadIdx.x / G, l = threadIdx.x % G;
+  constexpr int CS = 32 / G;  // columns side by side in a warp
+  const int warp = threadIdx.x >> 5, cs = slot % CS;
   const int nch = ngroups * LPG;
   for (int q = blockIdx.x / nch, ch = blockIdx.x % nch; q < nsn_l;
        next_task(q, ch, (int)gridDim.x / nch, (int)gridDim.x % nch, nch)) {
@@ -1176,8 +1295,20 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
       return r < w ? P[((size_t)r * (f + 1) + c) * G + l] : P[((size_t)w * (f + 1) + (size_t)(r - w) * w + c) * G + l];
     };
     // trailing entry (a, b) of the contribution block, and the carried right-hand side
-    auto CE = [&](int a, int b) -> T& { return cb[at32(g, L.sumcb, cbo + (long long)a * m + b, lane)]; };
+    const CbView<T> own = cb_view(cb, L.sumcb, g, cbo, m * m, lane, has_parent && L.sn_f[L.sn_parent[s]] > kBigFront);
+    auto CE = [&](int a, int b) -> T& { return own.p[(size_t)(a * m + b) * own.step]; };
     auto CR = [&](int a) -> T& { return cbr[at32(g, L.sumcbr, cbro + a, lane)]; };
+    // the large children's blocks of this task's lanes are contiguous: asked from DRAM now, so
+    // that the reads of the assembly, which hold 16 KB in flight per block, wait on L2 only
+    if (threadIdx.x == 0)
+      for (int ci = L.child_ptr[s]; ci < L.child_ptr[s + 1]; ++ci) {
+        if (L.sn_f[L.child_list[ci]] <= kBigFront) continue;
+        const ChildRef cr = L.child_ref[ci];
+        const CbView<T> from = cb_view(cb, L.sumcb, g, cr.cb_off, cr.m * cr.m, (ch % LPG) * G, true);
+        const size_t a0 = (size_t)from.p & ~(size_t)15;
+        const size_t a1 = ((size_t)(from.p + (size_t)cr.m * cr.m * (G > 2 ? G : 2)) + 15) & ~(size_t)15;
+        prefetch_l2(reinterpret_cast<const void*>(a0), (unsigned)(a1 - a0));
+      }
     for (int e = slot; e < npan; e += SLOTS) P[(size_t)e * G + l] = (T)0;
     __syncthreads();
     // the arrowhead: pivot rows and pivot columns, all in the panel
@@ -1201,92 +1332,50 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
       const ChildRef cr = L.child_ref[ci];
       const int mc = cr.m;
       const int* rel = L.relmap + cr.rel_ptr;
-      const int aw = first_at_least(rel, mc, w);
-      const T* src = cb + at32(g, L.sumcb, cr.cb_off, lane);
-      // entries (a_first + i, j), i rowlen + j < n, eight per thread at a time (their
-      // loads before their stores); (i, j) advance by SLOTS without divisions
-      auto add_panel = [&](int n, int a_first, int rowlen) {
-        if (n <= 0) return;
-        const int si = SLOTS / rowlen, sj = SLOTS % rowlen;
-        int i = slot / rowlen, j = slot % rowlen;
-        for (int e0 = slot; e0 < n; e0 += 8 * SLOTS) {
-          int r[8], c[8];
+      const int aw = warp_first_at_least(rel, mc, w);
+      const CbView<T> from = cb_view(cb, L.sumcb, g, cr.cb_off, mc * mc, lane, L.sn_f[L.child_list[ci]] > kBigFront);
+      const T* src = from.p;
+      const int es = from.step;
+      // a warp takes whole rows landing in pivot rows, 32 / G columns side by side, and of the
+      // other rows the columns landing in pivot columns; eight loads per thread before their adds
+      for (int a = warp; a < aw; a += 16) {
+        const int r = rel[a];
+        const T* row = src + (size_t)a * mc * es;
+        for (int b0 = cs; b0 < mc; b0 += 8 * CS) {
+          int c[8];
           T v[8];
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
-            const bool ok = e0 + u * SLOTS < n;
-            const int a = a_first + (ok ? i : 0), b = ok ? j : 0;
-            r[u] = rel[a];
+            const int b = min(b0 + u * CS, mc - 1);
             c[u] = rel[b];
-            v[u] = ok ? src[((size_t)a * mc + b) * 32] : (T)0;
-            next_task(i, j, si, sj, rowlen);
+            v[u] = row[(size_t)b * es];
           }
 #pragma unroll
           for (int u = 0; u < 8; ++u)
-            if (e0 + u * SLOTS < n) PE(r[u], c[u]) += v[u];
+            if (b0 + u * CS < mc) PE(r, c[u]) += v[u];
         }
-      };
-      add_panel(aw * mc, 0, mc);              // rows landing in pivot rows
-      add_panel((mc - aw) * aw, aw, aw);      // the other rows' pivot columns
+      }
+      for (int a = aw + warp; a < mc; a += 8 * 16)
+        for (int b = cs; b < aw; b += CS) {
+          const int c = rel[b];
+          int r[8];
+          T v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int au = min(a + u * 16, mc - 1);
+            r[u] = rel[au];
+            v[u] = src[(size_t)(au * mc + b) * es];
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (a + u * 16 < mc) PE(r[u], c) += v[u];
+        }
       if (with_rhs)
         for (int a = slot; a < aw; a += SLOTS) PE(rel[a], f) += cbr[at32(g, L.sumcbr, cr.cbr_off + a, lane)];
       __syncthreads();
     }
-    // LU of the panel, one pivot per barrier: rows p < i < w over columns p < j < ncols
-    // (top part) and rows i >= w over columns p < j < w (left part), each entry with
-    // the unscaled l_ip = F(i,p) / F(p,p) of its row; column p is scaled one pivot later
-    // (and after the loop for the last pivot), when no thread reads it any more
-    T inv_prev = (T)1;
-    for (int p = 0; p < w; ++p) {
-      T pk = PE(p, p);
-      if (bad_pivot(pk)) {
-        if (slot == 0) mark_singular(&status[g * 32 + lane]);
-        pk = (T)1;
-      }
-      const T inv = (T)1 / pk;
-      if (p > 0)
-        for (int i = p + slot; i < f; i += SLOTS) PE(i, p - 1) *= inv_prev;
-      // four entries per thread at a time, loads before stores: the updated entries
-      // (i > p, j > p) are distinct and none of them is in row p or column p, which the
-      // updates read
-      // rows of the part start at `base` (shared-memory index of column 0 of its first
-      // row, row stride rstride entries); entry e = i rowlen + j' of the part is row i,
-      // column p + 1 + j'; (i, j') advance by SLOTS without divisions
-      auto update = [&](int n, int base, int rstride, int rowlen) {
-        if (n <= 0) return;
-        const int si = SLOTS / rowlen, sj = SLOTS % rowlen;
-        int i = slot / rowlen, j = slot % rowlen;
-        const T* prow = P + ((size_t)p * (f + 1) + p + 1) * G + l;  // u_pj, j > p
-        for (int e0 = slot; e0 < n; e0 += 4 * SLOTS) {
-          int at[4], jc[4];
-          T lp[4], up[4], bv[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const bool ok = e0 + u * SLOTS < n;
-            const int row = base + (ok ? i : 0) * rstride;
-            at[u] = row + p + 1 + (ok ? j : 0);
-            jc[u] = ok ? j : 0;
-            lp[u] = P[(size_t)(row + p) * G + l];
-            up[u] = prow[(size_t)jc[u] * G];
-            bv[u] = P[(size_t)at[u] * G + l];
-            next_task(i, j, si, sj, rowlen);
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (e0 + u * SLOTS < n) P[(size_t)at[u] * G + l] = bv[u] - (lp[u] * inv) * up[u];
-        }
-      };
-      // top part: rows p+1 .. w-1, columns p+1 .. ncols-1
-      update((w - 1 - p) * (ncols - 1 - p), (p + 1) * (f + 1), f + 1, ncols - 1 - p);
-      // left part: rows w .. f-1, columns p+1 .. w-1
-      update(m * (w - 1 - p), w * (f + 1), w, w - 1 - p);
-      inv_prev = inv;
-      __syncthreads();
-    }
-    if (w > 0) {
-      for (int i = w + slot; i < f; i += SLOTS) PE(i, w - 1) *= inv_prev;
-      __syncthreads();
-    }
+    // (the pivots' inverses where the slabs come later, if these have the room)
+    panel_lu<T, G>(P, w <= scap ? P + (size_t)pcap * G : nullptr, f, w, ncols, slot, l, SLOTS, &status[g * 32 + lane]);
     // The trailing block (and the carried right-hand side as its column m), S rows at a
     // time in shared memory after the panel: zeroed, given the children's entries that
     // fall in those rows (a child's rows map in increasing order, so they are one range
@@ -1306,28 +1395,27 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
           const ChildRef cr = L.child_ref[ci];
           const int mc = cr.m;
           const int* rel = L.relmap + cr.rel_ptr;
-          const int aw = first_at_least(rel, mc, w);
-          const int lo = first_at_least(rel, mc, w + a0), hi = first_at_least(rel, mc, w + a0 + sr);
-          const int rowlen = mc - aw, n = (hi - lo) * rowlen;
-          const T* src = cb + at32(g, L.sumcb, cr.cb_off, lane);
-          if (n > 0) {
-            const int si = SLOTS / rowlen, sj = SLOTS % rowlen;
-            int i = slot / rowlen, j = slot % rowlen;
-            for (int e0 = slot; e0 < n; e0 += 8 * SLOTS) {
-              int at[8];
-              T v[8], t[8];
+          const int lo = warp_first_at_least(rel, mc, w + a0), hi = warp_first_at_least(rel, mc, w + a0 + sr);
+          if (lo == hi) continue;  // (the same for the whole block)
+          const int aw = warp_first_at_least(rel, mc, w);
+          const CbView<T> from = cb_view(cb, L.sumcb, g, cr.cb_off, mc * mc, lane, L.sn_f[L.child_list[ci]] > kBigFront);
+          const T* src = from.p;
+          const int es = from.step;
+          for (int a = lo + warp; a < hi; a += 16) {
+            T* dst = Sb + ((rel[a] - w - a0) * mcols - w) * G;
+            const T* row = src + (size_t)a * mc * es;
+            for (int b0 = aw + cs; b0 < mc; b0 += 8 * CS) {
+              int c[8];
+              T v[8];
 #pragma unroll
               for (int u = 0; u < 8; ++u) {
-                const bool ok = e0 + u * SLOTS < n;
-                const int a = lo + (ok ? i : 0), b = aw + (ok ? j : 0);
-                at[u] = (rel[a] - w - a0) * mcols + (rel[b] - w);
-                v[u] = ok ? src[((size_t)a * mc + b) * 32] : (T)0;
-                t[u] = Sb[(size_t)at[u] * G];
-                next_task(i, j, si, sj, rowlen);
+                const int b = min(b0 + u * CS, mc - 1);
+                c[u] = rel[b] * G;
+                v[u] = row[(size_t)b * es];
               }
 #pragma unroll
               for (int u = 0; u < 8; ++u)
-                if (e0 + u * SLOTS < n) Sb[(size_t)at[u] * G] = t[u] + v[u];
+                if (b0 + u * CS < mc) dst[c[u]] += v[u];
             }
           }
           if (with_rhs)
@@ -1337,23 +1425,35 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
         }
         const int nta = (sr + 3) / 4, ntb = (bc + 3) / 4;
         for (int tt = slot; tt < nta * ntb; tt += SLOTS) {
-          const int ra = (tt / ntb) * 4, b0 = (tt % ntb) * 4;
+          // rows ra + ii, columns cb + jj ntb: a warp's tiles read adjacent columns (no bank
+          // conflicts); rows and columns past the end repeat the last one and are not stored
+          const int ra = (tt / ntb) * 4, cb = tt % ntb;
           T acc[4][4];
+          const T* lb[4];
+          const T* ub[4];
+          int at[4], to[4];
+#pragma unroll
+          for (int ii = 0; ii < 4; ++ii) {
+            const int r = min(ra + ii, sr - 1);
+            lb[ii] = P + ((size_t)w * (f + 1) + (size_t)(a0 + r) * w) * G + l;  // l of trailing row a0 + r
+            at[ii] = r * mcols;
+          }
+#pragma unroll
+          for (int jj = 0; jj < 4; ++jj) {
+            to[jj] = min(cb + jj * ntb, bc - 1);
+            ub[jj] = P + (size_t)(w + to[jj]) * G + l;  // u of column w + b (w + m: the right-hand side)
+          }
 #pragma unroll
           for (int ii = 0; ii < 4; ++ii)
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj)
-              acc[ii][jj] = (ra + ii < sr && b0 + jj < bc) ? Sb[((size_t)(ra + ii) * mcols + b0 + jj) * G] : (T)0;
-          // l of trailing rows a0 + ra + ii (left part, stride w); u of columns w + b0 + jj
-          // (top part; column w + m is the right-hand side f)
-          const T* lb = P + ((size_t)w * (f + 1) + (size_t)(a0 + ra) * w) * G + l;
-          const T* ub = P + (size_t)(w + b0) * G + l;
+            for (int jj = 0; jj < 4; ++jj) acc[ii][jj] = Sb[(size_t)(at[ii] + to[jj]) * G];
+#pragma unroll 2
           for (int p = 0; p < w; ++p) {
             T lv[4], uv[4];
 #pragma unroll
-            for (int ii = 0; ii < 4; ++ii) lv[ii] = ra + ii < sr ? lb[((size_t)ii * w + p) * G] : (T)0;
+            for (int ii = 0; ii < 4; ++ii) lv[ii] = lb[ii][p * G];
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) uv[jj] = b0 + jj < bc ? ub[((size_t)p * (f + 1) + jj) * G] : (T)0;
+            for (int jj = 0; jj < 4; ++jj) uv[jj] = ub[jj][p * (f + 1) * G];
 #pragma unroll
             for (int ii = 0; ii < 4; ++ii)
 #pragma unroll
@@ -1363,15 +1463,15 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
           for (int ii = 0; ii < 4; ++ii)
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj)
-              if (ra + ii < sr && b0 + jj < bc) Sb[((size_t)(ra + ii) * mcols + b0 + jj) * G] = acc[ii][jj];
+              if (ra + ii < sr && cb + jj * ntb < bc) Sb[(size_t)(at[ii] + to[jj]) * G] = acc[ii][jj];
         }
         __syncthreads();
         {
-          const int si = SLOTS / m, sj = SLOTS % m;
-          int i = slot / m, j = slot % m;
-          for (int e = slot; e < sr * m; e += SLOTS) {
-            CE(a0 + i, j) = Sb[((size_t)i * mcols + j) * G];
-            next_task(i, j, si, sj, m);
+          for (int i = warp; i < sr; i += 16) {
+            T* dst = own.p + (size_t)(a0 + i) * m * own.step;
+            const T* row = Sb + i * mcols * G;
+#pragma unroll 4
+            for (int j = cs; j < m; j += CS) dst[(size_t)j * own.step] = row[j * G];
           }
           if (with_rhs)
             for (int a = slot; a < sr; a += SLOTS) CR(a0 + a) = Sb[((size_t)a * mcols + m) * G];
@@ -1401,10 +1501,11 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big_gt(DevLU L, const int*
                                                        T* __restrict__ pan, T* __restrict__ cb,
                                                        T* __restrict__ cbr, T* __restrict__ x,
                                                        int* __restrict__ status,
-                                                       const int* __restrict__ group_active, int with_rhs) {
+                                                       const int* __restrict__ group_active, int with_rhs, int wcap) {
   constexpr int SLOTS = 512 / G, LPG = 32 / G;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* P = reinterpret_cast<T*>(smem_raw);
+  T* const pinv = reinterpret_cast<T*>(smem_raw);  // pivot inverses (wcap), then the panel
+  T* P = pinv + (size_t)wcap * G;
   const int slot = threadIdx.x / G, l = threadIdx.x % G;
   const int nch = ngroups * LPG;
   for (int q = blockIdx.x / nch, ch = blockIdx.x % nch; q < nsn_l;
@@ -1425,7 +1526,8 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big_gt(DevLU L, const int*
       return r < w ? P[((size_t)r * (f + 1) + c) * G + l] : P[((size_t)w * (f + 1) + (size_t)(r - w) * w + c) * G + l];
     };
     // trailing entry (a, b) of the contribution block, and the carried right-hand side
-    auto CE = [&](int a, int b) -> T& { return cb[at32(g, L.sumcb, cbo + (long long)a * m + b, lane)]; };
+    const CbView<T> own = cb_view(cb, L.sumcb, g, cbo, m * m, lane, has_parent && L.sn_f[L.sn_parent[s]] > kBigFront);
+    auto CE = [&](int a, int b) -> T& { return own.p[(size_t)(a * m + b) * own.step]; };
     auto CR = [&](int a) -> T& { return cbr[at32(g, L.sumcbr, cbro + a, lane)]; };
     const bool trail = has_parent && m > 0;
     for (int e = slot; e < npan; e += SLOTS) P[(size_t)e * G + l] = (T)0;
@@ -1458,7 +1560,9 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big_gt(DevLU L, const int*
       // entry e = a mc + b of the child's block; (a, b) advance by SLOTS without divisions
       const int sa = SLOTS / mc, sb = SLOTS % mc;
       int a = slot / mc, b = slot % mc;
-      const T* src = cb + at32(g, L.sumcb, cr.cb_off, lane);
+      const CbView<T> from = cb_view(cb, L.sumcb, g, cr.cb_off, mc * mc, lane, L.sn_f[L.child_list[ci]] > kBigFront);
+      const T* src = from.p;
+      const int es = from.step;
       for (int e0 = slot; e0 < mc * mc; e0 += B * SLOTS) {
         int r[B], c[B];
         T v[B], t[B];
@@ -1467,7 +1571,7 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big_gt(DevLU L, const int*
           const int e = e0 + u * SLOTS;
           r[u] = e < mc * mc ? rel[a] : 0;
           c[u] = e < mc * mc ? rel[b] : 0;
-          v[u] = e < mc * mc ? src[(size_t)e * 32] : (T)0;
+          v[u] = e < mc * mc ? src[(size_t)e * es] : (T)0;
           next_task(a, b, sa, sb, mc);
         }
 #pragma unroll
@@ -1489,61 +1593,7 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big_gt(DevLU L, const int*
         }
       __syncthreads();
     }
-    // LU of the panel, one pivot per barrier: rows p < i < w over columns p < j < ncols
-    // (top part) and rows i >= w over columns p < j < w (left part), each entry with
-    // the unscaled l_ip = F(i,p) / F(p,p) of its row; column p is scaled one pivot later
-    // (and after the loop for the last pivot), when no thread reads it any more
-    T inv_prev = (T)1;
-    for (int p = 0; p < w; ++p) {
-      T pk = PE(p, p);
-      if (bad_pivot(pk)) {
-        if (slot == 0) mark_singular(&status[g * 32 + lane]);
-        pk = (T)1;
-      }
-      const T inv = (T)1 / pk;
-      if (p > 0)
-        for (int i = p + slot; i < f; i += SLOTS) PE(i, p - 1) *= inv_prev;
-      // four entries per thread at a time, loads before stores: the updated entries
-      // (i > p, j > p) are distinct and none of them is in row p or column p, which the
-      // updates read
-      // rows of the part start at `base` (shared-memory index of column 0 of its first
-      // row, row stride rstride entries); entry e = i rowlen + j' of the part is row i,
-      // column p + 1 + j'; (i, j') advance by SLOTS without divisions
-      auto update = [&](int n, int base, int rstride, int rowlen) {
-        if (n <= 0) return;
-        const int si = SLOTS / rowlen, sj = SLOTS % rowlen;
-        int i = slot / rowlen, j = slot % rowlen;
-        const T* prow = P + ((size_t)p * (f + 1) + p + 1) * G + l;  // u_pj, j > p
-        for (int e0 = slot; e0 < n; e0 += 4 * SLOTS) {
-          int at[4], jc[4];
-          T lp[4], up[4], bv[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const bool ok = e0 + u * SLOTS < n;
-            const int row = base + (ok ? i : 0) * rstride;
-            at[u] = row + p + 1 + (ok ? j : 0);
-            jc[u] = ok ? j : 0;
-            lp[u] = P[(size_t)(row + p) * G + l];
-            up[u] = prow[(size_t)jc[u] * G];
-            bv[u] = P[(size_t)at[u] * G + l];
-            next_task(i, j, si, sj, rowlen);
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (e0 + u * SLOTS < n) P[(size_t)at[u] * G + l] = bv[u] - (lp[u] * inv) * up[u];
-        }
-      };
-      // top part: rows p+1 .. w-1, columns p+1 .. ncols-1
-      update((w - 1 - p) * (ncols - 1 - p), (p + 1) * (f + 1), f + 1, ncols - 1 - p);
-      // left part: rows w .. f-1, columns p+1 .. w-1
-      update(m * (w - 1 - p), w * (f + 1), w, w - 1 - p);
-      inv_prev = inv;
-      __syncthreads();
-    }
-    if (w > 0) {
-      for (int i = w + slot; i < f; i += SLOTS) PE(i, w - 1) *= inv_prev;
-      __syncthreads();
-    }
+    panel_lu<T, G>(P, pinv, f, w, ncols, slot, l, SLOTS, &status[g * 32 + lane]);
     // the Schur complement on the trailing block (and the carried right-hand side):
     // x - l_ip u_pj in pivot order
     if (trail) {
@@ -1869,7 +1919,7 @@ __global__ void k_acc_drain(unsigned long long* __restrict__ acc, double* __rest
 // [group][entry][32] <-> [case][entry] through a 32 x 32 tile in shared memory, so that both
 // sides move whole 128-byte lines (a thread per entry and case reads 16 of every 512 bytes).
 // Block (32, kTileRows): tile of 32 entries (blockIdx.x) of group blockIdx.y.  Gathering the
-// voltages of 1000 cases of 9241 buses: 69 -> 52 us (296 MB: 5.7 TB/s).
+// voltages of 1000 cases of 9241 buses: 69 -> 57 us (296 MB: 5.2 TB/s).
 constexpr int kTileRows = 8;
 inline dim3 tile_grid(int n, int ngroups) { return dim3((unsigned)((n + 31) / 32), (unsigned)ngroups); }
 

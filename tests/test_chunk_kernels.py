@@ -1,6 +1,7 @@
 """Kernels that keep a chunk of lanes on one block for a whole solve (kernels_chunk.cuh):
 their plan on the CPU, and on the GPU every lane count against the oracle at the sizes
-where a team, a chunk or a segment ends."""
+where a team, a chunk or a segment ends; and the two large-front kernels against each
+other."""
 import os
 import shutil
 import subprocess
@@ -75,3 +76,24 @@ def test_newton_chunks_match_oracle(gpu, monkeypatch, lanes, prec, n_bus, n_case
     for r in out[1:]:
         assert np.array_equal(r.v, out[0].v) and np.array_equal(r.iterations, out[0].iterations)
         assert np.array_equal(r.status, out[0].status) and np.array_equal(r.max_mis, out[0].max_mis)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", [m.FP64, m.MIXED])
+@pytest.mark.parametrize("n_bus,n_cases", [(900, 3), (1354, 35)])
+def test_large_front_kernels_agree(gpu, monkeypatch, prec, n_bus, n_cases):
+    """Trailing block in shared-memory slabs (kind 6) or in global memory (7): the same
+    panels, contribution blocks stored by lane pairs in either, bit for bit; against the
+    oracle at the parity tests' bar (both to max |F| < 1e-11)."""
+    buses, branches = m.synth_grid(n_bus, int(1.47 * n_bus), n_bus // 5, 0.1, seed=5, topology=1)
+    n1 = np.flatnonzero(~m.find_bridges(branches, n_bus))
+    cases = [[]] + [[int(b)] for b in n1[:n_cases - 1]]
+    ref = oracle.runpf(buses, branches, cases[:4], alg=m.NR, tol=1e-11)
+    out = []
+    for kind in ("6", "7"):
+        monkeypatch.setenv("MPF_FACTOR_KIND", kind)
+        with m.PowerFlow(buses, branches, tol=1e-11) as pf:
+            out.append(pf.runpf(cases, alg=m.NR, precision=prec))
+    assert out[0].converged.all()
+    assert np.array_equal(out[0].v, out[1].v) and np.array_equal(out[0].iterations, out[1].iterations)
+    assert np.abs(out[0].v[:len(ref["v"])] - ref["v"]).max() < 1e-8
