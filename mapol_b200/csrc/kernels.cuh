@@ -208,13 +208,9 @@ __device__ __forceinline__ double2 ycase(const DevGrid& d, const LaneOut& o, int
   return y;
 }
 
-// Ybus entry p of this case: ycase() on rows an outage touches, plus the change a
-// per-case control (tap or shunt susceptance) makes at p.
-// CTL = false compiles the correction out (kernels whose register budget is tight
-// have a variant per case; the others pass true and test d.y_slot).
-template <bool CTL = true>
-__device__ __forceinline__ double2 yentry(const DevGrid& d, const LaneOut& o, bool touched, int p, int g, int lane) {
-  double2 y = touched ? ycase(d, o, p, d.y_val[p]) : d.y_val[p];
+// y plus the change a per-case control (tap or shunt susceptance) makes at Ybus entry p
+template <bool CTL>
+__device__ __forceinline__ double2 yctl(const DevGrid& d, double2 y, int p, int g, int lane) {
   if (CTL && d.y_slot) {
     const int s = d.y_slot[p];
     if (s >= 0) {
@@ -224,6 +220,15 @@ __device__ __forceinline__ double2 yentry(const DevGrid& d, const LaneOut& o, bo
     }
   }
   return y;
+}
+
+// Ybus entry p of this case: ycase() on rows an outage touches, plus the change a
+// per-case control (tap or shunt susceptance) makes at p.
+// CTL = false compiles the correction out (kernels whose register budget is tight
+// have a variant per case; the others pass true and test d.y_slot).
+template <bool CTL = true>
+__device__ __forceinline__ double2 yentry(const DevGrid& d, const LaneOut& o, bool touched, int p, int g, int lane) {
+  return yctl<CTL>(d, touched ? ycase(d, o, p, d.y_val[p]) : d.y_val[p], p, g, lane);
 }
 
 // Branch k's four admittances (ff, ft, tf, tt) in this case: the base values, or the
@@ -325,7 +330,6 @@ __global__ void k_check(DevGrid d, int it_arg, int max_it, double tol) {
 // ---------------------------------------------------------------- Newton mismatch
 // grid (row blocks, groups); 8 warps per block; a warp = one bus row x 32 cases.
 constexpr int kRowsPerBlock = 64;
-constexpr int kYB = 2;  // Ybus entries per batch of loads in the mismatch row pass
 
 // With JAC, the same warp then writes the Jacobian entries of its row, reusing the
 // row's admittances, voltages and Ibus; the Jacobian of a case that converges on
@@ -378,76 +382,180 @@ __device__ __forceinline__ void jac_entry(const DevGrid& d, double* A, int g, in
   }
 }
 
+// J entries of an off-diagonal Ybus entry: the formulas above with I = 0, where dP/dVm and
+// dQ/dVm are -dQ/dVa and dP/dVa over |V_j|.  Ag: this lane's entry 0 of its group's J; jp.x is
+// there whenever any of the four is (a free bus has its Va).
+__device__ __forceinline__ float inv_abs(float c, float d) { return rsqrtf(c * c + d * d); }
+__device__ __forceinline__ double inv_abs(double c, double d) { return rsqrt(c * c + d * d); }
+template <typename T>
+__device__ __forceinline__ void jac_off(T* Ag, int4 jp, T yr, T yi, T c, T d, T a, T b, bool qrow_off, bool vmcol_off) {
+  const T yvr = yr * c - yi * d, yvi = yr * d + yi * c;
+  const T pa = b * yvr - a * yvi, qa = -b * yvi - a * yvr;
+  Ag[(long long)jp.x * 32] = pa;
+  if (jp.z >= 0) Ag[(long long)jp.z * 32] = qrow_off ? (T)0 : qa;
+  if (jp.y >= 0 || jp.w >= 0) {
+    const T inv = inv_abs(c, d);
+    if (jp.y >= 0) Ag[(long long)jp.y * 32] = vmcol_off ? (T)0 : -qa * inv;
+    if (jp.w >= 0) Ag[(long long)jp.w * 32] = qrow_off || vmcol_off ? (T)0 : pa * inv;
+  }
+}
+
+// What a block's rows share among their cases, staged in shared memory before the rows are
+// walked: per row its bus, Ybus range, place here, diagonal and variables; per Ybus entry its
+// column, base value and Jacobian positions.  The kernel issued 190 instructions per entry and
+// 32 cases (address arithmetic, loads of these arrays, the outages' registers spilled) and a
+// row was a chain of loads (row -> range -> column -> voltage -> Jacobian positions).  Staged
+// by four threads per row the chain is walked once per block; a row waits for its voltages
+// alone, asked for one entry ahead, and an off-diagonal entry's four J values come from two
+// products.  With the Jacobian, 1000 cases of 9241 buses, mixed: 425 -> 329 us (0.87 GB, 2.6
+// TB/s; still bound by issue, at 24 warps per SM: 80 registers without spills beat 64 with
+// them, 338); 256 of 2869, FP64: 72 -> 51.  Batches of 2 or 4 entries per round: 365 and 367.
+// kMisEntries: 64 rows of 7 entries, more than a block of a transmission grid has (4 to 5 per
+// row); a row that finds no room here, and all behind it, is read from global memory.
+constexpr int kMisEntries = 448;
+struct __align__(16) MisEntry {
+  int4 jp;
+  double2 y;
+  int col;
+};
+struct MisStage {
+  int4 row[kRowsPerBlock];  // bus (-1: not in this group's island), first Ybus entry, entries, place in e
+  int4 aux[kRowsPerBlock];  // diagonal's Ybus entry, jvar.x, jvar.y
+  int warp_sum[2];
+  MisEntry e[kMisEntries];
+};
+
+// Fills S for rows [r0, r0 + kRowsPerBlock) of mis_rows; every thread of the block calls it
+template <bool JAC>
+__device__ __forceinline__ void stage_rows(const DevGrid& d, MisStage& S, int r0, int g) {
+  static_assert(kRowsPerBlock == 64, "two warps hold a row per thread, four threads copy a row");
+  const int tid = threadIdx.x, lane = tid & 31;
+  int4 row = make_int4(-1, 0, 0, 0);
+  int upto = 0;
+  if (tid < kRowsPerBlock) {
+    if (r0 + tid < d.nfree) {
+      const int i = d.mis_rows[r0 + tid];
+      if (row_here(d, i, g)) {
+        const int p0 = d.y_rowptr[i];
+        const int2 jv = d.jvar[i];
+        row = make_int4(i, p0, d.y_rowptr[i + 1] - p0, 0);
+        S.aux[tid] = make_int4(d.y_diag[i], jv.x, jv.y, 0);
+      }
+    }
+    upto = row.z;
+#pragma unroll
+    for (int s = 1; s < 32; s *= 2) {
+      const int o = __shfl_up_sync(0xffffffffu, upto, s);
+      if (lane >= s) upto += o;
+    }
+    if (lane == 31) S.warp_sum[tid >> 5] = upto;
+  }
+  __syncthreads();
+  if (tid < kRowsPerBlock) {
+    row.w = upto - row.z + (tid >= 32 ? S.warp_sum[0] : 0);
+    S.row[tid] = row;
+  }
+  __syncthreads();
+  const int4 q = S.row[tid >> 2];
+  if (q.w + q.z <= kMisEntries)
+    for (int k = tid & 3; k < q.z; k += 4) {
+      MisEntry& e = S.e[q.w + k];
+      e.col = d.y_col[q.y + k];
+      e.y = d.y_val[q.y + k];
+      if (JAC) e.jp = d.jpos[q.y + k];
+    }
+  __syncthreads();
+}
+
 // One pass over the row: the off-diagonal J entries need no Ibus and are written
 // while Ibus accumulates; the diagonal entry follows once Ibus is complete.
 template <typename T, bool JAC, bool CTL, bool QL>
-__global__ void __launch_bounds__(256, 4) k_mismatch_nr(DevGrid d, T* x, T* A) {
+__global__ void __launch_bounds__(256, 3) k_mismatch_nr(DevGrid d, T* x, T* A) {
+  __shared__ MisStage S;
   const int g = blockIdx.y;
   if (!d.group_active[g]) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = g * 32 + lane;
-  LaneOut o;
-  load_outages(d, c, o);
+  stage_rows<JAC>(d, S, blockIdx.x * kRowsPerBlock, g);
+  // which of this warp's rows the lane's outages touch (bit r / 8); the outages themselves
+  // are read again where they are needed, their twelve registers are not there
+  unsigned touches = 0;
+  {
+    LaneOut o;
+    load_outages(d, c, o);
+#pragma unroll
+    for (int r = 0; r < kRowsPerBlock / 8; ++r)
+      if (S.row[warp + 8 * r].x >= 0 && row_touched(o, S.aux[warp + 8 * r].x)) touches |= 1u << r;
+  }
   double lmax = 0.0;
-  const int r1 = min(d.nfree, (blockIdx.x + 1) * kRowsPerBlock);
-  for (int r = blockIdx.x * kRowsPerBlock + warp; r < r1; r += 8) {
-    const int i = d.mis_rows[r];
-    if (!row_here(d, i, g)) continue;
-    double2 ib = make_double2(0.0, 0.0);
-    const int p0 = d.y_rowptr[i], p1 = d.y_rowptr[i + 1];
-    const bool touched = row_touched(o, d.y_diag[i]);
-    const double2 vi = d.V[at32(g, d.nb, i, lane)];
+  const double2* const Vg = d.V + at32(g, d.nb, 0, lane);
+  T* const Ag = JAC ? A + at32(g, d.nA_jac, 0, lane) : nullptr;
+  T* const xg = x + at32(g, d.n_jac, 0, lane);
+  for (int r = warp; r < kRowsPerBlock; r += 8) {
+    const int4 row = S.row[r], aux = S.aux[r];
+    const int i = row.x, n = row.z;
+    if (i < 0) continue;
+    const bool touched = touches >> (r >> 3) & 1u;
+    auto ybus = [&](int p, double2 base) {
+      if (touched) {
+        LaneOut o;
+#pragma unroll
+        for (int q = 0; q < kMaxOut; ++q) o.e[q] = d.out_br[q * d.ngroups * 32 + c];
+        base = ycase(d, o, p, base);
+      }
+      return yctl<CTL>(d, base, p, g, lane);
+    };
+    const double2 vi = Vg[(long long)i * 32];
+    double2 s = d.sbus_case ? d.sbus_case[at32(g, d.nb, i, lane)] : d.sbus0[i];
     const bool pvi = QL && still_pv(d, i, g, lane);
-    // kYB entries at a time: their column indices, then their voltages, are loaded
-    // before any of them is used, so the row's chain of dependent loads is one round
-    // trip per kYB entries (padding entries point at the diagonal and load nothing);
-    // Ibus accumulates in the row's order as before
-    for (int p = p0; p < p1; p += kYB) {
-      int jj[kYB];
-      double2 vv[kYB];
-#pragma unroll
-      for (int u = 0; u < kYB; ++u) jj[u] = p + u < p1 ? d.y_col[p + u] : i;
-#pragma unroll
-      for (int u = 0; u < kYB; ++u) vv[u] = jj[u] == i ? vi : d.V[at32(g, d.nb, jj[u], lane)];
-#pragma unroll
-      for (int u = 0; u < kYB; ++u) {
-        if (p + u >= p1) break;
-        const int j = jj[u];
-        const double2 y = yentry<CTL>(d, o, touched, p + u, g, lane);
-        const double2 v = vv[u];
+    // e(k): the row's entry k
+    auto row_pass = [&](auto e) {
+      double2 ib = make_double2(0.0, 0.0);
+      double2 vn = Vg[(long long)e(0).col * 32];  // the next entry's voltage, one entry ahead
+#pragma unroll 1
+      for (int k = 0; k < n; ++k) {
+        const MisEntry q = e(k);
+        const double2 v = vn;
+        if (k + 1 < n) vn = Vg[(long long)e(k + 1).col * 32];
+        const double2 y = ybus(row.y + k, q.y);
         ib.x += y.x * v.x - y.y * v.y;
         ib.y += y.x * v.y + y.y * v.x;
-        if (JAC && j != i) {
-          const int4 jp = d.jpos[p + u];
-          if (jp.x >= 0 || jp.y >= 0 || jp.z >= 0 || jp.w >= 0)
-            jac_entry(d, A, g, lane, jp, y, v, vi.x, vi.y, 0.0, 0.0, pvi, QL && still_pv(d, j, g, lane));
-        }
+        if (JAC && q.jp.x >= 0 && q.col != i)
+          jac_off<T>(Ag, q.jp, (T)y.x, (T)y.y, (T)v.x, (T)v.y, (T)vi.x, (T)vi.y, pvi, QL && still_pv(d, q.col, g, lane));
       }
-    }
-    double2 s = d.sbus_case ? d.sbus_case[at32(g, d.nb, i, lane)] : d.sbus0[i];
-    if (QL && !pvi && d.sw_index[i] >= 0) s.y = d.q_fix[at32(g, d.nsw, d.sw_index[i], lane)];
-    // mis = V conj(Ibus) - S
-    const double mr = vi.x * ib.x + vi.y * ib.y - s.x;
-    const double mi = vi.y * ib.x - vi.x * ib.y - s.y;
-    const int2 jv = d.jvar[i];
-    x[at32(g, d.n_jac, jv.x, lane)] = (T)mr;
-    double m = fabs(mr);
-    if (jv.y >= 0 && pvi) {
-      x[at32(g, d.n_jac, jv.y, lane)] = (T)0;  // Q of a PV bus is free: its row asks dVm = 0
-    } else if (jv.y >= 0) {
-      x[at32(g, d.n_jac, jv.y, lane)] = (T)mi;
-      m = fmax(m, fabs(mi));
-      if (mi != mi) m = INFINITY;
-    }
-    if (mr != mr) m = INFINITY;
-    lmax = fmax(lmax, finite_or_inf(m));
-    if (JAC) {
-      const int pd = d.y_diag[i];
-      const int4 jp = d.jpos[pd];
-      jac_entry(d, A, g, lane, jp, yentry<CTL>(d, o, touched, pd, g, lane), vi, vi.x, vi.y, ib.x, ib.y, pvi, pvi,
-                   true);
+      if (QL && !pvi && d.sw_index[i] >= 0) s.y = d.q_fix[at32(g, d.nsw, d.sw_index[i], lane)];
+      // mis = V conj(Ibus) - S
+      const double mr = vi.x * ib.x + vi.y * ib.y - s.x;
+      const double mi = vi.y * ib.x - vi.x * ib.y - s.y;
+      const int2 jv = make_int2(aux.y, aux.z);
+      xg[(long long)jv.x * 32] = (T)mr;
+      double m = fabs(mr);
+      if (jv.y >= 0 && pvi) {
+        xg[(long long)jv.y * 32] = (T)0;  // Q of a PV bus is free: its row asks dVm = 0
+      } else if (jv.y >= 0) {
+        xg[(long long)jv.y * 32] = (T)mi;
+        m = fmax(m, fabs(mi));
+        if (mi != mi) m = INFINITY;
+      }
+      if (mr != mr) m = INFINITY;
+      lmax = fmax(lmax, finite_or_inf(m));
+      if (JAC) {
+        const MisEntry q = e(aux.x - row.y);
+        jac_entry(d, A, g, lane, q.jp, ybus(aux.x, q.y), vi, vi.x, vi.y, ib.x, ib.y, pvi, pvi, true);
+      } else {
+        d.Ibus[at32(g, d.nb, i, lane)] = ib;
+      }
+    };
+    if (row.w + n <= kMisEntries) {
+      row_pass([&](int k) -> const MisEntry& { return S.e[row.w + k]; });
     } else {
-      d.Ibus[at32(g, d.nb, i, lane)] = ib;
+      row_pass([&](int k) {
+        MisEntry q;
+        q.col = d.y_col[row.y + k];
+        q.y = d.y_val[row.y + k];
+        q.jp = d.jpos[row.y + k];
+        return q;
+      });
     }
   }
   block_lane_max(lmax, &d.facc[c], d.status[c] == ST_RUNNING);

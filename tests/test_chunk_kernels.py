@@ -1,7 +1,7 @@
 """Kernels that keep a chunk of lanes on one block for a whole solve (kernels_chunk.cuh):
 their plan on the CPU, and on the GPU every lane count against the oracle at the sizes
-where a team, a chunk or a segment ends; and the two large-front kernels against each
-other."""
+where a team, a chunk or a segment ends; the two large-front kernels against each other;
+and the mismatch pass where its staged rows run out of room."""
 import os
 import shutil
 import subprocess
@@ -97,3 +97,20 @@ def test_large_front_kernels_agree(gpu, monkeypatch, prec, n_bus, n_cases):
     assert out[0].converged.all()
     assert np.array_equal(out[0].v, out[1].v) and np.array_equal(out[0].iterations, out[1].iterations)
     assert np.abs(out[0].v[:len(ref["v"])] - ref["v"]).max() < 1e-8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", [m.FP64, m.MIXED])
+@pytest.mark.parametrize("n_bus,per_bus", [(64, 1.5), (65, 3.2), (130, 6.0)])
+def test_mismatch_rows_beyond_the_staged(gpu, prec, n_bus, per_bus):
+    """64 rows of fewer than 7 Ybus entries are staged, denser blocks only in part; one row
+    more than a block.  autotune=0: the row kernel runs, not the whole-solve one.  Same bar
+    as the parity tests (both to max |F| < 1e-11)."""
+    buses, branches = m.synth_grid(n_bus, int(per_bus * n_bus), n_bus // 5, 0.1, seed=7, topology=1)
+    n1 = np.flatnonzero(~m.find_bridges(branches, n_bus))
+    cases = [[]] + [[int(b)] for b in n1[:5]] + [[int(n1[5]), int(n1[7])]]
+    ref = oracle.runpf(buses, branches, cases, alg=m.NR, tol=1e-11)
+    with m.PowerFlow(buses, branches, tol=1e-11, autotune=0) as pf:
+        res = pf.runpf(cases, alg=m.NR, precision=prec)
+    assert res.converged.all() and ref["converged"].all()
+    assert np.abs(res.v - ref["v"]).max() < 1e-8
