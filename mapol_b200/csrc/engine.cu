@@ -258,7 +258,7 @@ struct LUSystem {
   std::map<std::pair<int, int>, std::vector<FactorChoice>> tuned;
   // autotuned lane count of every backward-solve level launch (0 = one case per thread)
   std::map<std::pair<int, int>, std::vector<int>> tuned_bs;
-  std::vector<Launch> level_sched;   // one launch per level (adjoint solves of full FP64 batches), ascending
+  std::vector<Launch> level_sched;   // one launch per level (adjoint solves of full batches), ascending
   std::vector<int> ah_host, ah_loc_host;  // host copies of ah_ptr and ah_loc
   int nA = 0;
   // values per precision [0] = FP64, [1] = FP32
@@ -1992,20 +1992,26 @@ void launch_bsolve_t(const LUSystem& sys, int ngroups, const T* pan, T* x, const
 }
 
 // x <- (L U)^-T x for every lane: a block per chunk of lanes (k_subst_chunk), or for full
-// batches of plain FP64 whose x does not fit in shared memory a launch per level with a
-// case per thread.  1354 buses, whole adjoint, ms, level launches / chunks: FP64 4096 cases
-// 3.5 / 3.9, FP32 factors 4096 cases 6.2 / 5.2; 300 cases of 2869 buses 9.2 / 4.0, of 9241
-// buses 19.4 / 7.9; 500 of 300 buses 1.47 / 0.52.
-constexpr int kLevelSubstGroups = 64;
+// batches a launch per level with a case per thread.  The chunks save the levels' latency, but
+// they fill the GPU: level launches leave room for another handle's solve beside them, and
+// their fixed cost is spread over more cases.  ms per solve + adjoint, three handles in turn
+// (one alone), level launches / chunks:
+//   1354 buses, 4096 cases, FP32 11.0 (14.4) / 12.5 (13.2), FP64 12.5 (14.1) / 13.9 (14.4)
+//   700 x 4096 FP32 6.8 (9.1) / 8.5 (9.4);  300 x 4096 FP32 3.7 (5.1) / 3.6 (4.0)
+//   1354 x 2048 FP32 7.6 (10.8) / 7.8 (8.6), FP64 7.5 (9.0) / 8.0 (8.6);  2869 x 1000 FP32
+//   10.8 (18.7) / 11.3 (12.6);  2869 x 300 7.8 (15.4) / 7.6 (9.9);  300 x 1024 1.6 (2.6) / 1.2 (1.6)
+constexpr int kLevelSubstGroups = 128;             // groups of 32 lanes, twice in FP64
+constexpr long long kLevelSubstEntries = 1800000;  // and their LU entries
 template <typename T>
 void launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, const int* group_active, int device,
                     cudaStream_t st) {
-  const ChunkShape sh = choose_chunk({&S}, Prec<T>::G, sizeof(T), ngroups, 2);
-  if (sizeof(T) == 8 && !sh.xs && ngroups >= kLevelSubstGroups) {
+  const int words = ngroups * (int)sizeof(T) / 4;
+  if (!std::getenv("MPF_CHUNK_LANES") && words >= kLevelSubstGroups && words * S.sym.nnz >= kLevelSubstEntries) {
     launch_fsolve_t<T>(S, ngroups, pan, cbr, x, group_active, st);
     launch_bsolve_t<T>(S, ngroups, pan, x, group_active, st);
     return;
   }
+  const ChunkShape sh = choose_chunk({&S}, Prec<T>::G, sizeof(T), ngroups, 2);
   with_shape<T>(sh, [&](auto g, auto xs) {
     constexpr int G = decltype(g)::value;
     constexpr bool XS = decltype(xs)::value;
