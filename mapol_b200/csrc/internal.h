@@ -8,7 +8,20 @@
 
 #include "mpf.h"
 
+#ifdef __CUDACC__
+#define MPF_HD __host__ __device__
+#else
+#define MPF_HD
+#endif
+
 namespace mpf {
+
+// A block of len entries stored in lane pairs ([16 pairs][len][2 lanes], contribution blocks
+// between two large fronts): the values that hold lanes lane .. lane + G - 1 (lane a multiple of
+// G) are the pair_values(len, G) from pair_first(len, lane) on.  One lane's values lie among
+// its pair's.
+MPF_HD inline long long pair_first(long long len, int lane) { return (lane >> 1) * len * 2; }
+MPF_HD inline long long pair_values(long long len, int G) { return len * (G > 2 ? G : 2); }
 
 uint64_t splitmix64(uint64_t& x);
 

@@ -27,6 +27,8 @@
 
 #include <cuda_runtime.h>
 
+#include "internal.h"
+
 namespace mpfk {
 
 constexpr int kMaxOut = 4;  // outaged branches per case
@@ -1262,7 +1264,7 @@ struct CbView {
 template <typename T>
 __device__ __forceinline__ CbView<T> cb_view(T* cb, long long sumcb, int g, long long off, int len, int lane, bool paired) {
   T* base = cb + at32(g, sumcb, off, 0);
-  if (paired) return CbView<T>{base + (size_t)(lane >> 1) * len * 2 + (lane & 1), 2};
+  if (paired) return CbView<T>{base + mpf::pair_first(len, lane) + (lane & 1), 2};
   return CbView<T>{base + lane, 32};
 }
 
@@ -1412,9 +1414,11 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
       for (int ci = L.child_ptr[s]; ci < L.child_ptr[s + 1]; ++ci) {
         if (L.sn_f[L.child_list[ci]] <= kBigFront) continue;
         const ChildRef cr = L.child_ref[ci];
-        const CbView<T> from = cb_view(cb, L.sumcb, g, cr.cb_off, cr.m * cr.m, (ch % LPG) * G, true);
-        const size_t a0 = (size_t)from.p & ~(size_t)15;
-        const size_t a1 = ((size_t)(from.p + (size_t)cr.m * cr.m * (G > 2 ? G : 2)) + 15) & ~(size_t)15;
+        // (whole pairs: blocks start on 128 bytes, so the rounding to 16 stays inside)
+        const long long len = (long long)cr.m * cr.m;
+        const T* from = cb + at32(g, L.sumcb, cr.cb_off, 0) + mpf::pair_first(len, (ch % LPG) * G);
+        const size_t a0 = (size_t)from & ~(size_t)15;
+        const size_t a1 = ((size_t)(from + mpf::pair_values(len, G)) + 15) & ~(size_t)15;
         prefetch_l2(reinterpret_cast<const void*>(a0), (unsigned)(a1 - a0));
       }
     for (int e = slot; e < npan; e += SLOTS) P[(size_t)e * G + l] = (T)0;
