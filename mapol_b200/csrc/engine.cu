@@ -234,7 +234,8 @@ struct LUSystem {
   DevBuf sn_w, sn_f, sn_rptr, sn_rows, child_ptr, child_list, sn_parent, rel_ptr, relmap, ah_ptr, ah_loc;
   DevBuf pan_off, cb_off, cbr_off, lev_sn, child_ref, cb_in;
   DevBuf sn_island;                  // multi-island handles only
-  std::vector<int> h_sn_island;      // the same on the host (empty: one island)
+  std::vector<int> h_sn_island;      // the same on the host
+  int n_islands = 1;
   // sweep plans by (compact, lanes, value bytes, kilobytes per ring slot)
   std::map<std::tuple<bool, int, int, int>, std::unique_ptr<PlanBufs>> plans;
   // factorisation plans by (lanes, value bytes, kilobytes of shared memory)
@@ -297,9 +298,10 @@ struct LUSystem {
   // var_island (multi-island handles): island of each variable; a supernode's
   // variables all belong to one island (the matrix is block-diagonal by island)
   void setup(const LUSymbolic& s, const std::vector<int>& ahp, const std::vector<int>& ahl, int nA_,
-             const std::vector<int>* var_island = nullptr) {
+             int n_islands_ = 1, const std::vector<int>* var_island = nullptr) {
     sym = s;
     nA = nA_;
+    n_islands = n_islands_;
     if (var_island) {
       std::vector<int> si(s.nsn);
       for (int k = 0; k < s.nsn; ++k) {
@@ -477,7 +479,7 @@ struct LUSystem {
     if (it != plans.end()) return it->second.get();
     SweepPlan p;
     const bool ok = slot_kb > 0 && build_sweep_plan(sym, h_sn_island, compact, G, wsize, (size_t)slot_kb * 1024,
-                                                    kChunkScratch, p);
+                                                    kChunkScratch, p, n_islands);
     auto& slot = plans[key];
     if (ok) {
       slot = std::make_unique<PlanBufs>();
@@ -503,7 +505,7 @@ struct LUSystem {
     FactorPlan p;
     bool ok = false;
     // the largest ring slots that leave room for the rest
-    for (size_t slot = 24 * 1024; !ok && slot >= 3 * 1024 && h_sn_island.empty(); slot = slot * 2 / 3 / 16 * 16)
+    for (size_t slot = 24 * 1024; !ok && slot >= 3 * 1024 && n_islands == 1; slot = slot * 2 / 3 / 16 * 16)
       ok = (size_t)kb * 1024 > kRingSlots * slot &&
            build_factor_plan(sym, ah_host, ah_loc_host, G, wsize, slot, (size_t)kb * 1024 - kRingSlots * slot, p);
     auto& out = fplans[key];
@@ -1745,7 +1747,7 @@ void upload_newton(mpf_handle* h) {
       if (g.var_va[i] >= 0) vi[g.var_va[i]] = g.bus_island[i];
       if (g.var_vm[i] >= 0) vi[g.var_vm[i]] = g.bus_island[i];
     }
-    h->jac.setup(g.jac, g.ah_ptr, g.ah_loc, g.nnz_jac, &vi);
+    h->jac.setup(g.jac, g.ah_ptr, g.ah_loc, g.nnz_jac, g.n_islands, &vi);
   } else {
     h->jac.setup(g.jac, g.ah_ptr, g.ah_loc, g.nnz_jac);
   }
@@ -1779,7 +1781,7 @@ void upload_fd(mpf_handle* h, int variant) {
       for (int i = 0; i < g.nb; ++i)
         if (fs.var[i] >= 0) vi[fs.var[i]] = g.bus_island[i];
     }
-    sys.setup(fs.lu, fs.ah_ptr, fs.ah_loc, (int)fs.base.size(), g.n_islands > 1 ? &vi : nullptr);
+    sys.setup(fs.lu, fs.ah_ptr, fs.ah_loc, (int)fs.base.size(), std::max(g.n_islands, 1), g.n_islands > 1 ? &vi : nullptr);
     sys.group_island = h->jac.group_island;
     upload(fd.base, fs.base);
     std::vector<int4> pos(g.nbr);
@@ -2062,7 +2064,7 @@ constexpr long long kNrChunkEntries = 50000;
 template <typename T>
 NrShape choose_nr(LUSystem& S, int ngroups) {
   NrShape sh, best;
-  if (!S.h_sn_island.empty()) return best;
+  if (S.n_islands > 1) return best;
   for (const char* e : {"MPF_FACTOR_KIND", "MPF_BSOLVE_LANES", "MPF_BSOLVE_TOP"})
     if (std::getenv(e)) return best;  // testing: a level kernel is forced
   if (const char* e = std::getenv("MPF_NR_CHUNK")) {  // testing: 0 off, else the lanes per block

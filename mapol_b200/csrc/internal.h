@@ -166,8 +166,8 @@ inline bool solo_task(int w, int f) { return w <= kSoloPivots && f <= kSoloFront
 // carried entries that front row i adds, two per layer, children in order (-1: none).
 struct SweepPlan {
   std::vector<SweepStep> step;
-  std::vector<int> step_ptr;   // steps of each island
-  std::vector<int> down_ptr;   // of them, the first root-to-leaves step
+  std::vector<int> step_ptr;   // [islands + 1]: steps of each island (none where it has no supernode)
+  std::vector<int> down_ptr;   // [islands]: of them, the first root-to-leaves step
   std::vector<int> idx;
   int peak_cb = 0;             // carried entries alive at once (most over the islands)
   size_t scratch = 0;          // values per lane of shared memory the teams need
@@ -207,11 +207,13 @@ struct FactorPlan {
 bool build_factor_plan(const LUSymbolic& s, const std::vector<int>& ah_ptr, const std::vector<int>& ah_loc, int G,
                        int wsize, size_t slot, size_t smem, FactorPlan& out);
 
+// sn_island: each supernode's island (empty: one island); n_islands: how many there are, also
+// those without a supernode (0: as many as sn_island names).
 // compact_cb: carried entries get slots that are reused once the parent has read them (else
 // their storage in cbr).  G lanes of wsize-byte values; slot: most bytes of a step; scratch:
 // bytes for the teams' fronts.  False when a front does not fit the scratch.
 bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bool compact_cb, int G, int wsize,
-                      size_t slot, size_t scratch, SweepPlan& out);
+                      size_t slot, size_t scratch, SweepPlan& out, int n_islands = 0);
 
 // Everything that does not depend on the case batch.
 struct GridSymbolic {

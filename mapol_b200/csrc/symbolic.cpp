@@ -884,10 +884,13 @@ std::string build_symbolic(const mpf_bus* buses, int nb, const mpf_branch* br, i
 
 // ------------------------------------------------------------------ block plans
 bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bool compact_cb, int G, int wsize,
-                      size_t slot, size_t scratch, SweepPlan& out) {
+                      size_t slot, size_t scratch, SweepPlan& out, int n_islands) {
   out = SweepPlan();
   if (s.nnz >= INT_MAX) return false;
-  const int nisl = sn_island.empty() ? 1 : 1 + *std::max_element(sn_island.begin(), sn_island.end());
+  // an island without variables in this system (a slack bus alone; in B'', a grid whose other
+  // buses are all PV) has no supernode, but the kernels look its range of steps up
+  int nisl = std::max(n_islands, 1);
+  for (int k : sn_island) nisl = std::max(nisl, k + 1);
   std::vector<std::vector<int>> of_island(nisl);
   for (int n = 0; n < s.nsn; ++n) of_island[sn_island.empty() ? 0 : sn_island[n]].push_back(n);
   std::vector<int> cb(s.nsn, -1);
@@ -938,6 +941,7 @@ bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bo
       }
       free_list = merged;
     }
+    if (nlev == 0) out.down_ptr.push_back((int)out.step.size());
     for (int q = 0; q < 2 * nlev; ++q) {
       const bool up = q < nlev;
       if (q == nlev) out.down_ptr.push_back((int)out.step.size());

@@ -25,3 +25,7 @@ def run_native(tmp_path, name):
 
 def test_lane_pair_ranges_stay_inside_their_block(tmp_path):
     assert int(run_native(tmp_path, "lane_pairs_check").split()[1]) == 2 * 24 * (32 + 16 + 8)
+
+
+def test_islands_without_supernodes_have_their_step_range(tmp_path):
+    assert int(run_native(tmp_path, "island_plan_check").split()[1]) == 5 * 5 * 2
