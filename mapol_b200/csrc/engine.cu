@@ -237,9 +237,9 @@ struct LUSystem {
   std::vector<int> h_sn_island;      // the same on the host
   int n_islands = 1;
   // sweep plans by (compact, lanes, value bytes, kilobytes per ring slot)
-  std::map<std::tuple<bool, int, int, int>, std::unique_ptr<PlanBufs>> plans;
+  PlanCache<std::tuple<bool, int, int, int>, PlanBufs> plans;
   // factorisation plans by (lanes, value bytes, kilobytes of shared memory)
-  std::map<std::tuple<int, int, int>, std::unique_ptr<FactorBufs>> fplans;
+  PlanCache<std::tuple<int, int, int>, FactorBufs> fplans;
   const int* group_island = nullptr; // the handle's current per-group islands (or null)
   std::vector<Launch> factor_sched;  // ascending levels
   std::vector<LaunchDeps> factor_deps;
@@ -474,54 +474,46 @@ struct LUSystem {
   // The sweep plan for blocks of G lanes of wsize-byte values with ring slots of slot_kb KB,
   // kept on the device; null when a front does not fit the scratch
   const PlanBufs* plan(bool compact, int G, int wsize, int slot_kb) {
-    const auto key = std::make_tuple(compact, G, wsize, slot_kb);
-    auto it = plans.find(key);
-    if (it != plans.end()) return it->second.get();
-    SweepPlan p;
-    const bool ok = slot_kb > 0 && build_sweep_plan(sym, h_sn_island, compact, G, wsize, (size_t)slot_kb * 1024,
-                                                    kChunkScratch, p, n_islands);
-    auto& slot = plans[key];
-    if (ok) {
-      slot = std::make_unique<PlanBufs>();
+    return plans.get(std::make_tuple(compact, G, wsize, slot_kb), [&](PlanBufs& out) {
+      SweepPlan p;
+      if (slot_kb <= 0 || !build_sweep_plan(sym, h_sn_island, compact, G, wsize, (size_t)slot_kb * 1024, kChunkScratch, p,
+                                            n_islands))
+        return false;
       std::vector<int4> st(p.step.size());
       for (size_t k = 0; k < st.size(); ++k) st[k] = make_int4(p.step[k].e0, p.step[k].ne, p.step[k].i0, p.step[k].ni);
-      upload(slot->step, st);
-      upload(slot->step_ptr, p.step_ptr);
-      upload(slot->down_ptr, p.down_ptr);
-      upload(slot->idx, p.idx);
-      slot->scratch = p.scratch;
-      slot->slot = p.slot;
-      slot->peak_cb = p.peak_cb;
-    }
-    return slot.get();
+      upload(out.step, st);
+      upload(out.step_ptr, p.step_ptr);
+      upload(out.down_ptr, p.down_ptr);
+      upload(out.idx, p.idx);
+      out.scratch = p.scratch;
+      out.slot = p.slot;
+      out.peak_cb = p.peak_cb;
+      return true;
+    });
   }
 
   // The factorisation plan for blocks of G lanes of wsize-byte values with kb KB for its ring,
   // contribution blocks and fronts; null when they do not fit
   const FactorBufs* fplan(int G, int wsize, int kb) {
-    const auto key = std::make_tuple(G, wsize, kb);
-    auto it = fplans.find(key);
-    if (it != fplans.end()) return it->second.get();
-    FactorPlan p;
-    bool ok = false;
-    // the largest ring slots that leave room for the rest
-    for (size_t slot = 24 * 1024; !ok && slot >= 3 * 1024 && n_islands == 1; slot = slot * 2 / 3 / 16 * 16)
-      ok = (size_t)kb * 1024 > kRingSlots * slot &&
-           build_factor_plan(sym, ah_host, ah_loc_host, G, wsize, slot, (size_t)kb * 1024 - kRingSlots * slot, p);
-    auto& out = fplans[key];
-    if (ok) {
-      out = std::make_unique<FactorBufs>();
+    return fplans.get(std::make_tuple(G, wsize, kb), [&](FactorBufs& out) {
+      FactorPlan p;
+      bool ok = false;
+      // the largest ring slots that leave room for the rest
+      for (size_t slot = 24 * 1024; !ok && slot >= 3 * 1024 && n_islands == 1; slot = slot * 2 / 3 / 16 * 16)
+        ok = (size_t)kb * 1024 > kRingSlots * slot &&
+             build_factor_plan(sym, ah_host, ah_loc_host, G, wsize, slot, (size_t)kb * 1024 - kRingSlots * slot, p);
+      if (!ok) return false;
       std::vector<int4> st(p.step.size());
       for (size_t k = 0; k < st.size(); ++k) st[k] = make_int4(p.step[k].e0, p.step[k].ne, p.step[k].i0, p.step[k].ni);
-      upload(out->step, st);
-      upload(out->idx, p.idx);
-      out->n = (int)st.size();
-      out->peak_cb = p.peak_cb;
-      out->most = p.most;
-      out->slot = p.slot;
-      out->cycles = p.cycles;
-    }
-    return out.get();
+      upload(out.step, st);
+      upload(out.idx, p.idx);
+      out.n = (int)st.size();
+      out.peak_cb = p.peak_cb;
+      out.most = p.most;
+      out.slot = p.slot;
+      out.cycles = p.cycles;
+      return true;
+    });
   }
 
   // A launch's shared memory per team is set by its largest front, while its fronts'
@@ -1585,8 +1577,9 @@ struct mpf_handle {
 
   // mismatch rows grouped by island
   DevBuf isl_rows, isl_row_ptr;
+  bool isl_ready = false;
   ChunkRows chunk_rows() {
-    if (!isl_row_ptr.p) {
+    if (!isl_ready) {
       std::vector<int> rows, ptr{0};
       for (int k = 0; k < std::max(g.n_islands, 1); ++k) {
         for (int i : g.mis_rows)
@@ -1595,6 +1588,7 @@ struct mpf_handle {
       }
       upload(isl_rows, rows);
       upload(isl_row_ptr, ptr);
+      isl_ready = true;
     }
     return ChunkRows{isl_rows.as<int>(), isl_row_ptr.as<int>()};
   }

@@ -3,7 +3,10 @@
 #define MPF_INTERNAL_H_
 
 #include <cstdint>
+#include <map>
+#include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "mpf.h"
@@ -214,6 +217,28 @@ bool build_factor_plan(const LUSymbolic& s, const std::vector<int>& ah_ptr, cons
 // bytes for the teams' fronts.  False when a front does not fit the scratch.
 bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bool compact_cb, int G, int wsize,
                       size_t slot, size_t scratch, SweepPlan& out, int n_islands = 0);
+
+// Plans kept by what they depend on.  A plan enters the cache when it is complete: a build
+// that throws (an allocation or a copy that failed) leaves no trace and is tried again by the
+// next call; one that returns false (the planner refuses) is remembered as null.
+template <class Key, class Plan>
+class PlanCache {
+ public:
+  template <class Build>  // bool build(Plan&)
+  const Plan* get(const Key& key, Build&& build) {
+    auto it = plans_.find(key);
+    if (it == plans_.end()) {
+      auto p = std::make_unique<Plan>();
+      if (!build(*p)) p.reset();
+      it = plans_.emplace(key, std::move(p)).first;
+    }
+    return it->second.get();
+  }
+  void clear() { plans_.clear(); }
+
+ private:
+  std::map<Key, std::unique_ptr<Plan>> plans_;
+};
 
 // Everything that does not depend on the case batch.
 struct GridSymbolic {

@@ -29,3 +29,7 @@ def test_lane_pair_ranges_stay_inside_their_block(tmp_path):
 
 def test_islands_without_supernodes_have_their_step_range(tmp_path):
     assert int(run_native(tmp_path, "island_plan_check").split()[1]) == 5 * 5 * 2
+
+
+def test_plan_whose_upload_fails_is_built_again(tmp_path):
+    assert run_native(tmp_path, "plan_cache_check").strip() == "ok"
