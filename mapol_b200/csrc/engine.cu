@@ -74,12 +74,30 @@ struct DevBuf {
   T* as() const { return reinterpret_cast<T*>(p); }
 };
 
+// Uploads and fills go to the legacy stream, and a copy from pageable memory (or a fill) may
+// return before it has landed.  The streams the kernels run on are not ordered after that one:
+// every entry point that launches calls after_uploads() first (an event of the handle, 1 us where
+// a wait on the host takes 6), and so does one that launches on what it has just uploaded;
+// uploads_done() waits here, for plans that are built once.
+thread_local bool uploads_pending = false;
+void uploads_done() {
+  if (!uploads_pending) return;
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  uploads_pending = false;
+}
+
 // Copies v to the device, reusing b's allocation when it is large enough.
 template <class T>
 void upload(DevBuf& b, const std::vector<T>& v) {
   const size_t need = v.size() * sizeof(T);
   if (!b.p || b.bytes < need) b.alloc(need);
-  if (!v.empty()) CUDA_TRY(cudaMemcpy(b.p, v.data(), need, cudaMemcpyHostToDevice));
+  if (v.empty()) return;
+  uploads_pending = true;
+  CUDA_TRY(cudaMemcpy(b.p, v.data(), need, cudaMemcpyHostToDevice));
+}
+void fill(DevBuf& b, int byte, size_t n) {
+  uploads_pending = true;
+  CUDA_TRY(cudaMemset(b.p, byte, n));
 }
 
 // ------------------------------------------------------------------ LU system
@@ -485,6 +503,7 @@ struct LUSystem {
       upload(out.step_ptr, p.step_ptr);
       upload(out.down_ptr, p.down_ptr);
       upload(out.idx, p.idx);
+      uploads_done();
       out.scratch = p.scratch;
       out.slot = p.slot;
       out.peak_cb = p.peak_cb;
@@ -507,6 +526,7 @@ struct LUSystem {
       for (size_t k = 0; k < st.size(); ++k) st[k] = make_int4(p.step[k].e0, p.step[k].ne, p.step[k].i0, p.step[k].ni);
       upload(out.step, st);
       upload(out.idx, p.idx);
+      uploads_done();
       out.n = (int)st.size();
       out.peak_cb = p.peak_cb;
       out.most = p.most;
@@ -1574,6 +1594,8 @@ struct mpf_handle {
     }
   } nr_graph[2];
   cudaEvent_t t0 = nullptr, t1 = nullptr;
+  cudaEvent_t uploaded = nullptr;   // after the handle's latest uploads
+  bool uploads_running = false;     // nothing has waited for it on the host yet
 
   // mismatch rows grouped by island
   DevBuf isl_rows, isl_row_ptr;
@@ -1588,6 +1610,7 @@ struct mpf_handle {
       }
       upload(isl_rows, rows);
       upload(isl_row_ptr, ptr);
+      uploads_done();
       isl_ready = true;
     }
     return ChunkRows{isl_rows.as<int>(), isl_row_ptr.as<int>()};
@@ -1752,10 +1775,39 @@ int fail(mpf_handle* h, int code, const std::string& msg) {
   return code;
 }
 
+// This thread's uploads so far are behind the handle's event
+void mark_uploads(mpf_handle* h) {
+  if (!uploads_pending || !h->uploaded) return;
+  CUDA_TRY(cudaEventRecord(h->uploaded, cudaStreamLegacy));
+  h->uploads_running = true;
+  uploads_pending = false;
+}
+
+// What is launched on st from here on runs after the handle's uploads.  (A capture cannot hold
+// the event: there the wait is the host's, in the mode that allows it beside a capture.)
+void after_uploads(mpf_handle* h, cudaStream_t st) {
+  mark_uploads(h);
+  if (!h->uploads_running) return;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+  if (cs == cudaStreamCaptureStatusNone) {
+    CUDA_TRY(cudaStreamWaitEvent(st, h->uploaded, 0));
+    return;
+  }
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+  const cudaError_t e = cudaEventSynchronize(h->uploaded);
+  CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+  CUDA_TRY(e);
+  h->uploads_running = false;
+}
+
 template <class F>
 int guarded(mpf_handle* h, F&& f) {
   try {
-    return f();
+    const int rc = f();
+    mark_uploads(h);
+    return rc;
   } catch (const MpfError& e) {
     return fail(h, e.code, e.msg);
   } catch (const std::bad_alloc&) {
@@ -1794,6 +1846,7 @@ void upload_fd(mpf_handle* h, int variant) {
     for (int i = 0; i < g.nb; ++i) fv[i] = make_int2(g.bp[0].var[i], g.bpp[0].var[i]);
     upload(h->fdvar, fv);
   }
+  uploads_done();
   h->fd_ready[variant] = true;
 }
 
@@ -2576,6 +2629,7 @@ int32_t mpf_create(const mpf_bus* buses, int32_t n_bus, const mpf_branch* branch
     CUDA_TRY(cudaMallocHost(&h->h_any, sizeof(int)));
     CUDA_TRY(cudaEventCreate(&h->t0));
     CUDA_TRY(cudaEventCreate(&h->t1));
+    CUDA_TRY(cudaEventCreateWithFlags(&h->uploaded, cudaEventDisableTiming));
     upload(h->y_rowptr, g.y_rowptr);
     upload(h->y_col, g.y_col);
     upload(h->y_diag, g.y_diag);
@@ -2641,6 +2695,7 @@ int32_t mpf_destroy(mpf_handle* h) {
   if (h->h_any) cudaFreeHost(h->h_any);
   if (h->t0) cudaEventDestroy(h->t0);
   if (h->t1) cudaEventDestroy(h->t1);
+  if (h->uploaded) cudaEventDestroy(h->uploaded);
   delete h;
   return MPF_OK;
 }
@@ -2862,6 +2917,7 @@ int set_cases_impl(mpf_handle* h, int32_t n_cases, const int32_t* island_of_case
       upload(h->case_lane, case_lane);
     }
     if (sbus) {
+      after_uploads(h, h->own_stream);  // the lane maps are read below
       k_scatter_sbus<<<tile_grid(g.nb, ngroups), dim3(32, kTileRows), 0, h->own_stream>>>(
           g.nb, n_cases, multi ? h->lane_case.as<int>() : nullptr, h->Ibus.as<double2>(), h->sbus_case.as<double2>());
       CUDA_TRY(cudaGetLastError());
@@ -2880,10 +2936,10 @@ int set_cases_impl(mpf_handle* h, int32_t n_cases, const int32_t* island_of_case
       h->q_fix.alloc(n * sizeof(double));
       h->q_flag.alloc((size_t)lanes * sizeof(int));
       h->iter_base.alloc((size_t)lanes * sizeof(int));
-      CUDA_TRY(cudaMemset(h->pv_on.p, 1, n));
-      CUDA_TRY(cudaMemset(h->q_fix.p, 0, n * sizeof(double)));
-      CUDA_TRY(cudaMemset(h->q_flag.p, 0, (size_t)lanes * sizeof(int)));
-      CUDA_TRY(cudaMemset(h->iter_base.p, 0, (size_t)lanes * sizeof(int)));
+      fill(h->pv_on, 1, n);
+      fill(h->q_fix, 0, n * sizeof(double));
+      fill(h->q_flag, 0, (size_t)lanes * sizeof(int));
+      fill(h->iter_base, 0, (size_t)lanes * sizeof(int));
     }
     h->ncases = n_cases;
     h->ngroups = ngroups;
@@ -3036,6 +3092,7 @@ int32_t mpf_set_controls(mpf_handle* h, int32_t n_controls, const mpf_control* c
     C.noltc = (int)oltc.size();
     C.nshc = (int)shc.size();
     C.nslot = (int)slot_pos.size();
+    after_uploads(h, st);
     const DevCtl t = h->devctl();
     if (C.noltc > 0) {
       const size_t tot = (size_t)h->ngroups * C.noltc * 32;
@@ -3119,6 +3176,7 @@ int32_t mpf_get_bus_types(mpf_handle* h, uint8_t* types) {
       for (int i = 0; i < h->g.nb; ++i) bt[i] = (uint8_t)h->g.bus_type[i];
       upload(h->base_type, bt);
     }
+    after_uploads(h, st);
     const size_t total = (size_t)h->ncases * h->g.nb;
     DevBuf out;
     out.alloc(total);
@@ -3144,6 +3202,7 @@ int32_t mpf_solve(mpf_handle* h, int32_t alg, int32_t precision, void* stream) {
     h->last_stream = st;
     std::memset(&h->timing, 0, sizeof(h->timing));
     h->timer.reset(st);
+    after_uploads(h, st);
     CUDA_TRY(cudaEventRecord(h->t0, st));
     ensure_attrs<double>(h->device);
     ensure_attrs<float>(h->device);
@@ -3192,6 +3251,7 @@ int32_t mpf_get_results_device(mpf_handle* h, double* v, int32_t* iterations, ui
   return guarded(h, [&]() -> int {
     CUDA_TRY(cudaSetDevice(h->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : h->own_stream;
+    after_uploads(h, st);
     if (v) {
       k_gather_v<<<tile_grid(h->g.nb, h->ngroups), dim3(32, kTileRows), 0, st>>>(
           h->g.nb, h->ncases, h->dev().lane_case, h->V.as<double2>(), reinterpret_cast<double2*>(v));
@@ -3229,6 +3289,7 @@ int32_t mpf_get_results(mpf_handle* h, double* v, int32_t* iterations, uint8_t* 
     if (max_mis) CUDA_TRY(cudaMemcpyAsync(max_mis, d_mm, h->ncases * sizeof(double), cudaMemcpyDeviceToHost, st));
     if (status) CUDA_TRY(cudaMemcpyAsync(status, d_st, h->ncases, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
+    h->uploads_running = false;
     return MPF_OK;
   });
 }
@@ -3243,8 +3304,9 @@ int32_t mpf_mismatch(mpf_handle* h, const double* v, double* max_mis, void* stre
     const size_t need = (size_t)h->ncases * sizeof(unsigned long long);
     if (!h->eval_acc.p || h->eval_acc.bytes < need) {
       h->eval_acc.alloc(need);
-      CUDA_TRY(cudaMemset(h->eval_acc.p, 0, need));
+      fill(h->eval_acc, 0, need);
     }
+    after_uploads(h, st);
     const int nfree = (int)h->g.mis_rows.size();
     k_mismatch_eval<<<dim3((unsigned)((nfree + 255) / 256), (unsigned)std::min(h->ncases, 65535)), 256, 0, st>>>(
         h->dev(), reinterpret_cast<const double2*>(v), h->ncases, h->eval_acc.as<unsigned long long>());
@@ -3270,6 +3332,7 @@ int32_t mpf_mismatch_noalloc(mpf_handle* h, const double* v, double* max_mis, vo
     unsigned long long* acc = nullptr;
     CUDA_TRY(noalloc_scratch(h->device, &acc));
     cudaStream_t st = stream ? (cudaStream_t)stream : h->own_stream;
+    after_uploads(h, st);
     // the array keeps whatever the previous call left: clear this call's slots
     CUDA_TRY(cudaMemsetAsync(acc, 0, (size_t)h->ncases * sizeof(unsigned long long), st));
     const int nfree = (int)h->g.mis_rows.size();
@@ -3309,6 +3372,7 @@ int32_t mpf_branch_flows(mpf_handle* h, double* ploss, double* overload, double*
     CUDA_TRY(cudaSetDevice(h->device));
     cudaStream_t st_ = stream ? (cudaStream_t)stream : h->own_stream;
     CUDA_TRY(cudaStreamWaitEvent(st_, h->t1, 0));
+    after_uploads(h, st_);
     CUDA_TRY(cudaMemsetAsync(ploss, 0, (size_t)h->ncases * sizeof(double), st_));
     if (overload) CUDA_TRY(cudaMemsetAsync(overload, 0, (size_t)h->ncases * sizeof(double), st_));
     const dim3 grid((unsigned)((h->g.nbr + 63) / 64), (unsigned)h->ngroups);
@@ -3330,6 +3394,7 @@ int32_t mpf_adjoint(mpf_handle* h, int32_t precision, double* grad_p, double* gr
     CUDA_TRY(cudaSetDevice(h->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : h->own_stream;
     CUDA_TRY(cudaStreamWaitEvent(st, h->t1, 0));
+    after_uploads(h, st);
     ensure_attrs<double>(h->device);
     ensure_attrs<float>(h->device);
     if (precision == MPF_FP64) adjoint_impl<double>(h, st, grad_p, grad_q, grad_g, grad_b);

@@ -27,3 +27,21 @@ def test_multigrid_with_grids_of_pv_buses_only(gpu, order, alg, prec):
         assert np.abs(res.v - ref["v"][0]).max() < 1e-8
         if prec == m.FP64:
             assert (res.iterations == ref["iterations"][0]).all()
+
+
+def test_multigrid_injections_follow_the_new_lane_map(gpu):
+    """Batches of another split between the grids, one after the other on one handle: every
+    batch's injections reach its own lanes.  Tolerance as above."""
+    grids = [m.synth_grid(30, 41, 5, seed=2), m.synth_grid(118, 179, 53, 0.1, seed=3)]
+    rng = np.random.default_rng(5)
+    with m.MultiGrid(grids, tol=1e-10) as mg:
+        for counts in ((70, 3), (3, 70), (1, 200), (200, 1), (33, 33)):
+            sbus = [np.stack([b["p"], b["q"]], -1)[None] * rng.uniform(0.8, 1.1, (n, len(b), 1))
+                    for (b, _), n in zip(grids, counts)]
+            mg.set_cases([[[]] * n for n in counts], sbus)
+            mg.solve(m.NR, m.FP64)
+            for (buses, branches), s, res in zip(grids, sbus, mg.results()):
+                with m.PowerFlow(buses, branches, tol=1e-10) as pf:
+                    ref = pf.runpf([[]] * len(s), sbus=s)
+                assert res.converged.all() and ref.converged.all()
+                assert np.abs(res.v - ref.v).max() < 1e-8
