@@ -2918,8 +2918,8 @@ int set_cases_impl(mpf_handle* h, int32_t n_cases, const int32_t* island_of_case
     }
     if (sbus) {
       after_uploads(h, h->own_stream);  // the lane maps are read below
-      k_scatter_sbus<<<tile_grid(g.nb, ngroups), dim3(32, kTileRows), 0, h->own_stream>>>(
-          g.nb, n_cases, multi ? h->lane_case.as<int>() : nullptr, h->Ibus.as<double2>(), h->sbus_case.as<double2>());
+      k_scatter_sbus<<<tile_grid(g.nb, std::min(ngroups, kMaxGridRows)), dim3(32, kTileRows), 0, h->own_stream>>>(
+          g.nb, n_cases, ngroups, multi ? h->lane_case.as<int>() : nullptr, h->Ibus.as<double2>(), h->sbus_case.as<double2>());
       CUDA_TRY(cudaGetLastError());
       CUDA_TRY(cudaStreamSynchronize(h->own_stream));
     }
@@ -3013,8 +3013,8 @@ int32_t mpf_set_controls(mpf_handle* h, int32_t n_controls, const mpf_control* c
       CUDA_TRY(cudaMemcpyAsync(in, values, vbytes, cudaMemcpyHostToDevice, st));
       CUDA_TRY(cudaMemcpyAsync(C.vbase.p, b2.data(), nc * sizeof(double2), cudaMemcpyHostToDevice, st));
       CUDA_TRY(cudaMemsetAsync(C.bad.p, 0xff, sizeof first, st));
-      k_scatter_ctl<<<tile_grid(nc, h->ngroups), dim3(32, kTileRows), 0, st>>>(
-          nc, ncases, h->dev().lane_case, in, C.vbase.as<double2>(), C.val.as<double>(), C.bad.as<unsigned long long>());
+      k_scatter_ctl<<<tile_grid(nc, std::min(h->ngroups, kMaxGridRows)), dim3(32, kTileRows), 0, st>>>(
+          nc, ncases, h->ngroups, h->dev().lane_case, in, C.vbase.as<double2>(), C.val.as<double>(), C.bad.as<unsigned long long>());
       CUDA_TRY(cudaGetLastError());
       CUDA_TRY(cudaMemcpyAsync(&first, C.bad.p, sizeof first, cudaMemcpyDeviceToHost, st));
       CUDA_TRY(cudaStreamSynchronize(st));

@@ -2588,38 +2588,51 @@ __global__ void __launch_bounds__(32 * kTileRows) k_gather_v(int nb, int ncases,
   }
 }
 
-// Injections given case by case, [case][bus], into [group][bus][32] (0 in padding lanes)
-__global__ void __launch_bounds__(32 * kTileRows) k_scatter_sbus(int nb, int ncases, const int* __restrict__ lane_case,
+// Injections given case by case, [case][bus], into [group][bus][32] (0 in padding lanes).
+// (Batches that can only be evaluated may have more groups than a grid has rows.)
+constexpr int kMaxGridRows = 65535;
+__global__ void __launch_bounds__(32 * kTileRows) k_scatter_sbus(int nb, int ncases, int ngroups,
+                                                               const int* __restrict__ lane_case,
                                                                const double2* __restrict__ in, double2* __restrict__ out) {
   __shared__ double2 tile[32][33];
-  const int g = blockIdx.y, i0 = blockIdx.x * 32;
-  for (int r = threadIdx.y; r < 32; r += kTileRows) {
-    const int c = g * 32 + r, uc = lane_case ? lane_case[c] : (c < ncases ? c : -1);
-    tile[threadIdx.x][r] = uc >= 0 && i0 + (int)threadIdx.x < nb ? in[(size_t)uc * nb + i0 + threadIdx.x] : make_double2(0.0, 0.0);
+  const int i0 = blockIdx.x * 32;
+  for (int g = blockIdx.y; g < ngroups; g += gridDim.y) {
+    for (int r = threadIdx.y; r < 32; r += kTileRows) {
+      const int c = g * 32 + r, uc = lane_case ? lane_case[c] : (c < ncases ? c : -1);
+      tile[threadIdx.x][r] =
+          uc >= 0 && i0 + (int)threadIdx.x < nb ? in[(size_t)uc * nb + i0 + threadIdx.x] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32 && i0 + r < nb; r += kTileRows)
+      out[at32(g, nb, i0 + r, threadIdx.x)] = tile[r][threadIdx.x];
+    __syncthreads();
   }
-  __syncthreads();
-  for (int r = threadIdx.y; r < 32 && i0 + r < nb; r += kTileRows) out[at32(g, nb, i0 + r, threadIdx.x)] = tile[r][threadIdx.x];
 }
 
 // Control values given case by case, [case][control], into [group][control][32] (padding
 // lanes: base); bad gets the smallest 2 (lane nc + control) + (1: not positive, where the
 // kind asks for it; 0: not finite) of the values in error
-__global__ void __launch_bounds__(32 * kTileRows) k_scatter_ctl(int nc, int ncases, const int* __restrict__ lane_case,
+__global__ void __launch_bounds__(32 * kTileRows) k_scatter_ctl(int nc, int ncases, int ngroups,
+                                                              const int* __restrict__ lane_case,
                                                               const double* __restrict__ in, const double2* __restrict__ base,
                                                               double* __restrict__ out, unsigned long long* __restrict__ bad) {
   __shared__ double tile[32][33];
-  const int g = blockIdx.y, k0 = blockIdx.x * 32, k = k0 + threadIdx.x;
-  for (int r = threadIdx.y; r < 32 && k < nc; r += kTileRows) {
-    const int c = g * 32 + r, uc = lane_case ? lane_case[c] : (c < ncases ? c : -1);
-    const double2 b = base[k];  // base value; y = 1: must be positive
-    const double v = uc >= 0 ? in[(size_t)uc * nc + k] : b.x;
-    const bool finite = fabs(v) <= DBL_MAX;
-    if (!finite || (b.y != 0.0 && !(v > 0.0)))
-      atomicMin(bad, 2ull * ((unsigned long long)c * nc + k) + (finite ? 1 : 0));
-    tile[threadIdx.x][r] = v;
+  const int k0 = blockIdx.x * 32, k = k0 + threadIdx.x;
+  for (int g = blockIdx.y; g < ngroups; g += gridDim.y) {
+    for (int r = threadIdx.y; r < 32 && k < nc; r += kTileRows) {
+      const int c = g * 32 + r, uc = lane_case ? lane_case[c] : (c < ncases ? c : -1);
+      const double2 b = base[k];  // base value; y = 1: must be positive
+      const double v = uc >= 0 ? in[(size_t)uc * nc + k] : b.x;
+      const bool finite = fabs(v) <= DBL_MAX;
+      if (!finite || (b.y != 0.0 && !(v > 0.0)))
+        atomicMin(bad, 2ull * ((unsigned long long)c * nc + k) + (finite ? 1 : 0));
+      tile[threadIdx.x][r] = v;
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32 && k0 + r < nc; r += kTileRows)
+      out[at32(g, nc, k0 + r, threadIdx.x)] = tile[r][threadIdx.x];
+    __syncthreads();
   }
-  __syncthreads();
-  for (int r = threadIdx.y; r < 32 && k0 + r < nc; r += kTileRows) out[at32(g, nc, k0 + r, threadIdx.x)] = tile[r][threadIdx.x];
 }
 
 // flag |= 1 where a value is infinite or NaN

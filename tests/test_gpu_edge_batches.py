@@ -45,3 +45,38 @@ def test_multigrid_injections_follow_the_new_lane_map(gpu):
                     ref = pf.runpf([[]] * len(s), sbus=s)
                 assert res.converged.all() and ref.converged.all()
                 assert np.abs(res.v - ref.v).max() < 1e-8
+
+
+def test_batches_of_more_groups_than_a_grid_has_rows(gpu):
+    """65537 groups of 32 cases: too many to solve in one batch, but injections and controls are
+    accepted and mpf_mismatch evaluates them.  A two-bus line against its formula; both are a
+    handful of FP64 operations on values of order 10, so 1e-12 is 100 roundings."""
+    import torch
+
+    from mapol_b200._lib import lib
+
+    n = 65536 * 32 + 1
+    buses, branches = m.synth_grid(2, 1, 0, seed=3)
+    slack = int(np.flatnonzero(buses["type"] == 3)[0])
+    k = 1 - slack
+    rng = np.random.default_rng(1)
+    sbus = rng.uniform(-1.0, 1.0, (n, 2, 2))
+    shunt = rng.uniform(0.0, 0.5, n)
+    volts = rng.uniform(0.9, 1.1, (n, 2)) * np.exp(1j * rng.uniform(-0.3, 0.3, (n, 2)))
+    b = branches[0]
+    assert b["tap"] == 0.0 and b["shift"] == 0.0
+    ys = 1.0 / (b["r"] + 1j * b["x"])
+    vk, vs = volts[:, k], volts[:, slack]
+    v = torch.from_numpy(np.ascontiguousarray(np.stack([volts.real, volts.imag], -1))).cuda()
+    out = torch.zeros(n, dtype=torch.float64, device="cuda")
+    with m.PowerFlow(buses, branches) as pf:
+        pf.set_cases([[]] * n, sbus=sbus)
+        for controls in (False, True):
+            if controls:
+                pf.set_controls([(m.CTRL_SHC, k)], shunt[:, None])
+            yd = ys + 0.5j * b["b"] + buses["gsh"][k] + 1j * (shunt if controls else buses["bsh"][k])
+            f = vk * np.conj(yd * vk - ys * vs) - (sbus[:, k, 0] + 1j * sbus[:, k, 1])
+            ref = np.maximum(np.abs(f.real), np.abs(f.imag))
+            assert lib().mpf_mismatch(pf._h, v.data_ptr(), out.data_ptr(), None) == 0
+            torch.cuda.synchronize()
+            assert np.abs(out.cpu().numpy() - ref).max() < 1e-12 * max(1.0, np.abs(ys) * 10)
