@@ -243,7 +243,7 @@ struct FactorBufs {
 struct PlanBufs {
   DevBuf step, step_ptr, down_ptr, idx;
   size_t scratch = 0, slot = 0;  // as SweepPlan
-  int peak_cb = 0;
+  int peak_cb = 0, steps = 0;
   DevSweep dev() const { return DevSweep{step.as<int4>(), step_ptr.as<int>(), down_ptr.as<int>(), idx.as<int>()}; }
 };
 
@@ -277,7 +277,7 @@ struct LUSystem {
   std::map<std::pair<int, int>, std::vector<FactorChoice>> tuned;
   // autotuned lane count of every backward-solve level launch (0 = one case per thread)
   std::map<std::pair<int, int>, std::vector<int>> tuned_bs;
-  std::vector<Launch> level_sched;   // one launch per level (adjoint solves of full batches), ascending
+  std::vector<Launch> level_sched;   // one launch per level (fast-decoupled and adjoint solves of full batches), ascending
   std::vector<int> ah_host, ah_loc_host;  // host copies of ah_ptr and ah_loc
   int nA = 0;
   // values per precision [0] = FP64, [1] = FP32
@@ -507,6 +507,7 @@ struct LUSystem {
       out.scratch = p.scratch;
       out.slot = p.slot;
       out.peak_cb = p.peak_cb;
+      out.steps = (int)p.step.size();
       return true;
     });
   }
@@ -675,6 +676,7 @@ void ensure_attrs(int device) {
   CUDA_TRY(cudaFuncSetAttribute(k_mf_bsolve_chunk<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_bsolve_chunk<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_bsolve_chunk<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+  CUDA_TRY(cudaFuncSetAttribute(k_mf_fsolve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_fsolve_t<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_bsolve_t<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   CUDA_TRY(cudaFuncSetAttribute(k_mf_factor_big<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
@@ -1464,6 +1466,21 @@ void tune_bsolve(LUSystem& sys, int ngroups, const T* pan, T* x, const int* grou
   TuneCache& tc = tune_cache();
   std::lock_guard<std::mutex> lock(tc.mu);
   if (tc.bsolve.emplace(key, best).second) append_tune_file(line + "\n");
+}
+
+template <typename T>
+void launch_fsolve(const LUSystem& sys, int ngroups, const T* pan, T* cbr, T* x, const int* group_active,
+                   cudaStream_t st, int* nlaunch) {
+  for (const Launch& ln : sys.level_sched) {
+    const long long ntasks = (long long)ln.count * ngroups;
+    const int wpb = solve_warps<T>(ln.fcap, 32);
+    long long blocks = std::min<long long>((ntasks + wpb - 1) / wpb, 148LL * 32);
+    const size_t smem = (size_t)wpb * ln.fcap * 32 * sizeof(T);
+    k_mf_fsolve<T><<<(unsigned)blocks, 32 * wpb, smem, st>>>(sys.dev(), sys.lev_sn.as<int>() + ln.offset, ln.count, ngroups,
+                                                        ln.fcap, pan, cbr, x, group_active);
+    CUDA_TRY(cudaGetLastError());
+    ++*nlaunch;
+  }
 }
 
 // ------------------------------------------------------------------ timing
@@ -2369,11 +2386,43 @@ void launch_fd_chunk_g(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSyste
 }
 
 template <typename T>
-void launch_fd_chunk(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSystem& Bp, LUSystem& Bpp, cudaStream_t st) {
-  const ChunkShape sh = choose_chunk({&Bp, &Bpp}, Prec<T>::G, sizeof(T), h->ngroups, 1);
+void launch_fd_chunk(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSystem& Bp, LUSystem& Bpp,
+                     const ChunkShape& sh, cudaStream_t st) {
   with_shape<T>(sh, [&](auto g, auto xs) {
     launch_fd_chunk_g<T, decltype(g)::value, decltype(xs)::value>(h, d, fd, Bp, Bpp, sh, st);
   });
+}
+
+// Whether a fast-decoupled solve runs on one block per chunk of lanes, and its shape (G = 0: on
+// level launches), by estimated microseconds per iteration.  A block's iteration is its steps
+// (about 1 us each) and its panels' traffic, and the batch is so many waves of blocks; the
+// level launches pay about 8 us per launch and the batch's entries.  Fitted to 30 to 9241 buses
+// x 11 to 60000 cases in both precisions.  ms per solve, level launches / chunks:
+//   FP64: 30 buses x 5000 2.4 / 2.1, x 10000 2.4 / 3.9;  300 x 4000 8.0 / 5.8, x 8000 9.2 / 11.1
+//     1354 x 4096 18.7 / 17.0, x 8000 25.3 / 33.3;  2869 x 1500 25.5 / 21.1, x 3000 31.1 / 40.9
+//     9241 x 256 41.4 / 14.9, x 1000 55.6 / 44.9, x 2000 69.7 / 86.7
+//   FP32: 30 x 10000 2.5 / 2.0, x 20000 2.6 / 3.7;  300 x 8000 8.9 / 6.1, x 16000 11.1 / 11.7
+//     1354 x 8000 23.4 / 21.6;  2869 x 3000 27.1 / 24.7, x 4000 30.3 / 32.4
+//     9241 x 1000 43.5 / 34.4, x 1500 49.6 / 58.7
+template <typename T>
+ChunkShape choose_fd(LUSystem& Bp, LUSystem& Bpp, int ngroups) {
+  ChunkShape none;
+  if (const char* e = std::getenv("MPF_FD_CHUNK"))  // testing: 0 off
+    if (std::atoi(e) == 0) return none;
+  const double isl = Bp.n_islands;  // a lane's share: its own island
+  const double nnz = (double)(Bp.sym.nnz + Bpp.sym.nnz) / isl;
+  const int levels = Bp.sym.nlevels + Bpp.sym.nlevels;
+  const double level = 8.0 * (2 * levels + 6) + nnz * (sizeof(T) == 8 ? 0.013 : 0.007) + 1e-5 * nnz * 32.0 * ngroups;
+  auto chunks = [&](int G, double steps, bool xs) {
+    const int waves = (ngroups * (32 / G) + 147) / 148;
+    return waves * (steps / isl + nnz * (0.0025 + 0.0011 * G) * (xs ? 1.0 : 1.3));
+  };
+  const bool forced = std::getenv("MPF_CHUNK_LANES") != nullptr;  // testing
+  bool possible = forced;
+  for (int G = Prec<T>::G; G >= 1 && !possible; G /= 2) possible = chunks(G, 2.0 * levels, true) < level;
+  if (!possible) return none;
+  const ChunkShape sh = choose_chunk({&Bp, &Bpp}, Prec<T>::G, sizeof(T), ngroups, 1);
+  return forced || chunks(sh.G, sh.plan[0]->steps + sh.plan[1]->steps, sh.xs) < level ? sh : none;
 }
 
 template <typename T>
@@ -2434,15 +2483,66 @@ void solve_fd(mpf_handle* h, cudaStream_t st, int variant) {
                      S.x[P].as<T>(), d.status, d.group_active, 0, st, &nl);
   }
   tm.end(ev);
-  ev = tm.begin(FAM_SOLVE);
-  launch_fd_chunk<T>(h, d, fdd, Bp, Bpp, st);
-  ++nl;
+  const ChunkShape shape = choose_fd<T>(Bp, Bpp, h->ngroups);
+  if (shape.G > 0) {
+    ev = tm.begin(FAM_SOLVE);
+    launch_fd_chunk<T>(h, d, fdd, Bp, Bpp, shape, st);
+    ++nl;
+    tm.end(ev);
+    // the largest iteration count over the chunks
+    CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    h->timing.launches = nl;
+    h->timing.iterations_max = *h->h_any;
+    return;
+  }
+  if (h->opt.autotune)
+    for (int k = 0; k < 2; ++k) {
+      LUSystem& S = *systems[k];
+      tune_bsolve<T>(S, h->ngroups, S.pan[P].as<T>(), S.x[P].as<T>(), d.group_active, st);
+    }
+  T* xp = Bp.x[P].as<T>();
+  T* xq = Bpp.x[P].as<T>();
+  const int max_it = h->opt.max_it_fd;
+  auto mismatch = [&]() {
+    int e2 = tm.begin(FAM_MIS);
+    k_mismatch_fd<T><<<rg, 256, 0, st>>>(d, fdd, xp, xq);
+    CUDA_TRY(cudaGetLastError());
+    ++nl;
+    tm.end(e2);
+  };
+  mismatch();
+  ev = tm.begin(FAM_OTHER);
+  check(h, st, 0, max_it, &nl);
   tm.end(ev);
-  // the largest iteration count over the chunks
-  CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(cudaStreamSynchronize(st));
+  int i = 0;
+  if (any_active(h, st)) {
+    while (i < max_it) {
+      ++i;
+      for (int half = 0; half < 2; ++half) {
+        LUSystem& S = half == 0 ? Bp : Bpp;
+        ev = tm.begin(FAM_SOLVE);
+        launch_fsolve<T>(S, h->ngroups, S.pan[P].as<T>(), S.cbr[P].as<T>(), S.x[P].as<T>(), d.group_active, st, &nl);
+        launch_bsolve<T>(S, h->ngroups, S.pan[P].as<T>(), S.x[P].as<T>(), d.group_active, st, &nl);
+        tm.end(ev);
+        ev = tm.begin(FAM_UPD);
+        k_update_fd<T><<<rg, 256, 0, st>>>(d, fdd, xp, xq, half);
+        CUDA_TRY(cudaGetLastError());
+        ++nl;
+        tm.end(ev);
+        mismatch();
+        ev = tm.begin(FAM_OTHER);
+        // after the P half only convergence retires a case (fdpf.h:529-540); the
+        // iteration limit is tested after the Q half
+        check(h, st, i, half == 0 ? INT32_MAX : max_it, &nl);
+        tm.end(ev);
+        if (!any_active(h, st)) break;
+      }
+      if (*h->h_any == 0) break;
+    }
+  }
   h->timing.launches = nl;
-  h->timing.iterations_max = *h->h_any;
+  h->timing.iterations_max = i;
 }
 
 }  // namespace

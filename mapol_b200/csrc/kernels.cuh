@@ -595,6 +595,73 @@ struct DevFD {
   const int2* fdvar;   // [nb] (B' var, B'' var) or -1
 };
 
+// P = Re(mis)/|V| over PV/PQ, Q = Im(mis)/|V| over PQ (fdpf.h:369-414)
+template <typename T>
+__global__ void __launch_bounds__(256) k_mismatch_fd(DevGrid d, DevFD f, T* xp, T* xq) {
+  const int g = blockIdx.y;
+  if (!d.group_active[g]) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = g * 32 + lane;
+  LaneOut o;
+  load_outages(d, c, o);
+  double lmax = 0.0;
+  const int r1 = min(d.nfree, (blockIdx.x + 1) * kRowsPerBlock);
+  for (int r = blockIdx.x * kRowsPerBlock + warp; r < r1; r += 8) {
+    const int i = d.mis_rows[r];
+    if (!row_here(d, i, g)) continue;
+    double2 ib = make_double2(0.0, 0.0);
+    const bool touched = row_touched(o, d.y_diag[i]);
+    for (int p = d.y_rowptr[i]; p < d.y_rowptr[i + 1]; ++p) {
+      const double2 y = yentry(d, o, touched, p, g, lane);
+      const double2 v = d.V[at32(g, d.nb, d.y_col[p], lane)];
+      ib.x += y.x * v.x - y.y * v.y;
+      ib.y += y.x * v.y + y.y * v.x;
+    }
+    const double2 vi = d.V[at32(g, d.nb, i, lane)];
+    const double2 s = d.sbus_case ? d.sbus_case[at32(g, d.nb, i, lane)] : d.sbus0[i];
+    const double av = sqrt(vi.x * vi.x + vi.y * vi.y);
+    const double mr = (vi.x * ib.x + vi.y * ib.y - s.x) / av;
+    const double mi = (vi.y * ib.x - vi.x * ib.y - s.y) / av;
+    const int2 fv = f.fdvar[i];
+    xp[at32(g, f.n_bp, fv.x, lane)] = (T)mr;
+    double m = fabs(mr);
+    if (mr != mr) m = INFINITY;
+    if (fv.y >= 0) {
+      xq[at32(g, f.n_bpp, fv.y, lane)] = (T)mi;
+      m = fmax(m, fabs(mi));
+      if (mi != mi) m = INFINITY;
+    }
+    lmax = fmax(lmax, finite_or_inf(m));
+  }
+  block_lane_max(lmax, &d.facc[c], d.status[c] == ST_RUNNING);
+}
+
+// half updates (fdpf.h:416-448): Va -= dVa over PV/PQ (half 0), |V| -= dVm over PQ (half 1)
+template <typename T>
+__global__ void __launch_bounds__(256) k_update_fd(DevGrid d, DevFD f, const T* xp, const T* xq, int half) {
+  const int g = blockIdx.y;
+  if (!d.group_active[g]) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = g * 32 + lane;
+  if (d.status[c] != ST_RUNNING) return;
+  const int r1 = min(d.nfree, (blockIdx.x + 1) * kRowsPerBlock);
+  for (int r = blockIdx.x * kRowsPerBlock + warp; r < r1; r += 8) {
+    const int i = d.mis_rows[r];
+    if (!row_here(d, i, g)) continue;
+    const int2 fv = f.fdvar[i];
+    if (half == 1 && fv.y < 0) continue;
+    const size_t k = at32(g, d.nb, i, lane);
+    const double2 v = d.V[k];
+    double mag = sqrt(v.x * v.x + v.y * v.y);
+    double ang = vangle(v, d.angle_mode);
+    if (half == 0) ang -= (double)xp[at32(g, f.n_bp, fv.x, lane)];
+    else mag -= (double)xq[at32(g, f.n_bpp, fv.y, lane)];
+    double sn, cs;
+    sincos(ang, &sn, &cs);
+    d.V[k] = make_double2(mag * cs, mag * sn);
+  }
+}
+
 // B'/B'' values of every case: base arrowhead values, then minus the outaged
 // branches' contributions.  Thread per (entry, lane).
 template <typename T>
@@ -1756,6 +1823,45 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big_gt(DevLU L, const int*
   }
 }
 
+// Forward substitution with stored factors (fast-decoupled solves): thread per
+// case, warp per (supernode, group).  b accumulates in shared memory.
+template <typename T>
+__global__ void __launch_bounds__(128) k_mf_fsolve(DevLU L, const int* __restrict__ task_sn, int nsn_l,
+                                                   int ngroups, int fcap, const T* __restrict__ pan,
+                                                   T* __restrict__ cbr, T* __restrict__ x,
+                                                   const int* __restrict__ group_active) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  T* b = reinterpret_cast<T*>(smem_raw) + (size_t)warp * fcap * 32;
+  const long long ntasks = (long long)nsn_l * ngroups;
+  for (long long t = (long long)blockIdx.x * warps + warp; t < ntasks; t += (long long)gridDim.x * warps) {
+    const int s = task_sn[t / ngroups];
+    const int g = (int)(t % ngroups);
+    if (!group_active[g] || !task_here(L, s, g)) continue;
+    const int w = L.sn_w[s], f = L.sn_f[s];
+    const int* rows = L.sn_rows + L.sn_rptr[s];
+    for (int i = 0; i < f; ++i) b[i * 32 + lane] = (T)0;
+    for (int p = 0; p < w; ++p) b[p * 32 + lane] = x[at32(g, L.n, rows[p], lane)];
+    for (int ci = L.child_ptr[s]; ci < L.child_ptr[s + 1]; ++ci) {
+      const int ch = L.child_list[ci];
+      const int m = L.sn_f[ch] - L.sn_w[ch];
+      const int* rel = L.relmap + L.rel_ptr[ch];
+      for (int a = 0; a < m; ++a) b[rel[a] * 32 + lane] += cbr[at32(g, L.sumcbr, L.cbr_off[ch] + a, lane)];
+    }
+    const long long po = L.pan_off[s];
+    for (int p = 0; p < w; ++p) {
+      const T yp = b[p * 32 + lane];
+      for (int i = p + 1; i < w; ++i) b[i * 32 + lane] -= pan[at32(g, L.nnz, po + (long long)i * f + p, lane)] * yp;
+      for (int i = w; i < f; ++i)
+        b[i * 32 + lane] -= pan[at32(g, L.nnz, po + (long long)w * f + (long long)(i - w) * w + p, lane)] * yp;
+    }
+    for (int p = 0; p < w; ++p) x[at32(g, L.n, rows[p], lane)] = b[p * 32 + lane];
+    if (L.sn_parent[s] >= 0)
+      for (int a = 0; a < f - w; ++a) cbr[at32(g, L.sumcbr, L.cbr_off[s] + a, lane)] = b[(w + a) * 32 + lane];
+    __syncwarp();
+  }
+}
+
 // Backward substitution: thread per case, warp per (supernode, group).  The
 // supernode's front values of x (ancestors' solutions, final after the previous
 // launches, and its own forward-substituted y) are staged in shared memory first,
@@ -2200,7 +2306,7 @@ __global__ void k_adj_cast(size_t n_total, const double* __restrict__ b, T* __re
 
 // U^T z = g, supernodes bottom-up (thread per case, warp per (supernode, group)):
 // pivots in order, each pushes U(p, i) z_p into the later rows of its front; the
-// non-pivot rows travel to the parent as a carried vector.
+// non-pivot rows travel to the parent as a carried vector (as k_mf_fsolve).
 template <typename T>
 __global__ void __launch_bounds__(128) k_mf_fsolve_t(DevLU L, const int* __restrict__ task_sn, int nsn_l,
                                                      int ngroups, int fcap, const T* __restrict__ pan,
