@@ -161,7 +161,11 @@ typedef struct mpf_stats {
                                                   pivot rows of each supernode: what a backward
                                                   substitution reads) */
   int32_t ordering;                            /* MPF_ORDER_* the Newton system uses */
-  int32_t pad_;
+  uint8_t solve_lanes, solve_in_shared;        /* the last mpf_solve: cases per block where a block
+                                                  carries its cases through the whole solve (0:
+                                                  level launches), and 1 where their solution
+                                                  vectors stay in shared memory */
+  uint8_t adjoint_lanes, adjoint_in_shared;    /* the same of the last mpf_adjoint's substitutions */
 } mpf_stats;
 
 typedef struct mpf_handle mpf_handle;

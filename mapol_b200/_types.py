@@ -129,5 +129,8 @@ class Stats(ctypes.Structure):
         ("device_bytes", ctypes.c_int64),
         ("nnz_lu_upper", ctypes.c_int64),
         ("ordering", ctypes.c_int32),
-        ("pad_", ctypes.c_int32),
+        ("solve_lanes", ctypes.c_uint8),
+        ("solve_in_shared", ctypes.c_uint8),
+        ("adjoint_lanes", ctypes.c_uint8),
+        ("adjoint_in_shared", ctypes.c_uint8),
     ]

@@ -1611,6 +1611,9 @@ struct mpf_handle {
     }
   } nr_graph[2];
   cudaEvent_t t0 = nullptr, t1 = nullptr;
+  // the last solve's and the last adjoint's chunk kernels (mpf_stats): lanes per block (0: level
+  // launches) and x in shared memory
+  uint8_t solve_lanes = 0, solve_in_shared = 0, adjoint_lanes = 0, adjoint_in_shared = 0;
   cudaEvent_t uploaded = nullptr;   // after the handle's latest uploads
   bool uploads_running = false;     // nothing has waited for it on the host yet
 
@@ -2068,14 +2071,17 @@ void launch_bsolve_t(const LUSystem& sys, int ngroups, const T* pan, T* x, const
 //   10.8 (18.7) / 11.3 (12.6);  2869 x 300 7.8 (15.4) / 7.6 (9.9);  300 x 1024 1.6 (2.6) / 1.2 (1.6)
 constexpr int kLevelSubstGroups = 128;             // groups of 32 lanes, twice in FP64
 constexpr long long kLevelSubstEntries = 1800000;  // and their LU entries
+// Returns the chunks' shape (G = 0: level launches).
 template <typename T>
-void launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, const int* group_active, int device,
-                    cudaStream_t st) {
+ChunkShape launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, const int* group_active, int device,
+                          cudaStream_t st) {
   const int words = ngroups * (int)sizeof(T) / 4;
-  if (!std::getenv("MPF_CHUNK_LANES") && words >= kLevelSubstGroups && words * S.sym.nnz >= kLevelSubstEntries) {
+  const char* off = std::getenv("MPF_SUBST_CHUNK");  // testing: 0 off
+  if ((off && std::atoi(off) == 0) ||
+      (!std::getenv("MPF_CHUNK_LANES") && words >= kLevelSubstGroups && words * S.sym.nnz >= kLevelSubstEntries)) {
     launch_fsolve_t<T>(S, ngroups, pan, cbr, x, group_active, st);
     launch_bsolve_t<T>(S, ngroups, pan, x, group_active, st);
-    return;
+    return ChunkShape();
   }
   const ChunkShape sh = choose_chunk({&S}, Prec<T>::G, sizeof(T), ngroups, 2);
   with_shape<T>(sh, [&](auto g, auto xs) {
@@ -2087,6 +2093,7 @@ void launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, const 
     k_subst_chunk<T, G, XS, true><<<(unsigned)(ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(a, S.group_island);
     CUDA_TRY(cudaGetLastError());
   });
+  return sh;
 }
 
 // How k_nr_chunk runs the Newton system: lanes per block (0: it does not), shared memory
@@ -2207,6 +2214,8 @@ void solve_nr(mpf_handle* h, cudaStream_t st) {
   auto& gph = h->nr_graph[P];
   // (autotune = 0 keeps the level kernels of the fixed rule)
   const NrShape chunk = h->opt.autotune ? choose_nr<T>(J, h->ngroups) : NrShape();
+  h->solve_lanes = (uint8_t)chunk.G;
+  h->solve_in_shared = chunk.G > 0;
   // one Newton run over the running cases: mismatch at the current voltages, check,
   // then iterations until no case is running (first: also tune and capture)
   auto run_newton = [&](bool first) {
@@ -2484,6 +2493,8 @@ void solve_fd(mpf_handle* h, cudaStream_t st, int variant) {
   }
   tm.end(ev);
   const ChunkShape shape = choose_fd<T>(Bp, Bpp, h->ngroups);
+  h->solve_lanes = (uint8_t)shape.G;
+  h->solve_in_shared = shape.xs;
   if (shape.G > 0) {
     ev = tm.begin(FAM_SOLVE);
     launch_fd_chunk<T>(h, d, fdd, Bp, Bpp, shape, st);
@@ -2603,6 +2614,11 @@ void adjoint_impl(mpf_handle* h, cudaStream_t st, double* gp, double* gq, double
                    d.group_active, 0, st, &nl);
   const size_t nx = (size_t)lanes * J.sym.n;
   const dim3 bg((unsigned)((h->g.nbr + 63) / 64), (unsigned)h->ngroups);
+  auto substitute = [&]() {
+    const ChunkShape sh = launch_subst_t<T>(J, h->ngroups, pan, J.cbr[P].as<T>(), x, d.group_active, h->device, st);
+    h->adjoint_lanes = (uint8_t)sh.G;
+    h->adjoint_in_shared = sh.xs;
+  };
   auto gradients = [&](const auto* lam) {
     using L = std::remove_cv_t<std::remove_pointer_t<decltype(lam)>>;
     if (gp || gq) {
@@ -2619,7 +2635,7 @@ void adjoint_impl(mpf_handle* h, cudaStream_t st, double* gp, double* gq, double
     CUDA_TRY(cudaMemsetAsync(x, 0, nx * sizeof(T), st));
     k_adj_dldx<T><<<bg, 256, 0, st>>>(d, h->g.nbr, h->rating.as<double>(), x);
     CUDA_TRY(cudaGetLastError());
-    launch_subst_t<T>(J, h->ngroups, pan, J.cbr[P].as<T>(), x, d.group_active, h->device, st);
+    substitute();
     gradients(x);
   } else {
     // FP32 factors: solve, then refine with FP64 residuals of the FP64 Jacobian
@@ -2647,7 +2663,7 @@ void adjoint_impl(mpf_handle* h, cudaStream_t st, double* gp, double* gq, double
                                                  h->adj_colent.as<int2>(), A64, lam64, b64, x);
         CUDA_TRY(cudaGetLastError());
       }
-      launch_subst_t<T>(J, h->ngroups, pan, J.cbr[P].as<T>(), x, d.group_active, h->device, st);
+      substitute();
       k_adj_accumulate<T><<<eb, 256, 0, st>>>(nx, x, lam64, r > 0);
       CUDA_TRY(cudaGetLastError());
     }
@@ -2826,6 +2842,10 @@ int32_t mpf_get_stats(const mpf_handle* h, mpf_stats* st) {
   st->device_bytes = (int64_t)h->device_bytes();
   for (int s = 0; s < g.jac.nsn; ++s) st->nnz_lu_upper += (int64_t)g.jac.sn_w[s] * g.jac.sn_f[s];
   st->ordering = g.ordering;
+  st->solve_lanes = h->solve_lanes;
+  st->solve_in_shared = h->solve_in_shared;
+  st->adjoint_lanes = h->adjoint_lanes;
+  st->adjoint_in_shared = h->adjoint_in_shared;
   return MPF_OK;
 }
 

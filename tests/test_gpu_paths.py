@@ -70,3 +70,78 @@ def test_fast_decoupled_form_by_batch(gpu, prec, n_bus, n_cases, chunks):
         res = pf.runpf(outages(branches, n_bus, n_cases), alg=m.FDXB, precision=prec)
         assert res.converged.all()
         assert (pf.timing()["launches"] < 50) == chunks
+
+
+def lanes_that_run(n_bus, prec, lanes):
+    """Lanes per block a forced count gives: 0 (level launches) beyond 32 bytes of lanes, and where
+    the vectors, contribution blocks and fronts of that many lanes do not fit shared memory."""
+    if prec == m.FP64 and lanes == 8:
+        return 0
+    if n_bus == 700 and lanes == (4 if prec == m.FP64 else 8):
+        return 0
+    return lanes
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+@pytest.mark.parametrize("prec", [m.FP64, m.MIXED])
+@pytest.mark.parametrize("n_bus,n_cases", [(30, 1), (118, 33), (300, 70), (700, 9)])
+def test_forced_newton_lanes_are_the_ones_that_run(gpu, monkeypatch, lanes, prec, n_bus, n_cases):
+    """Tolerance: both sides stop at max |F| < 1e-11, so |dV| stays below the parity tests' 1e-8."""
+    monkeypatch.setenv("MPF_NR_CHUNK", str(lanes))
+    buses, branches = m.synth_grid(n_bus, int(1.5 * n_bus), max(2, n_bus // 6), 0.1, seed=4)
+    cases = outages(branches, n_bus, n_cases)
+    ref = oracle.runpf(buses, branches, cases, alg=m.NR, tol=1e-11)
+    with m.PowerFlow(buses, branches, tol=1e-11) as pf:
+        res = pf.runpf(cases, alg=m.NR, precision=prec)
+        st = pf.stats()
+    assert st["solve_lanes"] == lanes_that_run(n_bus, prec, lanes)
+    assert st["solve_in_shared"] == (st["solve_lanes"] > 0)
+    assert res.converged.all() and np.abs(res.v - ref["v"]).max() < 1e-8
+
+
+@pytest.mark.parametrize("in_shared", [True, False])
+@pytest.mark.parametrize("prec,lanes", [(m.FP64, 1), (m.FP64, 2), (m.FP64, 4), (m.MIXED, 1), (m.MIXED, 2),
+                                        (m.MIXED, 4), (m.MIXED, 8)])
+def test_forced_fast_decoupled_lanes_are_the_ones_that_run(gpu, monkeypatch, in_shared, prec, lanes):
+    monkeypatch.setenv("MPF_CHUNK_LANES", str(lanes))
+    if not in_shared:
+        monkeypatch.setenv("MPF_CHUNK_GLOBAL", "1")
+    for n_bus, n_cases in ((30, 1), (118, 33), (300, 70)):
+        buses, branches = grid(n_bus)
+        with m.PowerFlow(buses, branches) as pf:
+            assert pf.runpf(outages(branches, n_bus, n_cases), alg=m.FDXB, precision=prec).converged.all()
+            st = pf.stats()
+        assert (st["solve_lanes"], st["solve_in_shared"]) == (lanes, in_shared)
+
+
+# 160 cases of 8 lanes are 20 blocks, of 1 lane 160: one block per SM, or two with half of its
+# shared memory each.  The 900-bus uniform grid has supernodes larger than a ring slot, which are
+# read in place.
+@pytest.mark.parametrize("in_shared", [True, False])
+@pytest.mark.parametrize("prec,lanes", [(m.FP64, 1), (m.FP64, 2), (m.FP64, 4), (m.MIXED, 1), (m.MIXED, 2),
+                                        (m.MIXED, 4), (m.MIXED, 8)])
+@pytest.mark.parametrize("n_bus,n_cases,topology", [(30, 5, 0), (300, 160, 0), (900, 6, 1)])
+def test_adjoint_chunks_match_level_launches(gpu, monkeypatch, n_bus, n_cases, topology, prec, lanes, in_shared):
+    """Same factors, other order of the substitutions' sums: a backward error of about n 2^-53,
+    times a condition number of up to 1e5 here 1e-8 of the largest gradient.  (Mixed: both forms
+    are refined twice against the FP64 Jacobian, which leaves 1e-12.)"""
+    buses, branches = m.synth_grid(n_bus, int(1.45 * n_bus), n_bus // 5, 0.1, seed=5, topology=topology)
+    cases = outages(branches, n_bus, n_cases)
+    with m.PowerFlow(buses, branches, tol=1e-11) as pf:
+        pf.set_cases(cases)
+        pf.solve(m.NR, prec)
+        assert (pf.status() == m.runpf.CONVERGED).all()
+        pf.set_ratings(0.8 * np.abs(pf.branch_flows(flows=True)["sf"][0]))
+        monkeypatch.setenv("MPF_SUBST_CHUNK", "0")
+        ref = pf.adjoint(prec)
+        assert pf.stats()["adjoint_lanes"] == 0
+        monkeypatch.delenv("MPF_SUBST_CHUNK")
+        monkeypatch.setenv("MPF_CHUNK_LANES", str(lanes))
+        if not in_shared:
+            monkeypatch.setenv("MPF_CHUNK_GLOBAL", "1")
+        got = pf.adjoint(prec)
+        st = pf.stats()
+    assert (st["adjoint_lanes"], st["adjoint_in_shared"]) == (lanes, in_shared)
+    for k in ref:
+        assert np.abs(ref[k]).max() > 0.0
+        assert np.abs(got[k] - ref[k]).max() < 1e-8 * np.abs(ref[k]).max(), k
