@@ -2060,30 +2060,52 @@ void launch_bsolve_t(const LUSystem& sys, int ngroups, const T* pan, T* x, const
   }
 }
 
-// x <- (L U)^-T x for every lane: a block per chunk of lanes (k_subst_chunk), or for full
-// batches a launch per level with a case per thread.  The chunks save the levels' latency, but
-// they fill the GPU: level launches leave room for another handle's solve beside them, and
-// their fixed cost is spread over more cases.  ms per solve + adjoint, three handles in turn
-// (one alone), level launches / chunks:
-//   1354 buses, 4096 cases, FP32 11.0 (14.4) / 12.5 (13.2), FP64 12.5 (14.1) / 13.9 (14.4)
-//   700 x 4096 FP32 6.8 (9.1) / 8.5 (9.4);  300 x 4096 FP32 3.7 (5.1) / 3.6 (4.0)
-//   1354 x 2048 FP32 7.6 (10.8) / 7.8 (8.6), FP64 7.5 (9.0) / 8.0 (8.6);  2869 x 1000 FP32
-//   10.8 (18.7) / 11.3 (12.6);  2869 x 300 7.8 (15.4) / 7.6 (9.9);  300 x 1024 1.6 (2.6) / 1.2 (1.6)
-constexpr int kLevelSubstGroups = 128;             // groups of 32 lanes, twice in FP64
-constexpr long long kLevelSubstEntries = 1800000;  // and their LU entries
-// Returns the chunks' shape (G = 0: level launches).
+// Whether the adjoint's substitutions run on one block per chunk of lanes, and its shape (G = 0:
+// a launch per level with a case per thread), by estimated microseconds: the blocks' steps and
+// panels per wave, the levels' launches and the batch's entries.  Chunks save the levels'
+// latency but fill the GPU, where level launches leave room for another handle's solve: they
+// are taken below 0.7 of the level launches' estimate, which is where the gain of a handle
+// alone and the loss of three handles in turn (solve + adjoint each) cancel.  Fitted to 30 to
+// 9241 buses x 64 to 40000 cases.  ms per solve + adjoint alone (three in turn), level / chunks:
+//   FP64: 30 buses x 5000 0.80 (0.71) / 0.79 (0.74), x 20000 1.31 (1.14) / 1.54 (1.50)
+//     300 x 2000 3.23 (2.68) / 2.93 (2.66), x 8000 5.61 (4.96) / 5.82 (5.55)
+//     700 x 2000 5.07 (4.25) / 5.46 (4.96);  1354 x 1000 7.00 (5.74) / 6.16 (5.74)
+//     1354 x 4096 14.7 (13.2) / 15.0 (14.5);  9241 x 256 24.5 (17.9) / 19.0 (17.8)
+//   FP32: 30 x 5000 1.06 (0.90) / 0.90 (0.80), x 20000 1.46 (1.12) / 1.52 (1.38)
+//     300 x 4000 4.71 (3.39) / 3.66 (3.27), x 8000 5.99 (4.57) / 5.32 (4.88)
+//     1354 x 2048 10.3 (7.4) / 8.1 (7.4), x 4096 13.7 (10.6) / 12.6 (11.8)
+//     2869 x 1000 18.7 (11.6) / 12.6 (11.4);  9241 x 1000 47.4 (32.8) / 38.2 (35.4)
+template <typename T>
+ChunkShape choose_subst(LUSystem& S, int ngroups) {
+  ChunkShape none;
+  if (const char* e = std::getenv("MPF_SUBST_CHUNK"))  // testing: 0 off
+    if (std::atoi(e) == 0) return none;
+  const double isl = S.n_islands, nnz = (double)S.sym.nnz / isl;  // a lane's share: its own island
+  const double level = 19.0 * S.sym.nlevels + 0.021 * nnz + 5.3e-6 * nnz * 32.0 * ngroups;
+  auto chunks = [&](int G, double steps, bool xs) {
+    const int blocks = ngroups * (32 / G), fit = blocks > 148 ? 296 : 148;
+    return (blocks + fit - 1) / fit *
+           (1.65 * steps / isl + 0.0116 * nnz * G * sizeof(T) / 32.0 * (xs ? 1.0 : 1.3));
+  };
+  const bool forced = std::getenv("MPF_CHUNK_LANES") != nullptr;  // testing
+  bool possible = forced;
+  for (int G = Prec<T>::G; G >= 1 && !possible; G /= 2)
+    possible = chunks(G, 2.0 * S.sym.nlevels, true) < 0.7 * level;
+  if (!possible) return none;
+  const ChunkShape sh = choose_chunk({&S}, Prec<T>::G, sizeof(T), ngroups, 2);
+  return forced || chunks(sh.G, sh.plan[0]->steps, sh.xs) < 0.7 * level ? sh : none;
+}
+
+// x <- (L U)^-T x for every lane.  Returns the chunks' shape (G = 0: level launches).
 template <typename T>
 ChunkShape launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, const int* group_active, int device,
                           cudaStream_t st) {
-  const int words = ngroups * (int)sizeof(T) / 4;
-  const char* off = std::getenv("MPF_SUBST_CHUNK");  // testing: 0 off
-  if ((off && std::atoi(off) == 0) ||
-      (!std::getenv("MPF_CHUNK_LANES") && words >= kLevelSubstGroups && words * S.sym.nnz >= kLevelSubstEntries)) {
+  const ChunkShape sh = choose_subst<T>(S, ngroups);
+  if (sh.G == 0) {
     launch_fsolve_t<T>(S, ngroups, pan, cbr, x, group_active, st);
     launch_bsolve_t<T>(S, ngroups, pan, x, group_active, st);
-    return ChunkShape();
+    return sh;
   }
-  const ChunkShape sh = choose_chunk({&S}, Prec<T>::G, sizeof(T), ngroups, 2);
   with_shape<T>(sh, [&](auto g, auto xs) {
     constexpr int G = decltype(g)::value;
     constexpr bool XS = decltype(xs)::value;

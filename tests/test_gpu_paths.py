@@ -145,3 +145,17 @@ def test_adjoint_chunks_match_level_launches(gpu, monkeypatch, n_bus, n_cases, t
     for k in ref:
         assert np.abs(ref[k]).max() > 0.0
         assert np.abs(got[k] - ref[k]).max() < 1e-8 * np.abs(ref[k]).max(), k
+
+
+@pytest.mark.parametrize("prec,n_bus,n_cases,chunks", [(m.FP64, 30, 1000, True), (m.FP64, 30, 20000, False),
+                                                       (m.MIXED, 30, 2500, True), (m.MIXED, 30, 60000, False),
+                                                       (m.FP64, 300, 500, True), (m.FP64, 300, 12000, False)])
+def test_adjoint_form_by_batch(gpu, prec, n_bus, n_cases, chunks):
+    """A factor of two or more from the line on either side."""
+    buses, branches = grid(n_bus)
+    with m.PowerFlow(buses, branches) as pf:
+        pf.set_cases(outages(branches, n_bus, n_cases))
+        pf.solve(m.NR, prec)
+        pf.set_ratings(np.full(len(branches), 0.2))
+        pf.adjoint(prec)
+        assert (pf.stats()["adjoint_lanes"] > 0) == chunks
