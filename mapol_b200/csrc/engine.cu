@@ -237,6 +237,7 @@ struct FactorBufs {
   size_t most = 0, slot = 0;
   double cycles = 0.0;
   DevFactor dev() const { return DevFactor{step.as<int4>(), idx.as<int>(), n}; }
+  size_t bytes() const { return step.bytes + idx.bytes; }
 };
 
 // A block's substitution steps (SweepPlan) on the device
@@ -245,6 +246,7 @@ struct PlanBufs {
   size_t scratch = 0, slot = 0;  // as SweepPlan
   int peak_cb = 0, steps = 0;
   DevSweep dev() const { return DevSweep{step.as<int4>(), step_ptr.as<int>(), down_ptr.as<int>(), idx.as<int>()}; }
+  size_t bytes() const { return step.bytes + step_ptr.bytes + down_ptr.bytes + idx.bytes; }
 };
 
 struct LUSystem {
@@ -1725,7 +1727,7 @@ struct mpf_handle {
                            &any_active, &vout, &small_out, &fdvar, &eval_acc, &it_ctr, &br_dy,
                            &adj_status, &bus_island, &br_island, &group_island, &lane_case, &case_lane,
                            &sw_index, &sw_bus, &q_lim, &base_type, &pv_on, &q_fix, &q_flag, &iter_base, &case_cut,
-                           &adj_colptr, &adj_colent, &adj_b64, &adj_lam64};
+                           &adj_colptr, &adj_colent, &adj_b64, &adj_lam64, &isl_rows, &isl_row_ptr};
     for (auto p : all) b += p->bytes;
     b += ctl.bytes();
     const LUSystem* systems[] = {&jac, &bp[0], &bp[1], &bpp[0], &bpp[1]};
@@ -1734,8 +1736,10 @@ struct mpf_handle {
       const DevBuf* idx[] = {&s->sn_w, &s->sn_f, &s->sn_rptr, &s->sn_rows, &s->child_ptr, &s->child_list,
                              &s->sn_parent, &s->rel_ptr, &s->relmap, &s->ah_ptr, &s->ah_loc, &s->pan_off,
                              &s->cb_off, &s->cbr_off, &s->lev_sn, &s->top_sn, &s->top_lev_ptr,
-                             &s->child_ref, &s->cb_in};
+                             &s->child_ref, &s->cb_in, &s->sn_island};
       for (auto q : idx) b += q->bytes;
+      s->plans.each([&](const PlanBufs& p) { b += p.bytes(); });
+      s->fplans.each([&](const FactorBufs& p) { b += p.bytes(); });
     }
     for (int v = 0; v < 2; ++v) b += fdp[v].base.bytes + fdp[v].br_apos.bytes + fdp[v].br_bval.bytes +
                                      fdpp[v].base.bytes + fdpp[v].br_apos.bytes + fdpp[v].br_bval.bytes;

@@ -235,6 +235,11 @@ class PlanCache {
     return it->second.get();
   }
   void clear() { plans_.clear(); }
+  template <class F>  // f(const Plan&) for every plan kept
+  void each(F&& f) const {
+    for (const auto& p : plans_)
+      if (p.second) f(*p.second);
+  }
 
  private:
   std::map<Key, std::unique_ptr<Plan>> plans_;

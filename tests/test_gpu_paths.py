@@ -159,3 +159,20 @@ def test_adjoint_form_by_batch(gpu, prec, n_bus, n_cases, chunks):
         pf.set_ratings(np.full(len(branches), 0.2))
         pf.adjoint(prec)
         assert (pf.stats()["adjoint_lanes"] > 0) == chunks
+
+
+def test_device_bytes_count_the_plans(gpu, monkeypatch):
+    """The same batch on level launches and on chunks: the chunks' plans and row lists are device
+    memory of the handle, at least one index per entry of the grid's Ybus diagonal."""
+    buses, branches = grid(300)
+    cases = outages(branches, 300, 64)
+    held = {}
+    for alg, env in ((m.NR, "MPF_NR_CHUNK"), (m.FDXB, "MPF_FD_CHUNK")):
+        for on in ("0", "1"):
+            monkeypatch.setenv(env, on)
+            with m.PowerFlow(buses, branches) as pf:
+                assert pf.runpf(cases, alg=alg).converged.all()
+                assert (pf.stats()["solve_lanes"] > 0) == (on == "1")
+                held[alg, on] = pf.stats()["device_bytes"]
+        monkeypatch.delenv(env)
+        assert held[alg, "1"] > held[alg, "0"] + 4 * 300
