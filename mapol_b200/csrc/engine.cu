@@ -244,7 +244,7 @@ struct FactorBufs {
 struct PlanBufs {
   DevBuf step, step_ptr, down_ptr, idx;
   size_t scratch = 0, slot = 0;  // as SweepPlan
-  int peak_cb = 0, steps = 0;
+  int steps = 0;
   DevSweep dev() const { return DevSweep{step.as<int4>(), step_ptr.as<int>(), down_ptr.as<int>(), idx.as<int>()}; }
   size_t bytes() const { return step.bytes + step_ptr.bytes + down_ptr.bytes + idx.bytes; }
 };
@@ -260,6 +260,9 @@ struct LUSystem {
   PlanCache<std::tuple<bool, int, int, int>, PlanBufs> plans;
   // factorisation plans by (lanes, value bytes, kilobytes of shared memory)
   PlanCache<std::tuple<int, int, int>, FactorBufs> fplans;
+  // what is known of them before any is built
+  int sweep_cb = 0;
+  FactorNeeds fneeds;
   const int* group_island = nullptr; // the handle's current per-group islands (or null)
   std::vector<Launch> factor_sched;  // ascending levels
   std::vector<LaunchDeps> factor_deps;
@@ -349,6 +352,8 @@ struct LUSystem {
     upload(ah_loc, ahl);
     ah_host = ahp;
     ah_loc_host = ahl;
+    sweep_cb = sweep_peak_cb(s, h_sn_island);
+    fneeds = factor_needs(s, ahp);
     std::vector<long long> po(s.pan_off.begin(), s.pan_off.end()), co(s.cb_off.begin(), s.cb_off.end()),
         ro(s.cbr_off.begin(), s.cbr_off.end());
     upload(pan_off, po);
@@ -508,7 +513,6 @@ struct LUSystem {
       uploads_done();
       out.scratch = p.scratch;
       out.slot = p.slot;
-      out.peak_cb = p.peak_cb;
       out.steps = (int)p.step.size();
       return true;
     });
@@ -523,6 +527,7 @@ struct LUSystem {
       // the largest ring slots that leave room for the rest
       for (size_t slot = 24 * 1024; !ok && slot >= 3 * 1024 && n_islands == 1; slot = slot * 2 / 3 / 16 * 16)
         ok = (size_t)kb * 1024 > kRingSlots * slot &&
+             fneeds.fits(G, wsize, slot, (size_t)kb * 1024 - kRingSlots * slot) &&
              build_factor_plan(sym, ah_host, ah_loc_host, G, wsize, slot, (size_t)kb * 1024 - kRingSlots * slot, p);
       if (!ok) return false;
       std::vector<int4> st(p.step.size());
@@ -1968,11 +1973,8 @@ inline bool chunk_shape(const std::vector<LUSystem*>& sys, int G, int wsize, boo
   size_t held = kChunkScratch;
   if (want_xs) {
     for (LUSystem* s : sys) {
-      // any slot size gives the carried entries' slots
-      const PlanBufs* p = s->plan(true, G, wsize, 64);
-      if (!p) return false;
       out.xcap = std::max(out.xcap, (s->sym.n + 3) / 4 * 4);
-      out.ccap = std::max(out.ccap, (p->peak_cb + 3) / 4 * 4);
+      out.ccap = std::max(out.ccap, (s->sweep_cb + 3) / 4 * 4);
     }
     held += (size_t)(out.xcap + out.ccap) * G * wsize;
     out.xs = true;
@@ -2174,10 +2176,14 @@ NrShape choose_nr(LUSystem& S, int ngroups) {
   const double lanes = 32.0 * ngroups;
   double bt = 0.9 * (60.0 + 6.0 * (S.factor_sched.size() + S.bsolve_sched.size()) +
                      1e-5 * sizeof(T) / 4.0 * (double)S.sym.nnz * lanes);
-  for (int G = Prec<T>::G; G >= 1; G /= 2) {
-    if (!nr_shape(S, G, sizeof(T), sh)) continue;
+  auto chunks = [&](int G, double cycles) {
     const int waves = (ngroups * (32 / G) + 147) / 148;
-    const double t = fp64 * waves * (20.0 + 2.2 * sh.fac->cycles / 1900.0 + 0.02 * S.sym.n * G);
+    return fp64 * waves * (20.0 + 2.2 * cycles / 1900.0 + 0.02 * S.sym.n * G);
+  };
+  for (int G = Prec<T>::G; G >= 1; G /= 2) {
+    // (no plan is built where the least it could cost is too much)
+    if (chunks(G, S.fneeds.cycles) >= bt || !nr_shape(S, G, sizeof(T), sh)) continue;
+    const double t = chunks(G, sh.fac->cycles);
     if (t < bt) {
       bt = t;
       best = sh;

@@ -205,10 +205,24 @@ struct FactorPlan {
   size_t slot = 0;             // bytes of the largest step
   double cycles = 0.0;         // estimated clock cycles of a factorisation
 };
+// What every factorisation plan needs, whatever its lanes: a plan that does not fit() is refused
+// without being built.  cycles: less than any plan's.
+struct FactorNeeds {
+  int peak_cb = 0;             // as FactorPlan
+  size_t front = 0;            // values per lane of the largest front
+  double cycles = 0.0;
+  std::vector<std::pair<int64_t, int64_t>> tasks;  // a step of one supernode: arrowhead values, ints
+  bool fits(int G, int wsize, size_t slot, size_t smem) const;
+};
+FactorNeeds factor_needs(const LUSymbolic& s, const std::vector<int>& ah_ptr);
+
 // G lanes of wsize-byte values; slot: most bytes of a step; smem: bytes for contribution blocks
 // and fronts.  False when they do not fit.
 bool build_factor_plan(const LUSymbolic& s, const std::vector<int>& ah_ptr, const std::vector<int>& ah_loc, int G,
                        int wsize, size_t slot, size_t smem, FactorPlan& out);
+
+// SweepPlan::peak_cb of the plans with compact carried entries (any lanes and slot)
+int sweep_peak_cb(const LUSymbolic& s, const std::vector<int>& sn_island);
 
 // sn_island: each supernode's island (empty: one island); n_islands: how many there are, also
 // those without a supernode (0: as many as sn_island names).

@@ -883,6 +883,108 @@ std::string build_symbolic(const mpf_bus* buses, int nb, const mpf_branch* br, i
 }
 
 // ------------------------------------------------------------------ block plans
+namespace {
+// An island's supernodes by level, in panel order: level l is sn[lev[l]] .. sn[lev[l + 1]]
+struct IslandLevels {
+  std::vector<int> sn, lev;
+};
+std::vector<IslandLevels> island_levels(const LUSymbolic& s, const std::vector<int>& sn_island, int nisl) {
+  std::vector<IslandLevels> out(nisl);
+  for (int n = 0; n < s.nsn; ++n) out[sn_island.empty() ? 0 : sn_island[n]].sn.push_back(n);
+  for (IslandLevels& il : out) {
+    std::sort(il.sn.begin(), il.sn.end(), [&](int a, int b) {
+      return s.sn_level[a] != s.sn_level[b] ? s.sn_level[a] < s.sn_level[b] : s.pan_off[a] < s.pan_off[b];
+    });
+    il.lev.assign(1, 0);
+    for (size_t k = 1; k <= il.sn.size(); ++k)
+      if (k == il.sn.size() || s.sn_level[il.sn[k]] != s.sn_level[il.sn[k - 1]]) il.lev.push_back((int)k);
+    if (il.sn.empty()) il.lev.assign(1, 0);
+  }
+  return out;
+}
+
+// Slots of len(n) values by first fit, for blocks that live from their supernode's level to its
+// parent's (roots have none); at[n]: supernode n's.  The most alive at once.
+template <class Len>
+int first_fit(const LUSymbolic& s, const std::vector<int>& sn, const std::vector<int>& lev, Len len, std::vector<int>& at) {
+  std::vector<std::pair<int, int>> free_list{{0, INT_MAX}};  // (offset, length), ascending
+  int peak = 0;
+  for (size_t lv = 0; lv + 1 < lev.size(); ++lv) {
+    for (int k = lev[lv]; k < lev[lv + 1]; ++k) {
+      const int n = sn[k];
+      if (s.sn_parent[n] < 0) continue;
+      const int m = len(n);
+      for (auto& fr : free_list)
+        if (fr.second >= m) {
+          at[n] = fr.first;
+          fr.first += m;
+          fr.second -= m;
+          break;
+        }
+      peak = std::max(peak, at[n] + m);
+    }
+    for (int k = lev[lv]; k < lev[lv + 1]; ++k)
+      for (int c = s.child_ptr[sn[k]]; c < s.child_ptr[sn[k] + 1]; ++c) {
+        const int ch = s.child_list[c];
+        free_list.push_back({at[ch], len(ch)});
+      }
+    std::sort(free_list.begin(), free_list.end());
+    std::vector<std::pair<int, int>> merged;
+    for (auto& fr : free_list) {
+      if (fr.second == 0) continue;
+      if (!merged.empty() && merged.back().first + merged.back().second == fr.first) merged.back().second += fr.second;
+      else merged.push_back(fr);
+    }
+    free_list = merged;
+  }
+  return peak;
+}
+
+size_t step_bytes(int64_t ne, size_t ni, int G, int wsize) { return (size_t)((ne * G * wsize + 15) / 16 * 16) + ni * 4; }
+// values per lane of a front, and of a contribution block with its carried right-hand side
+size_t front_area(int f) { return (size_t)(f * plan_front_stride(f) + 3) / 4 * 4; }
+int block_values(int m) { return (m * m + m + 3) / 4 * 4; }
+}  // namespace
+
+int sweep_peak_cb(const LUSymbolic& s, const std::vector<int>& sn_island) {
+  int nisl = 1, peak = 0;
+  for (int k : sn_island) nisl = std::max(nisl, k + 1);
+  std::vector<int> cb(s.nsn, -1);
+  for (const IslandLevels& il : island_levels(s, sn_island, nisl))
+    peak = std::max(peak, first_fit(s, il.sn, il.lev, [&](int n) { return s.sn_f[n] - s.sn_w[n]; }, cb));
+  return peak;
+}
+
+FactorNeeds factor_needs(const LUSymbolic& s, const std::vector<int>& ah_ptr) {
+  FactorNeeds out;
+  std::vector<int> cb(s.nsn, -1);
+  out.peak_cb = first_fit(s, s.lev_sn, s.lev_ptr, [&](int n) { return block_values(s.sn_f[n] - s.sn_w[n]); }, cb);
+  std::vector<double> chain(s.nlevels, 0.0);
+  for (int n = 0; n < s.nsn; ++n) {
+    const int w = s.sn_w[n], f = s.sn_f[n];
+    int64_t ints = kStepInts + 8 + (ah_ptr[n + 1] - ah_ptr[n]) + w;
+    for (int c = s.child_ptr[n]; c < s.child_ptr[n + 1]; ++c) {
+      const int64_t m = s.sn_f[s.child_list[c]] - s.sn_w[s.child_list[c]];
+      ints += 2 + m * m + m;
+    }
+    out.tasks.push_back({ah_ptr[n + 1] - ah_ptr[n], (ints + 3) / 4 * 4});
+    out.front = std::max(out.front, front_area(f));
+    // the least of build_factor_plan's cost() over its teams and lanes
+    const double least = f <= 16 ? 900.0 + w * (f <= 8 ? 220.0 : 330.0)
+                                 : 900.0 + w * 500.0 + 10.0 * (0.6 * w * f * f + 3.0 * f * f) / kChunkThreads;
+    chain[s.sn_level[n]] = std::max(chain[s.sn_level[n]], least);
+  }
+  for (double c : chain) out.cycles += c;
+  return out;
+}
+
+bool FactorNeeds::fits(int G, int wsize, size_t slot, size_t smem) const {
+  if (smem / ((size_t)G * wsize) < peak_cb + front) return false;
+  for (const auto& t : tasks)
+    if (step_bytes(t.first, (size_t)t.second, G, wsize) > slot) return false;
+  return true;
+}
+
 bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bool compact_cb, int G, int wsize,
                       size_t slot, size_t scratch, SweepPlan& out, int n_islands) {
   out = SweepPlan();
@@ -891,55 +993,19 @@ bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bo
   // buses are all PV) has no supernode, but the kernels look its range of steps up
   int nisl = std::max(n_islands, 1);
   for (int k : sn_island) nisl = std::max(nisl, k + 1);
-  std::vector<std::vector<int>> of_island(nisl);
-  for (int n = 0; n < s.nsn; ++n) of_island[sn_island.empty() ? 0 : sn_island[n]].push_back(n);
+  const std::vector<IslandLevels> levels = island_levels(s, sn_island, nisl);
   std::vector<int> cb(s.nsn, -1);
   out.step_ptr.assign(1, 0);
-  auto bytes_of = [&](int64_t ne, size_t ni) { return (size_t)((ne * G * wsize + 15) / 16 * 16) + ni * 4; };
+  auto bytes_of = [&](int64_t ne, size_t ni) { return step_bytes(ne, ni, G, wsize); };
   for (int isl = 0; isl < nisl; ++isl) {
-    // the island's supernodes by level, in panel order
-    std::vector<int> sn = of_island[isl];
-    std::sort(sn.begin(), sn.end(), [&](int a, int b) {
-      return s.sn_level[a] != s.sn_level[b] ? s.sn_level[a] < s.sn_level[b] : s.pan_off[a] < s.pan_off[b];
-    });
-    std::vector<int> lev{0};
-    for (size_t k = 1; k <= sn.size(); ++k)
-      if (k == sn.size() || s.sn_level[sn[k]] != s.sn_level[sn[k - 1]]) lev.push_back((int)k);
-    if (sn.empty()) lev.assign(1, 0);
+    const std::vector<int>&sn = levels[isl].sn, &lev = levels[isl].lev;
     const int nlev = (int)lev.size() - 1;
-    // carried entries: slots by first fit over the levels at which they are alive
-    std::vector<std::pair<int, int>> free_list{{0, INT_MAX}};  // (offset, length), ascending
-    for (int lv = 0; lv < nlev; ++lv) {
-      for (int k = lev[lv]; k < lev[lv + 1]; ++k) {
-        const int n = sn[k], m = s.sn_f[n] - s.sn_w[n];
-        if (s.sn_parent[n] < 0) continue;
-        if (!compact_cb) {
-          cb[n] = (int)s.cbr_off[n];
-          continue;
-        }
-        for (auto& fr : free_list)
-          if (fr.second >= m) {
-            cb[n] = fr.first;
-            fr.first += m;
-            fr.second -= m;
-            break;
-          }
-        out.peak_cb = std::max(out.peak_cb, cb[n] + m);
-      }
-      if (!compact_cb) continue;
-      for (int k = lev[lv]; k < lev[lv + 1]; ++k)
-        for (int c = s.child_ptr[sn[k]]; c < s.child_ptr[sn[k] + 1]; ++c) {
-          const int ch = s.child_list[c];
-          free_list.push_back({cb[ch], s.sn_f[ch] - s.sn_w[ch]});
-        }
-      std::sort(free_list.begin(), free_list.end());
-      std::vector<std::pair<int, int>> merged;
-      for (auto& fr : free_list) {
-        if (fr.second == 0) continue;
-        if (!merged.empty() && merged.back().first + merged.back().second == fr.first) merged.back().second += fr.second;
-        else merged.push_back(fr);
-      }
-      free_list = merged;
+    // carried entries
+    if (compact_cb) {
+      out.peak_cb = std::max(out.peak_cb, first_fit(s, sn, lev, [&](int n) { return s.sn_f[n] - s.sn_w[n]; }, cb));
+    } else {
+      for (int n : sn)
+        if (s.sn_parent[n] >= 0) cb[n] = (int)s.cbr_off[n];
     }
     if (nlev == 0) out.down_ptr.push_back((int)out.step.size());
     for (int q = 0; q < 2 * nlev; ++q) {
@@ -1063,47 +1129,17 @@ bool build_factor_plan(const LUSymbolic& s, const std::vector<int>& ah_ptr, cons
   if (s.nnz >= INT_MAX) return false;
   const int nv = std::max(1, G * wsize / 16);  // threads per entry
   const int warps = kChunkThreads / 32;
-  auto area = [](int f) { return (size_t)(f * ((f + 1) | 1) + 3) / 4 * 4; };  // front_stride()
   // clock cycles of one front: its barriers and round trips in shared memory, its entries
   auto cost = [&](int w, int f, int team) {
     if (team == 32 && f <= (G * wsize <= 16 ? 16 : 8)) return 900.0 + w * (f <= 8 ? 220.0 : 330.0) + 10.0 * nv * 3.0 * f * f / team;
     return 900.0 + w * (team == 32 ? 600.0 : 500.0) + 10.0 * nv * (0.6 * w * f * f + 3.0 * f * f) / team;
   };
-  // contribution blocks (and their carried right-hand sides): slots by first fit over the
-  // levels at which they are alive
+  // contribution blocks (and their carried right-hand sides)
   std::vector<int> cb(s.nsn, -1);
-  std::vector<std::pair<int, int>> free_list{{0, INT_MAX}};
-  for (int lv = 0; lv < s.nlevels; ++lv) {
-    for (int k = s.lev_ptr[lv]; k < s.lev_ptr[lv + 1]; ++k) {
-      const int n = s.lev_sn[k], m = s.sn_f[n] - s.sn_w[n];
-      if (s.sn_parent[n] < 0) continue;
-      const int len = (m * m + m + 3) / 4 * 4;
-      for (auto& fr : free_list)
-        if (fr.second >= len) {
-          cb[n] = fr.first;
-          fr.first += len;
-          fr.second -= len;
-          break;
-        }
-      out.peak_cb = std::max(out.peak_cb, cb[n] + len);
-    }
-    for (int k = s.lev_ptr[lv]; k < s.lev_ptr[lv + 1]; ++k)
-      for (int c = s.child_ptr[s.lev_sn[k]]; c < s.child_ptr[s.lev_sn[k] + 1]; ++c) {
-        const int ch = s.child_list[c], m = s.sn_f[ch] - s.sn_w[ch];
-        free_list.push_back({cb[ch], (m * m + m + 3) / 4 * 4});
-      }
-    std::sort(free_list.begin(), free_list.end());
-    std::vector<std::pair<int, int>> merged;
-    for (auto& fr : free_list) {
-      if (fr.second == 0) continue;
-      if (!merged.empty() && merged.back().first + merged.back().second == fr.first) merged.back().second += fr.second;
-      else merged.push_back(fr);
-    }
-    free_list = merged;
-  }
+  out.peak_cb = first_fit(s, s.lev_sn, s.lev_ptr, [&](int n) { return block_values(s.sn_f[n] - s.sn_w[n]); }, cb);
   if ((size_t)out.peak_cb * G * wsize >= smem) return false;
   const size_t cap = smem / ((size_t)G * wsize) - out.peak_cb;  // values per lane for the fronts
-  auto bytes_of = [&](int64_t ne, size_t ni) { return (size_t)((ne * G * wsize + 15) / 16 * 16) + ni * 4; };
+  auto bytes_of = [&](int64_t ne, size_t ni) { return step_bytes(ne, ni, G, wsize); };
   // supernodes are numbered level by level, so a level's arrowheads are adjacent
   std::vector<int> lev{0};
   for (int n = 1; n <= s.nsn; ++n)
@@ -1156,7 +1192,7 @@ bool build_factor_plan(const LUSymbolic& s, const std::vector<int>& ah_ptr, cons
           return std::make_pair(w, f);
         };
         const auto wb = worst(0, nbig), wsm = worst(nbig, n);
-        const size_t bs = area(wb.second), ss = area(wsm.second);
+        const size_t bs = front_area(wb.second), ss = front_area(wsm.second);
         for (int lteam : {5, 7, 8, 9}) {
           const int team = 1 << lteam;
           if (team > kChunkThreads || (nbig == 0) != (lteam == 5)) continue;

@@ -33,3 +33,8 @@ def test_islands_without_supernodes_have_their_step_range(tmp_path):
 
 def test_plan_whose_upload_fails_is_built_again(tmp_path):
     assert run_native(tmp_path, "plan_cache_check").strip() == "ok"
+
+
+def test_plans_are_refused_only_where_they_cannot_fit(tmp_path):
+    out = run_native(tmp_path, "plan_needs_check").split()
+    assert int(out[1]) > 100 and int(out[3]) > 30 and int(out[5]) > 40, out
