@@ -139,7 +139,9 @@ typedef struct mpf_options {
 #define MPF_ORDER_MIN_FILL_WEIGHTED 3
 
 /* Per-kernel device time of the last mpf_solve (CUDA events on the solve stream),
- * milliseconds, summed over all launches of that kernel in the solve. */
+ * milliseconds, summed over all launches of that kernel in the solve.  A fast-decoupled solve
+ * on chunks (mpf_stats.solve_lanes > 0) is one launch: its time is divided as its blocks' clock
+ * cycles are between mismatches with their checks, substitutions and updates. */
 typedef struct mpf_timing {
   double total_ms;
   double mismatch_ms, jacobian_ms, factor_ms, solve_ms, update_ms, other_ms;

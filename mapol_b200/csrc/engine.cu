@@ -1587,7 +1587,10 @@ struct mpf_handle {
   bool have_cases = false, have_results = false;
   int last_alg = -1, last_prec = -1;
   cudaStream_t last_stream = nullptr;  // stream of the last solve / result copy
-  int* h_any = nullptr;  // pinned
+  int* h_any = nullptr;  // pinned, a LoopRecord's bytes
+  // shares of mismatch, substitution and update in solve_ms of the last solve (fast-decoupled on
+  // chunks is one launch); all 0: the families have launches of their own
+  double phase_share[kFdPhases] = {};
   EventTimer timer;
   mpf_timing timing;
   // captured Newton iteration per precision [FP64, FP32]
@@ -2532,11 +2535,16 @@ void solve_fd(mpf_handle* h, cudaStream_t st, int variant) {
     launch_fd_chunk<T>(h, d, fdd, Bp, Bpp, shape, st);
     ++nl;
     tm.end(ev);
-    // the largest iteration count over the chunks
-    CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    // the largest iteration count over the chunks, and where their time went
+    CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(LoopRecord), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
+    LoopRecord rec;
+    std::memcpy(&rec, h->h_any, sizeof rec);
+    double cycles = 0.0;
+    for (unsigned long long c : rec.cycles) cycles += (double)c;
+    for (int k = 0; k < kFdPhases; ++k) h->phase_share[k] = cycles > 0.0 ? (double)rec.cycles[k] / cycles : 0.0;
     h->timing.launches = nl;
-    h->timing.iterations_max = *h->h_any;
+    h->timing.iterations_max = rec.iterations;
     return;
   }
   if (h->opt.autotune)
@@ -2774,7 +2782,7 @@ int32_t mpf_create(const mpf_bus* buses, int32_t n_bus, const mpf_branch* branch
       if (!lim.empty()) return fail(h.get(), MPF_ERR_BAD_INPUT, lim);
     }
     CUDA_TRY(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
-    CUDA_TRY(cudaMallocHost(&h->h_any, sizeof(int)));
+    CUDA_TRY(cudaMallocHost(&h->h_any, sizeof(LoopRecord)));
     CUDA_TRY(cudaEventCreate(&h->t0));
     CUDA_TRY(cudaEventCreate(&h->t1));
     CUDA_TRY(cudaEventCreateWithFlags(&h->uploaded, cudaEventDisableTiming));
@@ -2825,7 +2833,7 @@ int32_t mpf_create(const mpf_bus* buses, int32_t n_bus, const mpf_branch* branch
     }
     upload_newton(h.get());
     h->any_active.alloc(sizeof(int));
-    h->it_ctr.alloc(sizeof(int));
+    h->it_ctr.alloc(sizeof(LoopRecord));
     return MPF_OK;
   });
   *out = h.release();
@@ -3353,6 +3361,7 @@ int32_t mpf_solve(mpf_handle* h, int32_t alg, int32_t precision, void* stream) {
     cudaStream_t st = stream ? (cudaStream_t)stream : h->own_stream;
     h->last_stream = st;
     std::memset(&h->timing, 0, sizeof(h->timing));
+    std::fill(h->phase_share, h->phase_share + kFdPhases, 0.0);
     h->timer.reset(st);
     after_uploads(h, st);
     CUDA_TRY(cudaEventRecord(h->t0, st));
@@ -3382,6 +3391,12 @@ int32_t mpf_get_timing(mpf_handle* h, mpf_timing* t) {
     CUDA_TRY(cudaEventSynchronize(h->t1));
     double ms[FAM_N];
     h->timer.collect(ms);
+    if (h->phase_share[PH_SUBST] > 0.0) {
+      const double all = ms[FAM_SOLVE];
+      ms[FAM_MIS] = all * h->phase_share[PH_MIS];
+      ms[FAM_SOLVE] = all * h->phase_share[PH_SUBST];
+      ms[FAM_UPD] = all * h->phase_share[PH_UPD];
+    }
     float tot = 0.f;
     CUDA_TRY(cudaEventElapsedTime(&tot, h->t0, h->t1));
     h->timing.total_ms = tot;

@@ -39,6 +39,15 @@ __device__ __forceinline__ size_t at32(int g, long long n, long long e, int lane
   return ((size_t)g * (size_t)n + (size_t)e) * 32 + lane;
 }
 
+// What a solve that needs no host between its iterations leaves for the host, in one read-back:
+// the iterations, and for mpf_timing the clock cycles that the blocks of a fast-decoupled solve
+// spent on mismatches (and checks), substitutions and updates
+enum { PH_MIS = 0, PH_SUBST = 1, PH_UPD = 2, kFdPhases = 3 };
+struct LoopRecord {
+  int iterations, pad;
+  unsigned long long cycles[kFdPhases];
+};
+
 struct DevGrid {
   int nb, nfree, ngroups, n_jac, nA_jac;
   int angle_mode;
@@ -65,7 +74,7 @@ struct DevGrid {
   unsigned long long* facc; // running max |F| (bits of a non-negative double)
   int* group_active;        // [ngroups]
   int* any_active;          // [1]
-  int* it_ptr;              // [1] Newton iterations done (graph replays read it)
+  int* it_ptr;              // iterations done (graph replays read it), the first field of a LoopRecord
   // per-case controls (null when none are set)
   const int* y_slot;        // [nnzY] control slot of a Ybus position or -1
   const double2* ctl_dy;    // [g][nslot][32] change of the Ybus entry at each slot
@@ -289,6 +298,7 @@ __global__ void k_init(DevGrid d, int ncases) {
   }
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.ngroups; g += gridDim.x * blockDim.x)
     d.group_active[g] = 1;
+  if (blockIdx.x == 0 && threadIdx.x < kFdPhases) reinterpret_cast<LoopRecord*>(d.it_ptr)->cycles[threadIdx.x] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) *d.it_ptr = 0;
 }
 

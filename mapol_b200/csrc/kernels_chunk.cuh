@@ -497,6 +497,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_fd_chunk(const __grid_cons
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[kChunkThreads / 32 * G];
   __shared__ int st[G];
+  __shared__ long long clk[kFdPhases + 1];  // cycles of each phase; when the current one began
   T* const sx = reinterpret_cast<T*>(smem_raw);
   T* const xs = XS ? sx + (size_t)(a.xcap + a.ccap) * G : sx;  // the teams' fronts
   const Ring R{reinterpret_cast<unsigned char*>(xs + (size_t)a.scratch * G), a.slot};
@@ -541,17 +542,31 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_fd_chunk(const __grid_cons
     sweep_begin<T, G>(a.sw[half], sp[0], sp[1], R, pan0(half));
   };
   begin(0);
+  auto lap = [&](int phase) {  // the time since the last lap was this phase's
+    if (threadIdx.x == 0) {
+      const long long now = clock64();
+      clk[phase] += now - clk[kFdPhases];
+      clk[kFdPhases] = now;
+    }
+  };
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < kFdPhases; ++k) clk[k] = 0;
+    clk[kFdPhases] = clock64();
+  }
   int it = 0, half = 0;
 #pragma unroll 1
   for (;;) {
     mismatch(half);
     // after the P half only convergence retires a case (fdpf.h:529-540); the iteration limit
     // is tested after the Q half (and at the start point)
-    if (!check(it, half == 1 ? INT_MAX : max_it)) break;
+    const bool on = check(it, half == 1 ? INT_MAX : max_it);
+    lap(PH_MIS);
+    if (!on) break;
     if (half == 0) ++it;
     const ChunkVec<T> v = vec(half);
     const int* sp = a.sw[half].step_ptr + island;
     sweep_run<T, G, S, false>(a.sw[half], sp[0], sp[1], R, xs, pan0(half), v);
+    lap(PH_SUBST);
     // the next half step's first panels come in while the voltages are updated
     begin(1 - half);
     if (st[l] == ST_RUNNING)
@@ -571,11 +586,16 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_fd_chunk(const __grid_cons
         d.V[k] = make_double2(mag * cs, mag * sn);
       }
     __syncthreads();
+    lap(PH_UPD);
     half = 1 - half;
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");  // the copies of a half step not taken
   if (threadIdx.x < G) d.status[c] = st[threadIdx.x];
-  if (threadIdx.x == 0) atomicMax(d.it_ptr, it);
+  if (threadIdx.x == 0) {
+    atomicMax(d.it_ptr, it);
+    for (int k = 0; k < kFdPhases; ++k)
+      atomicAdd(&reinterpret_cast<LoopRecord*>(d.it_ptr)->cycles[k], (unsigned long long)clk[k]);
+  }
 }
 
 // ---------------------------------------------------------------- Newton on one block

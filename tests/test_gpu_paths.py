@@ -176,3 +176,20 @@ def test_device_bytes_count_the_plans(gpu, monkeypatch):
                 held[alg, on] = pf.stats()["device_bytes"]
         monkeypatch.delenv(env)
         assert held[alg, "1"] > held[alg, "0"] + 4 * 300
+
+
+@pytest.mark.parametrize("use_graph", [2, 1, 0])
+@pytest.mark.parametrize("chunk", ["0", "1"])
+def test_fast_decoupled_times_by_family(gpu, monkeypatch, chunk, use_graph):
+    """Either form reports what mismatches, substitutions and updates took, and no more than the
+    solve."""
+    monkeypatch.setenv("MPF_FD_CHUNK", chunk)
+    buses, branches = grid(300)
+    with m.PowerFlow(buses, branches, use_graph=use_graph) as pf:
+        for _ in range(2):
+            assert pf.runpf(outages(branches, 300, 64), alg=m.FDXB).converged.all()
+        t = pf.timing()
+        assert (pf.stats()["solve_lanes"] > 0) == (chunk == "1")
+    parts = [t[k] for k in ("mismatch_ms", "solve_ms", "update_ms", "jacobian_ms", "factor_ms")]
+    assert min(parts) > 0.0 and sum(parts) + t["other_ms"] <= 1.001 * t["total_ms"]
+    assert t["solve_ms"] > t["update_ms"]
