@@ -80,3 +80,37 @@ def test_batches_of_more_groups_than_a_grid_has_rows(gpu):
             assert lib().mpf_mismatch(pf._h, v.data_ptr(), out.data_ptr(), None) == 0
             torch.cuda.synchronize()
             assert np.abs(out.cpu().numpy() - ref).max() < 1e-12 * max(1.0, np.abs(ys) * 10)
+
+
+def test_injections_laid_out_on_the_host_and_on_the_device(gpu):
+    """Few injections are laid out on the host, more on the device: the same mismatches of the same
+    cases, bit for bit, alone and as the first of a larger batch, and both refuse a value that is
+    not finite and keep the batch they had."""
+    import torch
+
+    from mapol_b200._lib import lib
+
+    buses, branches = m.synth_grid(300, 411, 69, 0.1, seed=2)
+    rng = np.random.default_rng(3)
+    n_small, n_large = 33, 400  # two groups: 19200 with padding lanes; the host takes 16384
+    sbus = np.stack([buses["p"], buses["q"]], -1)[None] * rng.uniform(0.5, 1.5, (n_large, 300, 2))
+    flat = np.stack([buses["vm"], np.zeros(300)], -1)
+    with m.PowerFlow(buses, branches) as pf:
+
+        def mismatch(n):
+            v = torch.from_numpy(np.repeat(flat[None], n, 0)).cuda()
+            out = torch.zeros(n, dtype=torch.float64, device="cuda")
+            assert lib().mpf_mismatch(pf._h, v.data_ptr(), out.data_ptr(), None) == 0
+            torch.cuda.synchronize()
+            return out.cpu().numpy()
+
+        pf.set_cases([[]] * n_large, sbus=sbus)
+        large = mismatch(n_large)
+        for n in (1, 27, 32, n_small, n_large):
+            pf.set_cases([[]] * n, sbus=sbus[:n])
+            assert np.array_equal(mismatch(n), large[:n])
+            bad = sbus[:n].copy()
+            bad[n - 1, 299, 1] = np.inf
+            with pytest.raises(m.MpfError, match="non-finite"):
+                pf.set_cases([[]] * n, sbus=bad)
+            assert np.array_equal(mismatch(n), large[:n])
