@@ -12,7 +12,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <functional>
 #include <map>
 #include <memory>
 #include <array>
@@ -2120,10 +2119,10 @@ ChunkShape launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, 
   with_shape<T>(sh, [&](auto g, auto xs) {
     constexpr int G = decltype(g)::value;
     constexpr bool XS = decltype(xs)::value;
-    allow_chunk_smem<k_subst_chunk<T, G, XS, true>>(device);
+    allow_chunk_smem<k_subst_chunk<T, G, XS>>(device);
     SubstChunk<T> a{sh.plan[0]->dev(), S.sym.n, S.sym.nnz, S.sym.cbr_off.back(), pan, cbr, x,
                     sh.xcap, sh.ccap, sh.scratch, sh.slot};
-    k_subst_chunk<T, G, XS, true><<<(unsigned)(ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(a, S.group_island);
+    k_subst_chunk<T, G, XS><<<(unsigned)(ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(a, S.group_island);
     CUDA_TRY(cudaGetLastError());
   });
   return sh;
@@ -2256,134 +2255,134 @@ void solve_nr(mpf_handle* h, cudaStream_t st) {
   // one Newton run over the running cases: mismatch at the current voltages, check,
   // then iterations until no case is running (first: also tune and capture)
   auto run_newton = [&](bool first) {
-  if (!first) CUDA_TRY(cudaMemsetAsync(h->it_ctr.p, 0, sizeof(int), st));
-  const bool tuned = !first || !h->opt.autotune || (J.tuned.count({P, h->ngroups}) && J.tuned_bs.count({P, h->ngroups}));
-  int it = 0;
-  if (chunk.G == 0 || !tuned) {
-  ev = tm.begin(FAM_MIS);
-  launch_mismatch_nr<T>(d, rg, st, x, A, max_it > 0);
-  ++nl;
-  tm.end(ev);
-  ev = tm.begin(FAM_OTHER);
-  check(h, st, 0, max_it, &nl);
-  tm.end(ev);
-  }
-  // pick the factorisation kernels of this batch size (first solve only), before
-  // the iteration is captured (the chunk kernel needs none, the adjoint does)
-  if (!tuned && max_it > 0 && any_active(h, st)) {
-    tune_factor<T>(J, h->ngroups, A, pan, cb, cbr, x, d.status, d.group_active, st);
-    tune_bsolve<T>(J, h->ngroups, pan, x, d.group_active, st);
-  }
-  if (chunk.G > 0) {
-    auto part = [&](int what, int fam) {
-      const int e = tm.begin(fam);
-      if (what == NR_MISMATCH) CUDA_TRY(cudaMemsetAsync(h->any_active.p, 0, sizeof(int), st));
-      launch_nr_chunk<T>(h, chunk, d, what, st);
-      tm.end(e);
+    if (!first) CUDA_TRY(cudaMemsetAsync(h->it_ctr.p, 0, sizeof(int), st));
+    const bool tuned = !first || !h->opt.autotune || (J.tuned.count({P, h->ngroups}) && J.tuned_bs.count({P, h->ngroups}));
+    int it = 0;
+    if (chunk.G == 0 || !tuned) {
+      ev = tm.begin(FAM_MIS);
+      launch_mismatch_nr<T>(d, rg, st, x, A, max_it > 0);
       ++nl;
-    };
-    if (h->opt.use_graph == 2) {
-      part(NR_ALL, FAM_OTHER);
+      tm.end(ev);
+      ev = tm.begin(FAM_OTHER);
+      check(h, st, 0, max_it, &nl);
+      tm.end(ev);
+    }
+    // pick the factorisation kernels of this batch size (first solve only), before
+    // the iteration is captured (the chunk kernel needs none, the adjoint does)
+    if (!tuned && max_it > 0 && any_active(h, st)) {
+      tune_factor<T>(J, h->ngroups, A, pan, cb, cbr, x, d.status, d.group_active, st);
+      tune_bsolve<T>(J, h->ngroups, pan, x, d.group_active, st);
+    }
+    if (chunk.G > 0) {
+      auto part = [&](int what, int fam) {
+        const int e = tm.begin(fam);
+        if (what == NR_MISMATCH) CUDA_TRY(cudaMemsetAsync(h->any_active.p, 0, sizeof(int), st));
+        launch_nr_chunk<T>(h, chunk, d, what, st);
+        tm.end(e);
+        ++nl;
+      };
+      if (h->opt.use_graph == 2) {
+        part(NR_ALL, FAM_OTHER);
+        CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        it = *h->h_any;
+      } else {  // the same in parts, for the kernel families' times
+        part(NR_MISMATCH, FAM_MIS);
+        while (it < max_it && any_active(h, st)) {
+          part(NR_FACTOR, FAM_FACT);
+          part(NR_SOLVE, FAM_SOLVE);
+          part(NR_UPDATE, FAM_UPD);
+          part(NR_MISMATCH, FAM_MIS);
+          ++it;
+        }
+      }
+      it_total += it;
+      return;
+    }
+    const bool dev_loop = h->opt.use_graph == 2;
+    if (h->opt.use_graph) {
+      // the captured kernels hold every device pointer of d by value: capture again
+      // when any of them (or the LU buffers) changed since
+      const void* key[4] = {A, pan, cb, x};
+      if ((gph.exec[0] || gph.loop_exec) &&
+          (gph.ngroups != h->ngroups || std::memcmp(gph.key, key, sizeof(key)) != 0 ||
+           std::memcmp(&gph.dkey, &d, sizeof(d)) != 0))
+        gph.release();
+      if (!gph.captured(dev_loop)) {
+        // capture on a private stream (the caller's may be the legacy one)
+        cudaStream_t cs;
+        CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+        if (!dev_loop) {
+          for (int part = 0; part < 4; ++part) {
+            CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+            gph.launches[part] = enqueue_nr_part<T>(h, part, cs, A, pan, cb, cbr, x);
+            CUDA_TRY(cudaStreamEndCapture(cs, &gph.graph[part]));
+            CUDA_TRY(cudaGraphInstantiate(&gph.exec[part], gph.graph[part], 0));
+          }
+        } else {
+          // head: the condition at entry; then a while node running the four parts and
+          // the condition again.  The update kernel counts iterations on the device, so
+          // the loop ends after at most max_it bodies whatever the cases do.
+          CUDA_TRY(cudaGraphCreate(&gph.loop_graph, 0));
+          cudaGraphConditionalHandle hc;
+          CUDA_TRY(cudaGraphConditionalHandleCreate(&hc, gph.loop_graph, 0, 0));
+          CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, gph.loop_graph, nullptr, nullptr, 0,
+                                                 cudaStreamCaptureModeThreadLocal));
+          k_loop_cond<<<1, 1, 0, cs>>>(hc, h->any_active.as<int>(), d.it_ptr, max_it);
+          CUDA_TRY(cudaGetLastError());
+          CUDA_TRY(cudaStreamEndCapture(cs, &gph.loop_graph));
+          cudaGraphNode_t head;
+          size_t nn = 1;
+          CUDA_TRY(cudaGraphGetNodes(gph.loop_graph, &head, &nn));
+          if (nn != 1) throw MpfError{MPF_ERR_CUDA, "device loop: the head graph should hold one kernel"};
+          cudaGraphNodeParams cp = {};
+          cp.type = cudaGraphNodeTypeConditional;
+          cp.conditional.handle = hc;
+          cp.conditional.type = cudaGraphCondTypeWhile;
+          cp.conditional.size = 1;
+          cudaGraphNode_t loop;
+          CUDA_TRY(cudaGraphAddNode(&loop, gph.loop_graph, &head, 1, &cp));
+          cudaGraph_t body = cp.conditional.phGraph_out[0];
+          CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+          int nlb = 0;
+          for (int part = 0; part < 4; ++part) nlb += enqueue_nr_part<T>(h, part, cs, A, pan, cb, cbr, x);
+          k_loop_cond<<<1, 1, 0, cs>>>(hc, h->any_active.as<int>(), d.it_ptr, max_it);
+          CUDA_TRY(cudaGetLastError());
+          CUDA_TRY(cudaStreamEndCapture(cs, &body));
+          CUDA_TRY(cudaGraphInstantiate(&gph.loop_exec, gph.loop_graph, 0));
+          gph.loop_launches = nlb + 1;
+        }
+        CUDA_TRY(cudaStreamDestroy(cs));
+        std::memcpy(gph.key, key, sizeof(key));
+        std::memcpy(&gph.dkey, &d, sizeof(d));
+        gph.ngroups = h->ngroups;
+      }
+    }
+    if (dev_loop) {
+      // one launch for all iterations; their count is read back once
+      const int e = tm.begin(FAM_OTHER);
+      CUDA_TRY(cudaGraphLaunch(gph.loop_exec, st));
+      tm.end(e);
       CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
       CUDA_TRY(cudaStreamSynchronize(st));
       it = *h->h_any;
-    } else {  // the same in parts, for the kernel families' times
-      part(NR_MISMATCH, FAM_MIS);
-      while (it < max_it && any_active(h, st)) {
-        part(NR_FACTOR, FAM_FACT);
-        part(NR_SOLVE, FAM_SOLVE);
-        part(NR_UPDATE, FAM_UPD);
-        part(NR_MISMATCH, FAM_MIS);
-        ++it;
+      nl += 1 + it * gph.loop_launches;
+    }
+    while (!dev_loop && it < max_it && any_active(h, st)) {
+      int e[4];
+      for (int part = 0; part < 4; ++part) {
+        e[part] = tm.begin(kFam[part]);
+        if (h->opt.use_graph) {
+          CUDA_TRY(cudaGraphLaunch(gph.exec[part], st));
+          nl += gph.launches[part];
+        } else {
+          nl += enqueue_nr_part<T>(h, part, st, A, pan, cb, cbr, x);
+        }
+        tm.end(e[part]);
       }
+      ++it;
     }
     it_total += it;
-    return;
-  }
-  const bool dev_loop = h->opt.use_graph == 2;
-  if (h->opt.use_graph) {
-    // the captured kernels hold every device pointer of d by value: capture again
-    // when any of them (or the LU buffers) changed since
-    const void* key[4] = {A, pan, cb, x};
-    if ((gph.exec[0] || gph.loop_exec) &&
-        (gph.ngroups != h->ngroups || std::memcmp(gph.key, key, sizeof(key)) != 0 ||
-         std::memcmp(&gph.dkey, &d, sizeof(d)) != 0))
-      gph.release();
-    if (!gph.captured(dev_loop)) {
-      // capture on a private stream (the caller's may be the legacy one)
-      cudaStream_t cs;
-      CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-      if (!dev_loop) {
-        for (int part = 0; part < 4; ++part) {
-          CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-          gph.launches[part] = enqueue_nr_part<T>(h, part, cs, A, pan, cb, cbr, x);
-          CUDA_TRY(cudaStreamEndCapture(cs, &gph.graph[part]));
-          CUDA_TRY(cudaGraphInstantiate(&gph.exec[part], gph.graph[part], 0));
-        }
-      } else {
-        // head: the condition at entry; then a while node running the four parts and
-        // the condition again.  The update kernel counts iterations on the device, so
-        // the loop ends after at most max_it bodies whatever the cases do.
-        CUDA_TRY(cudaGraphCreate(&gph.loop_graph, 0));
-        cudaGraphConditionalHandle hc;
-        CUDA_TRY(cudaGraphConditionalHandleCreate(&hc, gph.loop_graph, 0, 0));
-        CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, gph.loop_graph, nullptr, nullptr, 0,
-                                               cudaStreamCaptureModeThreadLocal));
-        k_loop_cond<<<1, 1, 0, cs>>>(hc, h->any_active.as<int>(), d.it_ptr, max_it);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaStreamEndCapture(cs, &gph.loop_graph));
-        cudaGraphNode_t head;
-        size_t nn = 1;
-        CUDA_TRY(cudaGraphGetNodes(gph.loop_graph, &head, &nn));
-        if (nn != 1) throw MpfError{MPF_ERR_CUDA, "device loop: the head graph should hold one kernel"};
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = hc;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t loop;
-        CUDA_TRY(cudaGraphAddNode(&loop, gph.loop_graph, &head, 1, &cp));
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        int nlb = 0;
-        for (int part = 0; part < 4; ++part) nlb += enqueue_nr_part<T>(h, part, cs, A, pan, cb, cbr, x);
-        k_loop_cond<<<1, 1, 0, cs>>>(hc, h->any_active.as<int>(), d.it_ptr, max_it);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaStreamEndCapture(cs, &body));
-        CUDA_TRY(cudaGraphInstantiate(&gph.loop_exec, gph.loop_graph, 0));
-        gph.loop_launches = nlb + 1;
-      }
-      CUDA_TRY(cudaStreamDestroy(cs));
-      std::memcpy(gph.key, key, sizeof(key));
-      std::memcpy(&gph.dkey, &d, sizeof(d));
-      gph.ngroups = h->ngroups;
-    }
-  }
-  if (dev_loop) {
-    // one launch for all iterations; their count is read back once
-    const int e = tm.begin(FAM_OTHER);
-    CUDA_TRY(cudaGraphLaunch(gph.loop_exec, st));
-    tm.end(e);
-    CUDA_TRY(cudaMemcpyAsync(h->h_any, d.it_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    it = *h->h_any;
-    nl += 1 + it * gph.loop_launches;
-  }
-  while (!dev_loop && it < max_it && any_active(h, st)) {
-    int e[4];
-    for (int part = 0; part < 4; ++part) {
-      e[part] = tm.begin(kFam[part]);
-      if (h->opt.use_graph) {
-        CUDA_TRY(cudaGraphLaunch(gph.exec[part], st));
-        nl += gph.launches[part];
-      } else {
-        nl += enqueue_nr_part<T>(h, part, st, A, pan, cb, cbr, x);
-      }
-      tm.end(e[part]);
-    }
-    ++it;
-  }
-  it_total += it;
   };
   run_newton(true);
   // reactive limits: switch the violating PV buses of converged cases to PQ and run

@@ -1614,9 +1614,9 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
         }
         const int nta = (sr + 3) / 4, ntb = (bc + 3) / 4;
         for (int tt = slot; tt < nta * ntb; tt += SLOTS) {
-          // rows ra + ii, columns cb + jj ntb: a warp's tiles read adjacent columns (no bank
+          // rows ra + ii, columns col + jj ntb: a warp's tiles read adjacent columns (no bank
           // conflicts); rows and columns past the end repeat the last one and are not stored
-          const int ra = (tt / ntb) * 4, cb = tt % ntb;
+          const int ra = (tt / ntb) * 4, col = tt % ntb;
           T acc[4][4];
           const T* lb[4];
           const T* ub[4];
@@ -1629,7 +1629,7 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
           }
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj) {
-            to[jj] = min(cb + jj * ntb, bc - 1);
+            to[jj] = min(col + jj * ntb, bc - 1);
             ub[jj] = P + (size_t)(w + to[jj]) * G + l;  // u of column w + b (w + m: the right-hand side)
           }
 #pragma unroll
@@ -1652,7 +1652,7 @@ __global__ void __launch_bounds__(512, 1) k_mf_factor_big(DevLU L, const int* __
           for (int ii = 0; ii < 4; ++ii)
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj)
-              if (ra + ii < sr && cb + jj * ntb < bc) Sb[(size_t)(at[ii] + to[jj]) * G] = acc[ii][jj];
+              if (ra + ii < sr && col + jj * ntb < bc) Sb[(size_t)(at[ii] + to[jj]) * G] = acc[ii][jj];
         }
         __syncthreads();
         {
@@ -2426,51 +2426,51 @@ __global__ void __launch_bounds__(256) k_adj_grad_branch(DevGrid d, int nbr, int
   const bool ok = case_of_lane(d, c, ncases) >= 0 && d.status[c] == ST_CONVERGED;
   __shared__ double tg[32][33], tb[32][33];
   for (int k0 = blockIdx.x * 64; k0 < min(nbr, (int)(blockIdx.x + 1) * 64); k0 += 32) {
-  for (int q = warp; q < 32 && k0 + q < nbr; q += 8) {
-    const int k = k0 + q;
-    double rg = 0.0, rb = 0.0;
-    if (ok && branch_here(d, k, grp) && !outaged(o, k)) {
-      const int2 ft = d.br_ft[k];
-      double2 y[4], a[4];
-      branch_y(d, k, grp, lane, y);
-      const int jc = d.br_ctl ? d.br_ctl[k] : -1;
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        a[q] = jc < 0 ? br_dy[4 * k + q] : d.ctl_bdy[at32(grp, 4 * d.noltc, 4 * jc + q, lane)];
-      const double2 vf = d.V[at32(grp, d.nb, ft.x, lane)], vt = d.V[at32(grp, d.nb, ft.y, lane)];
-      // Df = Vf conj(a_ff Vf + a_ft Vt), Dt = Vt conj(a_tf Vf + a_tt Vt)
-      const double2 u = make_double2(a[0].x * vf.x - a[0].y * vf.y + a[1].x * vt.x - a[1].y * vt.y,
-                                     a[0].x * vf.y + a[0].y * vf.x + a[1].x * vt.y + a[1].y * vt.x);
-      const double2 Df = make_double2(vf.x * u.x + vf.y * u.y, vf.y * u.x - vf.x * u.y);
-      const double2 u2 = make_double2(a[2].x * vf.x - a[2].y * vf.y + a[3].x * vt.x - a[3].y * vt.y,
-                                      a[2].x * vf.y + a[2].y * vf.x + a[3].x * vt.y + a[3].y * vt.x);
-      const double2 Dt = make_double2(vt.x * u2.x + vt.y * u2.y, vt.y * u2.x - vt.x * u2.y);
-      // explicit part through this branch's own Sf
-      const double2 yv = make_double2(y[0].x * vf.x - y[0].y * vf.y + y[1].x * vt.x - y[1].y * vt.y,
-                                      y[0].x * vf.y + y[0].y * vf.x + y[1].x * vt.y + y[1].y * vt.x);
-      const double2 S = make_double2(vf.x * yv.x + vf.y * yv.y, vf.y * yv.x - vf.x * yv.y);
-      const double aS = sqrt(S.x * S.x + S.y * S.y);
-      const double E = aS - 0.9 * rating[k];
-      if (E > 0.0) {
-        const double cc = 2.0 * E / aS;
-        rg += cc * (S.x * Df.x + S.y * Df.y);
-        rb += cc * (S.x * Df.y - S.y * Df.x);
+    for (int q = warp; q < 32 && k0 + q < nbr; q += 8) {
+      const int k = k0 + q;
+      double rg = 0.0, rb = 0.0;
+      if (ok && branch_here(d, k, grp) && !outaged(o, k)) {
+        const int2 ft = d.br_ft[k];
+        double2 y[4], a[4];
+        branch_y(d, k, grp, lane, y);
+        const int jc = d.br_ctl ? d.br_ctl[k] : -1;
+  #pragma unroll
+        for (int q = 0; q < 4; ++q)
+          a[q] = jc < 0 ? br_dy[4 * k + q] : d.ctl_bdy[at32(grp, 4 * d.noltc, 4 * jc + q, lane)];
+        const double2 vf = d.V[at32(grp, d.nb, ft.x, lane)], vt = d.V[at32(grp, d.nb, ft.y, lane)];
+        // Df = Vf conj(a_ff Vf + a_ft Vt), Dt = Vt conj(a_tf Vf + a_tt Vt)
+        const double2 u = make_double2(a[0].x * vf.x - a[0].y * vf.y + a[1].x * vt.x - a[1].y * vt.y,
+                                       a[0].x * vf.y + a[0].y * vf.x + a[1].x * vt.y + a[1].y * vt.x);
+        const double2 Df = make_double2(vf.x * u.x + vf.y * u.y, vf.y * u.x - vf.x * u.y);
+        const double2 u2 = make_double2(a[2].x * vf.x - a[2].y * vf.y + a[3].x * vt.x - a[3].y * vt.y,
+                                        a[2].x * vf.y + a[2].y * vf.x + a[3].x * vt.y + a[3].y * vt.x);
+        const double2 Dt = make_double2(vt.x * u2.x + vt.y * u2.y, vt.y * u2.x - vt.x * u2.y);
+        // explicit part through this branch's own Sf
+        const double2 yv = make_double2(y[0].x * vf.x - y[0].y * vf.y + y[1].x * vt.x - y[1].y * vt.y,
+                                        y[0].x * vf.y + y[0].y * vf.x + y[1].x * vt.y + y[1].y * vt.x);
+        const double2 S = make_double2(vf.x * yv.x + vf.y * yv.y, vf.y * yv.x - vf.x * yv.y);
+        const double aS = sqrt(S.x * S.x + S.y * S.y);
+        const double E = aS - 0.9 * rating[k];
+        if (E > 0.0) {
+          const double cc = 2.0 * E / aS;
+          rg += cc * (S.x * Df.x + S.y * Df.y);
+          rb += cc * (S.x * Df.y - S.y * Df.x);
+        }
+        const int2 vfv = d.jvar[ft.x], vtv = d.jvar[ft.y];
+        const double lPf = vfv.x >= 0 ? (double)lam[at32(grp, d.n_jac, vfv.x, lane)] : 0.0;
+        const double lQf = vfv.y >= 0 ? (double)lam[at32(grp, d.n_jac, vfv.y, lane)] : 0.0;
+        const double lPt = vtv.x >= 0 ? (double)lam[at32(grp, d.n_jac, vtv.x, lane)] : 0.0;
+        const double lQt = vtv.y >= 0 ? (double)lam[at32(grp, d.n_jac, vtv.y, lane)] : 0.0;
+        rg -= lPf * Df.x + lQf * Df.y + lPt * Dt.x + lQt * Dt.y;
+        rb -= lPf * Df.y - lQf * Df.x + lPt * Dt.y - lQt * Dt.x;
       }
-      const int2 vfv = d.jvar[ft.x], vtv = d.jvar[ft.y];
-      const double lPf = vfv.x >= 0 ? (double)lam[at32(grp, d.n_jac, vfv.x, lane)] : 0.0;
-      const double lQf = vfv.y >= 0 ? (double)lam[at32(grp, d.n_jac, vfv.y, lane)] : 0.0;
-      const double lPt = vtv.x >= 0 ? (double)lam[at32(grp, d.n_jac, vtv.x, lane)] : 0.0;
-      const double lQt = vtv.y >= 0 ? (double)lam[at32(grp, d.n_jac, vtv.y, lane)] : 0.0;
-      rg -= lPf * Df.x + lQf * Df.y + lPt * Dt.x + lQt * Dt.y;
-      rb -= lPf * Df.y - lQf * Df.x + lPt * Dt.y - lQt * Dt.x;
+      tg[q][lane] = rg;
+      tb[q][lane] = rb;
     }
-    tg[q][lane] = rg;
-    tb[q][lane] = rb;
-  }
-  __syncthreads();
-  if (gg) write_tile(d, tg, grp, k0, nbr, ncases, gg, warp, 8);
-  if (gb) write_tile(d, tb, grp, k0, nbr, ncases, gb, warp, 8);
-  __syncthreads();
+    __syncthreads();
+    if (gg) write_tile(d, tg, grp, k0, nbr, ncases, gg, warp, 8);
+    if (gb) write_tile(d, tb, grp, k0, nbr, ncases, gb, warp, 8);
+    __syncthreads();
   }
 }
 

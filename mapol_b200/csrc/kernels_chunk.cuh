@@ -11,7 +11,7 @@
 // panels and index lists, stored in the order of the walk) streams through a ring buffer in
 // shared memory with cp.async, two steps ahead.  A step then costs a barrier and its
 // arithmetic.  Small supernodes (most of them) take 1 to 8 threads per lane without barriers,
-// and the few larger fronts of a step run beside them on teams of 32 to 1024 threads.
+// and the few larger fronts of a step run beside them on teams of 32 to 512 threads.
 #pragma once
 
 #include "internal.h"
@@ -291,9 +291,10 @@ __device__ __forceinline__ void sweep_begin(const DevSweep& P, int s0, int s1, c
 }
 
 // The steps [s0, s1) by the block, after sweep_begin (TR: with the transposed factors): an
-// island's whole range is both substitutions, from its down_ptr the second one.  pan0: the panels at the chunk's first lane; v: x and the carried entries at
-// this thread's lane (threadIdx.x % G); xs: the teams' fronts.  Ends with a block barrier;
-// every copy it started has landed.
+// island's whole range is both substitutions, from its down_ptr the second one.  pan0: the
+// panels at the chunk's first lane; v: x and the carried entries at this thread's lane
+// (threadIdx.x % G); xs: the teams' fronts.  Ends with a block barrier; every copy it started
+// has landed.
 template <typename T, int G, int S, bool TR>
 __device__ __forceinline__ void sweep_run(const DevSweep& P, int s0, int s1, const Ring& R, T* xs, const T* pan0,
                                           const ChunkVec<T>& v) {
@@ -361,8 +362,8 @@ __device__ __forceinline__ void sweep_run(const DevSweep& P, int s0, int s1, con
   __syncthreads();
 }
 
-// Both substitutions with the (transposed, TR) factors of one system for a chunk of lanes:
-// x in place.  XS: x and the carried entries in shared memory.
+// Both substitutions with the transposed factors of one system (the adjoint's) for a chunk of
+// lanes: x in place.  XS: x and the carried entries in shared memory.
 template <typename T>
 struct SubstChunk {
   DevSweep sw;
@@ -373,7 +374,7 @@ struct SubstChunk {
   T* x;
   int xcap, ccap, scratch, slot;  // as FdChunk
 };
-template <typename T, int G, bool XS, bool TR>
+template <typename T, int G, bool XS>
 __global__ void __launch_bounds__(kChunkThreads, 2) k_subst_chunk(const __grid_constant__ SubstChunk<T> a,
                                                                   const int* __restrict__ group_island) {
   constexpr int LPG = 32 / G, S = XS ? G : 32;
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(kChunkThreads, 2) k_subst_chunk(const __grid_c
     for (int i = threadIdx.x / G; i < a.n; i += kChunkThreads / G) sx[i * G + l] = gx[(size_t)i * 32];
   const ChunkVec<T> v = XS ? ChunkVec<T>{sx + l, sx + (size_t)a.xcap * G + l}
                            : ChunkVec<T>{gx, a.cbr + at32(g, a.sumcbr, 0, lane0 + l)};
-  sweep_run<T, G, S, TR>(a.sw, s0, s1, R, xs, pan0, v);
+  sweep_run<T, G, S, true>(a.sw, s0, s1, R, xs, pan0, v);
   if (XS)
     for (int i = threadIdx.x / G; i < a.n; i += kChunkThreads / G) gx[(size_t)i * 32] = sx[i * G + l];
 }

@@ -1079,8 +1079,7 @@ bool build_sweep_plan(const LUSymbolic& s, const std::vector<int>& sn_island, bo
           // clock cycles: a task's latency, its pivots with a barrier each, its work over
           // the team's threads
           double best = -1.0;
-          for (int team : {32, 128, 256, 512, 1024}) {
-            if (team > kChunkThreads) break;
+          for (int team : {32, 128, 256, kChunkThreads}) {
             const int nt = std::min(std::min(kChunkThreads / team, room), st.nbig);
             if (nt < 1) break;
             const double t = (double)((st.nbig + nt - 1) / nt) *
