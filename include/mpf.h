@@ -113,17 +113,27 @@ typedef struct mpf_options {
   int32_t angle_mode;  /* 0: atan2 (default); 1: atan(y/x) as cuCangle in
                           src/util/complexUtils.h:21-23 (loses the quadrant) */
   int32_t device;      /* CUDA device ordinal, default 0 */
-  int32_t use_graph;   /* 2: the whole Newton loop as one CUDA graph whose while node
-                          tests "any case running" and the iteration count on the device
-                          (one read-back per solve; mpf_timing then reports the loop in
-                          other_ms) (default 2); 1: the Newton iteration as captured CUDA
-                          graphs, the host reads one flag per iteration and mpf_timing
-                          splits the solve by kernel family; 0: direct launches.  All
-                          three give the same results bit for bit. */
+  int32_t use_graph;   /* how a Newton solve on level launches is driven.  2: the whole loop as
+                          one CUDA graph whose while node tests "any case running" and the
+                          iteration count on the device (one read-back per solve; mpf_timing
+                          then reports the loop in other_ms) (default 2); 1: the Newton
+                          iteration as captured CUDA graphs, the host reads one flag per
+                          iteration and mpf_timing splits the solve by kernel family; 0:
+                          direct launches.  A Newton solve on chunks (autotune) uses no
+                          graph: 2 is one launch for the whole solve (its time in other_ms),
+                          1 and 0 a launch per part of an iteration, timed by family.  All
+                          give the same results bit for bit.  Fast-decoupled solves do not
+                          look at it. */
   int32_t autotune;    /* 1: time the candidate kernels of every factorisation launch on
                           the first solve of a batch size and keep the fastest, and run
-                          Newton on one block per chunk of cases where that is faster
-                          (default 1); 0: level launches by a fixed heuristic */
+                          Newton on one block per chunk of cases where that is estimated to
+                          be faster (default 1); 0: Newton on level launches by a fixed
+                          heuristic.  The iterations of fast-decoupled solves and the
+                          adjoint's substitutions choose between chunks and level launches
+                          by their own estimate, whatever this says (mpf_stats tells which
+                          ran).  The form depends on the batch size, and sums are ordered
+                          differently in each: a case's voltages may differ in their last
+                          bits between batches of different sizes. */
   int32_t ordering;    /* fill-reducing bus order of the Newton system, MPF_ORDER_*:
                           0 automatic (default), 1 minimum degree, 2 minimum fill,
                           3 minimum fill weighted by variables per bus */

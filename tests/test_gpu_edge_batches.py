@@ -114,3 +114,30 @@ def test_injections_laid_out_on_the_host_and_on_the_device(gpu):
             with pytest.raises(m.MpfError, match="non-finite"):
                 pf.set_cases([[]] * n, sbus=bad)
             assert np.array_equal(mismatch(n), large[:n])
+
+
+def test_evaluation_captured_right_after_new_cases(gpu):
+    """mpf_mismatch_noalloc in a stream capture, called while the uploads of mpf_set_cases may still
+    run: the replay gives what the plain call gives."""
+    import torch
+
+    from mapol_b200._lib import lib
+
+    buses, branches, cases = m.workload("cfg1_300bus")
+    flat = np.repeat(np.stack([buses["vm"] * np.cos(buses["va"]), buses["vm"] * np.sin(buses["va"])], -1)[None], 64, 0)
+    v = torch.from_numpy(flat).cuda()
+    ref = torch.zeros(64, dtype=torch.float64, device="cuda")
+    got = torch.zeros(64, dtype=torch.float64, device="cuda")
+    with m.PowerFlow(buses, branches) as pf:
+        pf.set_cases(cases[:64])
+        assert lib().mpf_mismatch_noalloc(pf._h, v.data_ptr(), ref.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+        side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        pf.set_cases(cases[:64])
+        with torch.cuda.graph(graph, stream=side):
+            rc = lib().mpf_mismatch_noalloc(pf._h, v.data_ptr(), got.data_ptr(), side.cuda_stream)
+        assert rc == 0, lib().mpf_last_error(pf._h)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(got.cpu().numpy(), ref.cpu().numpy()) and (ref > 0).all()
+        del graph
