@@ -414,14 +414,15 @@ __device__ __forceinline__ void jac_off(T* Ag, int4 jp, T yr, T yi, T c, T d, T 
 
 // What a block's rows share among their cases, staged in shared memory before the rows are
 // walked: per row its bus, Ybus range, place here, diagonal and variables; per Ybus entry its
-// column, base value and Jacobian positions.  The kernel issued 190 instructions per entry and
+// column, base value and Jacobian positions.  The kernel issued 173 instructions per entry and
 // 32 cases (address arithmetic, loads of these arrays, the outages' registers spilled) and a
 // row was a chain of loads (row -> range -> column -> voltage -> Jacobian positions).  Staged
 // by four threads per row the chain is walked once per block; a row waits for its voltages
 // alone, asked for one entry ahead, and an off-diagonal entry's four J values come from two
-// products.  With the Jacobian, 1000 cases of 9241 buses, mixed: 425 -> 329 us (0.87 GB, 2.6
-// TB/s; still bound by issue, at 24 warps per SM: 80 registers without spills beat 64 with
-// them, 338); 256 of 2869, FP64: 72 -> 51.  Batches of 2 or 4 entries per round: 365 and 367.
+// products (120 instructions).  With the Jacobian, 1000 cases of 9241 buses, mixed: 425 -> 329
+// us (0.87 GB, 2.6 TB/s; still bound by issue, at 24 warps per SM: 80 registers without spills
+// beat 64 with them, 338); 256 of 2869, FP64: 72 -> 51.  Batches of 2 or 4 entries per round:
+// 365 and 367.
 // kMisEntries: 64 rows of 7 entries, more than a block of a transmission grid has (4 to 5 per
 // row); a row that finds no room here, and all behind it, is read from global memory.
 constexpr int kMisEntries = 448;
@@ -1328,9 +1329,9 @@ __global__ void __launch_bounds__(TEAM == 32 ? 288 : TEAM, TT > 0 ? 2 : (TEAM > 
 // Contribution blocks between two large fronts are stored [lane pair][entry][2] instead of
 // [entry][32]: a large front's task owns 1 to 4 lanes, which are 4 to 16 bytes of every
 // 128-byte row, so its reads and writes of the m x m block moved 32-byte sectors for them, one
-// line per entry (80% of the kernel's time); paired, a warp's accesses are contiguous.  Solve
-// of 250 cases of the uniform 1354-bus grid, mixed: 49.2 -> 34.6 ms, and 30.2 with the blocks
-// asked from DRAM at the task's start.
+// line per entry; paired, a warp's accesses are contiguous.  Solve of 250 cases of the uniform
+// 1354-bus grid, mixed: 49.2 -> 34.6 ms, and 30.2 with the blocks asked from DRAM at the task's
+// start.
 // Entry e of lane `lane` of the block at off (len entries): p[e * step].
 constexpr int kBigFront = 167;  // fronts above this many rows are large (kFmaxAll)
 template <typename T>

@@ -477,7 +477,8 @@ __device__ __forceinline__ double chunk_mismatch_fd(const DevGrid& d, const DevF
 // check, then up to max_it iterations of two half steps (forward and backward
 // substitution with the stored factors of B' / B'', update, mismatch, check).  Replaces
 // a launch per level for each of the four substitutions of an iteration and a host read
-// of the "any case running" flag per half step.
+// of the "any case running" flag per half step; large
+// batches, whose waves of blocks take longer than that, keep the level launches (choose_fd).
 // XS: x and the carried entries of the half step in shared memory (else in the systems' arrays)
 template <typename T>
 struct FdChunk {  // [0]: B' (P half steps), [1]: B'' (Q half steps)
