@@ -1809,17 +1809,19 @@ int fail(mpf_handle* h, int code, const std::string& msg) {
 }
 
 // This thread's uploads so far are behind the handle's event
-void mark_uploads(mpf_handle* h) {
-  if (!uploads_pending || !h->uploaded) return;
-  CUDA_TRY(cudaEventRecord(h->uploaded, cudaStreamLegacy));
+cudaError_t mark_uploads(mpf_handle* h) {
+  if (!uploads_pending || !h->uploaded) return cudaSuccess;
+  const cudaError_t e = cudaEventRecord(h->uploaded, cudaStreamLegacy);
+  if (e != cudaSuccess) return e;
   h->uploads_running = true;
   uploads_pending = false;
+  return cudaSuccess;
 }
 
 // What is launched on st from here on runs after the handle's uploads.  (A capture cannot hold
 // the event: there the wait is the host's, in the mode that allows it beside a capture.)
 void after_uploads(mpf_handle* h, cudaStream_t st) {
-  mark_uploads(h);
+  CUDA_TRY(mark_uploads(h));
   if (!h->uploads_running) return;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(st, &cs));
@@ -1837,17 +1839,21 @@ void after_uploads(mpf_handle* h, cudaStream_t st) {
 
 template <class F>
 int guarded(mpf_handle* h, F&& f) {
-  try {
-    const int rc = f();
-    mark_uploads(h);
-    return rc;
-  } catch (const MpfError& e) {
-    return fail(h, e.code, e.msg);
-  } catch (const std::bad_alloc&) {
-    return fail(h, MPF_ERR_OOM, "host allocation failed");
-  } catch (const std::exception& e) {
-    return fail(h, MPF_ERR_INTERNAL, e.what());
-  }
+  auto run = [&]() -> int {
+    try {
+      return f();
+    } catch (const MpfError& e) {
+      return fail(h, e.code, e.msg);
+    } catch (const std::bad_alloc&) {
+      return fail(h, MPF_ERR_OOM, "host allocation failed");
+    } catch (const std::exception& e) {
+      return fail(h, MPF_ERR_INTERNAL, e.what());
+    }
+  };
+  const int rc = run();
+  // (also after a failure: what it has uploaded belongs to this handle)
+  const cudaError_t e = mark_uploads(h);
+  return rc == MPF_OK && e != cudaSuccess ? fail(h, MPF_ERR_CUDA, cudaGetErrorString(e)) : rc;
 }
 
 void upload_fd(mpf_handle* h, int variant) {
