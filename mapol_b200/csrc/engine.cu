@@ -2006,7 +2006,8 @@ inline bool chunk_shape(const std::vector<LUSystem*>& sys, int G, int wsize, boo
 }
 
 // Widest chunk (at most a 32-byte sector of lanes) that fits and gives at least half of the SMs
-// a block (fewer, wider chunks read the plan less often; below half, a second wave is still free)
+// a block (fewer, wider chunks read the plan less often; below half, a second wave is still
+// free); G = 0 when no plan fits
 inline ChunkShape choose_chunk(const std::vector<LUSystem*>& sys, int widest, int wsize, int ngroups, int resident) {
   ChunkShape sh;
   auto budget = [&](int G) { return resident > 1 && ngroups * (32 / G) > 148 ? kChunkSmem / resident : kChunkSmem; };
@@ -2020,7 +2021,7 @@ inline ChunkShape choose_chunk(const std::vector<LUSystem*>& sys, int widest, in
     for (int xs = 1; xs >= 0; --xs)
       if (chunk_shape(sys, G, wsize, xs == 1, budget(G), sh)) return sh;
   }
-  throw MpfError{MPF_ERR_INTERNAL, "no chunk plan fits shared memory"};
+  return ChunkShape();
 }
 
 // Once per device: a kernel's permission to take the chunk kernels' shared memory
@@ -2109,6 +2110,7 @@ ChunkShape choose_subst(LUSystem& S, int ngroups) {
     possible = chunks(G, 2.0 * S.sym.nlevels, true) < 0.7 * level;
   if (!possible) return none;
   const ChunkShape sh = choose_chunk({&S}, Prec<T>::G, sizeof(T), ngroups, 2);
+  if (sh.G == 0) return none;
   return forced || chunks(sh.G, sh.plan[0]->steps, sh.xs) < 0.7 * level ? sh : none;
 }
 
@@ -2473,6 +2475,7 @@ ChunkShape choose_fd(LUSystem& Bp, LUSystem& Bpp, int ngroups) {
   for (int G = Prec<T>::G; G >= 1 && !possible; G /= 2) possible = chunks(G, 2.0 * levels, true) < level;
   if (!possible) return none;
   const ChunkShape sh = choose_chunk({&Bp, &Bpp}, Prec<T>::G, sizeof(T), ngroups, 1);
+  if (sh.G == 0) return none;
   return forced || chunks(sh.G, sh.plan[0]->steps + sh.plan[1]->steps, sh.xs) < level ? sh : none;
 }
 
