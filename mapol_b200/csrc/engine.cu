@@ -2448,11 +2448,13 @@ void launch_fd_chunk(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSystem&
 
 // Whether a fast-decoupled solve runs on one block per chunk of lanes, and its shape (G = 0: on
 // level launches), by estimated microseconds per iteration.  A block's iteration is its steps
-// (about 1 us each) and its panels' traffic, and the batch is so many waves of blocks; the
-// level launches pay about 8 us per launch and the batch's entries.  Fitted to 30 to 9241 buses
-// x 11 to 60000 cases in both precisions.  ms per solve, level launches / chunks:
-//   FP64: 30 buses x 5000 2.4 / 2.1, x 10000 2.4 / 3.9;  300 x 4000 8.0 / 5.8, x 8000 9.2 / 11.1
-//     1354 x 4096 18.7 / 17.0, x 8000 25.3 / 33.3;  2869 x 1500 25.5 / 21.1, x 3000 31.1 / 40.9
+// (0.85 us each, and 6 beside them) and its panels' traffic (1.45 times as long with x in global
+// memory), and the batch is so many waves of blocks; the level launches pay about 8 us per
+// launch and the batch's entries.  Fitted to 30 to 9241 buses x 11 to 60000 cases in both
+// precisions.  ms per solve, level launches / chunks:
+//   FP64: 11 buses x 7680 1.3 / 1.5;  30 x 5000 2.4 / 2.1, x 10000 2.4 / 3.9
+//     300 x 4000 8.0 / 5.8, x 8000 9.2 / 11.1;  1354 x 4096 18.7 / 17.0, x 8000 25.3 / 33.3
+//     2869 x 1500 25.5 / 21.1, x 3000 31.1 / 40.9
 //     9241 x 256 41.4 / 14.9, x 1000 55.6 / 44.9, x 2000 69.7 / 86.7
 //   FP32: 30 x 10000 2.5 / 2.0, x 20000 2.6 / 3.7;  300 x 8000 8.9 / 6.1, x 16000 11.1 / 11.7
 //     1354 x 8000 23.4 / 21.6;  2869 x 3000 27.1 / 24.7, x 4000 30.3 / 32.4
@@ -2468,7 +2470,7 @@ ChunkShape choose_fd(LUSystem& Bp, LUSystem& Bpp, int ngroups) {
   const double level = 8.0 * (2 * levels + 6) + nnz * (sizeof(T) == 8 ? 0.013 : 0.007) + 1e-5 * nnz * 32.0 * ngroups;
   auto chunks = [&](int G, double steps, bool xs) {
     const int waves = (ngroups * (32 / G) + 147) / 148;
-    return waves * (steps / isl + nnz * (0.0025 + 0.0011 * G) * (xs ? 1.0 : 1.3));
+    return waves * (6.0 + 0.85 * steps / isl + nnz * (0.0025 + 0.0011 * G) * (xs ? 1.0 : 1.45));
   };
   const bool forced = std::getenv("MPF_CHUNK_LANES") != nullptr;  // testing
   bool possible = forced;

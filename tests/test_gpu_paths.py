@@ -62,7 +62,8 @@ def test_fast_decoupled_level_launches_on_several_grids_with_controls(gpu, monke
 
 @pytest.mark.parametrize("prec,n_bus,n_cases,chunks", [(m.FP64, 30, 2500, True), (m.FP64, 30, 20000, False),
                                                        (m.MIXED, 30, 40000, False), (m.FP64, 300, 2000, True),
-                                                       (m.FP64, 300, 16000, False)])
+                                                       (m.FP64, 300, 16000, False), (m.FP64, 11, 2000, True),
+                                                       (m.FP64, 11, 16000, False)])
 def test_fast_decoupled_form_by_batch(gpu, prec, n_bus, n_cases, chunks):
     """A factor of two or more from the line on either side."""
     buses, branches = grid(n_bus)
