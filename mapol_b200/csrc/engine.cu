@@ -2170,8 +2170,12 @@ inline bool nr_shape(LUSystem& S, int G, int wsize, NrShape& out) {
 // FP64 0.43 / 0.15 (1); 118 x 167 mixed 0.78 / 0.24 (2); 300 x 257 mixed 1.55 / 0.55 (2), x
 // 1024 1.90 / 0.93 (8), FP64 2.09 / 1.63 (4); 700 x 300 mixed 2.49 / 1.92 (4), x 1000 3.45 /
 // 3.88 (4); 1354 x 200 mixed 3.38 / 2.56 (2), x 1000 4.62 / 10.2 (2).  No grid above
-// kNrChunkEntries LU entries gains (2869 buses x 20 cases 4.0 / 6.0).
+// kNrChunkEntries LU entries gains (2869 buses x 20 cases 4.0 / 6.0), and no chunk whose lanes'
+// LU is above kNrChunkBytes, which leaves its plan short ring slots and few fronts side by side
+// (reactive limits, all rounds, level / chunks: 1600 buses x 5 FP64 9.2 / 11.5, x 150 mixed on 2
+// lanes 10.7 / 11.9; below it 1354 x 5 FP64 10.0 / 10.1, x 150 mixed on 2 lanes 11.0 / 10.0).
 constexpr long long kNrChunkEntries = 50000;
+constexpr size_t kNrChunkBytes = 300000;
 template <typename T>
 NrShape choose_nr(LUSystem& S, int ngroups) {
   NrShape sh, best;
@@ -2194,6 +2198,7 @@ NrShape choose_nr(LUSystem& S, int ngroups) {
   };
   for (int G = Prec<T>::G; G >= 1; G /= 2) {
     // (no plan is built where the least it could cost is too much)
+    if ((size_t)S.sym.nnz * G * sizeof(T) > kNrChunkBytes) continue;
     if (chunks(G, S.fneeds.cycles) >= bt || !nr_shape(S, G, sizeof(T), sh)) continue;
     const double t = chunks(G, sh.fac->cycles);
     if (t < bt) {

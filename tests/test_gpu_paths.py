@@ -194,3 +194,18 @@ def test_fast_decoupled_times_by_family(gpu, monkeypatch, chunk, use_graph):
     parts = [t[k] for k in ("mismatch_ms", "solve_ms", "update_ms", "jacobian_ms", "factor_ms")]
     assert min(parts) > 0.0 and sum(parts) + t["other_ms"] <= 1.001 * t["total_ms"]
     assert t["solve_ms"] > t["update_ms"]
+
+
+@pytest.mark.parametrize("prec,n_bus,n_cases,chunks", [(m.FP64, 1600, 5, False), (m.MIXED, 1600, 5, True),
+                                                       (m.FP64, 300, 64, True), (m.FP64, 300, 8000, False)])
+def test_newton_form_with_reactive_limits(gpu, prec, n_bus, n_cases, chunks):
+    """A block's LU above 300,000 bytes, or a batch of many waves, keeps the level launches."""
+    buses, branches = m.synth_grid(n_bus, int(1.5 * n_bus), n_bus // 5, 0.1, seed=3)
+    with m.PowerFlow(buses, branches) as pf:
+        pf.set_q_limits(np.full(n_bus, -0.3), np.full(n_bus, 0.3))
+        pf.set_cases(outages(branches, n_bus, n_cases))
+        pf.solve(m.NR, prec)
+        st = pf.stats()
+        assert (st["solve_lanes"] > 0) == chunks
+        if n_bus == 1600:
+            assert 8 * st["nnz_lu"] > 300000 > 4 * st["nnz_lu"]
