@@ -73,17 +73,14 @@ struct DevBuf {
   T* as() const { return reinterpret_cast<T*>(p); }
 };
 
-// Uploads and fills go to the legacy stream, and a copy from pageable memory (or a fill) may
-// return before it has landed.  The streams the kernels run on are not ordered after that one:
-// every entry point that launches calls after_uploads() first (an event of the handle, 1 us where
-// a wait on the host takes 6), and so does one that launches on what it has just uploaded;
-// uploads_done() waits here, for plans that are built once.
-thread_local bool uploads_pending = false;
-void uploads_done() {
-  if (!uploads_pending) return;
-  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
-  uploads_pending = false;
-}
+// Uploads and fills go to the own stream of the handle whose entry point runs (guarded()), so
+// what is launched there needs no wait; a copy from pageable memory may return before it has
+// landed, so a launch on another stream calls after_uploads() first.
+struct Uploads {
+  cudaStream_t stream = nullptr;
+  bool any = false;  // since after_uploads() or the entry point's start
+};
+thread_local Uploads uploads;
 
 // Copies v to the device, reusing b's allocation when it is large enough.
 template <class T>
@@ -91,12 +88,12 @@ void upload(DevBuf& b, const std::vector<T>& v) {
   const size_t need = v.size() * sizeof(T);
   if (!b.p || b.bytes < need) b.alloc(need);
   if (v.empty()) return;
-  uploads_pending = true;
-  CUDA_TRY(cudaMemcpy(b.p, v.data(), need, cudaMemcpyHostToDevice));
+  uploads.any = true;
+  CUDA_TRY(cudaMemcpyAsync(b.p, v.data(), need, cudaMemcpyHostToDevice, uploads.stream));
 }
 void fill(DevBuf& b, int byte, size_t n) {
-  uploads_pending = true;
-  CUDA_TRY(cudaMemset(b.p, byte, n));
+  uploads.any = true;
+  CUDA_TRY(cudaMemsetAsync(b.p, byte, n, uploads.stream));
 }
 
 // ------------------------------------------------------------------ LU system
@@ -511,7 +508,6 @@ struct LUSystem {
       upload(out.step_ptr, p.step_ptr);
       upload(out.down_ptr, p.down_ptr);
       upload(out.idx, p.idx);
-      uploads_done();
       out.scratch = p.scratch;
       out.slot = p.slot;
       out.steps = (int)p.step.size();
@@ -535,7 +531,6 @@ struct LUSystem {
       for (size_t k = 0; k < st.size(); ++k) st[k] = make_int4(p.step[k].e0, p.step[k].ne, p.step[k].i0, p.step[k].ni);
       upload(out.step, st);
       upload(out.idx, p.idx);
-      uploads_done();
       out.n = (int)st.size();
       out.peak_cb = p.peak_cb;
       out.most = p.most;
@@ -1625,8 +1620,8 @@ struct mpf_handle {
   // the last solve's and the last adjoint's chunk kernels (mpf_stats): lanes per block (0: level
   // launches) and x in shared memory
   uint8_t solve_lanes = 0, solve_in_shared = 0, adjoint_lanes = 0, adjoint_in_shared = 0;
-  cudaEvent_t uploaded = nullptr;   // after the handle's latest uploads
-  bool uploads_running = false;     // nothing has waited for it on the host yet
+  cudaEvent_t uploaded = nullptr;   // recorded on own_stream for launches on other streams
+  bool uploads_running = false;     // the host has not waited for the latest uploads yet
 
   // mismatch rows grouped by island
   DevBuf isl_rows, isl_row_ptr;
@@ -1641,7 +1636,6 @@ struct mpf_handle {
       }
       upload(isl_rows, rows);
       upload(isl_row_ptr, ptr);
-      uploads_done();
       isl_ready = true;
     }
     return ChunkRows{isl_rows.as<int>(), isl_row_ptr.as<int>()};
@@ -1808,30 +1802,22 @@ int fail(mpf_handle* h, int code, const std::string& msg) {
   return code;
 }
 
-// This thread's uploads so far are behind the handle's event
-cudaError_t mark_uploads(mpf_handle* h) {
-  if (!uploads_pending || !h->uploaded) return cudaSuccess;
-  const cudaError_t e = cudaEventRecord(h->uploaded, cudaStreamLegacy);
-  if (e != cudaSuccess) return e;
-  h->uploads_running = true;
-  uploads_pending = false;
-  return cudaSuccess;
-}
-
 // What is launched on st from here on runs after the handle's uploads.  (A capture cannot hold
 // the event: there the wait is the host's, in the mode that allows it beside a capture.)
 void after_uploads(mpf_handle* h, cudaStream_t st) {
-  CUDA_TRY(mark_uploads(h));
-  if (!h->uploads_running) return;
+  h->uploads_running |= uploads.any;
+  uploads.any = false;
+  if (!h->uploads_running || st == h->own_stream) return;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(st, &cs));
   if (cs == cudaStreamCaptureStatusNone) {
+    CUDA_TRY(cudaEventRecord(h->uploaded, h->own_stream));
     CUDA_TRY(cudaStreamWaitEvent(st, h->uploaded, 0));
     return;
   }
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
-  const cudaError_t e = cudaEventSynchronize(h->uploaded);
+  const cudaError_t e = cudaStreamSynchronize(h->own_stream);
   CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
   CUDA_TRY(e);
   h->uploads_running = false;
@@ -1839,21 +1825,25 @@ void after_uploads(mpf_handle* h, cudaStream_t st) {
 
 template <class F>
 int guarded(mpf_handle* h, F&& f) {
-  auto run = [&]() -> int {
-    try {
-      return f();
-    } catch (const MpfError& e) {
-      return fail(h, e.code, e.msg);
-    } catch (const std::bad_alloc&) {
-      return fail(h, MPF_ERR_OOM, "host allocation failed");
-    } catch (const std::exception& e) {
-      return fail(h, MPF_ERR_INTERNAL, e.what());
+  // this call's uploads are the handle's, also when it fails
+  struct Scope {
+    mpf_handle* h;
+    Uploads outer;
+    explicit Scope(mpf_handle* h_) : h(h_), outer(uploads) { uploads = Uploads{h->own_stream, false}; }
+    ~Scope() {
+      h->uploads_running |= uploads.any;
+      uploads = outer;
     }
-  };
-  const int rc = run();
-  // (also after a failure: what it has uploaded belongs to this handle)
-  const cudaError_t e = mark_uploads(h);
-  return rc == MPF_OK && e != cudaSuccess ? fail(h, MPF_ERR_CUDA, cudaGetErrorString(e)) : rc;
+  } scope(h);
+  try {
+    return f();
+  } catch (const MpfError& e) {
+    return fail(h, e.code, e.msg);
+  } catch (const std::bad_alloc&) {
+    return fail(h, MPF_ERR_OOM, "host allocation failed");
+  } catch (const std::exception& e) {
+    return fail(h, MPF_ERR_INTERNAL, e.what());
+  }
 }
 
 void upload_fd(mpf_handle* h, int variant) {
@@ -1885,7 +1875,6 @@ void upload_fd(mpf_handle* h, int variant) {
     for (int i = 0; i < g.nb; ++i) fv[i] = make_int2(g.bp[0].var[i], g.bpp[0].var[i]);
     upload(h->fdvar, fv);
   }
-  uploads_done();
   h->fd_ready[variant] = true;
 }
 
@@ -2116,9 +2105,11 @@ ChunkShape choose_subst(LUSystem& S, int ngroups) {
 
 // x <- (L U)^-T x for every lane.  Returns the chunks' shape (G = 0: level launches).
 template <typename T>
-ChunkShape launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, const int* group_active, int device,
+ChunkShape launch_subst_t(mpf_handle* h, LUSystem& S, const T* pan, T* cbr, T* x, const int* group_active,
                           cudaStream_t st) {
+  const int ngroups = h->ngroups;
   const ChunkShape sh = choose_subst<T>(S, ngroups);
+  after_uploads(h, st);
   if (sh.G == 0) {
     launch_fsolve_t<T>(S, ngroups, pan, cbr, x, group_active, st);
     launch_bsolve_t<T>(S, ngroups, pan, x, group_active, st);
@@ -2127,7 +2118,7 @@ ChunkShape launch_subst_t(LUSystem& S, int ngroups, const T* pan, T* cbr, T* x, 
   with_shape<T>(sh, [&](auto g, auto xs) {
     constexpr int G = decltype(g)::value;
     constexpr bool XS = decltype(xs)::value;
-    allow_chunk_smem<k_subst_chunk<T, G, XS>>(device);
+    allow_chunk_smem<k_subst_chunk<T, G, XS>>(h->device);
     SubstChunk<T> a{sh.plan[0]->dev(), S.sym.n, S.sym.nnz, S.sym.cbr_off.back(), pan, cbr, x,
                     sh.xcap, sh.ccap, sh.scratch, sh.slot};
     k_subst_chunk<T, G, XS><<<(unsigned)(ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(a, S.group_island);
@@ -2215,6 +2206,8 @@ void launch_nr_chunk(mpf_handle* h, const NrShape& sh, const DevGrid& d, int wha
   LUSystem& J = h->jac;
   const NrChunk<T> a{sh.fac->dev(), sh.sw->dev(),     J.sym.n,  J.nA,    J.sym.nnz, J.A[P].as<T>(), J.pan[P].as<T>(),
                      J.x[P].as<T>(), sh.xcap, sh.scratch, sh.slot, sh.fslot, sh.cbs,    sh.fronts};
+  const ChunkRows rows = h->chunk_rows();
+  after_uploads(h, st);
   ChunkShape cs;
   cs.G = sh.G;
   with_shape<T>(cs, [&](auto g, auto) {
@@ -2223,7 +2216,7 @@ void launch_nr_chunk(mpf_handle* h, const NrShape& sh, const DevGrid& d, int wha
       constexpr bool CTL = decltype(ctl)::value, QL = decltype(ql)::value;
       allow_chunk_smem<k_nr_chunk<T, G, CTL, QL>>(h->device);
       k_nr_chunk<T, G, CTL, QL><<<(unsigned)(h->ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(
-          d, a, h->chunk_rows(), what, h->opt.max_it_nr, h->opt.tol);
+          d, a, rows, what, h->opt.max_it_nr, h->opt.tol);
       CUDA_TRY(cudaGetLastError());
     };
     if (d.sw_index) d.y_slot ? go(std::true_type(), std::true_type()) : go(std::false_type(), std::true_type());
@@ -2438,8 +2431,10 @@ void launch_fd_chunk_g(mpf_handle* h, const DevGrid& d, const DevFD& fd, LUSyste
   a.ccap = sh.ccap;
   a.scratch = sh.scratch;
   a.slot = sh.slot;
+  const ChunkRows rows = h->chunk_rows();
+  after_uploads(h, st);
   k_fd_chunk<T, G, XS><<<(unsigned)(h->ngroups * (32 / G)), kChunkThreads, sh.smem, st>>>(
-      d, fd, a, h->chunk_rows(), h->opt.max_it_fd, h->opt.tol);
+      d, fd, a, rows, h->opt.max_it_fd, h->opt.tol);
   CUDA_TRY(cudaGetLastError());
 }
 
@@ -2490,6 +2485,7 @@ template <typename T>
 void solve_fd(mpf_handle* h, cudaStream_t st, int variant) {
   constexpr int P = Prec<T>::idx;
   upload_fd(h, variant);
+  after_uploads(h, st);
   LUSystem& Bp = h->bp[variant];
   LUSystem& Bpp = h->bpp[variant];
   Bp.ensure_values(P, h->ngroups);
@@ -2672,7 +2668,7 @@ void adjoint_impl(mpf_handle* h, cudaStream_t st, double* gp, double* gq, double
   const size_t nx = (size_t)lanes * J.sym.n;
   const dim3 bg((unsigned)((h->g.nbr + 63) / 64), (unsigned)h->ngroups);
   auto substitute = [&]() {
-    const ChunkShape sh = launch_subst_t<T>(J, h->ngroups, pan, J.cbr[P].as<T>(), x, d.group_active, h->device, st);
+    const ChunkShape sh = launch_subst_t<T>(h, J, pan, J.cbr[P].as<T>(), x, d.group_active, st);
     h->adjoint_lanes = (uint8_t)sh.G;
     h->adjoint_in_shared = sh.xs;
   };
@@ -2799,6 +2795,7 @@ int32_t mpf_create(const mpf_bus* buses, int32_t n_bus, const mpf_branch* branch
       if (!lim.empty()) return fail(h.get(), MPF_ERR_BAD_INPUT, lim);
     }
     CUDA_TRY(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
+    uploads.stream = h->own_stream;
     CUDA_TRY(cudaMallocHost(&h->h_any, sizeof(LoopRecord)));
     CUDA_TRY(cudaEventCreate(&h->t0));
     CUDA_TRY(cudaEventCreate(&h->t1));

@@ -141,3 +141,36 @@ def test_evaluation_captured_right_after_new_cases(gpu):
         torch.cuda.synchronize()
         assert np.array_equal(got.cpu().numpy(), ref.cpu().numpy()) and (ref > 0).all()
         del graph
+
+
+@pytest.mark.parametrize("prec", [m.FP64, m.MIXED])
+@pytest.mark.parametrize("alg", [m.NR, m.FDXB])
+@pytest.mark.parametrize("n_cases", [40, 9000])
+def test_first_solves_on_other_streams(gpu, alg, prec, n_cases):
+    """A new handle's first solve and adjoint on streams of the caller, which have to wait for the
+    tables and plans that the calls themselves upload: bit for bit what its own stream gives.
+    (40 cases run on chunks, 9000 on level launches.)"""
+    import torch
+
+    from mapol_b200._lib import lib
+
+    buses, branches = m.synth_grid(118, 179, 53, 0.1, seed=3)
+    n1 = np.flatnonzero(~m.find_bridges(branches, 118))
+    cases = [[int(b)] for b in np.resize(n1, n_cases)]
+    sbus = np.repeat(np.stack([buses["p"], buses["q"]], -1)[None], n_cases, 0) * np.linspace(0.9, 1.0, n_cases)[:, None, None]
+    out = []
+    for streams in ((None, None), (torch.cuda.Stream(), torch.cuda.Stream())):
+        ptrs = [s.cuda_stream if s else None for s in streams]
+        grads = [torch.zeros((n_cases, n), dtype=torch.float64, device="cuda") for n in (118, 118, 179, 179)]
+        torch.cuda.synchronize()
+        with m.PowerFlow(buses, branches) as pf:
+            pf.set_cases(cases, sbus=sbus)
+            pf.solve(alg, prec, stream=ptrs[0])
+            pf.set_ratings(np.full(179, 0.3))
+            assert lib().mpf_adjoint(pf._h, prec, *[g.data_ptr() for g in grads], ptrs[1]) == 0
+            torch.cuda.synchronize()
+            res = pf.results()
+            assert res.converged.all()
+            out.append([res.v, res.iterations] + [g.cpu().numpy() for g in grads])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
